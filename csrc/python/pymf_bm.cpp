@@ -3,6 +3,7 @@
 #include <pybind11/stl.h>
 
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 
 #include "pymf_parts.h"
@@ -24,6 +25,74 @@ struct BigMemory {
 };
 
 uint32_t g_worldSize = 0;
+
+// The value of a non-negative Python int that fits 64 bits, read from its 30-bit digits; false: take the general way.
+inline bool SmallUnsigned(PyObject *o, uint64_t *v)
+{
+#if PY_VERSION_HEX >= 0x030C0000 && PY_VERSION_HEX < 0x030E0000 && PYLONG_BITS_IN_DIGIT == 30
+    if (!PyLong_CheckExact(o)) {
+        return false;
+    }
+    const _PyLongValue &lv = reinterpret_cast<PyLongObject *>(o)->long_value;
+    if ((lv.lv_tag & 3) == 2) {
+        return false;  // negative
+    }
+    const size_t digits = lv.lv_tag >> 3;
+    if (digits > 2) {
+        return false;
+    }
+    *v = (lv.lv_tag & 3) == 1 ? 0 : (digits == 2 ? (uint64_t)lv.ob_digit[0] | (uint64_t)lv.ob_digit[1] << 30 : (uint64_t)lv.ob_digit[0]);
+    return true;
+#else
+    return false;
+#endif
+}
+
+// Addresses or sizes handed over as a Python sequence, as a plain array. A KV batch is thousands of elements long, so lists and
+// tuples are read in place: the general conversion into a growing vector measured 20 ns an element (240 us of the 520 us that
+// a call of 3 x 3904 elements took), this one about 2 ns.
+class U64Array {
+public:
+    explicit U64Array(const py::handle &seq)
+    {
+        PyObject *o = seq.ptr();
+        if (!PyList_Check(o) && !PyTuple_Check(o)) {
+            general_ = Cast<std::vector<uint64_t>>(seq);
+            data_ = general_.data();
+            size_ = general_.size();
+            return;
+        }
+        size_ = (size_t)PySequence_Fast_GET_SIZE(o);
+        own_.reset(new uint64_t[size_ > 0 ? size_ : 1]);
+        data_ = own_.get();
+        for (size_t i = 0; i < size_; i++) {
+            PyObject *e = PySequence_Fast_GET_ITEM(o, (Py_ssize_t)i);
+            if (!SmallUnsigned(e, &own_[i])) {
+                own_[i] = Cast<uint64_t>(e);
+                if (i >= size_ || (size_t)PySequence_Fast_GET_SIZE(o) != size_) {
+                    throw py::type_error("the sequence changed while it was read");  // an element's __index__ ran Python code
+                }
+            }
+        }
+    }
+    uint64_t *data() { return data_; }
+    size_t size() const { return size_; }
+
+private:
+    template <typename T>
+    static T Cast(const py::handle &h)
+    {
+        try {
+            return h.cast<T>();
+        } catch (const py::cast_error &) {
+            throw py::type_error("addresses and sizes are sequences of non-negative 64-bit integers");
+        }
+    }
+    std::vector<uint64_t> general_;
+    std::unique_ptr<uint64_t[]> own_;
+    uint64_t *data_{nullptr};
+    size_t size_{0};
+};
 
 }  // namespace
 
@@ -133,24 +202,26 @@ void BindBm(py::module_ &m)
             mf_copy_params p{(const void *)src, (void *)dst, (size_t)size};
             return mf_bm_copy_on_stream(b.h, &p, t, (void *)stream, flags);
         }, py::arg("src"), py::arg("dest"), py::arg("size"), py::arg("type"), py::arg("stream"), py::arg("flags") = 0, py::call_guard<py::gil_scoped_release>())
-        .def("copy_data_batch", [](BigMemory &b, std::vector<uint64_t> srcs, std::vector<uint64_t> dsts, std::vector<uint64_t> sizes, uint32_t count,
+        .def("copy_data_batch", [](BigMemory &b, const py::object &srcAddrs, const py::object &destAddrs, const py::object &byteSizes, uint32_t count,
                                    mf_bm_copy_type t, uint32_t flags) {
+            U64Array srcs(srcAddrs), dsts(destAddrs), sizes(byteSizes);
             if (srcs.size() < count || dsts.size() < count || sizes.size() < count) {
                 return (int32_t)MF_INVALID_PARAM;
             }
+            py::gil_scoped_release nogil;
             mf_batch_copy_params p{(void **)srcs.data(), (void **)dsts.data(), sizes.data(), count};
             return mf_bm_copy_batch(b.h, &p, t, flags);
-        }, py::arg("src_addrs"), py::arg("dest_addrs"), py::arg("sizes"), py::arg("count"), py::arg("type") = MF_BM_COPY_AUTO, py::arg("flags") = 0,
-             py::call_guard<py::gil_scoped_release>())
-        .def("copy_data_batch_on_stream", [](BigMemory &b, std::vector<uint64_t> srcs, std::vector<uint64_t> dsts, std::vector<uint64_t> sizes,
+        }, py::arg("src_addrs"), py::arg("dest_addrs"), py::arg("sizes"), py::arg("count"), py::arg("type") = MF_BM_COPY_AUTO, py::arg("flags") = 0)
+        .def("copy_data_batch_on_stream", [](BigMemory &b, const py::object &srcAddrs, const py::object &destAddrs, const py::object &byteSizes,
                                              mf_bm_copy_type t, uint64_t stream, uint32_t flags) {
+            U64Array srcs(srcAddrs), dsts(destAddrs), sizes(byteSizes);
             uint32_t count = (uint32_t)sizes.size();
             if (srcs.size() != count || dsts.size() != count) {
                 return (int32_t)MF_INVALID_PARAM;
             }
+            py::gil_scoped_release nogil;
             mf_batch_copy_params p{(void **)srcs.data(), (void **)dsts.data(), sizes.data(), count};
             return mf_bm_copy_batch_on_stream(b.h, &p, t, (void *)stream, flags);
-        }, py::arg("src_addrs"), py::arg("dest_addrs"), py::arg("sizes"), py::arg("type"), py::arg("stream"), py::arg("flags") = 0,
-             py::call_guard<py::gil_scoped_release>())
+        }, py::arg("src_addrs"), py::arg("dest_addrs"), py::arg("sizes"), py::arg("type"), py::arg("stream"), py::arg("flags") = 0)
         .def("wait", [](BigMemory &b) { return mf_bm_wait(b.h); }, py::call_guard<py::gil_scoped_release>());
 }
