@@ -87,11 +87,9 @@ constexpr size_t kArenaBase = 256;  // offsets handed out by the pool start here
 constexpr size_t kArenaDefault = 2u << 20;
 
 struct ThreadCtx {
-    volatile uint32_t *flag{nullptr};  // pinned host word, device-visible under the same address
-    uint32_t *counter{nullptr};        // device word, self-resetting
-    uint32_t seq{0};
     StageArena arena;
     std::vector<mf_copy_desc_t> scratch;
+    cudaEvent_t order{nullptr};  // see OrderAfterProducers
 };
 
 class KernelDataOp : public DataOperator {
@@ -104,8 +102,6 @@ public:
     {
         MF_CHECK_RET(cu::Available() && device_ >= 0, BM_NOT_SUPPORTED, "kernel engine: no GPU");
         MF_CUDA_CHECK_RET(cudaSetDevice(device_), BM_ERROR);
-        const char *e = std::getenv("MF_BATCH_SYNC");
-        flagSync_ = !(e != nullptr && std::strcmp(e, "stream") == 0);
         return BM_OK;
     }
 
@@ -120,15 +116,13 @@ public:
             return BM_NOT_SUPPORTED;
         }
         cudaStream_t s = opt.stream != nullptr ? (cudaStream_t)opt.stream : cu::ThreadStream(device_);
+        OrderAfterProducers(dir, opt, s);
         int rc = mf_k_xcopy(p.dest, p.src, p.dataSize, 0, (mf_stream_t)s);
         if (rc != MF_K_OK) {
             MF_ERROR("kernel engine: xcopy launch failed");
             return BM_ERROR;
         }
-        if (opt.flags & FLAG_ASYNC_COPY) {
-            return BM_OK;
-        }
-        return BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
+        return (opt.flags & FLAG_ASYNC_COPY) ? BM_OK : BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
     }
 
     int BatchDataCopy(const BatchCopyParams &p, CopyDirection dir, const ExtOptions &opt) override
@@ -137,25 +131,48 @@ public:
             return BM_NOT_SUPPORTED;
         }
         ThreadCtx *ctx = Ctx();
-        MF_CHECK_RET(ctx != nullptr, BM_ERROR, "kernel engine: cannot set up the per-thread batch context");
         cudaStream_t s = opt.stream != nullptr ? (cudaStream_t)opt.stream : cu::ThreadStream(device_);
-        // 1. Coalesce runs that are contiguous on both sides, split anything too long for a 32-bit length.
-        std::vector<mf_copy_desc_t> &d = ctx->scratch;
-        d.clear();
+        OrderAfterProducers(dir, opt, s);
+        // All addresses and lengths multiples of 16: the bulk-copy kernel, else the load/store kernel.
+        uint64_t total = 0, bits = 0;
+        for (uint32_t i = 0; i < p.batchSize; i++) {
+            total += p.dataSizes[i];
+            bits |= (uint64_t)p.sources[i] | (uint64_t)p.destinations[i] | p.dataSizes[i];
+        }
+        int rc = BM_OK;
+        if ((bits & 15) == 0) {
+            rc = BulkBatch(p, total, (mf_stream_t)s);
+        } else {
+            rc = LoadStoreBatch(p, ctx, s);
+        }
+        if (rc != BM_OK) {
+            return rc;
+        }
+        return (opt.flags & FLAG_ASYNC_COPY) ? BM_OK : BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
+    }
+
+    int Wait() override { return BoundedStreamSync(device_, nullptr, DefaultSyncTimeoutMs()); }
+
+private:
+    static constexpr uint32_t kChunkShift = 15;
+    static_assert((1u << kChunkShift) == MF_BATCH_CHUNK_BYTES, "chunk size of the load/store kernel");
+
+    // Calls emit(src, dst, len) for every run that is contiguous on both sides, cut where it is too long for a 32-bit length.
+    template <typename Emit>
+    static void Coalesce(const BatchCopyParams &p, const Emit &emit)
+    {
         constexpr uint64_t kMaxLen = 1ull << 31;
-        uint32_t chunks = 0;
-        auto push = [&](uint64_t src, uint64_t dst, uint64_t len) {
-            while (len > 0) {
-                uint64_t part = std::min(len, kMaxLen);
-                d.push_back(mf_copy_desc_t{src, dst, (uint32_t)part, 0});
-                src += part;
-                dst += part;
-                len -= part;
+        uint64_t curS = 0, curD = 0, curL = 0;
+        auto flush = [&]() {
+            for (; curL > kMaxLen; curS += kMaxLen, curD += kMaxLen, curL -= kMaxLen) {
+                emit(curS, curD, (uint32_t)kMaxLen);
+            }
+            if (curL != 0) {
+                emit(curS, curD, (uint32_t)curL);
             }
         };
-        uint64_t curS = 0, curD = 0, curL = 0;
         for (uint32_t i = 0; i < p.batchSize; i++) {
-            uint64_t sa = (uint64_t)p.sources[i], da = (uint64_t)p.destinations[i], len = p.dataSizes[i];
+            const uint64_t sa = (uint64_t)p.sources[i], da = (uint64_t)p.destinations[i], len = p.dataSizes[i];
             if (len == 0) {
                 continue;
             }
@@ -163,29 +180,59 @@ public:
                 curL += len;
                 continue;
             }
-            if (curL != 0) {
-                push(curS, curD, curL);
-            }
+            flush();
             curS = sa;
             curD = da;
             curL = len;
         }
-        if (curL != 0) {
-            push(curS, curD, curL);
-        }
+        flush();
+    }
+
+    // Pieces of the descriptor list ride in the parameters of one launch each; the first is short, so that the GPU starts early,
+    // and the list of the next is written while it works (32 requests of 122 blocks: 179 us with one staged table).
+    static int BulkBatch(const BatchCopyParams &p, uint64_t total, mf_stream_t s)
+    {
+        const uint32_t shift = mf_k_batch_bulk_shift(total), round = (1u << shift) - 1;
+        thread_local std::unique_ptr<mf_copy_desc_t[]> piece(new mf_copy_desc_t[MF_BULK_INLINE_MAX]);
+        mf_copy_desc_t *d = piece.get();
+        uint32_t n = 0, chunks = 0, room = MF_BULK_FIRST_PIECE;
+        int launched = 0, rc = MF_K_OK;
+        auto launch = [&]() {
+            if (rc == MF_K_OK && n != 0) {
+                rc = mf_k_batch_bulk(d, n, chunks, shift, launched, s);
+                launched = 1;
+                room = MF_BULK_INLINE_MAX;
+            }
+            n = chunks = 0;
+        };
+        Coalesce(p, [&](uint64_t src, uint64_t dst, uint32_t len) {
+            if (n == room) {
+                launch();
+            }
+            d[n++] = mf_copy_desc_t{src, dst, len, chunks};
+            chunks += (uint32_t)(((uint64_t)len + round) >> shift);
+        });
+        launch();
+        MF_CHECK_RET(rc == MF_K_OK, BM_ERROR, "kernel engine: batch launch failed");
+        return BM_OK;
+    }
+
+    int LoadStoreBatch(const BatchCopyParams &p, ThreadCtx *ctx, cudaStream_t s)
+    {
+        std::vector<mf_copy_desc_t> &d = ctx->scratch;
+        d.clear();
+        uint32_t chunks = 0;
+        Coalesce(p, [&](uint64_t src, uint64_t dst, uint32_t len) {
+            d.push_back(mf_copy_desc_t{src, dst, len, chunks});
+            chunks += (uint32_t)(((uint64_t)len + MF_BATCH_CHUNK_BYTES - 1) >> kChunkShift);
+        });
         if (d.empty()) {
             return BM_OK;
         }
-        for (auto &e : d) {
-            e.chunkStart = chunks;
-            chunks += (e.len + MF_BATCH_CHUNK_BYTES - 1) / MF_BATCH_CHUNK_BYTES;
-        }
-        const bool sync = !(opt.flags & FLAG_ASYNC_COPY);
-        const bool useFlag = sync && flagSync_ && opt.stream == nullptr;
         const mf_copy_desc_t *devTable = nullptr;
         uint64_t stagedOff = 0;
         if (d.size() > MF_BATCH_INLINE_MAX) {
-            // 2. Large tables: stage in pinned memory and copy to the device ahead of the kernel, on the same stream.
+            // Large tables: stage in pinned memory and copy to the device ahead of the kernel, on the same stream.
             // Table layout: descriptors, then one uint32 per chunk naming its descriptor.
             const size_t descBytes = d.size() * sizeof(mf_copy_desc_t);
             const size_t bytes = descBytes + (size_t)chunks * sizeof(uint32_t);
@@ -205,37 +252,41 @@ public:
             MF_CUDA_CHECK_RET(cudaMemcpyAsync(ctx->arena.dev + stagedOff, host, bytes, cudaMemcpyHostToDevice, s), BM_ERROR);
             devTable = reinterpret_cast<const mf_copy_desc_t *>(ctx->arena.dev + stagedOff);
         }
-        uint32_t seq = ++ctx->seq;
-        int rc = mf_k_batch_xcopy(d.data(), devTable, (uint32_t)d.size(), chunks, useFlag ? ctx->counter : nullptr,
-                                  useFlag ? ctx->flag : nullptr, seq, 0, (mf_stream_t)s);
+        int rc = mf_k_batch_xcopy(d.data(), devTable, (uint32_t)d.size(), chunks, 0, (mf_stream_t)s);
         if (stagedOff != 0) {
             StageRetire(ctx->arena, stagedOff, s);  // the range is free again once this kernel has run
         }
-        if (rc != MF_K_OK) {
-            MF_ERROR("kernel engine: batch launch failed");
-            return BM_ERROR;
-        }
-        if (!sync) {
-            return BM_OK;
-        }
-        if (useFlag) {
-            // 3. Completion word written by the last CTA; bounded poll, then fall back to the stream for the verdict.
-            uint64_t deadline = NowNs() + (uint64_t)DefaultSyncTimeoutMs() * 1000000ull;
-            uint32_t spins = 0;
-            while (*ctx->flag != seq) {
-                if ((++spins & 0x3ff) == 0 && NowNs() > deadline) {
-                    MF_ERROR("kernel engine: batch completion word not seen in time");
-                    return BM_TIMEOUT;
-                }
-            }
-            return BM_OK;
-        }
-        return BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
+        MF_CHECK_RET(rc == MF_K_OK, BM_ERROR, "kernel engine: batch launch failed");
+        return BM_OK;
     }
 
-    int Wait() override { return BoundedStreamSync(device_, nullptr, DefaultSyncTimeoutMs()); }
+    // A call without a stream runs on this thread's own stream, which does not wait for the default one. Where one side is the
+    // caller's own device buffer, what was queued for that buffer on the default stream (a producer, a fill) has to come first:
+    // a copy that starts within microseconds at high priority would overtake it. An idle default stream costs one query;
+    // copies between pool addresses, which the library alone places, are not ordered.
+    void OrderAfterProducers(CopyDirection dir, const ExtOptions &opt, cudaStream_t s)
+    {
+        if (opt.stream != nullptr || (SrcClassOf(dir) != PC_LOCAL_DEVICE && DstClassOf(dir) != PC_LOCAL_DEVICE)) {
+            return;
+        }
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(cudaStreamLegacy, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+            (void)cudaGetLastError();  // another thread captures a graph: the default stream must not be touched
+            return;
+        }
+        if (cudaStreamQuery(cudaStreamLegacy) == cudaErrorNotReady) {
+            ThreadCtx *ctx = Ctx();
+            if (ctx->order == nullptr && cudaEventCreateWithFlags(&ctx->order, cudaEventDisableTiming) != cudaSuccess) {
+                (void)cudaGetLastError();
+                cudaStreamSynchronize(cudaStreamLegacy);
+                return;
+            }
+            cudaEventRecord(ctx->order, cudaStreamLegacy);
+            cudaStreamWaitEvent(s, ctx->order, 0);
+        }
+        (void)cudaGetLastError();
+    }
 
-private:
     // Hands back the ranges whose kernels have finished; with `block` it waits for the oldest one.
     static void StageReclaim(StageArena &a, bool block)
     {
@@ -307,29 +358,15 @@ private:
     ThreadCtx *Ctx()
     {
         thread_local std::unordered_map<const KernelDataOp *, ThreadCtx> ctxs;
-        ThreadCtx &c = ctxs[this];
-        if (c.flag == nullptr) {
+        auto it = ctxs.find(this);
+        if (it == ctxs.end()) {
             cudaSetDevice(device_);
-            void *hp = nullptr;
-            if (cudaHostAlloc(&hp, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-                (void)cudaGetLastError();
-                return nullptr;
-            }
-            std::memset(hp, 0, 64);
-            void *dp = nullptr;
-            if (cudaMalloc(&dp, 64) != cudaSuccess || cudaMemset(dp, 0, 64) != cudaSuccess) {
-                (void)cudaGetLastError();
-                cudaFreeHost(hp);
-                return nullptr;
-            }
-            c.flag = (volatile uint32_t *)hp;
-            c.counter = (uint32_t *)dp;
+            it = ctxs.try_emplace(this).first;
         }
-        return &c;
+        return &it->second;
     }
 
     int device_;
-    bool flagSync_{true};
 };
 
 // =============================================================================================== copy engine
@@ -623,42 +660,53 @@ static uint64_t PeerCopyEngineMin()
     return v;
 }
 
-std::vector<std::shared_ptr<DataOperator>> ComposeDataOp::Candidates(CopyDirection dir, const ExtOptions &opt, uint64_t bytes, bool batch) const
+unsigned ComposeDataOp::Order(CopyDirection dir, const ExtOptions &opt, uint64_t bytes, bool batch, unsigned picked[kMaxEngines]) const
 {
     uint32_t mask = allowed_;
     if (tags_) {
         mask = tags_->AllowedOps(opt.srcRank, opt.dstRank, allowed_);
     }
-    // Rank order of preference for this call.
-    std::vector<uint32_t> order;
     constexpr uint32_t kCpuBits = OP_HOST_RDMA | OP_HOST_TCP | OP_HOST_URMA;
     constexpr uint64_t kCopyEngineMin = 1ull << 20;
+    // Ranking for this call, best first.
+    static constexpr uint32_t kHost[] = {kCpuBits, OP_COPY_ENGINE, OP_KERNEL_LDST}, kKernel[] = {OP_KERNEL_LDST, OP_COPY_ENGINE, kCpuBits},
+                              kNoKernel[] = {OP_COPY_ENGINE, kCpuBits, 0}, kEngine[] = {OP_COPY_ENGINE, OP_KERNEL_LDST, kCpuBits};
+    const uint32_t *order = kKernel;
     if (HostOnly(dir)) {
-        order = {kCpuBits, OP_COPY_ENGINE, OP_KERNEL_LDST};
+        order = kHost;
     } else if (opt.flags & FLAG_COPY_KERNEL) {
-        order = {OP_KERNEL_LDST, OP_COPY_ENGINE, kCpuBits};
+        order = kKernel;
     } else if (!opt.srcDeviceVisible || !opt.dstDeviceVisible) {
-        order = {OP_COPY_ENGINE, kCpuBits};
+        order = kNoKernel;
     } else if (TouchesHost(dir) && !batch && bytes >= kCopyEngineMin) {
-        order = {OP_COPY_ENGINE, OP_KERNEL_LDST, kCpuBits};  // big host legs: DMA engines saturate PCIe without SMs
+        order = kEngine;  // big host legs: DMA engines saturate PCIe without SMs
     } else if (!batch && opt.srcRank != opt.dstRank && PeerCopyEngineMin() != 0 && bytes >= PeerCopyEngineMin()) {
         // Opt-in (MF_PEER_COPY_ENGINE_MIN_MB): large single transfers between GPUs ride the copy engine, whose packets
         // carry about a tenth more payload over NVLink than writes issued by SMs can; the SMs stay free for compute.
-        order = {OP_COPY_ENGINE, OP_KERNEL_LDST, kCpuBits};
-    } else {
-        order = {OP_KERNEL_LDST, OP_COPY_ENGINE, kCpuBits};
+        order = kEngine;
     }
-    std::vector<std::shared_ptr<DataOperator>> out;
-    for (uint32_t want : order) {
-        for (auto &e : engines_) {
-            uint32_t t = e->Type();
-            bool isCpu = (t & kCpuBits) != 0;
+    unsigned n = 0;
+    for (int k = 0; k < 3; k++) {
+        for (unsigned i = 0; i < engines_.size() && n < kMaxEngines; i++) {
+            const uint32_t t = engines_[i]->Type();
+            const bool isCpu = (t & kCpuBits) != 0;
             // DEVICE_RDMA shares the kernel engine; host engines are always admissible for host-only legs.
-            bool permitted = isCpu ? (HostOnly(dir) || (mask & kCpuBits)) : ((mask & t) || (t == OP_KERNEL_LDST && (mask & OP_DEVICE_RDMA)));
-            if ((t & want) && permitted && e->Supports(dir, opt) && std::find(out.begin(), out.end(), e) == out.end()) {
-                out.push_back(e);
+            const bool permitted = isCpu ? (HostOnly(dir) || (mask & kCpuBits)) : ((mask & t) || (t == OP_KERNEL_LDST && (mask & OP_DEVICE_RDMA)));
+            if ((t & order[k]) && permitted && engines_[i]->Supports(dir, opt) && std::find(picked, picked + n, i) == picked + n) {
+                picked[n++] = i;
             }
         }
+    }
+    return n;
+}
+
+std::vector<std::shared_ptr<DataOperator>> ComposeDataOp::Candidates(CopyDirection dir, const ExtOptions &opt, uint64_t bytes, bool batch) const
+{
+    unsigned picked[kMaxEngines];
+    const unsigned n = Order(dir, opt, bytes, batch, picked);
+    std::vector<std::shared_ptr<DataOperator>> out;
+    for (unsigned k = 0; k < n; k++) {
+        out.push_back(engines_[picked[k]]);
     }
     return out;
 }
@@ -667,8 +715,10 @@ int ComposeDataOp::DataCopy(const CopyParams &p, CopyDirection dir, const ExtOpt
 {
     int ret = BM_NOT_SUPPORTED;
     MF_TRACE_SCOPE(MF_TP(TM_DATAOP, (int)dir), DirectionName(dir), &ret);
-    auto cands = Candidates(dir, opt, p.dataSize, false);
-    for (auto &e : cands) {
+    unsigned picked[kMaxEngines];
+    const unsigned n = Order(dir, opt, p.dataSize, false, picked);
+    for (unsigned k = 0; k < n; k++) {
+        DataOperator *e = engines_[picked[k]].get();
         ret = e->DataCopy(p, dir, opt);
         if (ret == BM_OK) {
             NoteServed(e->Type(), 1);
@@ -676,7 +726,7 @@ int ComposeDataOp::DataCopy(const CopyParams &p, CopyDirection dir, const ExtOpt
         }
         MF_WARN("data op: engine " << e->Name() << " failed (" << ret << ") for " << DirectionName(dir) << ", trying the next one");
     }
-    if (cands.empty()) {
+    if (n == 0) {
         MF_ERROR("data op: no engine can serve " << DirectionName(dir) << " between ranks " << opt.srcRank << " and " << opt.dstRank);
     }
     return ret;
@@ -690,8 +740,10 @@ int ComposeDataOp::BatchDataCopy(const BatchCopyParams &p, CopyDirection dir, co
     for (uint32_t i = 0; i < p.batchSize; i++) {
         bytes += p.dataSizes[i];
     }
-    auto cands = Candidates(dir, opt, bytes, true);
-    for (auto &e : cands) {
+    unsigned picked[kMaxEngines];
+    const unsigned n = Order(dir, opt, bytes, true, picked);
+    for (unsigned k = 0; k < n; k++) {
+        DataOperator *e = engines_[picked[k]].get();
         ret = e->BatchDataCopy(p, dir, opt);
         if (ret == BM_OK) {
             NoteServed(e->Type(), p.batchSize);
@@ -699,7 +751,7 @@ int ComposeDataOp::BatchDataCopy(const BatchCopyParams &p, CopyDirection dir, co
         }
         MF_WARN("data op: engine " << e->Name() << " failed (" << ret << ") for batch " << DirectionName(dir) << ", trying the next one");
     }
-    if (cands.empty()) {
+    if (n == 0) {
         MF_ERROR("data op: no engine can serve batch " << DirectionName(dir));
     }
     return ret;

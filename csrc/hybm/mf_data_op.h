@@ -2,7 +2,7 @@
 //
 // Interface after the reference's DataOperator (src/hybm/csrc/data_operation/hybm_data_operator.h:22-101). Engines:
 //   KernelDataOp      LD/ST copy kernels (mf_xcopy.cu) — every leg both of whose ends a GPU kernel can dereference: local
-//                     HBM, peer HBM over NVLink, pinned host pool. Batches are one launch with a completion word.
+//                     HBM, peer HBM over NVLink, pinned host pool. Batches are one launch.
 //                     Role of HostDataOpSDMA + the copy_extend kernels (data_operation/host/hybm_data_op_sdma.cpp).
 //   CopyEngineDataOp  cudaMemcpyAsync — legs that touch ordinary (unpinned) local host memory, and large host-pool legs.
 //                     Unlike the reference's LH↔G path (hybm_data_op_sdma.cpp:171-221) no temporary device buffer is
@@ -83,6 +83,10 @@ public:
     void SetEngines(std::vector<std::shared_ptr<DataOperator>> engines) { engines_ = std::move(engines); }
 
 private:
+    static constexpr unsigned kMaxEngines = 8;
+    // Indexes into engines_ in the order to try; returns how many.
+    unsigned Order(CopyDirection dir, const ExtOptions &opt, uint64_t bytes, bool batch, unsigned picked[kMaxEngines]) const;
+
     int device_;
     uint32_t allowed_;
     std::shared_ptr<TagInfo> tags_;

@@ -20,60 +20,83 @@ __device__ __forceinline__ void StStream16(void *p, const uint4 &v)
     asm volatile("st.global.L1::no_allocate.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-template <typename T>
-__device__ __forceinline__ T LdStream(const T *p)
+// Copies n aligned 16-byte vectors with THREADS cooperating threads (this thread is `tid`), UNROLL independent loads in flight per
+// thread before the first store; what is left at the end takes less than one trip and has the same loads in flight, each
+// under its own bound.
+template <int UNROLL, int THREADS>
+__device__ __forceinline__ void CopyVec(uint4 *__restrict__ dst, const uint4 *__restrict__ src, unsigned n, unsigned tid)
 {
-    return *p;
-}
-template <>
-__device__ __forceinline__ uint4 LdStream<uint4>(const uint4 *p)
-{
-    return LdStream16(p);
-}
-template <typename T>
-__device__ __forceinline__ void StStream(T *p, const T &v)
-{
-    *p = v;
-}
-template <>
-__device__ __forceinline__ void StStream<uint4>(uint4 *p, const uint4 &v)
-{
-    StStream16(p, v);
-}
-
-// Copies n elements of T with `nthreads` cooperating threads (this thread is `tid`), UNROLL independent loads in flight
-// per thread before the first store.
-template <typename T, int UNROLL>
-__device__ __forceinline__ void CopyVec(T *__restrict__ dst, const T *__restrict__ src, size_t n, unsigned tid, unsigned nthreads)
-{
-    size_t i = tid;
-    const size_t step = (size_t)nthreads * UNROLL;
-    for (; i + (size_t)(UNROLL - 1) * nthreads < n; i += step) {
-        T v[UNROLL];
+    dst += tid;
+    src += tid;
+    int left = (int)n - (int)tid;  // this thread's vectors are those below it in steps of THREADS
+    for (; left > 0; left -= UNROLL * THREADS, dst += UNROLL * THREADS, src += UNROLL * THREADS) {
+        uint4 v[UNROLL];
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
-            v[u] = LdStream<T>(src + i + (size_t)u * nthreads);
+            if (left > u * THREADS) {
+                v[u] = LdStream16(src + u * THREADS);
+            }
         }
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
-            StStream<T>(dst + i + (size_t)u * nthreads, v[u]);
+            if (left > u * THREADS) {
+                StStream16(dst + u * THREADS, v[u]);
+            }
         }
-    }
-    for (; i < n; i += nthreads) {
-        StStream<T>(dst + i, LdStream<T>(src + i));
     }
 }
 
-// Copies [src, src+n) to [dst, dst+n) with the threads (tid of nthreads). The destination is brought to a 16-byte
-// boundary with byte stores; the body then uses the widest vector that the *relative* alignment of the two pointers
-// allows (16 bytes when src and dst are congruent modulo 16).
-template <int UNROLL>
-__device__ __forceinline__ void CopySpan(unsigned char *dst, const unsigned char *src, size_t n, unsigned tid, unsigned nthreads)
+// The same through the L1: for vectors that two threads read.
+__device__ __forceinline__ uint4 LdShared16(const void *p)
 {
-    if (n == 0) {
-        return;
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// The 16 bytes that start `rel` (0..15) bytes into the 32 bytes of two neighbouring vectors: by two words, by one, by bits.
+__device__ __forceinline__ uint4 Realign16(const uint4 &a, const uint4 &b, unsigned rel)
+{
+    const bool two = (rel & 8) != 0, one = (rel & 4) != 0;
+    const uint32_t t0 = two ? a.z : a.x, t1 = two ? a.w : a.y, t2 = two ? b.x : a.z, t3 = two ? b.y : a.w, t4 = two ? b.z : b.x, t5 = two ? b.w : b.y;
+    const uint32_t w0 = one ? t1 : t0, w1 = one ? t2 : t1, w2 = one ? t3 : t2, w3 = one ? t4 : t3, w4 = one ? t5 : t4;
+    const unsigned bits = (rel & 3) * 8;
+    return make_uint4(__funnelshift_r(w0, w1, bits), __funnelshift_r(w1, w2, bits), __funnelshift_r(w2, w3, bits), __funnelshift_r(w3, w4, bits));
+}
+
+// nv 16-byte vectors to a 16-byte boundary from an address `rel` (1..15) bytes past `src`, a boundary. Memory is read and written
+// in aligned vectors only: an output takes the source vector that it starts in and the following one, which the L1 holds for the
+// neighbouring thread. Every source vector that is touched has at least one wanted byte, so nothing outside the pages of
+// the source is read. Narrow loads (two bytes for a bf16 slice at an odd element) need eight times the instructions.
+template <int UNROLL, int THREADS>
+__device__ __forceinline__ void CopyRealigned(uint4 *__restrict__ dst, const uint4 *__restrict__ src, unsigned nv, unsigned rel, unsigned tid)
+{
+    dst += tid;
+    src += tid;
+    for (int left = (int)nv - (int)tid; left > 0; left -= UNROLL * THREADS, dst += UNROLL * THREADS, src += UNROLL * THREADS) {
+        uint4 v[UNROLL], n[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) {
+            if (left > u * THREADS) {
+                v[u] = LdShared16(src + u * THREADS);
+                n[u] = LdShared16(src + u * THREADS + 1);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) {
+            if (left > u * THREADS) {
+                StStream16(dst + u * THREADS, Realign16(v[u], n[u], rel));
+            }
+        }
     }
-    size_t head = (16 - ((uintptr_t)dst & 15)) & 15;
+}
+
+// Copies [src, src+n), at most 1 GiB, to [dst, dst+n) with the threads (tid of THREADS). The destination is brought to a 16-byte
+// boundary with byte stores; the body moves in 16-byte vectors whatever the two addresses are modulo 16.
+template <int UNROLL, int THREADS>
+__device__ __forceinline__ void CopySpan(unsigned char *dst, const unsigned char *src, unsigned n, unsigned tid)
+{
+    unsigned head = (16 - (unsigned)((uintptr_t)dst & 15)) & 15;
     if (head > n) {
         head = n;
     }
@@ -83,25 +106,16 @@ __device__ __forceinline__ void CopySpan(unsigned char *dst, const unsigned char
     dst += head;
     src += head;
     n -= head;
+    const unsigned body = n & ~15u;
     const unsigned rel = (unsigned)((uintptr_t)src & 15);
-    size_t body;
+    uint4 *d16 = (uint4 *)dst;
+    const uint4 *s16 = (const uint4 *)(src - rel);
     if (rel == 0) {
-        body = n & ~(size_t)15;
-        CopyVec<uint4, UNROLL>((uint4 *)dst, (const uint4 *)src, body >> 4, tid, nthreads);
-    } else if ((rel & 7) == 0) {
-        body = n & ~(size_t)7;
-        CopyVec<uint2, UNROLL>((uint2 *)dst, (const uint2 *)src, body >> 3, tid, nthreads);
-    } else if ((rel & 3) == 0) {
-        body = n & ~(size_t)3;
-        CopyVec<uint32_t, UNROLL>((uint32_t *)dst, (const uint32_t *)src, body >> 2, tid, nthreads);
-    } else if ((rel & 1) == 0) {
-        body = n & ~(size_t)1;
-        CopyVec<uint16_t, UNROLL>((uint16_t *)dst, (const uint16_t *)src, body >> 1, tid, nthreads);
+        CopyVec<UNROLL, THREADS>(d16, s16, body >> 4, tid);
     } else {
-        body = n;
-        CopyVec<unsigned char, UNROLL>(dst, src, body, tid, nthreads);
+        CopyRealigned<UNROLL / 2, THREADS>(d16, s16, body >> 4, rel, tid);
     }
-    const size_t tail = n - body;
+    const unsigned tail = n - body;
     if (tid < tail) {
         dst[body + tid] = src[body + tid];
     }

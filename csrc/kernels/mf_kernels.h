@@ -39,11 +39,16 @@ enum { MF_BATCH_INLINE_MAX = 168, MF_BATCH_CHUNK_BYTES = 32768 };
 // Batch of `count` independent copies in ONE launch. Descriptors must have chunkStart filled (prefix sum of
 // ceil(len / MF_BATCH_CHUNK_BYTES)); totalChunks is the grand total. count <= MF_BATCH_INLINE_MAX travels in the kernel
 // parameters; larger batches must pass `descsDev`, a device-readable copy of the table that is followed directly by
-// uint32 map[totalChunks] giving each chunk's descriptor index. `doneCounter` (device, zero
-// before first use, self-resetting) and `hostFlag` (pinned host word, may be NULL) implement completion signalling:
-// the last CTA stores `flagValue` to *hostFlag with system-scope release semantics.
-int mf_k_batch_xcopy(const mf_copy_desc_t *descs, const mf_copy_desc_t *descsDev, uint32_t count, uint32_t totalChunks,
-                     uint32_t *doneCounter, volatile uint32_t *hostFlag, uint32_t flagValue, int ctas, mf_stream_t stream);
+// uint32 map[totalChunks] giving each chunk's descriptor index.
+int mf_k_batch_xcopy(const mf_copy_desc_t *descs, const mf_copy_desc_t *descsDev, uint32_t count, uint32_t totalChunks, int ctas, mf_stream_t stream);
+
+// The same for batches whose addresses and lengths are all multiples of 16 bytes, through the bulk copy engine of the SMs. Chunks
+// are 1 << chunkShift bytes (10..15; mf_k_batch_bulk_shift picks it from the size of the batch), chunkStart and totalChunks count
+// those. At most MF_BULK_INLINE_MAX descriptors travel in the kernel parameters of a launch; a longer batch is launched in
+// pieces, each numbered from chunk 0, on one stream with nothing in between, `chained` set from the second on.
+enum { MF_BULK_FIRST_PIECE = 504, MF_BULK_INLINE_MAX = 1344 };
+uint32_t mf_k_batch_bulk_shift(uint64_t totalBytes);
+int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint32_t totalChunks, uint32_t chunkShift, int chained, mf_stream_t stream);
 
 // ------------------------------------------------------------------------------------------------ allreduce + RMSNorm (K4)
 

@@ -3,19 +3,21 @@
 // mf_xcopy_kernel        one contiguous copy, any alignment. Contract of the reference's hybm_copy_kernel
 //                        (src/hybm/csrc/copy_extend/hybm_copy_kernel.cpp:44-83): split the byte range over the grid in
 //                        aligned shares and move each share load→store; bit-exact result.
-// mf_batch_xcopy_kernel  N independent {src,dst,len} copies in one launch plus a completion word. Contract of
+// mf_batch_xcopy_kernel  N independent {src,dst,len} copies in one launch. Contract of
 //                        hybm_batch_copy_kernel and its parameter-slot protocol (hybm_copy_kernel.cpp:85-124,
 //                        src/hybm/csrc/data_operation/host/hybm_data_op_sdma.cpp:504-543). Differences by design:
 //                        work is balanced by BYTES (fixed-size chunks found by binary search over a prefix table)
-//                        rather than by descriptor index, small tables ride in the kernel parameters, and completion is
-//                        one counter + one system-scope release store instead of a chain of blocks spinning on each other
-//                        (no device-side wait exists in this kernel, so nothing can hang).
+//                        rather than by descriptor index, small tables ride in the kernel parameters, and completion is that
+//                        of the launch instead of a chain of blocks spinning on each other (a completion word in pinned host
+//                        memory needs a system-wide fence in every CTA and was seen 5 us later than the stream's own completion).
 // Blackwell mapping: 16-byte streaming loads with L1 bypass, 8 loads in flight per thread before the first store,
 // 512-thread CTAs at two per SM (128 KiB in flight per SM — enough to cover HBM3e and NVLink latency), persistent grid.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 
 #include "mf_copy_device.cuh"
 #include "mf_kernels.h"
@@ -24,18 +26,22 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kUnroll = 8;
-constexpr size_t kPdlMaxBytes = 32 * 1024;
+
+// Programmatic dependent launch: every copy kernel is launched with the stream-serialisation attribute, so the next one of the
+// stream may be scheduled while this one runs, and this one may have been scheduled while its predecessor ran; the wait returns
+// once the predecessor has completed and its writes are visible. Stream order is kept, only the launch latency between
+// back-to-back copies is hidden: 4.1 -> 2.2 us a copy up to 1 MiB, 6.2 -> 3.4 us at 8 MiB, 14.4 -> 13.0 us at 32 MiB. Without the
+// attribute both instructions do nothing.
+__device__ __forceinline__ void FollowPredecessor()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 __global__ void __launch_bounds__(kThreads, 2)
 mf_xcopy_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict__ src, size_t n, size_t tileBytes)
 {
-    // Programmatic dependent launch: when the host sets the stream-serialisation attribute (copies up to kPdlMaxBytes: beyond it the overlap measured no gain), the
-    // next kernel of the stream may be scheduled while this one runs, and this kernel may have been scheduled while its
-    // predecessor ran; the wait returns once the predecessor has completed and its writes are visible, so stream order
-    // is kept and only the launch latency between back-to-back copies is hidden. Without the attribute both
-    // instructions do nothing.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    FollowPredecessor();
     // Tile 0 is stretched by `lead` bytes so that every later tile starts on a 16-byte boundary of dst.
     const size_t lead = (16 - ((uintptr_t)dst & 15)) & 15;
     const size_t body = n > lead ? n - lead : 0;
@@ -46,7 +52,7 @@ mf_xcopy_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict
         if (end > n) {
             end = n;
         }
-        mf::dev::CopySpan<kUnroll>(dst + begin, src + begin, end - begin, threadIdx.x, kThreads);
+        mf::dev::CopySpan<kUnroll, kThreads>(dst + begin, src + begin, (unsigned)(end - begin), threadIdx.x);
     }
 }
 
@@ -55,12 +61,12 @@ mf_xcopy_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict
 // asynchronous copy engine of the SM (cp.async.bulk, no tensor map, no multicast) through a ring of shared-memory stages. One
 // thread issues loads, one thread issues stores; mbarriers hand tiles over. The SM's load/store units and register file stay out of the
 // data path, so the copy runs at what the memory system and NVLink deliver. Waits are bounded like everywhere else.
-// Default pipeline shapes, picked from a sweep of tile x stages x stores in flight x walk order x CTAs per SM on local HBM
-// copies (a shallow pipeline interleaves DRAM reads and writes more regularly than a deep one: 6 stages with 3 stores in
-// flight measured 3.11 TB/s at 1 GiB, the shapes below 3.30 TB/s, the copy engine 3.27 TB/s). Over NVLink every shape
-// runs at the link's rate. Large copies: 32 KiB tiles, 4 stages, 2 stores in flight, each CTA on one contiguous run.
-// Smaller ones: 16 KiB tiles, 4 stages, 1 store in flight, strided walk, two CTAs per SM so the last wave is short.
-constexpr size_t kTmaLargeBytes = 256u << 20;
+// Default pipeline shape, picked from a sweep of tile x stages x stores in flight x walk order x CTAs per SM on local HBM
+// copies (a shallow pipeline interleaves DRAM reads and writes more regularly than a deep one): 32 KiB tiles, 4 stages, 2
+// stores in flight, one CTA per SM, strided walk: 12.9 / 23.0 / 44.0 / 83.5 / 325 us at 32 / 64 / 128 / 256 / 1024 MiB, against 13.3 /
+// 25.4 / 50.0 / 97.5 / 376 us of the load/store kernel. Below kTmaMinBytes the load/store kernel is the faster one (3.6 and 6.2 us
+// at 8 and 16 MiB against 3.5 and 6.7 us, 3.1 against 3.3 us at 4 MiB). Over NVLink every shape runs at the link's rate.
+constexpr size_t kTmaMinBytes = 24u << 20;
 
 __device__ __forceinline__ uint32_t SmemU32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -113,6 +119,7 @@ mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__rest
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tmaSmemRaw) + 127) & ~(uintptr_t)127);
     __shared__ uint64_t full[kTmaMaxStages], empty[kTmaMaxStages];
     const uint32_t kTmaTile = shape.tile, kTmaStages = shape.stages, kTmaStoresInFlight = shape.inflight;
+    FollowPredecessor();
     // Unaligned head (up to the first 16-byte boundary of dst) and tail bytes go through ordinary loads/stores.
     const size_t head = n < 16 ? n : ((16 - ((uintptr_t)dst & 15)) & 15);
     const size_t body = (n - head) & ~(size_t)15;
@@ -184,10 +191,6 @@ mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__rest
 struct BatchInline {
     uint32_t count;
     uint32_t totalChunks;
-    uint32_t flagValue;
-    uint32_t pad;
-    uint32_t *doneCounter;
-    volatile uint32_t *hostFlag;
     mf_copy_desc_t d[MF_BATCH_INLINE_MAX];
 };
 static_assert(sizeof(BatchInline) <= 4096 + 32, "inline batch must fit the classic kernel parameter space");
@@ -217,42 +220,141 @@ __device__ __forceinline__ void BatchBody(const mf_copy_desc_t *__restrict__ d, 
         if (len > MF_BATCH_CHUNK_BYTES) {
             len = MF_BATCH_CHUNK_BYTES;
         }
-        mf::dev::CopySpan<4>((unsigned char *)(d[lo].dst + off), (const unsigned char *)(d[lo].src + off), len, threadIdx.x, kThreads);
-    }
-}
-
-__device__ __forceinline__ void BatchSignal(uint32_t *doneCounter, volatile uint32_t *hostFlag, uint32_t flagValue)
-{
-    if (doneCounter == nullptr) {
-        return;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence_system();  // this CTA's copies are visible system-wide before it is counted
-        unsigned prev = atomicAdd(doneCounter, 1u);
-        if (prev == gridDim.x - 1) {
-            *doneCounter = 0;  // self-reset for the next launch that uses this slot
-            __threadfence_system();
-            if (hostFlag != nullptr) {
-                asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(hostFlag), "r"(flagValue) : "memory");
-            }
-        }
+        mf::dev::CopySpan<4, kThreads>((unsigned char *)(d[lo].dst + off), (const unsigned char *)(d[lo].src + off), (unsigned)len, threadIdx.x);
     }
 }
 
 __global__ void __launch_bounds__(kThreads, 2) mf_batch_xcopy_inline_kernel(const __grid_constant__ BatchInline p)
 {
+    FollowPredecessor();
     BatchBody(p.d, p.count, p.totalChunks, nullptr);
-    BatchSignal(p.doneCounter, p.hostFlag, p.flagValue);
 }
 
 // The chunk → descriptor map follows the descriptor table in the same device buffer.
 __global__ void __launch_bounds__(kThreads, 2)
-mf_batch_xcopy_table_kernel(const mf_copy_desc_t *__restrict__ d, uint32_t count, uint32_t totalChunks, uint32_t *doneCounter,
-                            volatile uint32_t *hostFlag, uint32_t flagValue)
+mf_batch_xcopy_table_kernel(const mf_copy_desc_t *__restrict__ d, uint32_t count, uint32_t totalChunks)
 {
+    FollowPredecessor();
     BatchBody(d, count, totalChunks, reinterpret_cast<const uint32_t *>(d + count));
-    BatchSignal(doneCounter, hostFlag, flagValue);
+}
+
+// ---------------------------------------------------------------------------------------------- bulk-copy batch
+// Batches whose addresses and lengths are all multiples of 16 (KV blocks, pages): the same global → shared → global pipeline of
+// the SM's bulk copy engine, fed from the descriptor list. The batch is cut into chunks of 1 << chunkShift bytes and CTA b
+// owns the run [b * total / grid, (b + 1) * total / grid) of them, so CTAs differ by one chunk at most and every load of a small
+// batch is in flight at once; a CTA finds its first descriptor by a 128-way search and walks on from there.
+// A long list goes out as several launches, so that the GPU works on the first while the host prepares the next. The first
+// piece lets its dependents start only after its own wait, i.e. when everything before the batch is complete; the others therefore
+// begin at once, as SMs become free, and wait for the piece before them at their END, which keeps completion in stream order.
+struct BulkBatch {
+    uint32_t count;
+    uint32_t totalChunks;
+    uint32_t chunkShift;
+    uint32_t stages;
+    uint32_t inflight;
+    uint32_t chained;  // a further piece of the batch whose first piece was launched just before
+};
+template <int MAX>
+struct BulkBatchInline {
+    BulkBatch b;
+    mf_copy_desc_t d[MAX];
+};
+constexpr int kBulkThreads = 128;
+constexpr int kBulkSmemMax = 128 * 1024 + 128;
+
+__device__ __forceinline__ void BulkBatchBody(const BulkBatch &b, const mf_copy_desc_t *__restrict__ d)
+{
+    extern __shared__ unsigned char tmaSmemRaw[];
+    unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tmaSmemRaw) + 127) & ~(uintptr_t)127);
+    __shared__ uint64_t full[kTmaMaxStages], empty[kTmaMaxStages];
+    __shared__ uint64_t stageDst[kTmaMaxStages];
+    __shared__ uint32_t stageLen[kTmaMaxStages];
+    const uint32_t c0 = (uint32_t)((uint64_t)blockIdx.x * b.totalChunks / gridDim.x);
+    const uint32_t c1 = (uint32_t)((uint64_t)(blockIdx.x + 1) * b.totalChunks / gridDim.x);
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < b.stages; i++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(SmemU32(&full[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(SmemU32(&empty[i])));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (!b.chained) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // Last descriptor whose chunkStart <= c0 (chunkStart ascends, d[0] starts at 0).
+    uint32_t lo = 0, n = b.count;
+    while (n > 1) {
+        const uint32_t step = (n + kBulkThreads - 1) / kBulkThreads;
+        const uint32_t probe = threadIdx.x * step;
+        const int k = __syncthreads_count(probe < n && d[lo + probe].chunkStart <= c0);
+        lo += (uint32_t)(k - 1) * step;
+        n = min(step, n - (uint32_t)(k - 1) * step);
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        // Loader: the warp holds 32 descriptors and has the next 32 on the way; lane 0 issues.
+        uint32_t window = lo, cur = 0;
+        mf_copy_desc_t mine = d[min(window + lane, b.count - 1)], next = d[min(window + 32 + lane, b.count - 1)];
+        uint64_t src = __shfl_sync(0xffffffffu, mine.src, 0), dst = __shfl_sync(0xffffffffu, mine.dst, 0);
+        uint32_t len = __shfl_sync(0xffffffffu, mine.len, 0), start = __shfl_sync(0xffffffffu, mine.chunkStart, 0);
+        bool alive = true;
+        for (uint32_t c = c0, it = 0; c < c1; c++, it++) {
+            if (((uint64_t)(c - start) << b.chunkShift) >= len) {
+                if (++cur == 32) {
+                    window += 32;
+                    cur = 0;
+                    mine = next;
+                    next = d[min(window + 32 + lane, b.count - 1)];
+                }
+                src = __shfl_sync(0xffffffffu, mine.src, cur);
+                dst = __shfl_sync(0xffffffffu, mine.dst, cur);
+                len = __shfl_sync(0xffffffffu, mine.len, cur);
+                start = __shfl_sync(0xffffffffu, mine.chunkStart, cur);
+            }
+            if (lane == 0 && alive) {
+                const uint32_t st = it % b.stages, ph = (it / b.stages) & 1;
+                const uint32_t off = (c - start) << b.chunkShift;
+                const uint32_t bytes = min(len - off, 1u << b.chunkShift);
+                alive = MbarWaitParity(&empty[st], ph ^ 1);
+                if (alive) {
+                    stageDst[st] = dst + off;
+                    stageLen[st] = bytes;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemU32(&full[st])), "r"(bytes) : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     SmemU32(tiles + ((size_t)st << b.chunkShift))),
+                                 "l"(src + off), "r"(bytes), "r"(SmemU32(&full[st]))
+                                 : "memory");
+                }
+            }
+        }
+    } else if (threadIdx.x == 32) {
+        for (uint32_t it = 0; it < c1 - c0; it++) {
+            const uint32_t st = it % b.stages, ph = (it / b.stages) & 1;
+            if (!MbarWaitParity(&full[st], ph)) {
+                break;
+            }
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(stageDst[st]), "r"(SmemU32(tiles + ((size_t)st << b.chunkShift))),
+                         "r"(stageLen[st])
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            BulkWaitRead(b.inflight);
+            if (it >= b.inflight) {
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemU32(&empty[(it - b.inflight) % b.stages])) : "memory");
+            }
+        }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every store of this CTA has landed
+        if (b.chained) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+    }
+}
+
+template <int MAX>
+__global__ void __launch_bounds__(kBulkThreads, 1) mf_batch_bulk_inline_kernel(const __grid_constant__ BulkBatchInline<MAX> p)
+{
+    BulkBatchBody(p.b, p.d);
 }
 
 // ---------------------------------------------------------------------------------------------- test support
@@ -328,6 +430,57 @@ int SmCount()
     return cached[dev];
 }
 
+template <typename T>
+struct Same {
+    using type = T;
+};
+
+// Launches a copy kernel that begins with FollowPredecessor(). MF_XCOPY_PDL=0 turns the overlap off (read once).
+template <typename... Params>
+int LaunchCopy(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, mf_stream_t stream, const typename Same<Params>::type &...args)
+{
+    static const bool usePdl = []() {
+        const char *e = getenv("MF_XCOPY_PDL");
+        return !(e != nullptr && e[0] == '0');
+    }();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = usePdl ? 1 : 0;
+    void *params[] = {(void *)&args...};
+    if (cudaLaunchKernelExC(&cfg, (const void *)kernel, params) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MF_K_LAUNCH_FAILED;
+    }
+    return MF_K_OK;
+}
+
+// Dynamic shared memory above 48 KiB has to be allowed once per kernel and device.
+template <auto KERNEL>
+bool AllowSmem(size_t bytes)
+{
+    static std::atomic<bool> allowed[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (!allowed[dev].load(std::memory_order_relaxed)) {
+        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        allowed[dev].store(true, std::memory_order_relaxed);
+    }
+    return true;
+}
+
 int LaunchResult()
 {
     cudaError_t e = cudaGetLastError();
@@ -351,21 +504,15 @@ static bool ShapeValid(const TmaShape &sh)
 
 static int LaunchTma(void *dst, const void *src, size_t n, const TmaShape &shape, int ctas, int sms, mf_stream_t stream)
 {
-    static size_t attrBytes = 0;
     const size_t smem = (size_t)shape.stages * shape.tile + 128;
-    if (smem > attrBytes) {
-        if (cudaFuncSetAttribute(mf_xcopy_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return MF_K_LAUNCH_FAILED;
-        }
-        attrBytes = smem;
+    if (!AllowSmem<mf_xcopy_tma_kernel>(220 * 1024 + 128)) {
+        return MF_K_LAUNCH_FAILED;
     }
     size_t tiles = (n + shape.tile - 1) / shape.tile;
     const size_t perSm = smem <= 110u * 1024 ? 2 : 1;  // two CTAs fit an SM when their tiles take less than half its shared memory
     const size_t full = (size_t)sms * perSm;
     size_t grid = ctas > 0 ? (size_t)ctas : (tiles < full ? tiles : full);
-    mf_xcopy_tma_kernel<<<(unsigned)grid, 128, smem, (cudaStream_t)stream>>>((unsigned char *)dst, (const unsigned char *)src, n, shape);
-    return LaunchResult();
+    return LaunchCopy(mf_xcopy_tma_kernel, (unsigned)grid, 128, smem, stream, (unsigned char *)dst, (const unsigned char *)src, n, shape);
 }
 
 // The bulk-copy kernel with an explicit pipeline shape, for tuning sweeps. Same preconditions as the automatic path: both
@@ -400,11 +547,7 @@ extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, mf_str
         const char *e = getenv("MF_XCOPY_TMA");
         return !(e != nullptr && e[0] == '0');
     }();
-    static const bool usePdl = []() {
-        const char *e = getenv("MF_XCOPY_PDL");
-        return !(e != nullptr && e[0] == '0');
-    }();
-    if (useTma && ctas >= 0 && n >= (4u << 20) && ((((uintptr_t)dst) ^ ((uintptr_t)src)) & 15) == 0) {
+    if (useTma && ctas >= 0 && n >= kTmaMinBytes && ((((uintptr_t)dst) ^ ((uintptr_t)src)) & 15) == 0) {
         // MF_XCOPY_SHAPE="tile,stages,inflight,blocked" overrides the pipeline shape (read once).
         static const TmaShape forced = []() {
             TmaShape sh{0, 0, 0, 0};
@@ -418,42 +561,26 @@ extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, mf_str
             }
             return sh;
         }();
-        const TmaShape shape = forced.tile != 0 ? forced : (n >= kTmaLargeBytes ? TmaShape{32 * 1024, 4, 2, 1} : TmaShape{16 * 1024, 4, 1, 0});
+        const TmaShape shape = forced.tile != 0 ? forced : TmaShape{32 * 1024, 4, 2, 0};
         return LaunchTma(dst, src, n, shape, ctas, sms, stream);
     }
     if (ctas < 0) {
         ctas = -ctas == 1 ? 0 : -ctas;  // negative: force the load/store kernel (with |ctas| CTAs, -1 = automatic)
     }
     const size_t maxCtas = (size_t)sms * 2;
-    // Tile = what one CTA moves per loop trip. Large copies use 64 KiB (8 × 16 B per thread); mid-size copies shrink the
-    // tile so that every SM gets work; 8 KiB is the floor (one 16-byte vector per thread).
-    size_t tile = 64 * 1024;
-    while (tile > 8 * 1024 && n / tile < maxCtas) {
-        tile >>= 1;
-    }
+    // Tile = what one CTA moves per loop trip: 64 KiB (8 x 16 B per thread) at most, 8 KiB (one 16-byte vector per thread)
+    // at least, and in between just as much as puts the whole copy into one wave with every load in flight at once (a power of
+    // two there left a second or third wave for a few CTAs).
+    const size_t tgt = ctas > 0 ? (size_t)ctas : maxCtas;
+    size_t tile = ((n + tgt - 1) / tgt + 511) & ~(size_t)511;
+    tile = tile < 8 * 1024 ? 8 * 1024 : (tile > 64 * 1024 ? 64 * 1024 : tile);
     size_t ntiles = (n + tile - 1) / tile;
     size_t grid = ctas > 0 ? (size_t)ctas : (ntiles < maxCtas ? ntiles : maxCtas);
-    // Back-to-back small copies are bound by the launch-to-launch gap, not by bytes: up to kPdlMaxBytes the kernel is
-    // launched with programmatic stream serialisation (measured on two B200s over NVLink: 4.1 us -> 2.5-2.9 us per 4-16 KiB
-    // copy, against 3.1-3.6 us for the copy engine; from 64 KiB on the overlap no longer pays).
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (usePdl && n <= kPdlMaxBytes) ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, mf_xcopy_kernel, (unsigned char *)dst, (const unsigned char *)src, n, tile) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return MF_K_LAUNCH_FAILED;
-    }
-    return MF_K_OK;
+    return LaunchCopy(mf_xcopy_kernel, (unsigned)grid, kThreads, 0, stream, (unsigned char *)dst, (const unsigned char *)src, n, tile);
 }
 
 extern "C" int mf_k_batch_xcopy(const mf_copy_desc_t *descs, const mf_copy_desc_t *descsDev, uint32_t count, uint32_t totalChunks,
-                                uint32_t *doneCounter, volatile uint32_t *hostFlag, uint32_t flagValue, int ctas, mf_stream_t stream)
+                                int ctas, mf_stream_t stream)
 {
     if (count == 0 || totalChunks == 0) {
         return MF_K_OK;
@@ -468,21 +595,56 @@ extern "C" int mf_k_batch_xcopy(const mf_copy_desc_t *descs, const mf_copy_desc_
         BatchInline p;
         p.count = count;
         p.totalChunks = totalChunks;
-        p.flagValue = flagValue;
-        p.pad = 0;
-        p.doneCounter = doneCounter;
-        p.hostFlag = hostFlag;
         for (uint32_t i = 0; i < count; i++) {
             p.d[i] = descs[i];
         }
-        mf_batch_xcopy_inline_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>(p);
-        return LaunchResult();
+        return LaunchCopy(mf_batch_xcopy_inline_kernel, grid, kThreads, 0, stream, p);
     }
     if (descsDev == nullptr) {
         return MF_K_INVALID;
     }
-    mf_batch_xcopy_table_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>(descsDev, count, totalChunks, doneCounter, hostFlag, flagValue);
-    return LaunchResult();
+    return LaunchCopy(mf_batch_xcopy_table_kernel, grid, kThreads, 0, stream, descsDev, count, totalChunks);
+}
+
+// Chunk size of a batch: with fewer bytes to share, smaller chunks spread them over more SMs (measured for 0.9, 2.9, 9, 36 and 288 MB
+// of KV blocks: 8 KiB 3.5 / 4.5 / 7.4 / 23.0 / 123 us, 16 KiB 3.7 / 4.2 / 6.2 / 19.8 / 113 us, 32 KiB 4.0 / 4.2 / 6.2 / 20.2 / 103 us).
+extern "C" uint32_t mf_k_batch_bulk_shift(uint64_t totalBytes) { return totalBytes >= (64ull << 20) ? 15 : (totalBytes >= (2ull << 20) ? 14 : 13); }
+
+template <int MAX>
+static int LaunchBulkInline(const BulkBatch &b, const mf_copy_desc_t *descs, unsigned grid, size_t smem, mf_stream_t stream)
+{
+    if (!AllowSmem<mf_batch_bulk_inline_kernel<MAX>>(kBulkSmemMax)) {
+        return MF_K_LAUNCH_FAILED;
+    }
+    BulkBatchInline<MAX> p;
+    p.b = b;
+    memcpy(p.d, descs, b.count * sizeof(mf_copy_desc_t));
+    return LaunchCopy(mf_batch_bulk_inline_kernel<MAX>, grid, kBulkThreads, smem, stream, p);
+}
+
+extern "C" int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint32_t totalChunks, uint32_t chunkShift, int chained, mf_stream_t stream)
+{
+    if (count == 0 || totalChunks == 0) {
+        return MF_K_OK;
+    }
+    const int sms = SmCount();
+    if (sms <= 0) {
+        return MF_K_LAUNCH_FAILED;
+    }
+    if (descs == nullptr || count > MF_BULK_INLINE_MAX || chunkShift < 10 || chunkShift > 15) {
+        return MF_K_INVALID;
+    }
+    // 128 KiB of stages and one CTA per SM: two or three smaller CTAs were never faster.
+    const uint32_t stages = chunkShift >= 15 ? 4 : 8, inflight = stages / 2;
+    const size_t smem = ((size_t)stages << chunkShift) + 128;
+    const unsigned grid = totalChunks < (unsigned)sms ? totalChunks : (unsigned)sms;
+    const BulkBatch b{count, totalChunks, chunkShift, stages, inflight, chained ? 1u : 0u};
+    // The launch copies the whole parameter block: 4 KiB cost nothing measurable, 32 KiB 3.5 us, so three sizes.
+    if (count <= 168) {
+        return LaunchBulkInline<168>(b, descs, grid, smem, stream);
+    }
+    return count <= MF_BULK_FIRST_PIECE ? LaunchBulkInline<MF_BULK_FIRST_PIECE>(b, descs, grid, smem, stream)
+                                        : LaunchBulkInline<MF_BULK_INLINE_MAX>(b, descs, grid, smem, stream);
 }
 
 extern "C" int mf_k_fill_pattern(void *dst, size_t n, uint64_t seed, mf_stream_t stream)
@@ -549,7 +711,7 @@ extern "C" unsigned long long mf_k_checksum_host(const void *buf, size_t n)
 }
 
 // ---------------------------------------------------------------------------------------------- batch copy without any allocation
-// See mf_xcopy_noalloc.h. The descriptor table, the chunk map and the completion counter of this variant live in the array
+// See mf_xcopy_noalloc.h. The descriptor table and the chunk map of this variant live in the array
 // below instead of in memory obtained from cudaMalloc. Every GPU that loads the library carries the array until exit.
 #include "mf_xcopy_noalloc.h"
 
@@ -558,9 +720,7 @@ extern "C" unsigned long long mf_k_checksum_host(const void *buf, size_t n)
 
 namespace {
 
-constexpr size_t kNoAllocHeader = 256;  // completion counter, padded so that the table stays 256-byte aligned
-constexpr size_t kNoAllocBytes =
-    kNoAllocHeader + (size_t)MF_NOALLOC_MAX_COPIES * sizeof(mf_copy_desc_t) + (size_t)MF_NOALLOC_MAX_CHUNKS * sizeof(uint32_t);
+constexpr size_t kNoAllocBytes = (size_t)MF_NOALLOC_MAX_COPIES * sizeof(mf_copy_desc_t) + (size_t)MF_NOALLOC_MAX_CHUNKS * sizeof(uint32_t);
 
 static __device__ __align__(256) unsigned char g_noAllocScratch[kNoAllocBytes];
 
@@ -633,11 +793,10 @@ extern "C" int mf_batch_xcopy_noalloc(const uint64_t *srcs, const uint64_t *dsts
     }
     cudaStream_t s = (cudaStream_t)stream;
     const size_t descBytes = (size_t)count * sizeof(mf_copy_desc_t);
-    // The array keeps whatever the previous call left in it: the counter has to start at zero, the table and the map are
-    // overwritten for exactly the part this call uses.
-    if (cudaMemsetAsync(base, 0, kNoAllocHeader, s) != cudaSuccess ||
-        cudaMemcpyAsync(base + kNoAllocHeader, g_noAllocDescs, descBytes, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemcpyAsync(base + kNoAllocHeader + descBytes, g_noAllocMap, (size_t)chunks * sizeof(uint32_t), cudaMemcpyHostToDevice, s) != cudaSuccess) {
+    // The array keeps whatever the previous call left in it: the table and the map are overwritten for exactly the part this
+    // call uses.
+    if (cudaMemcpyAsync(base, g_noAllocDescs, descBytes, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaMemcpyAsync(base + descBytes, g_noAllocMap, (size_t)chunks * sizeof(uint32_t), cudaMemcpyHostToDevice, s) != cudaSuccess) {
         fprintf(stderr, "mf_batch_xcopy_noalloc: staging the copy table failed: %s\n", cudaGetErrorString(cudaGetLastError()));
         return MF_K_LAUNCH_FAILED;
     }
@@ -647,7 +806,5 @@ extern "C" int mf_batch_xcopy_noalloc(const uint64_t *srcs, const uint64_t *dsts
     }
     const unsigned maxCtas = (unsigned)sms * 2;
     const unsigned grid = chunks < maxCtas ? (unsigned)chunks : maxCtas;
-    mf_batch_xcopy_table_kernel<<<grid, kThreads, 0, s>>>(reinterpret_cast<const mf_copy_desc_t *>(base + kNoAllocHeader), count, (uint32_t)chunks,
-                                                         reinterpret_cast<uint32_t *>(base), nullptr, 0);
-    return LaunchResult();
+    return LaunchCopy(mf_batch_xcopy_table_kernel, grid, kThreads, 0, (mf_stream_t)s, reinterpret_cast<const mf_copy_desc_t *>(base), count, (uint32_t)chunks);
 }

@@ -472,7 +472,7 @@ void BindNative(py::module_ &m)
         if (d.size() > MF_BATCH_INLINE_MAX) {
             return (int)MF_K_TOO_LARGE;
         }
-        return mf_k_batch_xcopy(d.data(), nullptr, (uint32_t)d.size(), chunks, nullptr, nullptr, 0, ctas, (mf_stream_t)stream);
+        return mf_k_batch_xcopy(d.data(), nullptr, (uint32_t)d.size(), chunks, ctas, (mf_stream_t)stream);
     }, py::arg("srcs"), py::arg("dsts"), py::arg("sizes"), py::arg("ctas") = 0, py::arg("stream") = 0);
     // Any number of copies up to the limits of the allocation-free entry point; tables longer than the inline limit run
     // through the table kernel.

@@ -1,0 +1,140 @@
+"""Edges of the copy kernels on one GPU, bytes against bytes: vectors put together from two neighbours at every relative alignment,
+tiles and their remainders, batches around the list lengths at which a launch takes a larger parameter block or a further piece,
+chunk remainders, batches that are not aligned, and an enqueued copy that follows the copy which writes its source."""
+import numpy as np
+import pytest
+
+from conftest import free_port
+
+pytestmark = pytest.mark.gpu
+
+KiB, MiB = 1 << 10, 1 << 20
+
+
+@pytest.fixture(scope="module")
+def pool():
+    import torch
+
+    from memfabric_hybrid_b200.parallel.pool import open_pool
+
+    torch.cuda.set_device(0)
+    p = open_pool(0, 1, 0, 192 * MiB, store_url=f"tcp://127.0.0.1:{free_port()}")
+    yield p
+    p.close()
+
+
+def _regions(pool, n):
+    import torch
+
+    from memfabric_hybrid_b200.utils.tensors import device_tensor_from_gva
+
+    src, dst = device_tensor_from_gva(pool.hbm(), n), device_tensor_from_gva(pool.hbm() + 96 * MiB, n)
+    src.random_(0, 256, generator=torch.Generator(device="cuda").manual_seed(n & 0xFFFF))
+    dst.fill_(0xA5)
+    torch.cuda.synchronize()
+    return src, dst
+
+
+@pytest.mark.parametrize("rel", range(16))
+@pytest.mark.parametrize("n", [31, 8 * KiB + 1, 148 * 2 * 8 * KiB + 17, 20 * MiB + 5])
+def test_every_relative_alignment(mf, pool, rel, n):
+    import torch
+
+    src, dst = _regions(pool, n + 64)
+    for doff in (0, 5):
+        dst.fill_(0xA5)
+        torch.cuda.synchronize()
+        soff = (rel + doff) % 16
+        assert pool.handle.copy_data(pool.hbm() + soff, pool.hbm() + 96 * MiB + 16 + doff, n, mf.bm.BmCopyType.G2G, 0) == 0, mf.get_last_err_msg()
+        lo = 16 + doff
+        assert torch.equal(dst[lo:lo + n], src[soff:soff + n])
+        assert bool((dst[:lo] == 0xA5).all()) and bool((dst[lo + n:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("n", [24 * MiB - 16, 24 * MiB, 24 * MiB + 16, 32 * KiB * 148 * 5 + 48])
+def test_both_sides_of_the_bulk_copy_threshold(mf, pool, n):
+    import torch
+
+    src, dst = _regions(pool, n + 64)
+    assert pool.handle.copy_data(pool.hbm() + 7, pool.hbm() + 96 * MiB + 23, n, mf.bm.BmCopyType.G2G, 0) == 0, mf.get_last_err_msg()
+    assert torch.equal(dst[23:23 + n], src[7:7 + n])
+    assert bool((dst[:23] == 0xA5).all()) and bool((dst[23 + n:] == 0xA5).all())
+
+
+def _batch(rng, count, unit, top, aligned=16):
+    """Blocks of 1..top units in a shuffled order with gaps between them: offsets and sizes in bytes."""
+    sizes = (rng.integers(1, top + 1, count) * unit).astype(np.int64)
+    slot = top * unit + 32
+    offs = rng.permutation(count).astype(np.int64) * slot + rng.integers(0, 2, count) * aligned
+    return offs, sizes, slot * count
+
+
+@pytest.mark.parametrize("stream", [False, True])
+@pytest.mark.parametrize("unit,top", [(16, 3), (16, 600), (8 * KiB, 1), (4112, 7)])
+@pytest.mark.parametrize("count", [1, 2, 32, 33, 168, 169, 504, 505, 504 + 1344, 504 + 1344 + 1, 3000])
+def test_bulk_batches(mf, pool, count, unit, top, stream):
+    import torch
+
+    if count * (top * unit + 32) > 90 * MiB:
+        pytest.skip("larger than the region")
+    rng = np.random.default_rng(count * 7 + unit)
+    so, sizes, span = _batch(rng, count, unit, top)
+    do = rng.permutation(count).astype(np.int64) * (top * unit + 32)
+    src, dst = _regions(pool, span + 64)
+    srcs, dsts = [int(pool.hbm() + o) for o in so], [int(pool.hbm() + 96 * MiB + o) for o in do]
+    szs = [int(z) for z in sizes]
+    if stream:
+        assert pool.handle.copy_data_batch_on_stream(srcs, dsts, szs, mf.bm.BmCopyType.G2G, torch.cuda.current_stream().cuda_stream, 0) == 0
+        torch.cuda.synchronize()
+    else:
+        assert pool.handle.copy_data_batch(srcs, dsts, szs, count, mf.bm.BmCopyType.G2G, 0) == 0, mf.get_last_err_msg()
+    s, d = src.cpu().numpy(), dst.cpu().numpy()
+    want = np.full_like(d, 0xA5)
+    for a, b, z in zip(so, do, sizes):
+        want[b:b + z] = s[a:a + z]
+    assert (d == want).all()
+
+
+@pytest.mark.parametrize("count", [3, 168, 169, 1000])
+@pytest.mark.parametrize("shift", [1, 2, 8])
+def test_batches_off_the_16_byte_grid(mf, pool, count, shift):
+    rng = np.random.default_rng(count + shift)
+    so, sizes, span = _batch(rng, count, 100, 50, aligned=shift)
+    do = rng.permutation(count).astype(np.int64) * (50 * 100 + 32)
+    src, dst = _regions(pool, span + 64)
+    assert pool.handle.copy_data_batch([int(pool.hbm() + o) for o in so], [int(pool.hbm() + 96 * MiB + o) for o in do], [int(z) for z in sizes], count,
+                                       mf.bm.BmCopyType.G2G, 0) == 0, mf.get_last_err_msg()
+    s, d = src.cpu().numpy(), dst.cpu().numpy()
+    want = np.full_like(d, 0xA5)
+    for a, b, z in zip(so, do, sizes):
+        want[b:b + z] = s[a:a + z]
+    assert (d == want).all()
+
+
+@pytest.mark.parametrize("kind", ["small", "shifted", "bulk", "batch"])
+def test_enqueued_copies_keep_stream_order(mf, pool, kind):
+    """Forty hops, each reading what the one before wrote: a copy that overlaps its predecessor's end must not read too early."""
+    import torch
+
+    from memfabric_hybrid_b200.utils.tensors import device_tensor_from_gva
+
+    n = {"small": 3000, "shifted": 3 * MiB + 1, "bulk": 25 * MiB, "batch": 8 * MiB}[kind]
+    step = 2 if kind == "shifted" else 0
+    base, hop, G2G = pool.hbm(), 40 * MiB, mf.bm.BmCopyType.G2G
+    first = device_tensor_from_gva(base, n)
+    first.random_(0, 256, generator=torch.Generator(device="cuda").manual_seed(4))
+    want = first.clone()
+    st = torch.cuda.current_stream().cuda_stream
+    at = base
+    for i in range(40):
+        to = base + (hop if i % 2 == 0 else 0) + step * (i + 1)
+        if kind == "batch":
+            blk = n // 2048
+            order = np.random.default_rng(i).permutation(2048)
+            rc = pool.handle.copy_data_batch_on_stream([int(at + o * blk) for o in order], [int(to + o * blk) for o in order], [blk] * 2048, G2G, st, 0)
+        else:
+            rc = pool.handle.copy_data_on_stream(at, to, n, G2G, st, 0)
+        assert rc == 0, mf.get_last_err_msg()
+        at = to
+    torch.cuda.synchronize()
+    assert torch.equal(device_tensor_from_gva(at, n), want)
