@@ -105,15 +105,26 @@ public:
         uint64_t total = ReservedBytes();
         uint64_t want = VaManager::Instance().FindFreeWindow(total, hint);
         MF_CHECK_RET(want != 0, BM_MALLOC_FAILED, "device segment: GVA window exhausted");
+        // The driver prefers a hole that freed memory left in one of its own address blocks to the hint. What it offers instead
+        // is kept until the end, so that the next try finds the hole taken and comes to the hint.
+        std::vector<CUdeviceptr> offered;
         CUdeviceptr got = 0;
-        CUresult r = d->MemAddressReserve(&got, total, GRANULE, (CUdeviceptr)want, 0);
+        CUresult r = CUDA_SUCCESS;
+        for (int tries = 0; tries < 16; tries++) {
+            r = d->MemAddressReserve(&got, total, GRANULE, (CUdeviceptr)want, 0);
+            if (r != CUDA_SUCCESS || (uint64_t)got == want) {
+                break;
+            }
+            offered.push_back(got);
+        }
+        for (CUdeviceptr o : offered) {
+            d->MemAddressFree(o, total);
+        }
         if (r != CUDA_SUCCESS) {
             MF_WARN("device segment: cuMemAddressReserve(0x" << std::hex << want << std::dec << ") failed: " << cu::ErrStr(r));
             return BM_ERROR;
         }
         if ((uint64_t)got != want) {
-            // The hint was not honoured: this address cannot be shared, give it back.
-            d->MemAddressFree(got, total);
             MF_WARN("device segment: asked for 0x" << std::hex << want << " but the driver offered 0x" << (uint64_t)got << std::dec);
             return BM_ERROR;
         }
