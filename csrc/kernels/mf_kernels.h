@@ -175,14 +175,17 @@ typedef struct {
     int cap;                  // rows of the receive buffer (and of y)
     int retRows;              // rows of every rank's landing zone (max tokens * K)
     int reserved;
+    const int *sendSlot;      // optional, both: [T, K] as filled by dispatch and [T, K] weights as given to it. With them a rank gathers the
+    const float *topkW;       // outputs of its own experts directly. The same choice on every rank.
 } mf_moe_combine_args_t;
 
 // H: hidden (multiple of 128), K: experts per token, E: experts in total (multiple of the rank count). Both kernels are
 // cooperative launches; epoch must grow by one per call and channel on every rank alike (epoch 0: taken from args.epochState).
 int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int E, uint32_t channel,
                       uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream);
+// direct: the argument blocks carry sendSlot and topkW.
 int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int EL, uint32_t channel,
-                     uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream);
+                     uint64_t epoch, uint64_t timeoutNs, int ctas, int direct, mf_stream_t stream);
 
 // ------------------------------------------------------------------------------------------------ weight reshard (K6)
 

@@ -42,6 +42,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxExperts = 1024;
+constexpr int kMaxTopk = 32;
 // A token routed to several experts of one owner crosses the link once and is replicated by the owner when the call moves at
 // least this many (token, expert) pairs per rank on average; below it the scan of the receive buffer that the replication
 // needs costs more than the link time it saves (measured on two GPUs, top-8 of 64 experts: 128 tokens per rank 45 us without
@@ -111,9 +112,12 @@ __device__ __forceinline__ int4 mf_ld_meta(const int4 *p)
     return make_int4((int)u.x, (int)u.y, (int)u.z, (int)u.w);
 }
 
-// Two CTAs per SM (71 KB of shared memory and at most 128 registers each): a warp works on one token at a time through chains
-// of dependent loads, shuffles and stores, so the kernel lives on the number of warps in flight, not on any one unit.
-__global__ void __launch_bounds__(kThreads, 2)
+// A CTA works on one token at a time: every thread quantises 16 consecutive elements (32 bytes in, 16 out, the eight lanes of a
+// 128-element block share the maximum) and stores them straight from registers to every row that gets them, while warp 0
+// finds the rows. One warp per token with a stage in shared memory took 28 dependent loads a token; with one CTA per token and
+// four per SM the small call is a few latencies long (128 tokens: 55 -> 15 us on one rank) and the large one is bound by its stores
+// (4096 tokens, top-8 of 32 experts on one rank, 300 MB: 158 -> 75 us).
+__global__ void __launch_bounds__(kThreads, 4)
 mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, int K, int E, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
     cg::grid_group grid = cg::this_grid();
@@ -131,10 +135,13 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
     int *sendBase = reinterpret_cast<int *>(smem);                              // [E]
     int *totals = sendBase + kMaxExperts;                                       // [E] pairs per expert over all sources
     int *starts = totals + kMaxExperts;                                         // [E] first row of the expert on its owner
-    unsigned char *stage = smem + (size_t)3 * kMaxExperts * sizeof(int);        // per warp: H bytes fp8 + nblk floats
-    const size_t stagePerWarp = (size_t)H + (size_t)nblk * 4;
+    __shared__ int2 target[2][kMaxTopk];  // per parity of the token: row on the owner (-1: none) and owner of each pair
     __shared__ int abortFlag;
     __shared__ int grandTotal;
+    __shared__ int overflow;  // rows did not fit an owner's buffer: reported when no CTA reads the status any more to see whether to go on
+    if (threadIdx.x == 0) {
+        overflow = 0;
+    }
     if (mf_check_bounds_enabled(m) &&
         !(mf_shm_in_own_window(m, a.cnt, (uint64_t)(a.arrive != nullptr ? 2 : 1) * R * E * 4) &&
           (a.arrive == nullptr || mf_shm_in_own_window(m, a.arrive, (uint64_t)(a.cap / 128) * 4)) && mf_shm_in_own_window(m, a.recvX, (uint64_t)a.cap * H) &&
@@ -155,15 +162,29 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
         }
     }
     const int pairs = a.T * K;
-    for (int i = blockIdx.x * kThreads + threadIdx.x; i < pairs; i += gridDim.x * kThreads) {
-        const int e = a.topkIdx[i];
-        if (e >= 0 && e < E) {
-            atomicAdd(&a.localCnt[e], 1);
+    if (blockIdx.x * kThreads < pairs) {
+        for (int e = threadIdx.x; e < E; e += kThreads) {
+            totals[e] = 0;
+        }
+        __syncthreads();
+        for (int i = blockIdx.x * kThreads + threadIdx.x; i < pairs; i += gridDim.x * kThreads) {
+            const int e = a.topkIdx[i];
+            if (e >= 0 && e < E) {
+                atomicAdd(&totals[e], 1);
+            }
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < E; e += kThreads) {
+            if (totals[e] != 0) {
+                atomicAdd(&a.localCnt[e], totals[e]);
+            }
         }
     }
     __threadfence();
     grid.sync();
-    if (blockIdx.x == 0) {
+    if (R == 1) {
+        myCnt = a.localCnt;  // one rank: its own histogram is the count matrix, there is nobody to publish it to or wait for
+    } else if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < E * R; i += kThreads) {
             const int r = i / E, e = i % E;
             int *peerCnt = mf_shm_peer(m, const_cast<int *>(myCnt), (uint32_t)r);
@@ -175,7 +196,9 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
             FailD(a.status, rc);
         }
     }
-    grid.sync();
+    if (R > 1) {
+        grid.sync();
+    }
     const bool dead = ReadAbort(a.status, &abortFlag) != 0;
     bool dedup = false;
 
@@ -219,7 +242,7 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
             }
         }
         __syncthreads();
-        dedup = !arrival && (long long)grandTotal >= (long long)R * (a.dedupMinPairs > 0 ? a.dedupMinPairs : kDedupMinPairsPerRank);
+        dedup = !arrival && R > 1 && (long long)grandTotal >= (long long)R * (a.dedupMinPairs > 0 ? a.dedupMinPairs : kDedupMinPairsPerRank);
         if (blockIdx.x == 0) {
             // What the GEMM and combine consume never points past the receive buffer: an expert that starts beyond the
             // capacity is published empty, one that straddles it is cut. The senders skip the same rows.
@@ -233,142 +256,147 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
                 const int off = starts[last] + ((totals[last] + 127) & ~127);
                 a.expertOffset[EL] = min(off, a.cap);
                 if (off > a.cap) {
-                    FailD(a.status, MF_DEV_ERR_BOUNDS);
+                    overflow = 1;
                 }
             }
         }
         __syncthreads();
 
         // ---- (c) quantise each token once, store it to the owners of its experts
-        unsigned char *myStage = stage + (size_t)warp * stagePerWarp;
-        uint32_t *myScale = reinterpret_cast<uint32_t *>(myStage + H);
-        const int warpsTotal = gridDim.x * kWarps;
-        for (int t = blockIdx.x * kWarps + warp; t < a.T; t += warpsTotal) {
-            const __nv_bfloat16 *row = reinterpret_cast<const __nv_bfloat16 *>(a.x) + (size_t)t * H;
-            for (int b0 = 0; b0 < nblk; b0 += 2) {
-                // Lanes 0-15 own block b0, lanes 16-31 block b0+1; with an odd block count the upper half idles through the
-                // same instructions (no divergent shuffles).
-                const int blk = b0 + (lane >> 4);
-                const bool active = blk < nblk;
-                const int off = (active ? blk : b0) * 128 + (lane & 15) * 8;
-                uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-                if (active) {
-                    raw = *reinterpret_cast<const uint4 *>(row + off);
-                }
-                const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw);
-                float f[8];
-                float amax = 0.f;
+        const int pieces = H / 16;
+        for (int t = blockIdx.x, turn = 0; t < a.T; t += gridDim.x, turn ^= 1) {
+            const unsigned char *row = reinterpret_cast<const unsigned char *>(a.x) + (size_t)t * H * 2;
+            int2 *to = target[turn];
+            uint4 raw[2][2];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float2 v = __bfloat1622float2(h[i]);
-                    f[2 * i] = v.x;
-                    f[2 * i + 1] = v.y;
-                    amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
-                }
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) {
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                }
-                // Scale = smallest power of two >= amax / 448, as a biased exponent byte; multiplying by its reciprocal is exact.
-                const uint32_t eb = Ue8m0Ceil(amax * (1.f / 448.f));
-                const float inv = __uint_as_float((254u - eb) << 23);
-                uint2 packed;
-                unsigned short *ps = reinterpret_cast<unsigned short *>(&packed);
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    ps[i] = __nv_cvt_float2_to_fp8x2(make_float2(f[2 * i] * inv, f[2 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-                }
-                if (active) {
-                    *reinterpret_cast<uint2 *>(myStage + off) = packed;
-                    if ((lane & 15) == 0) {
-                        myScale[blk] = eb * 0x01010101u;  // the same exponent for the four 32-element steps of the block
-                    }
+            for (int i = 0; i < 2; i++) {
+                const int p = threadIdx.x + i * kThreads;
+                if (p < pieces) {
+                    raw[i][0] = *reinterpret_cast<const uint4 *>(row + (size_t)p * 32);
+                    raw[i][1] = *reinterpret_cast<const uint4 *>(row + (size_t)p * 32 + 16);
                 }
             }
-            __syncwarp();
-            // Lane k owns pair (t, k): its row on the owner, and whether it leads the pairs of this token on that owner.
-            int myE = -1, mySlot = -1, myOwner = -1;
-            float myW = 0.f;
-            if (lane < K) {
-                myE = a.topkIdx[t * K + lane];
-                myW = a.topkW[t * K + lane];
-                if (myE >= 0 && myE < E) {
-                    mySlot = sendBase[myE] + atomicAdd(&a.cursor[myE], 1);
-                    myOwner = myE / EL;
-                    if (mySlot >= a.cap) {
-                        if (a.status != nullptr) {
-                            atomicCAS(a.status, 0, MF_DEV_ERR_BOUNDS);
+            int mySlot = -1, myOwner = -1;
+            if (warp == 0) {
+                // Lane k owns pair (t, k): its row on the owner, and whether it leads the pairs of this token on that owner.
+                float myW = 0.f;
+                if (lane < K) {
+                    const int myE = a.topkIdx[t * K + lane];
+                    myW = a.topkW[t * K + lane];
+                    if (myE >= 0 && myE < E) {
+                        mySlot = sendBase[myE] + atomicAdd(&a.cursor[myE], 1);
+                        myOwner = myE / EL;
+                        if (mySlot >= a.cap) {
+                            overflow = 1;
+                            mySlot = -1;  // the owner's buffer is full: this pair is dropped and the call reports the overflow
                         }
-                        mySlot = -1;  // the owner's buffer is full: this pair is dropped and the call reports the overflow
+                    }
+                    if (a.sendSlot != nullptr) {
+                        a.sendSlot[t * K + lane] = mySlot;
                     }
                 }
-                if (a.sendSlot != nullptr) {
-                    a.sendSlot[t * K + lane] = mySlot;
-                }
-            }
-            // Pairs of one (token, owner) form groups of up to 1 + MF_MOE_MAX_SIBLINGS in k order; the first of a group leads it.
-            int before = 0, nsib = 0;
-            int2 sib[MF_MOE_MAX_SIBLINGS];
-            for (int j = 0; j < K; j++) {
-                const int oj = __shfl_sync(0xffffffffu, myOwner, j);
-                const int sj = __shfl_sync(0xffffffffu, mySlot, j);
-                const float wj = __shfl_sync(0xffffffffu, myW, j);
-                if (mySlot >= 0 && sj >= 0 && oj == myOwner && j != lane) {
-                    if (j < lane) {
+                // Pairs of one (token, owner) form groups of up to 1 + MF_MOE_MAX_SIBLINGS in k order; the first of a group leads it.
+                int before = 0, nsib = 0;
+                const uint32_t leadDst = (uint32_t)(mySlot >= 0 ? myOwner : me);
+                for (int j = 0; j < K; j++) {
+                    const int oj = __shfl_sync(0xffffffffu, myOwner, j);
+                    const int sj = __shfl_sync(0xffffffffu, mySlot, j);
+                    if (mySlot >= 0 && sj >= 0 && oj == myOwner && j < lane) {
                         before++;
-                    } else if (nsib < MF_MOE_MAX_SIBLINGS) {
-                        sib[nsib++] = make_int2(sj, __float_as_int(wj));
                     }
                 }
+                const bool leader = mySlot >= 0 && before % (MF_MOE_MAX_SIBLINGS + 1) == 0;
+                int2 *sd = mf_shm_peer(m, a.recvSib, leadDst) + (size_t)(mySlot >= 0 ? mySlot : 0) * MF_MOE_MAX_SIBLINGS;
+                for (int j = 0; j < K; j++) {
+                    const int oj = __shfl_sync(0xffffffffu, myOwner, j);
+                    const int sj = __shfl_sync(0xffffffffu, mySlot, j);
+                    const float wj = __shfl_sync(0xffffffffu, myW, j);
+                    if (leader && sj >= 0 && oj == myOwner && j > lane && nsib < MF_MOE_MAX_SIBLINGS) {
+                        sd[nsib++] = make_int2(sj, __float_as_int(wj));
+                    }
+                }
+                // In a large call only the leader of a (token, owner) group carries the payload over the link; the owner copies it
+                // into the followers' rows after everything has landed (phase (e)): a token routed to several experts of one
+                // other rank crosses NVLink once. Rows of this rank itself are written here one and all.
+                if (lane < K) {
+                    to[lane] = make_int2(dedup && myOwner != me && !leader ? -1 : mySlot, myOwner);
+                }
+                if (mySlot >= 0) {
+                    // Followers of a (token, owner) group are marked; the leader carries the number of siblings and their rows.
+                    const int kField = lane | (leader ? (nsib << 8) : MF_MOE_META_FOLLOWER);
+                    mf_shm_peer(m, a.recvMeta, (uint32_t)myOwner)[mySlot] = make_int4(me, t, kField, __float_as_int(myW));
+                }
             }
-            const bool leader = mySlot >= 0 && before % (MF_MOE_MAX_SIBLINGS + 1) == 0;
-            // In a large call only the leader of a (token, owner) group carries the payload over the link; the owner copies it
-            // into the followers' rows after everything has landed (phase (e)): a token routed to several experts of one rank
-            // crosses NVLink once.
-            const uint32_t leadMask = __ballot_sync(0xffffffffu, leader);
-            for (int k = 0; k < K; k++) {
-                const int slot = __shfl_sync(0xffffffffu, mySlot, k);
-                if (slot < 0 || (dedup && (leadMask >> k & 1u) == 0)) {
-                    continue;
-                }
-                const uint32_t d = (uint32_t)__shfl_sync(0xffffffffu, myOwner, k);
-                unsigned char *dx = reinterpret_cast<unsigned char *>(mf_shm_peer(m, a.recvX, d)) + (size_t)slot * H;
-                uint32_t *ds = mf_shm_peer(m, a.recvSf, d) + (size_t)slot * nblk;
-                for (int v = lane; v < H / 16; v += 32) {
-                    mf_st16(dx + (size_t)v * 16, *reinterpret_cast<const uint4 *>(myStage + (size_t)v * 16));
-                }
-                for (int v = lane; v < nblk; v += 32) {
-                    ds[v] = myScale[v];
-                }
-            }
-            if (mySlot >= 0) {
-                const uint32_t d = (uint32_t)myOwner;
-                // Followers of a (token, owner) group are marked; the leader carries the number of siblings and their rows.
-                const int kField = lane | (leader ? (nsib << 8) : MF_MOE_META_FOLLOWER);
-                mf_shm_peer(m, a.recvMeta, d)[mySlot] = make_int4(me, t, kField, __float_as_int(myW));
-                if (leader) {
-                    int2 *sd = mf_shm_peer(m, a.recvSib, d) + (size_t)mySlot * MF_MOE_MAX_SIBLINGS;
-                    for (int i = 0; i < nsib; i++) {
-                        sd[i] = sib[i];
+            __syncthreads();  // the targets are known; those of the token after next go into the same place only after the next round
+            for (int p0 = 0; p0 < pieces; p0 += 2 * kThreads) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int p = p0 + threadIdx.x + i * kThreads;
+                    const bool active = p < pieces;
+                    if (p0 > 0 && active) {
+                        raw[i][0] = *reinterpret_cast<const uint4 *>(row + (size_t)p * 32);
+                        raw[i][1] = *reinterpret_cast<const uint4 *>(row + (size_t)p * 32 + 16);
+                    }
+                    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(raw[i]);
+                    __nv_bfloat162 m2 = __float2bfloat162_rn(0.f);
+                    if (active) {
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                            m2 = __hmax2(m2, __habs2(h[q]));
+                        }
+                    }
+                    const float2 ends = __bfloat1622float2(m2);
+                    float amax = fmaxf(ends.x, ends.y);
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) {
+                        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                    }
+                    if (!active) {
+                        continue;
+                    }
+                    // Scale = smallest power of two >= amax / 448, as a biased exponent byte; multiplying by its reciprocal is exact.
+                    const uint32_t eb = Ue8m0Ceil(amax * (1.f / 448.f));
+                    const float inv = __uint_as_float((254u - eb) << 23);
+                    uint4 packed;
+                    unsigned short *ps = reinterpret_cast<unsigned short *>(&packed);
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const float2 f = __bfloat1622float2(h[q]);
+                        ps[q] = __nv_cvt_float2_to_fp8x2(make_float2(f.x * inv, f.y * inv), __NV_SATFINITE, __NV_E4M3);
+                    }
+                    for (int k = 0; k < K; k++) {
+                        const int2 d = to[k];
+                        if (d.x < 0) {
+                            continue;
+                        }
+                        mf_st16(reinterpret_cast<unsigned char *>(mf_shm_peer(m, a.recvX, (uint32_t)d.y)) + (size_t)d.x * H + (size_t)p * 16, packed);
+                        if ((lane & 7) == 0) {
+                            // the same exponent for the four 32-element steps of the block
+                            mf_shm_peer(m, a.recvSf, (uint32_t)d.y)[(size_t)d.x * nblk + (p >> 3)] = eb * 0x01010101u;
+                        }
                     }
                 }
             }
             if (arrival) {
-                // Everything this warp stored for the token is visible system-wide before any of its rows is counted.
+                // Everything this CTA stored for the token is visible system-wide before any of its rows is counted.
                 __threadfence_system();
-                __syncwarp();
+                __syncthreads();
                 if (mySlot >= 0) {
                     atomicAdd_system(mf_shm_peer(m, a.arrive, (uint32_t)myOwner) + (mySlot >> 7), 1);
                 }
             }
-            __syncwarp();
         }
     }
     // ---- (d) everything I sent is visible before my arrival is; when all have arrived, all receive buffers are complete
-    __threadfence_system();
+    if (R > 1) {
+        __threadfence_system();
+    }
     grid.sync();
+    if (overflow != 0) {
+        FailD(a.status, MF_DEV_ERR_BOUNDS);
+    }
     if (blockIdx.x == 0) {
-        if (!dead && !arrival) {
+        if (!dead && !arrival && R > 1) {
             int rc = mf_barrier_cta(m, channel, 0, 2 * epoch, timeoutNs);
             if (rc != MF_DEV_OK) {
                 FailD(a.status, rc);
@@ -384,7 +412,7 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
         FinishEpochD(a, epochArg, epoch);
         return;  // every row came with its payload (in arrival mode the consumers wait on the tile counters)
     }
-    // ---- (e) every leader row that arrived here is copied into the rows of its followers (local memory only)
+    // ---- (e) every leader row that arrived here from another rank is copied into the rows of its followers (local memory only)
     grid.sync();
     if (dead || ReadAbort(a.status, &abortFlag) != 0) {
         FinishEpochD(a, epochArg, epoch);
@@ -404,7 +432,7 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
             }
             const int4 meta = mf_ld_meta(a.recvMeta + r);
             const int nsib = (meta.z >> 8) & 0xff;
-            if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || nsib == 0 || nsib > MF_MOE_MAX_SIBLINGS) {
+            if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || meta.x == me || nsib == 0 || nsib > MF_MOE_MAX_SIBLINGS) {
                 continue;
             }
             const int2 *sd = a.recvSib + (size_t)r * MF_MOE_MAX_SIBLINGS;
@@ -445,10 +473,88 @@ mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, i
     FinishEpochD(a, epochArg, epoch);
 }
 
+// Eight fp32 values as bf16, and two such vectors added to fp32 sums.
+__device__ __forceinline__ uint4 PackRow(const float (&v)[8])
+{
+    uint4 pk;
+    __nv_bfloat162 *hp = reinterpret_cast<__nv_bfloat162 *>(&pk);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        hp[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+    }
+    return pk;
+}
+
+__device__ __forceinline__ void AddRow(float (&acc)[2][8], const uint4 (&raw)[2])
+{
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[c]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float2 f = __bfloat1622float2(h[q]);
+            acc[c][2 * q] += f.x;
+            acc[c][2 * q + 1] += f.y;
+        }
+    }
+}
+
+// Weighted sum of up to `left` rows of y, in ascending lane order over the lanes in `group`, each of which holds a row and its
+// weight. Four rows of two vectors are in flight per lane (the rows of a group lie far apart: latency, not bandwidth, would
+// pace a one-at-a-time loop).
+__device__ __forceinline__ void GatherGroup(float (&part)[2][8], uint32_t group, int left, int myRow, float myW, const void *y, size_t rowBytes, int rows,
+                                            int v0, int vecs)
+{
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        part[0][q] = part[1][q] = 0.f;
+    }
+    while (group != 0 && left > 0) {
+        uint4 raw[4][2];
+        float w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const bool any = group != 0 && left > 0;
+            const int j = any ? __ffs(group) - 1 : 0;
+            const int row = __shfl_sync(0xffffffffu, myRow, j);
+            w[i] = __shfl_sync(0xffffffffu, myW, j);
+            group &= group - 1;
+            left--;
+            raw[i][0] = raw[i][1] = make_uint4(0u, 0u, 0u, 0u);
+            if (any && row >= 0 && row < rows) {
+                const char *rowp = reinterpret_cast<const char *>(y) + (size_t)row * rowBytes + (size_t)v0 * 16;
+                if (v0 < vecs) {
+                    raw[i][0] = mf_ld16(rowp);
+                }
+                if (v0 + 32 < vecs) {
+                    raw[i][1] = mf_ld16(rowp + 512);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[i][c]);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float2 f = __bfloat1622float2(h[q]);
+                    part[c][2 * q] = fmaf(w[i], f.x, part[c][2 * q]);
+                    part[c][2 * q + 1] = fmaf(w[i], f.y, part[c][2 * q + 1]);
+                }
+            }
+        }
+    }
+}
+
+// Bound by the traffic of the expert outputs. A rank's own pairs are gathered by token from where dispatch put them: no landing
+// zone is written and read for them and no receive buffer is scanned for leaders (7 of 8 of its rows are followers when one rank
+// owns all experts). One rank, top-8, hidden 7168: 128 tokens 63 -> 8 us, 4096 tokens (530 MB) 247 -> 90 us.
+// ALONE: one rank with sendSlot and topkW and at most eight pairs a token; nothing waits on anything, so it is an ordinary launch.
+template <bool ALONE>
 __global__ void __launch_bounds__(kThreads, 3)
 mf_moe_combine_kernel(const mf_moe_combine_args_t *__restrict__ args, int H, int K, int EL, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
-    cg::grid_group grid = cg::this_grid();
     const mf_moe_combine_args_t a = args[blockIdx.y];
     const uint64_t epoch = ResolveEpochD(a, epochArg);
     if (epoch == 0) {
@@ -466,26 +572,29 @@ mf_moe_combine_kernel(const mf_moe_combine_args_t *__restrict__ args, int H, int
         FinishEpochD(a, epochArg, epoch);
         return;
     }
-    for (int i = threadIdx.x; i <= EL; i += kThreads) {
+    for (int i = threadIdx.x; i <= EL && !ALONE; i += kThreads) {
         offs[i] = a.expertOffset[i];
         if (i < EL) {
             cnts[i] = a.expertCount[i];
         }
     }
     __syncthreads();
-    const int rows = min(offs[EL], a.cap);
+    const int rows = ALONE ? 0 : min(offs[EL], a.cap);
     const int vecs = H / 8;
     const uint32_t R = m->rankCount;
     // A call whose dispatch failed (overflow, timeout) moves no data; it still walks through the barriers so that the
     // peers' waits complete.
     const bool dead = ReadAbort(a.status, &abortFlag) != 0;
+    // The rows that this rank computed for its own tokens need no landing zone: dispatch left their places in sendSlot, and the
+    // source gathers them itself below.
+    const bool direct = ALONE || (a.sendSlot != nullptr && a.topkW != nullptr);
 
     // ---- push: one row per (token, owner): the leader's output plus its siblings', weighted, to the source rank's
     //      landing zone [token][k of the leader][:]
-    // Work unit = (row, chunk of 128 vectors): a leader with many siblings is spread over several warps.
-    const int chunks = (vecs + 127) / 128;
-    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)rows * chunks && !dead; u += warpsTotal) {
-        const int r = (int)(u / chunks), ch = (int)(u % chunks);
+    // Work unit = (row, chunk of 64 vectors): a leader with many siblings is spread over several warps.
+    const int units = (vecs + 63) / 64;
+    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)rows * units && !dead && !ALONE; u += warpsTotal) {
+        const int r = (int)(u / units), v0 = (int)(u % units) * 64 + lane;
         int el = 0;
         while (el + 1 < EL && offs[el + 1] <= r) {
             el++;
@@ -496,147 +605,103 @@ mf_moe_combine_kernel(const mf_moe_combine_args_t *__restrict__ args, int H, int
         const int4 meta = a.recvMeta[r];
         const uint32_t src = (uint32_t)meta.x;
         const int k = meta.z & 0xff, nsib = (meta.z >> 8) & 0xff;
-        if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || src >= R || meta.y < 0 || k >= K || (long long)meta.y * K + k >= a.retRows ||
+        if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || src >= R || (direct && src == m->rankId) || meta.y < 0 || k >= K || (long long)meta.y * K + k >= a.retRows ||
             nsib > MF_MOE_MAX_SIBLINGS) {
             continue;
         }
-        const int2 *sd = a.recvSib + (size_t)r * MF_MOE_MAX_SIBLINGS;
-        int rowOf[MF_MOE_MAX_SIBLINGS + 1];
-        float wOf[MF_MOE_MAX_SIBLINGS + 1];
-        rowOf[0] = r;
-        wOf[0] = __int_as_float(meta.w);
-        int n = 1;
-        for (int i = 0; i < nsib; i++) {
-            const int2 e = sd[i];
-            if (e.x >= 0 && e.x < rows) {
-                rowOf[n] = e.x;
-                wOf[n] = __int_as_float(e.y);
-                n++;
-            }
+        // Lane 0 holds the leader's row, lanes 1..nsib those of its siblings.
+        int2 mine = make_int2(r, meta.w);
+        if (lane >= 1 && lane <= nsib) {
+            mine = a.recvSib[(size_t)r * MF_MOE_MAX_SIBLINGS + lane - 1];
         }
+        float part[2][8];
+        GatherGroup(part, (2u << nsib) - 1, MF_MOE_MAX_SIBLINGS + 1, mine.x, __int_as_float(mine.y), a.y, (size_t)H * 2, rows, v0, vecs);
         char *dst = reinterpret_cast<char *>(mf_shm_peer(m, a.retY, src)) + ((size_t)meta.y * K + k) * H * 2;
-        // The lane's four vectors of the chunk are loaded together for every addend, so that four 16-byte loads per lane are
-        // in flight (the rows of a group lie far apart: latency, not bandwidth, would pace a one-at-a-time loop).
-        const int vEnd = min(vecs, (ch + 1) * 128);
-        const int v0 = ch * 128 + lane;
-        float acc[4][8];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                acc[j][q] = 0.f;
-            }
+        if (v0 < vecs) {
+            mf_st16(dst + (size_t)v0 * 16, PackRow(part[0]));
         }
-        for (int i = 0; i < n; i++) {
-            const char *rowp = reinterpret_cast<const char *>(a.y) + (size_t)rowOf[i] * H * 2;
-            uint4 raw[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                raw[j] = v0 + 32 * j < vEnd ? mf_ld16(rowp + (size_t)(v0 + 32 * j) * 16) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            const float w = wOf[i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[j]);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float2 f = __bfloat1622float2(h[q]);
-                    acc[j][2 * q] = fmaf(w, f.x, acc[j][2 * q]);
-                    acc[j][2 * q + 1] = fmaf(w, f.y, acc[j][2 * q + 1]);
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (v0 + 32 * j < vEnd) {
-                uint4 pk;
-                __nv_bfloat162 *hp = reinterpret_cast<__nv_bfloat162 *>(&pk);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    hp[q] = __floats2bfloat162_rn(acc[j][2 * q], acc[j][2 * q + 1]);
-                }
-                mf_st16(dst + (size_t)(v0 + 32 * j) * 16, pk);
-            }
+        if (v0 + 32 < vecs) {
+            mf_st16(dst + (size_t)(v0 + 32) * 16, PackRow(part[1]));
         }
     }
-    __threadfence_system();
-    grid.sync();
-    if (blockIdx.x == 0) {
-        int rc = mf_barrier_cta(m, channel, 0, epoch, timeoutNs);
-        if (rc != MF_DEV_OK) {
-            FailD(a.status, rc);
+    if (!ALONE) {
+        __threadfence_system();
+        cg::grid_group grid = cg::this_grid();
+        grid.sync();
+        if (blockIdx.x == 0) {
+            int rc = mf_barrier_cta(m, channel, 0, epoch, timeoutNs);
+            if (rc != MF_DEV_OK) {
+                FailD(a.status, rc);
+            }
         }
+        grid.sync();
     }
-    grid.sync();
     if (ReadAbort(a.status, &abortFlag) != 0) {
         FinishEpochD(a, epochArg, epoch);
         return;
     }
-    // ---- add the owners' partial sums (fp32, fixed order): pair k carries one iff no earlier pair of the token has the same owner
-    const int ELg = EL;
-    for (int t = blockIdx.x * kWarps + warp; t < a.T; t += warpsTotal) {
-        const char *base = reinterpret_cast<const char *>(a.retY) + (size_t)t * K * H * 2;
-        char *o = reinterpret_cast<char *>(a.out) + (size_t)t * H * 2;
-        uint32_t leaders = 0;
-        for (int k = 0; k < K; k++) {
-            const int e = a.topkIdx[t * K + k];
-            if (e < 0 || e >= ELg * (int)R) {
-                continue;
-            }
-            int before = 0;
-            for (int j = 0; j < k; j++) {
-                const int ej = a.topkIdx[t * K + j];
-                if (ej >= 0 && ej < ELg * (int)R && ej / ELg == e / ELg) {
-                    before++;
+    // ---- add the owners' partial sums (fp32, fixed order): pair k carries one iff no earlier pair of its group (the pairs of the
+    //      token on one owner, eight at most, in k order) does. Work unit = (token, chunk of 64 vectors).
+    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)a.T * units; u += warpsTotal) {
+        const int t = (int)(u / units), v0 = (int)(u % units) * 64 + lane, v1 = v0 + 32;
+        const bool has0 = v0 < vecs, has1 = v1 < vecs;
+        // Lane k holds pair k: where its partial sum or its expert's output stands and which lanes belong to its group.
+        int myOwner = -1, mySlot = -1;
+        float myW = 0.f;
+        if (lane < K) {
+            const int e = a.topkIdx[t * K + lane];
+            if (e >= 0 && e < EL * (int)R) {
+                myOwner = e / EL;
+                if (direct && myOwner == (int)m->rankId) {
+                    mySlot = a.sendSlot[t * K + lane];
+                    myW = a.topkW[t * K + lane];
                 }
-            }
-            if (before % (MF_MOE_MAX_SIBLINGS + 1) == 0) {
-                leaders |= 1u << k;
             }
         }
-        // Four vectors per lane and trip, loaded together for every partial sum (same reason as above).
-        for (int vb = lane; vb < vecs; vb += 128) {
-            float acc[4][8];
+        uint32_t same = 0;
+        for (int j = 0; j < K; j++) {
+            same |= __shfl_sync(0xffffffffu, myOwner, j) == myOwner ? 1u << j : 0u;
+        }
+        const int before = __popc(same & ((1u << lane) - 1));
+        uint32_t leaders = __ballot_sync(0xffffffffu, myOwner >= 0 && before % (MF_MOE_MAX_SIBLINGS + 1) == 0);
+        char *o = reinterpret_cast<char *>(a.out) + ((size_t)t * H + (size_t)v0 * 8) * 2;
+        float acc[2][8];
+        if (ALONE) {  // one group holds everything
+            GatherGroup(acc, __ballot_sync(0xffffffffu, myOwner >= 0), MF_MOE_MAX_SIBLINGS + 1, mySlot, myW, a.y, (size_t)H * 2, a.cap, v0, vecs);
+            leaders = 0;
+        } else {
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    acc[j][q] = 0.f;
-                }
+            for (int q = 0; q < 8; q++) {
+                acc[0][q] = acc[1][q] = 0.f;
             }
-            for (int k = 0; k < K; k++) {
-                if ((leaders >> k & 1u) == 0) {
-                    continue;
+        }
+        for (; leaders != 0; leaders &= leaders - 1) {
+            const int k = __ffs(leaders) - 1;
+            const int owner = __shfl_sync(0xffffffffu, myOwner, k);
+            if (!direct || owner != (int)m->rankId) {
+                const char *rowp = reinterpret_cast<const char *>(a.retY) + ((size_t)t * K + k) * H * 2;
+                uint4 raw[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+                if (has0) {
+                    raw[0] = mf_ld16_coherent(rowp + (size_t)v0 * 16);
                 }
-                const char *rowp = base + (size_t)k * H * 2;
-                uint4 raw[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    raw[j] = vb + 32 * j < vecs ? mf_ld16_coherent(rowp + (size_t)(vb + 32 * j) * 16) : make_uint4(0u, 0u, 0u, 0u);
+                if (has1) {
+                    raw[1] = mf_ld16_coherent(rowp + (size_t)v1 * 16);
                 }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[j]);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        float2 f = __bfloat1622float2(h[i]);
-                        acc[j][2 * i] += f.x;
-                        acc[j][2 * i + 1] += f.y;
-                    }
-                }
+                AddRow(acc, raw);
+                continue;
             }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (vb + 32 * j < vecs) {
-                    uint4 pk;
-                    __nv_bfloat162 *hp = reinterpret_cast<__nv_bfloat162 *>(&pk);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        hp[i] = __floats2bfloat162_rn(acc[j][2 * i], acc[j][2 * i + 1]);
-                    }
-                    mf_st16(o + (size_t)(vb + 32 * j) * 16, pk);
-                }
-            }
+            // This group's outputs are here: weighted in k order, and rounded like a partial sum that travels.
+            float part[2][8];
+            const uint32_t group = __shfl_sync(0xffffffffu, same, k) & (0xffffffffu << k);
+            GatherGroup(part, group, MF_MOE_MAX_SIBLINGS + 1, mySlot, myW, a.y, (size_t)H * 2, a.cap, v0, vecs);
+            uint4 rounded[2] = {PackRow(part[0]), PackRow(part[1])};
+            AddRow(acc, rounded);
+        }
+        if (has0) {
+            mf_st16(o, PackRow(acc[0]));
+        }
+        if (has1) {
+            mf_st16(o + 512, PackRow(acc[1]));
         }
     }
     FinishEpochD(a, epochArg, epoch);
@@ -690,21 +755,13 @@ extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmu
                                  uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
 {
     if (argsDev == nullptr || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || H <= 0 || H % 128 != 0 || K < 1 ||
-        K > 32 || E < rankCount || E % rankCount != 0 || E > kMaxExperts || channel >= MF_SIGNAL_CHANNELS) {
+        K > kMaxTopk || E < rankCount || E % rankCount != 0 || E > kMaxExperts || channel >= MF_SIGNAL_CHANNELS) {
         return MF_K_INVALID;
     }
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
-    const size_t smem = (size_t)3 * kMaxExperts * sizeof(int) + (size_t)kWarps * ((size_t)H + (size_t)(H / 128) * 4);
-    static size_t attrSmem = 0;
-    if (smem > attrSmem) {
-        if (cudaFuncSetAttribute(mf_moe_dispatch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return MF_K_TOO_LARGE;
-        }
-        attrSmem = smem;
-    }
+    const size_t smem = (size_t)3 * kMaxExperts * sizeof(int);
     int cap = CoopCap((const void *)mf_moe_dispatch_kernel, smem);
     if (cap <= 0) {
         return MF_K_LAUNCH_FAILED;
@@ -727,7 +784,7 @@ extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmu
 }
 
 extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int EL, uint32_t channel,
-                                uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+                                uint64_t epoch, uint64_t timeoutNs, int ctas, int direct, mf_stream_t stream)
 {
     if (argsDev == nullptr || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || H <= 0 || H % 8 != 0 || K < 1 || K > 32 ||
         EL < 1 || EL > kMaxExperts || channel >= MF_SIGNAL_CHANNELS) {
@@ -736,7 +793,9 @@ extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmula
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
-    int cap = CoopCap((const void *)mf_moe_combine_kernel, 0);
+    const bool alone = direct != 0 && rankCount == 1 && K <= MF_MOE_MAX_SIBLINGS + 1;
+    const void *kernel = alone ? (const void *)mf_moe_combine_kernel<true> : (const void *)mf_moe_combine_kernel<false>;
+    int cap = CoopCap(kernel, 0);
     if (cap <= 0) {
         return MF_K_LAUNCH_FAILED;
     }
@@ -749,7 +808,8 @@ extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmula
     }
     void *kargs[] = {(void *)&argsDev, (void *)&H, (void *)&K, (void *)&EL, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
     dim3 g((unsigned)grid, (unsigned)nEmulatedRanks, 1), b(kThreads, 1, 1);
-    cudaError_t e = cudaLaunchCooperativeKernel((const void *)mf_moe_combine_kernel, g, b, kargs, 0, (cudaStream_t)stream);
+    cudaError_t e = alone ? cudaLaunchKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream)
+                          : cudaLaunchCooperativeKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return MF_K_LAUNCH_FAILED;

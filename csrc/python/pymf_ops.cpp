@@ -96,8 +96,11 @@ void BindOps(py::module_ &m)
             py::arg("recv_sib"), py::arg("local_cnt"), py::arg("cursor"), py::arg("expert_offset"), py::arg("expert_count"), py::arg("send_slot"),
             py::arg("status"), py::arg("T"), py::arg("cap"), py::arg("arrive") = 0, py::arg("dedup_min_pairs") = 0, py::arg("epoch_state") = 0);
     ops.def("pack_moe_combine_args", [](uint64_t meta, uint64_t y, uint64_t recvMeta, uint64_t recvSib, uint64_t expertOffset, uint64_t expertCount,
-                                        uint64_t retY, uint64_t topkIdx, uint64_t out, uint64_t status, int T, int cap, int retRows, uint64_t epochState) {
+                                        uint64_t retY, uint64_t topkIdx, uint64_t out, uint64_t status, int T, int cap, int retRows, uint64_t epochState,
+                                        uint64_t sendSlot, uint64_t topkW) {
         mf_moe_combine_args_t a{};
+        a.sendSlot = (const int *)sendSlot;
+        a.topkW = (const float *)topkW;
         a.epochState = (unsigned long long *)epochState;
         a.meta = (const void *)meta;
         a.y = (const void *)y;
@@ -114,7 +117,8 @@ void BindOps(py::module_ &m)
         a.retRows = retRows;
         return py::bytes((const char *)&a, sizeof(a));
     }, py::arg("meta"), py::arg("y"), py::arg("recv_meta"), py::arg("recv_sib"), py::arg("expert_offset"), py::arg("expert_count"), py::arg("ret_y"),
-            py::arg("topk_idx"), py::arg("out"), py::arg("status"), py::arg("T"), py::arg("cap"), py::arg("ret_rows"), py::arg("epoch_state") = 0);
+            py::arg("topk_idx"), py::arg("out"), py::arg("status"), py::arg("T"), py::arg("cap"), py::arg("ret_rows"), py::arg("epoch_state") = 0,
+            py::arg("send_slot") = 0, py::arg("topk_w") = 0);
     ops.def("moe_dispatch", [](uint64_t argsDev, int nEmulated, int rankCount, int H, int K, int E, uint32_t channel, uint64_t epoch, uint64_t timeoutNs,
                                int ctas, uint64_t stream) {
         return mf_k_moe_dispatch((const mf_moe_dispatch_args_t *)argsDev, nEmulated, rankCount, H, K, E, channel, epoch, timeoutNs, ctas,
@@ -122,11 +126,11 @@ void BindOps(py::module_ &m)
     }, py::arg("args_dev"), py::arg("n_emulated"), py::arg("rank_count"), py::arg("H"), py::arg("K"), py::arg("E"), py::arg("channel"), py::arg("epoch"),
             py::arg("timeout_ns") = 0, py::arg("ctas") = 0, py::arg("stream") = 0);
     ops.def("moe_combine", [](uint64_t argsDev, int nEmulated, int rankCount, int H, int K, int EL, uint32_t channel, uint64_t epoch, uint64_t timeoutNs,
-                              int ctas, uint64_t stream) {
-        return mf_k_moe_combine((const mf_moe_combine_args_t *)argsDev, nEmulated, rankCount, H, K, EL, channel, epoch, timeoutNs, ctas,
+                              int ctas, uint64_t stream, int direct) {
+        return mf_k_moe_combine((const mf_moe_combine_args_t *)argsDev, nEmulated, rankCount, H, K, EL, channel, epoch, timeoutNs, ctas, direct,
                                 (mf_stream_t)stream);
     }, py::arg("args_dev"), py::arg("n_emulated"), py::arg("rank_count"), py::arg("H"), py::arg("K"), py::arg("EL"), py::arg("channel"), py::arg("epoch"),
-            py::arg("timeout_ns") = 0, py::arg("ctas") = 0, py::arg("stream") = 0);
+            py::arg("timeout_ns") = 0, py::arg("ctas") = 0, py::arg("stream") = 0, py::arg("direct") = 0);
     ops.attr("RESHARD_DESC_BYTES") = (int)sizeof(mf_reshard_desc_t);
     ops.attr("RESHARD_ARGS_BYTES") = (int)sizeof(mf_reshard_args_t);
     ops.def("pack_reshard_desc", [](uint64_t srcFlatOff, uint64_t dstOff, uint64_t scaleOff, uint32_t colsFull, uint32_t r0, uint32_t c0, uint32_t nrows,

@@ -154,7 +154,7 @@ class FusedMoE(_MoEBase):
                                         self._epoch_d.data_ptr() if self.device_epochs else 0)
         c = _ops.pack_moe_combine_args(h.meta_ptr, st.y.data_ptr(), st.recv_m.data_ptr(), st.recv_sib.data_ptr(), st.expert_offset.data_ptr(),
                                        st.expert_count.data_ptr(), st.ret_y.data_ptr(), idx.data_ptr(), st.out.data_ptr(), st.status.data_ptr(), T,
-                                       st.cap, st.max_rows_ret, self._epoch_c.data_ptr() if self.device_epochs else 0)
+                                       st.cap, st.max_rows_ret, self._epoch_c.data_ptr() if self.device_epochs else 0, st.send_slot.data_ptr(), w.data_ptr())
         self._dargs.copy_(torch.frombuffer(bytearray(d), dtype=torch.uint8))
         self._cargs.copy_(torch.frombuffer(bytearray(c), dtype=torch.uint8))
         self._key = key
@@ -165,8 +165,7 @@ class FusedMoE(_MoEBase):
         T = x.shape[0]
         self._pack(x, idx, w, T)
         s = stream or torch.cuda.current_stream()
-        # One warp per token: small batches get a small grid (its grid-wide barriers are cheaper), large ones every SM.
-        ctas = max(1, min(1 << 16, (T + 7) // 8))
+        ctas = max(1, T)  # one CTA per token: small batches get a small grid (its grid-wide barriers are cheaper), large ones every SM
         rc = _ops.moe_dispatch(self._dargs.data_ptr(), 1, self.world, self.hidden, self.topk, self.n_experts, CH_DISPATCH,
                                0 if self.device_epochs else self.heap.next_epoch(CH_DISPATCH), self.timeout_ns, ctas, s.cuda_stream)
         if rc != 0:
@@ -180,9 +179,11 @@ class FusedMoE(_MoEBase):
         import torch
 
         s = stream or torch.cuda.current_stream()
-        ctas = max(1, min(1 << 16, (T * self.topk * ((self.hidden // 8 + 127) // 128) + 7) // 8))  # one warp per 2 KiB piece of a returned row
+        # one warp per 2 KiB piece of a returned row; alone, a rank has no rows to return and one warp sums each 1 KiB of a token
+        pieces = T * ((self.hidden // 8 + 63) // 64) if self.world == 1 else T * self.topk * ((self.hidden // 8 + 127) // 128)
+        ctas = max(1, min(1 << 16, (pieces + 7) // 8))
         rc = _ops.moe_combine(self._cargs.data_ptr(), 1, self.world, self.hidden, self.topk, self.el, CH_COMBINE,
-                              0 if self.device_epochs else self.heap.next_epoch(CH_COMBINE), self.timeout_ns, ctas, s.cuda_stream)
+                              0 if self.device_epochs else self.heap.next_epoch(CH_COMBINE), self.timeout_ns, ctas, s.cuda_stream, 1)
         if rc != 0:
             raise RuntimeError(f"moe_combine launch failed ({rc})")
         self.launches += 1
@@ -239,7 +240,7 @@ class EmulatedMoE(_MoEBase):
                                              st.arrive.data_ptr() if self.overlap else 0, self.dedup_min_pairs)
             c += _ops.pack_moe_combine_args(rk.meta_ptr, st.y.data_ptr(), st.recv_m.data_ptr(), st.recv_sib.data_ptr(), st.expert_offset.data_ptr(),
                                             st.expert_count.data_ptr(), st.ret_y.data_ptr(), idxs[r].data_ptr(), st.out.data_ptr(), st.status.data_ptr(),
-                                            T, st.cap, st.max_rows_ret)
+                                            T, st.cap, st.max_rows_ret, 0, st.send_slot.data_ptr(), ws[r].data_ptr())
         dargs = torch.frombuffer(bytearray(d), dtype=torch.uint8).cuda()
         cargs = torch.frombuffer(bytearray(c), dtype=torch.uint8).cuda()
         s = torch.cuda.current_stream().cuda_stream
@@ -252,7 +253,7 @@ class EmulatedMoE(_MoEBase):
             return None, status
         for r in range(n):
             self._experts(self.states[r], *self.weights[r])
-        rc = _ops.moe_combine(cargs.data_ptr(), n, R, self.hidden, self.topk, self.el, CH_COMBINE, self.eheap.next_epoch(CH_COMBINE), timeout_ns, 0, s)
+        rc = _ops.moe_combine(cargs.data_ptr(), n, R, self.hidden, self.topk, self.el, CH_COMBINE, self.eheap.next_epoch(CH_COMBINE), timeout_ns, 0, s, 1)
         if rc != 0:
             raise RuntimeError(f"moe_combine launch failed ({rc})")
         torch.cuda.synchronize()
