@@ -13,9 +13,9 @@
 //              multimem.st: each GPU moves ~1x the tensor per direction instead of ~2x.
 // Accumulation is fp32 in rank order, so every rank computes bit-identical results. All cross-rank waits are bounded:
 // on expiry the kernel stores an error code to *status and every CTA leaves through the normal exit.
-// The launcher takes an array of per-rank argument blocks: production passes one; tests that emulate R ranks on a single
-// GPU pass R and the kernel runs them as gridDim.y slices of one cooperative launch (separate launches that wait on one
-// another are never used).
+// A rank passes its argument block by value; tests that emulate R ranks on a single GPU pass an array of R blocks in device memory
+// and the kernel runs them as gridDim.y slices of one cooperative launch (separate launches that wait on one another are
+// never used). One rank alone has nobody to wait for and runs a kernel without barriers that reads and writes everything once.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -192,14 +192,102 @@ __device__ __forceinline__ void FinishEpoch(const mf_allreduce_args_t &a, uint64
     }
 }
 
+// ------------------------------------------------------------------------------------------------ one rank
+
+// A row per CTA: residual + x, rounded, stored, normalised from registers. Latency-bound up to a few hundred rows (32 x 8192: 3 us
+// against 9 us of the one-shot kernel with its flag round trip), beyond that bound by the traffic of x, residual and both
+// results; the two-shot kernel wrote the new residual and read it back between grid barriers.
+template <int VPT>
+__global__ void __launch_bounds__(kThreads, 2)
+mf_residual_rmsnorm_kernel(const mf_allreduce_args_t a, int T, int H, float eps)
+{
+    // See the copy kernels: only the launch latency overlaps with the predecessor, nothing is read before it is complete.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const MfDeviceMeta *m = reinterpret_cast<const MfDeviceMeta *>(a.meta);
+    const int vecsPerRow = H / 8;
+    const size_t rowOff = (size_t)blockIdx.x * H * 2;
+    uint4 xv[VPT], rv[VPT], wv[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; k++) {
+        const int vec = (int)threadIdx.x + k * kThreads;
+        if (vec < vecsPerRow) {
+            xv[k] = mf_ld16((const char *)a.x + rowOff + (size_t)vec * 16);
+            if (a.residual != nullptr) {
+                rv[k] = mf_ld16((const char *)a.residual + rowOff + (size_t)vec * 16);
+            }
+            wv[k] = *reinterpret_cast<const uint4 *>((const char *)a.weight + (size_t)vec * 16);
+        }
+    }
+    if (mf_check_bounds_enabled(m) && !mf_shm_in_own_window(m, a.x, (uint64_t)T * H * 2)) {
+        Fail(a, MF_DEV_ERR_BOUNDS);
+        return;
+    }
+    float ss = 0.f;
+    Acc8 acc[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; k++) {
+        const int vec = (int)threadIdx.x + k * kThreads;
+        if (vec < vecsPerRow) {
+            Unpack(xv[k], acc[k].v);
+            if (a.residual != nullptr) {
+                float res[8];
+                Unpack(rv[k], res);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    acc[k].v[i] += res[i];
+                }
+            }
+            const uint4 h = Pack(acc[k].v);
+            Unpack(h, acc[k].v);
+            if (a.residualOut != nullptr) {
+                mf_st16((char *)a.residualOut + rowOff + (size_t)vec * 16, h);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                ss += acc[k].v[i] * acc[k].v[i];
+            }
+        }
+    }
+    // Every warp adds up all warps' sums itself: one barrier.
+    __shared__ float warpSums[kThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        warpSums[threadIdx.x >> 5] = ss;
+    }
+    __syncthreads();
+    ss = (threadIdx.x & 31) < kThreads / 32 ? warpSums[threadIdx.x & 31] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    }
+    const float rstd = rsqrtf(ss / (float)H + eps);
+#pragma unroll
+    for (int k = 0; k < VPT; k++) {
+        const int vec = (int)threadIdx.x + k * kThreads;
+        if (vec < vecsPerRow) {
+            float w[8], o[8];
+            Unpack(wv[k], w);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                o[i] = acc[k].v[i] * rstd * w[i];
+            }
+            mf_st16((char *)a.out + rowOff + (size_t)vec * 16, Pack(o));
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ one-shot
 
 template <int VPT, bool TAIL>
 __global__ void __launch_bounds__(kThreads, 1)
-mf_allreduce_rmsnorm_oneshot_kernel(const mf_allreduce_args_t *__restrict__ args, int T, int H, float eps, uint32_t channel, uint64_t epochArg,
+mf_allreduce_rmsnorm_oneshot_kernel(const mf_allreduce_args_t own, const mf_allreduce_args_t *__restrict__ emulated, int T, int H, float eps, uint32_t channel, uint64_t epochArg,
                                     uint64_t timeoutNs)
 {
-    const mf_allreduce_args_t a = args[blockIdx.y];
+    const mf_allreduce_args_t a = emulated != nullptr ? emulated[blockIdx.y] : own;
     const MfDeviceMeta *m = reinterpret_cast<const MfDeviceMeta *>(a.meta);
     const int vecsPerRow = H / 8;
     const uint64_t epoch = ResolveEpoch(a, epochArg);
@@ -255,11 +343,11 @@ mf_allreduce_rmsnorm_oneshot_kernel(const mf_allreduce_args_t *__restrict__ args
 // RC: compile-time upper bound of the rank count (2, 4 or 8; 0 = any) so that the peer vectors of a trip live in registers.
 template <bool NVLS, int VPT, int RC>
 __global__ void __launch_bounds__(kThreads, 1)
-mf_allreduce_rmsnorm_twoshot_kernel(const mf_allreduce_args_t *__restrict__ args, int T, int H, float eps, uint32_t channel, uint64_t epochArg,
+mf_allreduce_rmsnorm_twoshot_kernel(const mf_allreduce_args_t own, const mf_allreduce_args_t *__restrict__ emulated, int T, int H, float eps, uint32_t channel, uint64_t epochArg,
                                     uint64_t timeoutNs)
 {
     cg::grid_group grid = cg::this_grid();
-    const mf_allreduce_args_t a = args[blockIdx.y];
+    const mf_allreduce_args_t a = emulated != nullptr ? emulated[blockIdx.y] : own;
     const MfDeviceMeta *m = reinterpret_cast<const MfDeviceMeta *>(a.meta);
     const uint32_t R = m->rankCount, me = m->rankId;
     const int vecsPerRow = H / 8;
@@ -473,21 +561,48 @@ int CoopCapacity(const void *kernel)
 
 }  // namespace
 
-extern "C" int mf_k_allreduce_rmsnorm(const mf_allreduce_args_t *argsDev, int nEmulatedRanks, int rankCount, int T, int H, float eps, int algo,
-                                      uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+static int LaunchOneRank(const mf_allreduce_args_t &a, int T, int H, float eps, mf_stream_t stream)
 {
-    if (argsDev == nullptr || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || T <= 0 || H <= 0 || H % 8 != 0 ||
+    const int vecsPerRow = H / 8;
+    auto kernel = vecsPerRow <= kThreads       ? mf_residual_rmsnorm_kernel<1>
+                  : vecsPerRow <= 2 * kThreads ? mf_residual_rmsnorm_kernel<2>
+                                               : mf_residual_rmsnorm_kernel<4>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)T);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, a, T, H, eps) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MF_K_LAUNCH_FAILED;
+    }
+    return MF_K_OK;
+}
+
+// argsHost: the block of a real rank, by value; argsDev: nEmulatedRanks blocks in device memory. One of the two.
+static int LaunchAllReduce(const mf_allreduce_args_t *argsHost, const mf_allreduce_args_t *argsDev, int nEmulatedRanks, int rankCount, int T, int H,
+                           float eps, int algo, uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    if ((argsHost == nullptr) == (argsDev == nullptr) || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || T <= 0 || H <= 0 || H % 8 != 0 ||
         H > kThreads * kMaxVpt * 8 || channel >= MF_SIGNAL_CHANNELS) {
         return MF_K_INVALID;  // epoch 0 = device-resident epoch (args->epochState), see the header
     }
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
+    if (argsHost != nullptr && rankCount == 1) {
+        return LaunchOneRank(*argsHost, T, H, eps, stream);
+    }
+    const mf_allreduce_args_t own = argsHost != nullptr ? *argsHost : mf_allreduce_args_t{};
     const size_t bytes = (size_t)T * H * 2;
     if (algo == MF_AR_AUTO) {
         algo = bytes <= (512u << 10) ? MF_AR_ONESHOT : MF_AR_TWOSHOT;
     }
-    void *kargs[] = {(void *)&argsDev, (void *)&T, (void *)&H, (void *)&eps, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
+    void *kargs[] = {(void *)&own, (void *)&argsDev, (void *)&T, (void *)&H, (void *)&eps, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
     // Vectors per thread per row are a compile-time constant so that a row lives in registers.
     const int vecsPerRow = H / 8;
     const void *kernel = vecsPerRow <= kThreads       ? PickKernel<1>(algo, rankCount)
@@ -527,4 +642,16 @@ extern "C" int mf_k_allreduce_rmsnorm(const mf_allreduce_args_t *argsDev, int nE
         return MF_K_LAUNCH_FAILED;
     }
     return MF_K_OK;
+}
+
+extern "C" int mf_k_allreduce_rmsnorm(const mf_allreduce_args_t *argsDev, int nEmulatedRanks, int rankCount, int T, int H, float eps, int algo,
+                                      uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    return LaunchAllReduce(nullptr, argsDev, nEmulatedRanks, rankCount, T, H, eps, algo, channel, epoch, timeoutNs, ctas, stream);
+}
+
+extern "C" int mf_k_allreduce_rmsnorm_rank(const mf_allreduce_args_t *argsHost, int rankCount, int T, int H, float eps, int algo, uint32_t channel,
+                                           uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    return LaunchAllReduce(argsHost, nullptr, 1, rankCount, T, H, eps, algo, channel, epoch, timeoutNs, ctas, stream);
 }

@@ -80,6 +80,9 @@ enum { MF_AR_AUTO = 0, MF_AR_ONESHOT = 1, MF_AR_TWOSHOT = 2, MF_AR_NVLS = 3, MF_
 // be used with host-side epochs any more). H: multiple of 8, at most 16384. timeoutNs 0 = 2 s.
 int mf_k_allreduce_rmsnorm(const mf_allreduce_args_t *argsDev, int nEmulatedRanks, int rankCount, int T, int H, float eps, int algo,
                            uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream);
+// The same for a real rank, its block passed by value: nothing has to be uploaded when a pointer changes, and a CUDA graph holds it.
+int mf_k_allreduce_rmsnorm_rank(const mf_allreduce_args_t *argsHost, int rankCount, int T, int H, float eps, int algo, uint32_t channel, uint64_t epoch,
+                                uint64_t timeoutNs, int ctas, mf_stream_t stream);
 
 // ------------------------------------------------------------------------------------------------ MoE expert FFN (K5b)
 
@@ -183,9 +186,13 @@ typedef struct {
 // cooperative launches; epoch must grow by one per call and channel on every rank alike (epoch 0: taken from args.epochState).
 int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int E, uint32_t channel,
                       uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream);
-// direct: the argument blocks carry sendSlot and topkW.
 int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int EL, uint32_t channel,
-                     uint64_t epoch, uint64_t timeoutNs, int ctas, int direct, mf_stream_t stream);
+                     uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream);
+// The same for a real rank, its block passed by value.
+int mf_k_moe_dispatch_rank(const mf_moe_dispatch_args_t *argsHost, int rankCount, int H, int K, int E, uint32_t channel, uint64_t epoch,
+                           uint64_t timeoutNs, int ctas, mf_stream_t stream);
+int mf_k_moe_combine_rank(const mf_moe_combine_args_t *argsHost, int rankCount, int H, int K, int EL, uint32_t channel, uint64_t epoch,
+                          uint64_t timeoutNs, int ctas, mf_stream_t stream);
 
 // ------------------------------------------------------------------------------------------------ weight reshard (K6)
 

@@ -23,8 +23,8 @@
 //           the owner.
 // The reference library names MoE dispatch/combine only as a use case of its symmetric heap (README.md:53 of the reference);
 // the flag/barrier discipline follows its sample kernel (example/shm/AllReduce/shm_all_reduce.cpp:69-112) with bounded waits.
-// Like the all-reduce, both kernels take an array of per-rank argument blocks so that tests can run all ranks of a fake
-// heap as gridDim.y slices of one cooperative launch on a single GPU.
+// Like the all-reduce, both kernels take a rank's argument block by value, or an array of blocks in device memory so that tests can
+// run all ranks of a fake heap as gridDim.y slices of one cooperative launch on a single GPU.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -117,11 +117,12 @@ __device__ __forceinline__ int4 mf_ld_meta(const int4 *p)
 // finds the rows. One warp per token with a stage in shared memory took 28 dependent loads a token; with one CTA per token and
 // four per SM the small call is a few latencies long (128 tokens: 55 -> 15 us on one rank) and the large one is bound by its stores
 // (4096 tokens, top-8 of 32 experts on one rank, 300 MB: 158 -> 75 us).
+template <bool EMULATED>
 __global__ void __launch_bounds__(kThreads, 4)
-mf_moe_dispatch_kernel(const mf_moe_dispatch_args_t *__restrict__ args, int H, int K, int E, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
+mf_moe_dispatch_kernel(const __grid_constant__ mf_moe_dispatch_args_t own, const mf_moe_dispatch_args_t *__restrict__ emulated, int H, int K, int E, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
     cg::grid_group grid = cg::this_grid();
-    const mf_moe_dispatch_args_t a = args[blockIdx.y];
+    const mf_moe_dispatch_args_t &a = EMULATED ? emulated[blockIdx.y] : own;
     const uint64_t epoch = ResolveEpochD(a, epochArg);
     if (epoch == 0) {
         FailD(a.status, MF_DEV_ERR_BOUNDS);  // neither an epoch argument nor a device-resident epoch
@@ -551,11 +552,11 @@ __device__ __forceinline__ void GatherGroup(float (&part)[2][8], uint32_t group,
 // zone is written and read for them and no receive buffer is scanned for leaders (7 of 8 of its rows are followers when one rank
 // owns all experts). One rank, top-8, hidden 7168: 128 tokens 63 -> 8 us, 4096 tokens (530 MB) 247 -> 90 us.
 // ALONE: one rank with sendSlot and topkW and at most eight pairs a token; nothing waits on anything, so it is an ordinary launch.
-template <bool ALONE>
+template <bool ALONE, bool EMULATED>
 __global__ void __launch_bounds__(kThreads, 3)
-mf_moe_combine_kernel(const mf_moe_combine_args_t *__restrict__ args, int H, int K, int EL, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
+mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const mf_moe_combine_args_t *__restrict__ emulated, int H, int K, int EL, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
-    const mf_moe_combine_args_t a = args[blockIdx.y];
+    const mf_moe_combine_args_t &a = EMULATED ? emulated[blockIdx.y] : own;
     const uint64_t epoch = ResolveEpochD(a, epochArg);
     if (epoch == 0) {
         FailD(a.status, MF_DEV_ERR_BOUNDS);  // neither an epoch argument nor a device-resident epoch
@@ -751,10 +752,11 @@ int CoopCap(const void *kernel, size_t smem)
 
 }  // namespace
 
-extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int E, uint32_t channel,
-                                 uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+// argsHost: the block of a real rank, by value; argsDev: nEmulatedRanks blocks in device memory. One of the two.
+static int LaunchDispatch(const mf_moe_dispatch_args_t *argsHost, const mf_moe_dispatch_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K,
+                          int E, uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
 {
-    if (argsDev == nullptr || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || H <= 0 || H % 128 != 0 || K < 1 ||
+    if ((argsHost == nullptr) == (argsDev == nullptr) || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || H <= 0 || H % 128 != 0 || K < 1 ||
         K > kMaxTopk || E < rankCount || E % rankCount != 0 || E > kMaxExperts || channel >= MF_SIGNAL_CHANNELS) {
         return MF_K_INVALID;
     }
@@ -762,7 +764,9 @@ extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmu
         timeoutNs = 2000000000ull;
     }
     const size_t smem = (size_t)3 * kMaxExperts * sizeof(int);
-    int cap = CoopCap((const void *)mf_moe_dispatch_kernel, smem);
+    const void *kernel = argsHost != nullptr ? (const void *)mf_moe_dispatch_kernel<false> : (const void *)mf_moe_dispatch_kernel<true>;
+    const mf_moe_dispatch_args_t own = argsHost != nullptr ? *argsHost : mf_moe_dispatch_args_t{};
+    int cap = CoopCap(kernel, smem);
     if (cap <= 0) {
         return MF_K_LAUNCH_FAILED;
     }
@@ -773,9 +777,9 @@ extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmu
     if (grid < 1) {
         return MF_K_TOO_LARGE;
     }
-    void *kargs[] = {(void *)&argsDev, (void *)&H, (void *)&K, (void *)&E, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
+    void *kargs[] = {(void *)&own, (void *)&argsDev, (void *)&H, (void *)&K, (void *)&E, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
     dim3 g((unsigned)grid, (unsigned)nEmulatedRanks, 1), b(kThreads, 1, 1);
-    cudaError_t e = cudaLaunchCooperativeKernel((const void *)mf_moe_dispatch_kernel, g, b, kargs, smem, (cudaStream_t)stream);
+    cudaError_t e = cudaLaunchCooperativeKernel(kernel, g, b, kargs, smem, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return MF_K_LAUNCH_FAILED;
@@ -783,18 +787,21 @@ extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmu
     return MF_K_OK;
 }
 
-extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int EL, uint32_t channel,
-                                uint64_t epoch, uint64_t timeoutNs, int ctas, int direct, mf_stream_t stream)
+static int LaunchCombine(const mf_moe_combine_args_t *argsHost, const mf_moe_combine_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K,
+                         int EL, uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
 {
-    if (argsDev == nullptr || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || H <= 0 || H % 8 != 0 || K < 1 || K > 32 ||
+    if ((argsHost == nullptr) == (argsDev == nullptr) || nEmulatedRanks < 1 || rankCount < 1 || rankCount > (int)MF_SIGNAL_MAX_RANKS || H <= 0 || H % 8 != 0 || K < 1 || K > 32 ||
         EL < 1 || EL > kMaxExperts || channel >= MF_SIGNAL_CHANNELS) {
         return MF_K_INVALID;
     }
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
-    const bool alone = direct != 0 && rankCount == 1 && K <= MF_MOE_MAX_SIBLINGS + 1;
-    const void *kernel = alone ? (const void *)mf_moe_combine_kernel<true> : (const void *)mf_moe_combine_kernel<false>;
+    const bool alone = argsHost != nullptr && argsHost->sendSlot != nullptr && argsHost->topkW != nullptr && rankCount == 1 && K <= MF_MOE_MAX_SIBLINGS + 1;
+    const void *kernel = alone                 ? (const void *)mf_moe_combine_kernel<true, false>
+                         : argsHost != nullptr ? (const void *)mf_moe_combine_kernel<false, false>
+                                               : (const void *)mf_moe_combine_kernel<false, true>;
+    const mf_moe_combine_args_t own = argsHost != nullptr ? *argsHost : mf_moe_combine_args_t{};
     int cap = CoopCap(kernel, 0);
     if (cap <= 0) {
         return MF_K_LAUNCH_FAILED;
@@ -806,7 +813,7 @@ extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmula
     if (grid < 1) {
         return MF_K_TOO_LARGE;
     }
-    void *kargs[] = {(void *)&argsDev, (void *)&H, (void *)&K, (void *)&EL, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
+    void *kargs[] = {(void *)&own, (void *)&argsDev, (void *)&H, (void *)&K, (void *)&EL, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
     dim3 g((unsigned)grid, (unsigned)nEmulatedRanks, 1), b(kThreads, 1, 1);
     cudaError_t e = alone ? cudaLaunchKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream)
                           : cudaLaunchCooperativeKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream);
@@ -815,4 +822,28 @@ extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmula
         return MF_K_LAUNCH_FAILED;
     }
     return MF_K_OK;
+}
+
+extern "C" int mf_k_moe_dispatch(const mf_moe_dispatch_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int E, uint32_t channel,
+                                 uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    return LaunchDispatch(nullptr, argsDev, nEmulatedRanks, rankCount, H, K, E, channel, epoch, timeoutNs, ctas, stream);
+}
+
+extern "C" int mf_k_moe_dispatch_rank(const mf_moe_dispatch_args_t *argsHost, int rankCount, int H, int K, int E, uint32_t channel, uint64_t epoch,
+                                      uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    return LaunchDispatch(argsHost, nullptr, 1, rankCount, H, K, E, channel, epoch, timeoutNs, ctas, stream);
+}
+
+extern "C" int mf_k_moe_combine(const mf_moe_combine_args_t *argsDev, int nEmulatedRanks, int rankCount, int H, int K, int EL, uint32_t channel,
+                                uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    return LaunchCombine(nullptr, argsDev, nEmulatedRanks, rankCount, H, K, EL, channel, epoch, timeoutNs, ctas, stream);
+}
+
+extern "C" int mf_k_moe_combine_rank(const mf_moe_combine_args_t *argsHost, int rankCount, int H, int K, int EL, uint32_t channel, uint64_t epoch,
+                                     uint64_t timeoutNs, int ctas, mf_stream_t stream)
+{
+    return LaunchCombine(argsHost, nullptr, 1, rankCount, H, K, EL, channel, epoch, timeoutNs, ctas, stream);
 }

@@ -9,6 +9,66 @@
 
 namespace py = pybind11;
 
+namespace {
+
+// What one AllReduceRMSNorm object keeps between calls.
+struct AllReducePlan {
+    mf_allreduce_args_t a{};
+    int world{1}, hidden{0};
+    float eps{0.f};
+    uint32_t channel{0};
+    uint64_t timeoutNs{0};
+};
+
+// What one MoE layer of a rank keeps between calls, and the launches of a call: in Python the four of them took about 60 us,
+// more than a small layer runs on the GPU.
+struct MoePlan {
+    mf_moe_dispatch_args_t d{};
+    mf_moe_combine_args_t c{};
+    void *h1Q{nullptr}, *h1Sf{nullptr};
+    int world{1}, hidden{0}, topk{0}, experts{0}, inter{0};
+    uint32_t dispatchChannel{0}, combineChannel{0};
+    uint64_t timeoutNs{0}, waitNs{0};
+    int *arrive{nullptr};
+
+    int Dispatch(uint64_t x, uint64_t idx, uint64_t w, int T, uint64_t epoch, bool overlap, int dedupMinPairs, uint64_t stream)
+    {
+        d.x = (const void *)x;
+        d.topkIdx = c.topkIdx = (const int *)idx;
+        d.topkW = c.topkW = (const float *)w;
+        d.T = T;
+        d.arrive = overlap ? arrive : nullptr;
+        d.dedupMinPairs = dedupMinPairs;
+        // One CTA per token: small batches get a small grid (its grid-wide barriers are cheaper), large ones every SM.
+        return mf_k_moe_dispatch_rank(&d, world, hidden, topk, experts, dispatchChannel, epoch, timeoutNs, T > 1 ? T : 1, (mf_stream_t)stream);
+    }
+    int Experts(uint64_t w13Q, uint64_t w13S, int w13Packed, uint64_t w2Q, uint64_t w2S, int w2Packed, bool overlap, uint64_t stream)
+    {
+        const int el = experts / world, rows = c.cap;
+        const int mode1 = MF_GEMM_EPI_SWIGLU_FP8 | (w13Packed ? (int)MF_GEMM_B_PACKED : 0), mode2 = MF_GEMM_EPI_BF16 | (w2Packed ? (int)MF_GEMM_B_PACKED : 0);
+        const int rc = overlap ? mf_k_moe_grouped_gemm_mx_gated(d.recvX, d.recvSf, (const void *)w13Q, (const float *)w13S, h1Q, h1Sf, d.expertOffset,
+                                                                d.expertCount, el, rows, 2 * inter, hidden, mode1, 0, arrive, waitNs, d.status, 0,
+                                                                (mf_stream_t)stream)
+                               : mf_k_moe_grouped_gemm_mx(d.recvX, d.recvSf, (const void *)w13Q, (const float *)w13S, h1Q, h1Sf, d.expertOffset,
+                                                          d.expertCount, el, rows, 2 * inter, hidden, mode1, 0, d.status, 0, (mf_stream_t)stream);
+        if (rc != MF_K_OK) {
+            return rc;
+        }
+        return mf_k_moe_grouped_gemm_mx(h1Q, (const uint32_t *)h1Sf, (const void *)w2Q, (const float *)w2S, const_cast<void *>(c.y), nullptr, d.expertOffset,
+                                        d.expertCount, el, rows, hidden, inter, mode2, 0, d.status, 0, (mf_stream_t)stream);
+    }
+    int Combine(int T, uint64_t epoch, uint64_t stream)
+    {
+        c.T = T;
+        // One warp per 1 KiB piece of a returned row; alone, a rank has no rows to return and one warp sums each 1 KiB of a token.
+        const long long pieces = (long long)T * (world == 1 ? 1 : topk) * ((hidden / 8 + 63) / 64);
+        const int ctas = (int)((pieces + 7) / 8 < 65536 ? (pieces + 7) / 8 : 65536);
+        return mf_k_moe_combine_rank(&c, world, hidden, topk, experts / world, combineChannel, epoch, timeoutNs, ctas > 1 ? ctas : 1, (mf_stream_t)stream);
+    }
+};
+
+}  // namespace
+
 void BindOps(py::module_ &m)
 {
     py::module_ ops = m.def_submodule("ops", "raw launchers of the fused kernels");
@@ -126,11 +186,11 @@ void BindOps(py::module_ &m)
     }, py::arg("args_dev"), py::arg("n_emulated"), py::arg("rank_count"), py::arg("H"), py::arg("K"), py::arg("E"), py::arg("channel"), py::arg("epoch"),
             py::arg("timeout_ns") = 0, py::arg("ctas") = 0, py::arg("stream") = 0);
     ops.def("moe_combine", [](uint64_t argsDev, int nEmulated, int rankCount, int H, int K, int EL, uint32_t channel, uint64_t epoch, uint64_t timeoutNs,
-                              int ctas, uint64_t stream, int direct) {
-        return mf_k_moe_combine((const mf_moe_combine_args_t *)argsDev, nEmulated, rankCount, H, K, EL, channel, epoch, timeoutNs, ctas, direct,
+                              int ctas, uint64_t stream) {
+        return mf_k_moe_combine((const mf_moe_combine_args_t *)argsDev, nEmulated, rankCount, H, K, EL, channel, epoch, timeoutNs, ctas,
                                 (mf_stream_t)stream);
     }, py::arg("args_dev"), py::arg("n_emulated"), py::arg("rank_count"), py::arg("H"), py::arg("K"), py::arg("EL"), py::arg("channel"), py::arg("epoch"),
-            py::arg("timeout_ns") = 0, py::arg("ctas") = 0, py::arg("stream") = 0, py::arg("direct") = 0);
+            py::arg("timeout_ns") = 0, py::arg("ctas") = 0, py::arg("stream") = 0);
     ops.attr("RESHARD_DESC_BYTES") = (int)sizeof(mf_reshard_desc_t);
     ops.attr("RESHARD_ARGS_BYTES") = (int)sizeof(mf_reshard_args_t);
     ops.def("pack_reshard_desc", [](uint64_t srcFlatOff, uint64_t dstOff, uint64_t scaleOff, uint32_t colsFull, uint32_t r0, uint32_t c0, uint32_t nrows,
@@ -156,6 +216,85 @@ void BindOps(py::module_ &m)
         return mf_k_reshard((const mf_reshard_args_t *)argsDev, nEmulated, rankCount, channel, epoch, timeoutNs, ctas, (mf_stream_t)stream);
     }, py::arg("args_dev"), py::arg("n_emulated"), py::arg("rank_count"), py::arg("channel"), py::arg("epoch"), py::arg("timeout_ns") = 0,
             py::arg("ctas") = 0, py::arg("stream") = 0);
+    py::class_<AllReducePlan>(ops, "AllReducePlan")
+        .def(py::init([](uint64_t meta, uint64_t residualOut, uint64_t out, uint64_t status, uint64_t epochState, int world, int hidden, float eps,
+                         uint32_t channel, uint64_t timeoutNs) {
+            AllReducePlan p;
+            p.a.meta = (const void *)meta;
+            p.a.residualOut = (void *)residualOut;
+            p.a.out = (void *)out;
+            p.a.status = (int *)status;
+            p.a.epochState = (unsigned long long *)epochState;
+            p.world = world;
+            p.hidden = hidden;
+            p.eps = eps;
+            p.channel = channel;
+            p.timeoutNs = timeoutNs;
+            return p;
+        }))
+        .def("run", [](const AllReducePlan &p, uint64_t x, uint64_t residual, uint64_t weight, int T, int algo, uint64_t epoch, int ctas, uint64_t stream) {
+            mf_allreduce_args_t a = p.a;
+            a.x = (const void *)x;
+            a.residual = (const void *)residual;
+            a.weight = (const void *)weight;
+            return mf_k_allreduce_rmsnorm_rank(&a, p.world, T, p.hidden, p.eps, algo, p.channel, epoch, p.timeoutNs, ctas, (mf_stream_t)stream);
+        });
+    py::class_<MoePlan>(ops, "MoePlan")
+        .def(py::init([](uint64_t meta, uint64_t cnt, uint64_t recvX, uint64_t recvSf, uint64_t recvMeta, uint64_t recvSib, uint64_t localCnt,
+                         uint64_t cursor, uint64_t expertOffset, uint64_t expertCount, uint64_t sendSlot, uint64_t arrive, uint64_t status, uint64_t h1Q,
+                         uint64_t h1Sf, uint64_t y, uint64_t retY, uint64_t out, int cap, int retRows, int world, int hidden, int topk, int experts,
+                         int inter, uint32_t dispatchChannel, uint32_t combineChannel, uint64_t timeoutNs, uint64_t waitNs, uint64_t epochD,
+                         uint64_t epochC) {
+            MoePlan p;
+            p.d.meta = p.c.meta = (const void *)meta;
+            p.d.cnt = (int *)cnt;
+            p.d.recvX = (void *)recvX;
+            p.d.recvSf = (uint32_t *)recvSf;
+            p.d.recvMeta = (int4 *)recvMeta;
+            p.c.recvMeta = (const int4 *)recvMeta;
+            p.d.recvSib = (int2 *)recvSib;
+            p.c.recvSib = (const int2 *)recvSib;
+            p.d.localCnt = (int *)localCnt;
+            p.d.cursor = (int *)cursor;
+            p.d.expertOffset = (int *)expertOffset;
+            p.c.expertOffset = (const int *)expertOffset;
+            p.d.expertCount = (int *)expertCount;
+            p.c.expertCount = (const int *)expertCount;
+            p.d.sendSlot = (int *)sendSlot;
+            p.c.sendSlot = (const int *)sendSlot;
+            p.d.status = p.c.status = (int *)status;
+            p.d.epochState = (unsigned long long *)epochD;
+            p.c.epochState = (unsigned long long *)epochC;
+            p.d.cap = p.c.cap = cap;
+            p.c.y = (const void *)y;
+            p.c.retY = (void *)retY;
+            p.c.out = (void *)out;
+            p.c.retRows = retRows;
+            p.h1Q = (void *)h1Q;
+            p.h1Sf = (void *)h1Sf;
+            p.arrive = (int *)arrive;
+            p.world = world;
+            p.hidden = hidden;
+            p.topk = topk;
+            p.experts = experts;
+            p.inter = inter;
+            p.dispatchChannel = dispatchChannel;
+            p.combineChannel = combineChannel;
+            p.timeoutNs = timeoutNs;
+            p.waitNs = waitNs;
+            return p;
+        }))
+        .def("dispatch", &MoePlan::Dispatch)
+        .def("experts", &MoePlan::Experts)
+        .def("combine", &MoePlan::Combine)
+        .def("run", [](MoePlan &p, uint64_t x, uint64_t idx, uint64_t w, int T, uint64_t w13Q, uint64_t w13S, int w13Packed, uint64_t w2Q, uint64_t w2S,
+                       int w2Packed, uint64_t epochD, uint64_t epochC, bool overlap, int dedupMinPairs, uint64_t stream) {
+            int rc = p.Dispatch(x, idx, w, T, epochD, overlap, dedupMinPairs, stream);
+            if (rc == MF_K_OK) {
+                rc = p.Experts(w13Q, w13S, w13Packed, w2Q, w2S, w2Packed, overlap, stream);
+            }
+            return rc == MF_K_OK ? p.Combine(T, epochC, stream) : rc;
+        });
     ops.def("allreduce_rmsnorm", [](uint64_t argsDev, int nEmulated, int rankCount, int T, int H, float eps, int algo, uint32_t channel, uint64_t epoch,
                                     uint64_t timeoutNs, int ctas, uint64_t stream) {
         return mf_k_allreduce_rmsnorm((const mf_allreduce_args_t *)argsDev, nEmulated, rankCount, T, H, eps, algo, channel, epoch, timeoutNs, ctas,

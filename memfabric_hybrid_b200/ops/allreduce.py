@@ -23,6 +23,7 @@ from typing import Optional
 
 from .. import _loader  # noqa: F401
 from .._loader import _pymf
+from ..utils.tensors import current_stream_handle
 
 _ops = _pymf.ops
 ALGOS = {"auto": _ops.AR_AUTO, "oneshot": _ops.AR_ONESHOT, "twoshot": _ops.AR_TWOSHOT, "nvls": _ops.AR_NVLS,
@@ -62,8 +63,6 @@ class AllReduceRMSNorm:
         dev = self._xs[0].device
         self.out = torch.empty(max_tokens, hidden, dtype=torch.bfloat16, device=dev)
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
-        self._args = [torch.empty(_ops.ALLREDUCE_ARGS_BYTES, dtype=torch.uint8, device=dev) for _ in range(2)]
-        self._args_key = [None, None]
         self.launches = 0
         self.device_epochs = device_epochs
         self._epoch_state = None
@@ -71,28 +70,17 @@ class AllReduceRMSNorm:
             # [0] = epoch of the last finished call, [1] = CTAs of the running call that have retired. Starts at the channel's
             # current host-side epoch (the same number on every rank), so that flags left by earlier host-epoch calls are stale.
             self._epoch_state = torch.tensor([heap.next_epoch(channel), 0], dtype=torch.int64, device=dev)
+        self._plan = _ops.AllReducePlan(heap.meta_ptr, self.residual_out.data_ptr(), self.out.data_ptr(), self.status.data_ptr(),
+                                        self._epoch_state.data_ptr() if device_epochs else 0, heap.world, hidden, eps, channel, timeout_ns)
+        self._x_ptrs = [x.data_ptr() for x in self._xs]
+        self._results = (max_tokens, (self.out, self.residual_out))  # views of the last token count: making them costs as much as a launch
 
     @property
     def x(self):
         """Input buffer of the next call (bf16 [max_tokens, hidden])."""
         return self._xs[self._cur]
 
-    def _pack(self, residual, weight):
-        import torch
-
-        c = self._cur
-        key = (residual.data_ptr() if residual is not None else 0, weight.data_ptr())
-        if key != self._args_key[c]:
-            blob = _ops.pack_allreduce_args(self.heap.meta_ptr, self._xs[c].data_ptr(), key[0], key[1], self.residual_out.data_ptr(),
-                                            self.out.data_ptr(), self.status.data_ptr(),
-                                            self._epoch_state.data_ptr() if self._epoch_state is not None else 0)
-            self._args[c].copy_(torch.frombuffer(bytearray(blob), dtype=torch.uint8), non_blocking=False)
-            self._args_key[c] = key
-        return self._args[c].data_ptr()
-
     def __call__(self, tokens: int, residual, weight, algo: str = "auto", ctas: int = 0, stream=None):
-        import torch
-
         if tokens > self.max_tokens:
             raise ValueError("tokens exceeds max_tokens")
         a = ALGOS[algo]
@@ -110,16 +98,17 @@ class AllReduceRMSNorm:
             raise ValueError("oneshot_notail needs double_buffer=True")
         if a == _ops.AR_NVLS and not self.heap.multicast_ptr:
             raise RuntimeError("the NVLS algorithm needs a heap created with nvls=True on a platform with multicast")
-        args = self._pack(residual, weight)
-        s = stream or torch.cuda.current_stream()
+        s = stream.cuda_stream if stream is not None else current_stream_handle()
         epoch = 0 if self.device_epochs else self.heap.next_epoch(self.channel)
-        rc = _ops.allreduce_rmsnorm(args, 1, self.heap.world, tokens, self.hidden, self.eps, a, self.channel, epoch, self.timeout_ns, ctas, s.cuda_stream)
+        rc = self._plan.run(self._x_ptrs[self._cur], residual.data_ptr() if residual is not None else 0, weight.data_ptr(), tokens, a, epoch, ctas, s)
         if rc != 0:
             raise RuntimeError(f"allreduce_rmsnorm launch failed ({rc})")
         self.launches += 1
         if self.double_buffer:
             self._cur = 1 - self._cur
-        return self.out[:tokens], self.residual_out[:tokens]
+        if self._results[0] != tokens:
+            self._results = (tokens, (self.out[:tokens], self.residual_out[:tokens]))
+        return self._results[1]
 
     def check_status(self) -> int:
         """Synchronises and returns the device status word (0 = fine, else MF_DEV_ERR_* | peer << 8)."""

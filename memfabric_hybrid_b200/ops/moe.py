@@ -15,8 +15,7 @@ while slower senders are still pushing (every pair then carries its payload over
 owner and the owner replicates it).
 
 CUDA graphs: with ``device_epochs=True`` the epochs that order the cross-rank flags of dispatch and combine live in device
-memory and are advanced by the kernels themselves, so a call of the layer may be captured into a graph and replayed (call it once
-eagerly with the same tensors first: the argument blocks are uploaded on first use). Every rank must use the same setting.
+memory and are advanced by the kernels themselves, so a call of the layer may be captured into a graph and replayed. Every rank must use the same setting.
 
 ``EmulatedMoE`` drives the same kernels for all ranks of an ``EmulatedHeap`` on one GPU (dispatch and combine each as one
 cooperative launch over all ranks; the per-rank GEMMs in between are ordinary launches) — this is how the multi-rank logic
@@ -28,6 +27,7 @@ from typing import List, Optional
 
 from .. import _loader  # noqa: F401
 from .._loader import _pymf
+from ..utils.tensors import current_stream_handle
 from . import fp8_gemm as F
 
 _ops = _pymf.ops
@@ -127,9 +127,6 @@ class FusedMoE(_MoEBase):
         cap = capacity_rows(max_tokens, topk, heap.world, self.el, capacity_factor)
         dev = torch.device("cuda", torch.cuda.current_device())
         self.st = _RankState(heap, heap.alloc, max_tokens, hidden, n_experts, topk, inter, cap, dev)
-        self._dargs = torch.empty(_ops.MOE_DISPATCH_ARGS_BYTES, dtype=torch.uint8, device=dev)
-        self._cargs = torch.empty(_ops.MOE_COMBINE_ARGS_BYTES, dtype=torch.uint8, device=dev)
-        self._key = None
         self.device_epochs = device_epochs
         self._epoch_d = self._epoch_c = None
         if device_epochs:
@@ -137,62 +134,68 @@ class FusedMoE(_MoEBase):
             # epochs (the same numbers on every rank) so that flags left by earlier calls are stale
             self._epoch_d = torch.tensor([heap.next_epoch(CH_DISPATCH), 0], dtype=torch.int64, device=dev)
             self._epoch_c = torch.tensor([heap.next_epoch(CH_COMBINE), 0], dtype=torch.int64, device=dev)
+        st = self.st
+        self._plan = _ops.MoePlan(heap.meta_ptr, st.cnt.data_ptr(), st.recv_x.data_ptr(), st.recv_s.data_ptr(), st.recv_m.data_ptr(),
+                                  st.recv_sib.data_ptr(), st.local_cnt.data_ptr(), st.cursor.data_ptr(), st.expert_offset.data_ptr(),
+                                  st.expert_count.data_ptr(), st.send_slot.data_ptr(), st.arrive.data_ptr(), st.status.data_ptr(), st.h1_q.data_ptr(),
+                                  st.h1_sf.data_ptr(), st.y.data_ptr(), st.ret_y.data_ptr(), st.out.data_ptr(), st.cap, st.max_rows_ret, heap.world, hidden,
+                                  topk, n_experts, inter, CH_DISPATCH, CH_COMBINE, timeout_ns, self.wait_ns,
+                                  self._epoch_d.data_ptr() if device_epochs else 0, self._epoch_c.data_ptr() if device_epochs else 0)
+        self._weights_checked = None
+        self._result = (max_tokens, st.out)
         torch.cuda.synchronize()
         heap.barrier()  # everybody's count matrix is zeroed before the first dispatch touches it
 
-    def _pack(self, x, idx, w, T):
-        import torch
+    def _weights(self):
+        """(address, scales' address, packed) of both projections. Shapes are looked at when a tensor is another than last time."""
+        t = (self.w13_q, self.w13_s, self.w2_q, self.w2_s)
+        if self._weights_checked is None or any(a is not b for a, b in zip(t, self._weights_checked)):
+            for q, s, n, k in ((t[0], t[1], 2 * self.inter, self.hidden), (t[2], t[3], self.hidden, self.inter)):
+                shape = (self.el, n // 32, k // 128, 32, 128) if q.dim() == 5 else (self.el, n, k)
+                assert tuple(q.shape) == shape and tuple(s.shape) == (self.el, n // 128, k // 128) and q.is_contiguous() and s.is_contiguous()
+            self._weights_checked = t
+        return t[0].data_ptr(), t[1].data_ptr(), int(t[0].dim() == 5), t[2].data_ptr(), t[3].data_ptr(), int(t[2].dim() == 5)
 
-        key = (x.data_ptr(), idx.data_ptr(), w.data_ptr(), T, self.overlap, self.dedup_min_pairs)
-        if key == self._key:
-            return
-        st, h = self.st, self.heap
-        d = _ops.pack_moe_dispatch_args(h.meta_ptr, x.data_ptr(), idx.data_ptr(), w.data_ptr(), st.cnt.data_ptr(), st.recv_x.data_ptr(), st.recv_s.data_ptr(),
-                                        st.recv_m.data_ptr(), st.recv_sib.data_ptr(), st.local_cnt.data_ptr(), st.cursor.data_ptr(), st.expert_offset.data_ptr(),
-                                        st.expert_count.data_ptr(), st.send_slot.data_ptr(), st.status.data_ptr(), T, st.cap,
-                                        st.arrive.data_ptr() if self.overlap else 0, self.dedup_min_pairs,
-                                        self._epoch_d.data_ptr() if self.device_epochs else 0)
-        c = _ops.pack_moe_combine_args(h.meta_ptr, st.y.data_ptr(), st.recv_m.data_ptr(), st.recv_sib.data_ptr(), st.expert_offset.data_ptr(),
-                                       st.expert_count.data_ptr(), st.ret_y.data_ptr(), idx.data_ptr(), st.out.data_ptr(), st.status.data_ptr(), T,
-                                       st.cap, st.max_rows_ret, self._epoch_c.data_ptr() if self.device_epochs else 0, st.send_slot.data_ptr(), w.data_ptr())
-        self._dargs.copy_(torch.frombuffer(bytearray(d), dtype=torch.uint8))
-        self._cargs.copy_(torch.frombuffer(bytearray(c), dtype=torch.uint8))
-        self._key = key
+    def _epoch(self, channel):
+        return 0 if self.device_epochs else self.heap.next_epoch(channel)
 
     def dispatch(self, x, idx, w, stream=None):
-        import torch
-
-        T = x.shape[0]
-        self._pack(x, idx, w, T)
-        s = stream or torch.cuda.current_stream()
-        ctas = max(1, T)  # one CTA per token: small batches get a small grid (its grid-wide barriers are cheaper), large ones every SM
-        rc = _ops.moe_dispatch(self._dargs.data_ptr(), 1, self.world, self.hidden, self.topk, self.n_experts, CH_DISPATCH,
-                               0 if self.device_epochs else self.heap.next_epoch(CH_DISPATCH), self.timeout_ns, ctas, s.cuda_stream)
+        s = stream.cuda_stream if stream is not None else current_stream_handle()
+        rc = self._plan.dispatch(x.data_ptr(), idx.data_ptr(), w.data_ptr(), x.shape[0], self._epoch(CH_DISPATCH), self.overlap, self.dedup_min_pairs, s)
         if rc != 0:
             raise RuntimeError(f"moe_dispatch launch failed ({rc})")
         self.launches += 1
 
     def experts(self, stream=None):
-        return self._experts(self.st, self.w13_q, self.w13_s, self.w2_q, self.w2_s, stream)
+        s = stream.cuda_stream if stream is not None else current_stream_handle()
+        rc = self._plan.experts(*self._weights(), self.overlap, s)
+        if rc != 0:
+            raise RuntimeError(f"moe_grouped_gemm_mx launch failed ({rc})")
+        self.launches += 2
+        return self.st.cap
 
     def combine(self, T, stream=None):
-        import torch
-
-        s = stream or torch.cuda.current_stream()
-        # one warp per 2 KiB piece of a returned row; alone, a rank has no rows to return and one warp sums each 1 KiB of a token
-        pieces = T * ((self.hidden // 8 + 63) // 64) if self.world == 1 else T * self.topk * ((self.hidden // 8 + 127) // 128)
-        ctas = max(1, min(1 << 16, (pieces + 7) // 8))
-        rc = _ops.moe_combine(self._cargs.data_ptr(), 1, self.world, self.hidden, self.topk, self.el, CH_COMBINE,
-                              0 if self.device_epochs else self.heap.next_epoch(CH_COMBINE), self.timeout_ns, ctas, s.cuda_stream, 1)
+        s = stream.cuda_stream if stream is not None else current_stream_handle()
+        rc = self._plan.combine(T, self._epoch(CH_COMBINE), s)
         if rc != 0:
             raise RuntimeError(f"moe_combine launch failed ({rc})")
         self.launches += 1
-        return self.st.out[:T]
+        return self._out(T)
+
+    def _out(self, T):
+        if self._result[0] != T:
+            self._result = (T, self.st.out[:T])
+        return self._result[1]
 
     def __call__(self, x, idx, w, stream=None):
-        self.dispatch(x, idx, w, stream)
-        self.experts(stream)
-        return self.combine(x.shape[0], stream)
+        T = x.shape[0]
+        s = stream.cuda_stream if stream is not None else current_stream_handle()
+        rc = self._plan.run(x.data_ptr(), idx.data_ptr(), w.data_ptr(), T, *self._weights(), self._epoch(CH_DISPATCH), self._epoch(CH_COMBINE),
+                            self.overlap, self.dedup_min_pairs, s)
+        if rc != 0:
+            raise RuntimeError(f"MoE layer launch failed ({rc})")
+        self.launches += 4
+        return self._out(T)
 
     def check_status(self) -> int:
         return int(self.st.status.item())
@@ -253,7 +256,7 @@ class EmulatedMoE(_MoEBase):
             return None, status
         for r in range(n):
             self._experts(self.states[r], *self.weights[r])
-        rc = _ops.moe_combine(cargs.data_ptr(), n, R, self.hidden, self.topk, self.el, CH_COMBINE, self.eheap.next_epoch(CH_COMBINE), timeout_ns, 0, s, 1)
+        rc = _ops.moe_combine(cargs.data_ptr(), n, R, self.hidden, self.topk, self.el, CH_COMBINE, self.eheap.next_epoch(CH_COMBINE), timeout_ns, 0, s)
         if rc != 0:
             raise RuntimeError(f"moe_combine launch failed ({rc})")
         torch.cuda.synchronize()

@@ -6,6 +6,14 @@ import ctypes
 import numpy as np
 
 
+def current_stream_handle() -> int:
+    """cudaStream_t of the calling thread's current stream on its current device, without building the Stream object (which
+    takes about as long as a kernel launch)."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 class _CudaBlob:
     """Minimal __cuda_array_interface__ provider for a raw device-visible address."""
 

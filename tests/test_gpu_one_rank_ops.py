@@ -1,0 +1,124 @@
+"""The operators on a heap of one rank, where they take their own ways: the MoE layer writes and gathers its rows directly, the layer
+epilogue runs without barriers. Sizes at the edges of the work split; against the PyTorch oracles."""
+import pytest
+
+from conftest import free_port
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def heap():
+    import torch
+
+    from memfabric_hybrid_b200.parallel.heap import SymmetricHeap
+
+    torch.cuda.set_device(0)
+    h = SymmetricHeap(0, 1, 0, 1 << 30, store_url=f"tcp://127.0.0.1:{free_port()}")
+    yield h
+    h.close()
+
+
+def _weights(E, H, I, seed):
+    import torch
+
+    from memfabric_hybrid_b200.ops import fp8_gemm as F
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    wg, wu = (torch.randn(E, I, H, generator=g, device="cuda") * H ** -0.5 for _ in range(2))
+    w2 = torch.randn(E, H, I, generator=g, device="cuda") * I ** -0.5
+    return F.quant_weight_mx_torch(F.interleave_gate_up(wg, wu)) + F.quant_weight_mx_torch(w2)
+
+
+def _check(out, ref):
+    scale = float(ref.abs().max()) + 1e-6
+    err = (out.float() - ref).abs()
+    # the bounds of the emulated-rank tests: a flipped e4m3 rounding of the intermediate moves single elements by a step
+    assert float(err.max()) <= 1e-1 * scale and float(err.mean()) <= 4e-3 * scale
+    assert float((err > 4e-2 * scale).float().mean()) < 1e-3
+
+
+# tokens: one, fewer and more than there are CTAs; hidden 128 (one block), 384 (three), 4096 (exactly one trip of a CTA), 4224 and 8320
+# (a second and a third trip); topk 1, 8 (one group) and 10 (a second group of pairs per token)
+@pytest.mark.parametrize("T,H,E,K,I", [(1, 128, 4, 2, 128), (3, 384, 8, 8, 128), (130, 512, 8, 1, 256), (700, 1024, 16, 8, 256), (40, 4096, 4, 4, 128),
+                                       (33, 4224, 4, 2, 128), (9, 8320, 4, 3, 128), (65, 512, 16, 10, 128), (64, 512, 16, 8, 384)])
+def test_moe_layer(heap, T, H, E, K, I):
+    import torch
+
+    from memfabric_hybrid_b200.ops.moe import FusedMoE, moe_reference, route
+
+    w = _weights(E, H, I, 3)
+    layer = FusedMoE(heap, T + 5, H, E, K, I, *w, capacity_factor=2.0)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    for turn in range(3):  # the scratch counters have to be clean for the next call, whatever its size
+        n = T if turn != 1 else max(1, T // 2)
+        x = torch.randn(n, H, generator=g, device="cuda").to(torch.bfloat16)
+        idx, tw = route(torch.randn(n, E, generator=g, device="cuda"), K)
+        out = layer(x, idx, tw)
+        assert layer.check_status() == 0
+        _check(out, moe_reference([x], [idx], [tw], [w], E, I)[0])
+        ref_call = out.clone()
+        layer.dispatch(x, idx, tw)  # the phases one by one give the same
+        layer.experts()
+        assert torch.equal(layer.combine(n), ref_call)
+    assert layer.launches == 3 * 8
+
+
+def test_moe_layer_skips_masked_pairs(heap):
+    """Pairs with expert -1 are not routed: their weight does not enter the sum, and tokens without any pair come out zero."""
+    import torch
+
+    from memfabric_hybrid_b200.ops.moe import FusedMoE, moe_reference, route
+
+    T, H, E, K, I = 50, 512, 8, 4, 128
+    w = _weights(E, H, I, 4)
+    layer = FusedMoE(heap, T, H, E, K, I, *w)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    idx, tw = route(torch.randn(T, E, generator=g, device="cuda"), K)
+    drop = torch.rand(T, K, generator=g, device="cuda") < 0.4
+    drop[7] = True
+    masked = torch.where(drop, torch.full_like(idx, -1), idx)
+    out = layer(x, masked, tw)
+    assert layer.check_status() == 0
+    _check(out, moe_reference([x], [idx], [torch.where(drop, torch.zeros_like(tw), tw)], [w], E, I)[0])
+    assert float(out[7].float().abs().max()) == 0.0
+
+
+def test_moe_overflow_is_reported_and_the_kernel_ends(heap):
+    """Everything goes to one expert of a layer whose receive buffer holds a fraction of it."""
+    import torch
+
+    from memfabric_hybrid_b200.ops.moe import FusedMoE
+
+    T, H, E, K, I = 1500, 256, 4, 2, 128
+    layer = FusedMoE(heap, T, H, E, K, I, *_weights(E, H, I, 5), capacity_factor=0.25)
+    x = torch.zeros(T, H, dtype=torch.bfloat16, device="cuda")
+    idx = torch.tensor([[0, 1]], dtype=torch.int32, device="cuda").repeat(T, 1)
+    layer(x, idx, torch.full((T, K), 0.5, device="cuda"))
+    assert layer.check_status() == 2  # MF_DEV_ERR_BOUNDS
+
+
+@pytest.mark.parametrize("T", [1, 7, 300, 4099])
+@pytest.mark.parametrize("H", [8, 2048, 4096, 4104, 8192, 16384])
+def test_epilogue(heap, T, H):
+    import torch
+
+    from memfabric_hybrid_b200.ops.allreduce import AllReduceRMSNorm, reference
+
+    if T * H > 300 * 16384 and H > 4104:
+        pytest.skip("heap space")
+    mark = heap._bump.used
+    ar = AllReduceRMSNorm(heap, T, H)
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    w = (1.0 + 0.1 * torch.randn(H, generator=g, device="cuda")).to(torch.bfloat16)
+    for n, with_res in ((T, True), (max(1, T // 2), False), (T, True)):
+        x = torch.randn(n, H, generator=g, device="cuda").to(torch.bfloat16)
+        res = torch.randn(n, H, generator=g, device="cuda").to(torch.bfloat16) if with_res else None
+        ar.x[:n].copy_(x)
+        out, h = ar(n, res, w)
+        ref_out, ref_h = reference([x], res, w, 1e-6)
+        assert out.shape == (n, H) and ar.check_status() == 0
+        assert torch.equal(h.float(), ref_h)  # one rounding of an exact sum of two bf16 numbers
+        torch.testing.assert_close(out.float(), ref_out, rtol=2 ** -7, atol=1e-6)  # bf16 rounding (2^-8) and 32-bit sums
+    heap._bump.used = mark
