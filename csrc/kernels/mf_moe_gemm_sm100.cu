@@ -4,15 +4,21 @@
 // fp32 scale per 128x128 block. The reference library has no GEMM (MoE is only named as a use case, README.md:53 of the
 // reference); the contract here is the DeepSeek-V3 block-scaled FFN of the workload definition.
 //
-// Mapping to the hardware, per CTA (one persistent CTA per SM, 320 threads):
-//   warp 0     TMA producer: cp.async.bulk.tensor 2-D loads of a 128x128-byte A tile and a 128x128-byte B tile per K-block
-//              into a 6-stage shared-memory ring (128-byte swizzle), completion on mbarriers. Loads are per-CTA, no multicast.
-//   warp 1     one elected thread issues tcgen05.mma.kind::f8f6f4 (M128 N128 K32, four per K-block) into one of four
-//              128-column TMEM accumulators (all 512 columns) and tcgen05.commit's to "stage free" and "partial ready" mbarriers.
-//   warps 2-9  read each K-block's partial product from TMEM (tcgen05.ld 32x32b, 64 columns per thread: warps 2-5 take the
-//              left half of the tile, warps 6-9 the right half), multiply by sa[row, kb] * sb[tile, kb] and add into fp32
-//              registers; the four TMEM buffers let the MMAs run up to three K-blocks ahead of this promotion. After the last
-//              K-block they apply the epilogue (plain, or SwiGLU on interleaved gate/up columns) and store bf16.
+// Mapping to the hardware, per CTA (one persistent CTA per SM; tiles of 128 x BN, BN = 256 or 128):
+//   warp 0     TMA producer: cp.async.bulk.tensor 2-D loads of a 128x128-byte A tile and a BNx128-byte B tile per K-block
+//              into a shared-memory ring (128-byte swizzle), completion on mbarriers. Loads are per-CTA, no multicast.
+//   warp 1     one elected thread issues tcgen05.mma.kind::f8f6f4 (M128, N = BN, K32, four per K-block) into one of 512 / BN
+//              TMEM accumulators (all 512 columns) and tcgen05.commit's to "stage free" and "partial ready" mbarriers.
+//   warps 4..  read each K-block's partial product from TMEM (tcgen05.ld 32x32b, 64 columns per thread: every four warps one
+//              64-column part of the tile), multiply by sa[row, kb] * sb[tile, kb] and add into fp32 registers (two columns per
+//              packed FMA) while the MMAs fill the other accumulators. After the last K-block they apply the epilogue (plain,
+//              or SwiGLU on interleaved gate/up columns) and store bf16.
+//   warps 2-3  bring the products sa * sb of four K-blocks at a time into a ring of two such groups, one group ahead and across
+//              tiles: a row's scales are a line of their own for every thread, and waiting for them once per K-block on the
+//              promotion path took longer than the MMAs. It also leaves the promotion threads few enough registers.
+// 8191 rows over 32 experts, SwiGLU GEMM N 4096 / K 7168: 486 -> 389 us; N 7168 / K 2048: 281 -> 215 us. What bounds it now: a partial
+// product is read from TMEM while the next one is made in the other accumulator, and the hand-over (commit, wait, load, arrive) is
+// not shorter than the MMAs of a K-block.
 // Tiles are enumerated on the device from group_offset/group_count (the host does not know the routing result), n fastest so
 // that concurrently running CTAs share an A tile and stream one expert's weights through L2.
 // Every mbarrier wait is bounded; on expiry the CTA sets *status, all roles drain and the CTA frees its TMEM and exits.
@@ -30,25 +36,37 @@ using namespace mf::sm100;
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 128;
-constexpr int kStages = 6;
-constexpr int kThreads = 320;
-constexpr int kAccBufs = 4;                      // TMEM accumulator buffers (128 columns each)
-constexpr int kEpiThreads = 256;                 // warps 2-9
-constexpr int kTileBytes = BM * BK;  // fp8: 16 KiB per operand tile
+constexpr int BM = 128, BK = 128;
+constexpr int HC = 64;               // columns per promotion thread
+constexpr int kTileBytes = BM * BK;  // fp8: 16 KiB of A per K-block
 constexpr int kMaxGroups = 256;
 constexpr uint32_t kTmemCols = 512;
 
+template <int BN>
+struct Cfg {
+    static constexpr int kStages = BN == 256 ? 4 : 6;
+    static constexpr int kAccBufs = (int)kTmemCols / BN;  // TMEM accumulator buffers
+    static constexpr int kEpiWarps = 4 * (BN / HC);       // warps 4 and up
+    static constexpr int kThreads = 128 + 32 * kEpiWarps;
+    static constexpr int kBTile = BN * BK;
+};
+
+template <int BN>
 struct SharedStorage {
-    alignas(1024) unsigned char a[kStages][kTileBytes];
-    alignas(1024) unsigned char b[kStages][kTileBytes];
-    uint64_t full[kStages];
-    uint64_t empty[kStages];
-    uint64_t tmemFull[kAccBufs];
-    uint64_t tmemEmpty[kAccBufs];
+    alignas(1024) unsigned char a[Cfg<BN>::kStages][kTileBytes];
+    alignas(1024) unsigned char b[Cfg<BN>::kStages][Cfg<BN>::kBTile];
+    float4 scale[2][BN / 128][BM];  // [group of four K-blocks][weight block][row]
+    uint64_t scaleFull[2];
+    uint64_t scaleEmpty[2];
+    uint64_t full[Cfg<BN>::kStages];
+    uint64_t empty[Cfg<BN>::kStages];
+    uint64_t tmemFull[Cfg<BN>::kAccBufs];
+    uint64_t tmemEmpty[Cfg<BN>::kAccBufs];
     uint32_t tmemBase;
     int abortFlag;
     int tilePrefix[kMaxGroups + 1];
+    int groupOffset[kMaxGroups];  // of the caller's tables: looked up for every tile by every role
+    int groupCount[kMaxGroups];
 };
 
 struct GemmParams {
@@ -59,40 +77,82 @@ struct GemmParams {
     const int *groupCount;
     int *status;
     int G, N, K, mode, outStride, rowsTotal;
+    int wideStores;  // out is 32-byte aligned: the epilogue stores whole sectors
+    int vecScales;   // the scales of four K-blocks of a row are one aligned 16-byte word
 };
+
+__device__ __forceinline__ uint32_t PackBf16(float lo, float hi)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// Sixteen bf16 of one row: one whole sector where the address allows it (the lanes of a warp store to 32 different rows).
+__device__ __forceinline__ void Store16(__nv_bfloat16 *o, const uint32_t (&pk)[8], bool wide)
+{
+    if (wide) {
+        StGlobal32B(o, pk);
+    } else {
+        reinterpret_cast<uint4 *>(o)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        reinterpret_cast<uint4 *>(o)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+    }
+}
+
+__device__ __forceinline__ uint64_t PackF32x2(float lo, float hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void UnpackF32x2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+// acc = a * b + acc on two floats at once, each as fmaf does it.
+__device__ __forceinline__ void FmaF32x2(uint64_t &acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 
 __device__ __forceinline__ float Silu(float x) { return x / (1.f + __expf(-x)); }
 
-__global__ void __launch_bounds__(kThreads, 1)
+template <int BN>
+__global__ void __launch_bounds__(Cfg<BN>::kThreads, 1)
 mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const GemmParams p)
 {
+    using C = Cfg<BN>;
     extern __shared__ unsigned char smemRaw[];
-    SharedStorage &s = *reinterpret_cast<SharedStorage *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
+    SharedStorage<BN> &s = *reinterpret_cast<SharedStorage<BN> *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KB = p.K / BK, NT = p.N / BN;
 
+    for (int g = threadIdx.x; g < p.G; g += C::kThreads) {
+        s.groupOffset[g] = p.groupOffset[g];
+        s.groupCount[g] = p.groupCount[g];
+        s.tilePrefix[g + 1] = ((s.groupCount[g] + BM - 1) / BM) * NT;
+    }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; i++) {
+        for (int i = 0; i < C::kStages; i++) {
             MbarInit(&s.full[i], 1);
             MbarInit(&s.empty[i], 1);
         }
-        for (int i = 0; i < kAccBufs; i++) {
+        for (int i = 0; i < C::kAccBufs; i++) {
             MbarInit(&s.tmemFull[i], 1);
-            MbarInit(&s.tmemEmpty[i], kEpiThreads / 32);  // one arrival per epilogue warp
+            MbarInit(&s.tmemEmpty[i], C::kEpiWarps);  // one arrival per promotion warp
+        }
+        for (int i = 0; i < 2; i++) {
+            MbarInit(&s.scaleFull[i], 2);
+            MbarInit(&s.scaleEmpty[i], C::kEpiWarps);
         }
         s.abortFlag = 0;
-        int acc = 0;
-        for (int g = 0; g < p.G; g++) {
-            s.tilePrefix[g] = acc;
-            acc += ((p.groupCount[g] + BM - 1) / BM) * NT;
-        }
-        s.tilePrefix[p.G] = acc;
         MbarInitFence();
         TmaPrefetchDesc(&tmapA);
         TmaPrefetchDesc(&tmapB);
     }
     if (warp == 0) {
         TmemAlloc(&s.tmemBase, kTmemCols);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int acc = 0;
+        s.tilePrefix[0] = 0;
+        for (int g = 0; g < p.G; g++) {
+            acc += s.tilePrefix[g + 1];
+            s.tilePrefix[g + 1] = acc;
+        }
     }
     TcFenceBefore();
     __syncthreads();
@@ -124,14 +184,14 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
             for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x) {
                 int g, mt, nt;
                 decode(tile, g, mt, nt);
-                const int rowA = p.groupOffset[g] + mt * BM;
+                const int rowA = s.groupOffset[g] + mt * BM;
                 const int rowB = g * p.N + nt * BN;
                 for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % kStages, ph = (it / kStages) & 1;
+                    const uint32_t st = it % C::kStages, ph = (it / C::kStages) & 1;
                     if (!MbarWaitBounded(&s.empty[st], ph ^ 1, abortFlag)) {
                         break;
                     }
-                    MbarExpectTx(&s.full[st], 2 * kTileBytes);
+                    MbarExpectTx(&s.full[st], kTileBytes + C::kBTile);
                     TmaLoad2D(s.a[st], &tmapA, &s.full[st], kb * BK, rowA);
                     TmaLoad2D(s.b[st], &tmapB, &s.full[st], kb * BK, rowB);
                 }
@@ -144,8 +204,8 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x) {
                 for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % kStages, ph = (it / kStages) & 1;
-                    const uint32_t buf = it % kAccBufs, bph = (it / kAccBufs) & 1;
+                    const uint32_t st = it % C::kStages, ph = (it / C::kStages) & 1;
+                    const uint32_t buf = it % C::kAccBufs, bph = (it / C::kAccBufs) & 1;
                     if (!MbarWaitBounded(&s.tmemEmpty[buf], bph ^ 1, abortFlag) || !MbarWaitBounded(&s.full[st], ph, abortFlag)) {
                         break;
                     }
@@ -163,85 +223,175 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
                 }
             }
         }
-    } else {
-        // ------------------------------------------------------------------ promotion + epilogue (8 warps: one row, 64 columns per thread)
-        const int quad = warp & 3;          // TMEM lanes this warp may touch: 32*quad .. 32*quad+31
-        const int half = (warp - 2) >> 2;   // 0: tile columns [0,64), 1: [64,128)
-        const int rowInTile = quad * 32 + lane;
-        constexpr int HC = BN / 2;
-        uint32_t it = 0;
-        for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x) {
+    } else if (warp < 4) {
+        // ------------------------------------------------------------------ scales: a work item is a tile and four of its K-blocks
+        const int row0 = (warp - 2) * (BM / 2) + lane;  // and row0 + 32
+        struct Words {
+            float a[2][4], b[BN / 128][4];
+        };
+        auto load4 = [&](const float *src, int kb0, bool valid, float (&f)[4]) {
+            if (p.vecScales) {
+                const float4 q = valid ? *reinterpret_cast<const float4 *>(src + kb0) : make_float4(0.f, 0.f, 0.f, 0.f);
+                f[0] = q.x;
+                f[1] = q.y;
+                f[2] = q.z;
+                f[3] = q.w;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    f[k] = valid && kb0 + k < KB ? src[kb0 + k] : 0.f;
+                }
+            }
+        };
+        auto fetch = [&](int tile, int kb0, Words &w) {
             int g, mt, nt;
             decode(tile, g, mt, nt);
-            const int row = p.groupOffset[g] + mt * BM + rowInTile;
-            // Rows past the end of A (group tables that overrun the buffer) are never read or written.
-            const bool valid = mt * BM + rowInTile < p.groupCount[g] && row < p.rowsTotal;
-            const float *sa = p.aScale + (size_t)row * KB;
-            const float *sb = p.bScale + ((size_t)g * NT + nt) * KB;
-            float acc[HC];
 #pragma unroll
-            for (int i = 0; i < HC; i++) {
-                acc[i] = 0.f;
+            for (int j = 0; j < 2; j++) {
+                const int rowInTile = row0 + 32 * j;
+                const int row = s.groupOffset[g] + mt * BM + rowInTile;
+                load4(p.aScale + (size_t)row * KB, kb0, mt * BM + rowInTile < s.groupCount[g] && row < p.rowsTotal, w.a[j]);
             }
-            float scaleNext = valid ? sa[0] * sb[0] : 0.f;
-            bool ok = true;
-            for (int kb = 0; kb < KB; kb++, it++) {
-                const uint32_t buf = it % kAccBufs, bph = (it / kAccBufs) & 1;
-                const float scale = scaleNext;
-                if (kb + 1 < KB) {
-                    scaleNext = valid ? sa[kb + 1] * sb[kb + 1] : 0.f;
+#pragma unroll
+            for (int c = 0; c < BN / 128; c++) {
+                load4(p.bScale + ((size_t)g * (p.N / 128) + (size_t)(nt * (BN / 128) + c)) * KB, kb0, true, w.b[c]);
+            }
+        };
+        Words cur, nxt;
+        uint32_t it = 0;
+        int tile = blockIdx.x, kb0 = 0;
+        bool have = tile < totalTiles;
+        if (have) {
+            fetch(tile, kb0, cur);
+        }
+        for (; have && *abortFlag == 0; it++) {
+            const int tileN = kb0 + 4 < KB ? tile : tile + (int)gridDim.x, kbN = kb0 + 4 < KB ? kb0 + 4 : 0;
+            const bool haveNext = tileN < totalTiles;
+            if (haveNext) {
+                fetch(tileN, kbN, nxt);
+            }
+            const uint32_t buf = it & 1, ph = (it >> 1) & 1;
+            if (!MbarWaitBounded(&s.scaleEmpty[buf], ph ^ 1, abortFlag)) {
+                break;
+            }
+#pragma unroll
+            for (int c = 0; c < BN / 128; c++) {
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    s.scale[buf][c][row0 + 32 * j] = make_float4(cur.a[j][0] * cur.b[c][0], cur.a[j][1] * cur.b[c][1], cur.a[j][2] * cur.b[c][2],
+                                                                 cur.a[j][3] * cur.b[c][3]);
                 }
+            }
+            __syncwarp();
+            if (lane == 0) {
+                MbarArrive(&s.scaleFull[buf]);
+            }
+            cur = nxt;
+            tile = tileN;
+            kb0 = kbN;
+            have = haveNext;
+        }
+    } else {
+        // ------------------------------------------------------------------ promotion + epilogue (one row, 64 columns per thread)
+        const int quad = warp & 3;         // TMEM lanes this warp may touch: 32*quad .. 32*quad+31
+        const int part = (warp - 4) >> 2;  // tile columns [64 * part, 64 * part + 64)
+        const int rowInTile = quad * 32 + lane;
+        uint64_t acc2[HC / 2];  // two fp32 sums each
+#pragma unroll
+        for (int i = 0; i < HC / 2; i++) {
+            acc2[i] = 0;
+        }
+        uint32_t it = 0, item = 0;
+        int tile = blockIdx.x, kb0 = 0;
+        while (tile < totalTiles && *abortFlag == 0) {
+            if (!MbarWaitBounded(&s.scaleFull[item & 1], (item >> 1) & 1, abortFlag)) {
+                break;
+            }
+            float4 scale = s.scale[item & 1][part / 2][rowInTile];
+            __syncwarp();
+            if (lane == 0) {
+                MbarArrive(&s.scaleEmpty[item & 1]);
+            }
+            item++;
+            const int n = min(4, KB - kb0);
+            bool ok = true;
+#pragma unroll 1
+            for (int k = 0; k < n; k++, it++) {
+                const uint32_t buf = it % C::kAccBufs, bph = (it / C::kAccBufs) & 1;
                 if (!MbarWaitBounded(&s.tmemFull[buf], bph, abortFlag)) {
                     ok = false;
                     break;
                 }
                 TcFenceAfter();
-                const uint32_t taddr = tmemBase + ((uint32_t)(quad * 32) << 16) + buf * BN + half * HC;
-                float v[HC];
-                TmemLd32Issue(taddr, v);
-                TmemLd32Issue(taddr + 32, v + 32);
-                TmemLdWait();
-                TcFenceBefore();
-                __syncwarp();
-                if (lane == 0) {
-                    MbarArrive(&s.tmemEmpty[buf]);  // the warp's values are in registers: one arrival per warp keeps the barrier cheap
-                }
+                const uint32_t taddr = tmemBase + ((uint32_t)(quad * 32) << 16) + buf * BN + part * HC;
+                const uint64_t sc = PackF32x2(scale.x, scale.x);
 #pragma unroll
-                for (int i = 0; i < HC; i++) {
-                    acc[i] = fmaf(v[i], scale, acc[i]);
+                for (int c = 0; c < HC; c += 16) {
+                    float v[16];
+                    TmemLd16Issue(taddr + c, v);
+                    TmemLdWait16(v);
+                    if (c == HC - 16) {
+                        TcFenceBefore();
+                        __syncwarp();
+                        if (lane == 0) {
+                            MbarArrive(&s.tmemEmpty[buf]);  // the warp's values are in registers: one arrival per warp keeps the barrier cheap
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        FmaF32x2(acc2[(c + i) / 2], PackF32x2(v[i], v[i + 1]), sc);
+                    }
                 }
+                scale = make_float4(scale.y, scale.z, scale.w, 0.f);
             }
             if (!ok) {
                 break;
             }
-            if (valid) {
-                if ((p.mode & 15) == MF_GEMM_EPI_SWIGLU) {
-                    // Each 64-column half of the tile holds 32 gate projections followed by the 32 matching up projections.
-                    __nv_bfloat16 *o = p.out + (size_t)row * p.outStride + nt * (BN / 2) + half * (HC / 2);
+            kb0 += 4;
+            if (kb0 >= KB) {
+                int g, mt, nt;
+                decode(tile, g, mt, nt);
+                const int row = s.groupOffset[g] + mt * BM + rowInTile;
+                // Rows past the end of A (group tables that overrun the buffer) are never read or written.
+                if (mt * BM + rowInTile < s.groupCount[g] && row < p.rowsTotal) {
+                    float acc[HC];
 #pragma unroll
-                    for (int j = 0; j < HC / 2; j += 8) {
-                        uint4 pk;
-                        __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            h[q] = __floats2bfloat162_rn(Silu(acc[j + 2 * q]) * acc[HC / 2 + j + 2 * q],
-                                                         Silu(acc[j + 2 * q + 1]) * acc[HC / 2 + j + 2 * q + 1]);
-                        }
-                        *reinterpret_cast<uint4 *>(o + j) = pk;
+                    for (int i = 0; i < HC; i += 2) {
+                        UnpackF32x2(acc2[i / 2], acc[i], acc[i + 1]);
                     }
-                } else {
-                    __nv_bfloat16 *o = p.out + (size_t)row * p.outStride + nt * BN + half * HC;
+                    const int col = nt * BN + part * HC;
+                    const bool swiglu = (p.mode & 15) == MF_GEMM_EPI_SWIGLU;
+                    __nv_bfloat16 *o = p.out + (size_t)row * p.outStride + (swiglu ? col / 2 : col);
+                    if (swiglu) {
+                        // Every 64 columns hold 32 gate projections followed by the 32 matching up projections.
 #pragma unroll
-                    for (int j = 0; j < HC; j += 8) {
-                        uint4 pk;
-                        __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
+                        for (int j = 0; j < HC / 2; j += 16) {
+                            uint32_t pk[8];
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            h[q] = __floats2bfloat162_rn(acc[j + 2 * q], acc[j + 2 * q + 1]);
+                            for (int q = 0; q < 8; q++) {
+                                const int c = j + 2 * q;
+                                pk[q] = PackBf16(Silu(acc[c]) * acc[HC / 2 + c], Silu(acc[c + 1]) * acc[HC / 2 + c + 1]);
+                            }
+                            Store16(o + j, pk, p.wideStores);
                         }
-                        *reinterpret_cast<uint4 *>(o + j) = pk;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < HC; j += 16) {
+                            uint32_t pk[8];
+#pragma unroll
+                            for (int q = 0; q < 8; q++) {
+                                pk[q] = PackBf16(acc[j + 2 * q], acc[j + 2 * q + 1]);
+                            }
+                            Store16(o + j, pk, p.wideStores);
+                        }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < HC / 2; i++) {
+                    acc2[i] = 0;
+                }
+                tile += gridDim.x;
+                kb0 = 0;
             }
         }
     }
@@ -259,55 +409,77 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
 
 // ---------------------------------------------------------------------------------------------- row quantisation (bf16 → fp8, 1x128 scales)
 
-__global__ void mf_quant_rows_fp8_kernel(const __nv_bfloat16 *__restrict__ x, unsigned char *__restrict__ q, float *__restrict__ scale, int rows, int K,
-                                         const int *__restrict__ rowLimit)
+// x / sc as IEEE division rounds it, from rcp = the rounded 1 / sc: with FMAs one correction step of the product is enough
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990). Needs 0 < sc < infinity and
+// a normal rcp; where the correction underflows, the quotient is far below the smallest e4m3 value.
+__device__ __forceinline__ float DivByRcp(float x, float sc, float rcp)
 {
-    // One warp per (row, group of 256 elements): lanes 0-15 and 16-31 each own one 128-element block, 8 elements per lane.
-    const int warpsPerBlock = blockDim.x >> 5;
+    const float q = x * rcp;
+    return q == 0.f ? q : fmaf(fmaf(-q, sc, x), rcp, q);  // the sum would lose the sign of a zero
+}
+
+constexpr int kQuantUnroll = 4;
+
+// Bound by DRAM: 12288 x 7168 in 57 us = 4.6 TB/s (96 us with one load in flight and divisions). K is a multiple of 128, so the rows are one sequence of 128-element blocks; sixteen lanes own a block, eight elements
+// each, and a warp takes 2 x kQuantUnroll consecutive blocks at once so that four 16-byte loads per lane are in flight.
+__global__ void __launch_bounds__(256) mf_quant_rows_fp8_kernel(const __nv_bfloat16 *__restrict__ x, unsigned char *__restrict__ q,
+                                                                float *__restrict__ scale, int rows, int blocksPerRow, const int *__restrict__ rowLimit)
+{
     const int lane = threadIdx.x & 31;
-    const int blocksPerRow = K / 128;
-    const int pairsPerRow = (blocksPerRow + 1) / 2;
-    const long long totalPairs = (long long)rows * pairsPerRow;
-    const int limit = rowLimit != nullptr ? *rowLimit : rows;
-    for (long long pr = (long long)blockIdx.x * warpsPerBlock + (threadIdx.x >> 5); pr < totalPairs; pr += (long long)gridDim.x * warpsPerBlock) {
-        const int row = (int)(pr / pairsPerRow);
-        if (row >= limit) {
-            continue;
-        }
-        // With an odd number of blocks per row the upper half-warp has no block in the last pair; it walks through the same
-        // instructions on a zero vector so that the full-mask shuffles below stay convergent.
-        const int blk = (int)(pr % pairsPerRow) * 2 + (lane >> 4);
-        const bool active = blk < blocksPerRow;
-        const size_t off = (size_t)row * K + (size_t)(active ? blk : 0) * 128 + (lane & 15) * 8;
-        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-        if (active) {
-            raw = *reinterpret_cast<const uint4 *>(x + off);
-        }
-        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw);
-        float f[8];
-        float amax = 0.f;
+    const int limit = rowLimit != nullptr ? min(*rowLimit, rows) : rows;
+    const long long total = (long long)limit * blocksPerRow;
+    constexpr int kStep = 2 * kQuantUnroll;
+    for (long long b0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kStep; b0 < total;
+         b0 += (long long)gridDim.x * (blockDim.x >> 5) * kStep) {
+        const long long first = b0 + (lane >> 4);
+        uint4 raw[kQuantUnroll];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float2 t = __bfloat1622float2(h[i]);
-            f[2 * i] = t.x;
-            f[2 * i + 1] = t.y;
-            amax = fmaxf(amax, fmaxf(fabsf(t.x), fabsf(t.y)));
+        for (int u = 0; u < kQuantUnroll; u++) {
+            raw[u] = make_uint4(0u, 0u, 0u, 0u);  // past the end: a zero vector, so that the full-mask shuffles below stay convergent
+            if (first + 2 * u < total) {
+                raw[u] = *reinterpret_cast<const uint4 *>(x + (first + 2 * u) * 128 + (lane & 15) * 8);
+            }
         }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        }
-        const float sc = fmaxf(amax, 1e-10f) * (1.f / 448.f);
-        uint2 packed;
-        unsigned short *ps = reinterpret_cast<unsigned short *>(&packed);
+        for (int u = 0; u < kQuantUnroll; u++) {
+            const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[u]);
+            float f[8];
+            float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            ps[i] = __nv_cvt_float2_to_fp8x2(make_float2(f[2 * i] / sc, f[2 * i + 1] / sc), __NV_SATFINITE, __NV_E4M3);
-        }
-        if (active) {
-            *reinterpret_cast<uint2 *>(q + off) = packed;
-            if ((lane & 15) == 0) {
-                scale[(size_t)row * blocksPerRow + blk] = sc;
+            for (int i = 0; i < 4; i++) {
+                float2 t = __bfloat1622float2(h[i]);
+                f[2 * i] = t.x;
+                f[2 * i + 1] = t.y;
+                amax = fmaxf(amax, fmaxf(fabsf(t.x), fabsf(t.y)));
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            }
+            const float sc = fmaxf(amax, 1e-10f) * (1.f / 448.f);
+            if (sc < __int_as_float(0x7f800000)) {
+                const float rcp = 1.f / sc;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    f[i] = DivByRcp(f[i], sc, rcp);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    f[i] = f[i] / sc;
+                }
+            }
+            uint2 packed;
+            unsigned short *ps = reinterpret_cast<unsigned short *>(&packed);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                ps[i] = __nv_cvt_float2_to_fp8x2(make_float2(f[2 * i], f[2 * i + 1]), __NV_SATFINITE, __NV_E4M3);
+            }
+            if (first + 2 * u < total) {
+                *reinterpret_cast<uint2 *>(q + (first + 2 * u) * 128 + (lane & 15) * 8) = packed;
+                if ((lane & 15) == 0) {
+                    scale[first + 2 * u] = sc;
+                }
             }
         }
     }
@@ -330,8 +502,8 @@ EncodeTiledFn GetEncodeTiled()
     return fn;
 }
 
-// [rows, K] uint8 row-major, boxes of 128 (K) x 128 (rows), 128-byte swizzle.
-bool MakeMap(CUtensorMap *m, const void *base, uint64_t rows, uint64_t K)
+// [rows, K] uint8 row-major, boxes of 128 (K) x boxRows, 128-byte swizzle.
+bool MakeMap(CUtensorMap *m, const void *base, uint64_t rows, uint64_t K, uint32_t boxRows)
 {
     EncodeTiledFn enc = GetEncodeTiled();
     if (enc == nullptr) {
@@ -339,10 +511,35 @@ bool MakeMap(CUtensorMap *m, const void *base, uint64_t rows, uint64_t K)
     }
     cuuint64_t dims[2] = {K, rows};
     cuuint64_t strides[1] = {K};
-    cuuint32_t box[2] = {BK, BM};
+    cuuint32_t box[2] = {BK, boxRows};
     cuuint32_t estr[2] = {1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN>
+int Launch(const void *a, const void *b, const GemmParams &p, int ctas, cudaStream_t stream)
+{
+    CUtensorMap mapA, mapB;
+    if (!MakeMap(&mapA, a, (uint64_t)p.rowsTotal, (uint64_t)p.K, BM) || !MakeMap(&mapB, b, (uint64_t)p.G * p.N, (uint64_t)p.K, BN)) {
+        return MF_K_LAUNCH_FAILED;
+    }
+    static bool attrSet = false;
+    const size_t smem = sizeof(SharedStorage<BN>) + 1024;
+    if (!attrSet) {
+        if (cudaFuncSetAttribute(mf_moe_grouped_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return MF_K_LAUNCH_FAILED;
+        }
+        attrSet = true;
+    }
+    const int sms = mf_k_sm_count();
+    if (sms <= 0) {
+        return MF_K_LAUNCH_FAILED;
+    }
+    const int grid = ctas > 0 && ctas < sms ? ctas : sms;
+    mf_moe_grouped_gemm_kernel<BN><<<grid, Cfg<BN>::kThreads, smem, stream>>>(mapA, mapB, p);
+    return cudaGetLastError() == cudaSuccess ? MF_K_OK : MF_K_LAUNCH_FAILED;
 }
 
 }  // namespace
@@ -351,15 +548,11 @@ extern "C" int mf_k_moe_grouped_gemm(const void *a, const float *aScale, const v
                                      const int *groupCount, int G, int rowsTotal, int N, int K, int mode, int *status, int ctas, mf_stream_t stream)
 {
     if (a == nullptr || b == nullptr || out == nullptr || aScale == nullptr || bScale == nullptr || groupOffset == nullptr || groupCount == nullptr ||
-        G < 1 || G > kMaxGroups || rowsTotal < 1 || N % BN != 0 || K % BK != 0 || N <= 0 || K <= 0) {
+        G < 1 || G > kMaxGroups || rowsTotal < 1 || N % 128 != 0 || K % BK != 0 || N <= 0 || K <= 0) {
         return MF_K_INVALID;
     }
     if (((uintptr_t)a & 15) || ((uintptr_t)b & 15) || ((uintptr_t)out & 15)) {
         return MF_K_INVALID;  // TMA base addresses and the 16-byte epilogue stores need 16-byte alignment
-    }
-    CUtensorMap mapA, mapB;
-    if (!MakeMap(&mapA, a, (uint64_t)rowsTotal, (uint64_t)K) || !MakeMap(&mapB, b, (uint64_t)G * N, (uint64_t)K)) {
-        return MF_K_LAUNCH_FAILED;
     }
     if (ctas < 0) {
         ctas = 0;
@@ -377,22 +570,14 @@ extern "C" int mf_k_moe_grouped_gemm(const void *a, const float *aScale, const v
     p.mode = mode;
     p.outStride = (mode & 15) == MF_GEMM_EPI_SWIGLU ? N / 2 : N;
     p.rowsTotal = rowsTotal;
-    static bool attrSet = false;
-    const size_t smem = sizeof(SharedStorage) + 1024;
-    if (!attrSet) {
-        if (cudaFuncSetAttribute(mf_moe_grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return MF_K_LAUNCH_FAILED;
-        }
-        attrSet = true;
-    }
-    int sms = mf_k_sm_count();
-    if (sms <= 0) {
-        return MF_K_LAUNCH_FAILED;
-    }
-    int grid = ctas > 0 && ctas < sms ? ctas : sms;
-    mf_moe_grouped_gemm_kernel<<<grid, kThreads, smem, (cudaStream_t)stream>>>(mapA, mapB, p);
-    return cudaGetLastError() == cudaSuccess ? MF_K_OK : MF_K_LAUNCH_FAILED;
+    p.wideStores = ((uintptr_t)out & 31) == 0 ? 1 : 0;
+    p.vecScales = (K / BK) % 4 == 0 && ((uintptr_t)aScale & 15) == 0 && ((uintptr_t)bScale & 15) == 0 ? 1 : 0;
+    // The wide tile reads A half as often and hands a partial product over half as often: one K-block takes 1050 cycles instead of
+    // 2 x 720. It pays from two m-tiles per expert on if every SM still gets two tiles (8191 rows over 32 experts, N 4096 / K 7168: 389
+    // against 455 us); below that the weights' stream is what counts and the finer tiles end more evenly (2048 rows: 201 against 197 us).
+    const long long mTiles = (rowsTotal + BM - 1) / BM;
+    const bool wide = N % 256 == 0 && mTiles >= 2LL * G && mTiles * (N / 256) >= 2LL * 148;
+    return wide ? Launch<256>(a, b, p, ctas, (cudaStream_t)stream) : Launch<128>(a, b, p, ctas, (cudaStream_t)stream);
 }
 
 extern "C" int mf_k_quant_rows_fp8(const void *x, void *q, float *scale, int rows, int K, const int *rowLimit, mf_stream_t stream)
@@ -400,11 +585,11 @@ extern "C" int mf_k_quant_rows_fp8(const void *x, void *q, float *scale, int row
     if (x == nullptr || q == nullptr || scale == nullptr || rows < 1 || K % 128 != 0) {
         return MF_K_INVALID;
     }
-    long long pairs = (long long)rows * ((K / 128 + 1) / 2);
-    long long blocks = (pairs + 7) / 8;
+    const long long perCta = 8LL * 2 * kQuantUnroll;  // eight warps
+    long long blocks = ((long long)rows * (K / 128) + perCta - 1) / perCta;
     if (blocks > 148 * 16) {
         blocks = 148 * 16;
     }
-    mf_quant_rows_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x, (unsigned char *)q, scale, rows, K, rowLimit);
+    mf_quant_rows_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x, (unsigned char *)q, scale, rows, K / 128, rowLimit);
     return cudaGetLastError() == cudaSuccess ? MF_K_OK : MF_K_LAUNCH_FAILED;
 }

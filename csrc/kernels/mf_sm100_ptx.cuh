@@ -146,6 +146,15 @@ __device__ __forceinline__ void TmemLd16Issue(uint32_t taddr, float *v)
         : "memory");
 }
 __device__ __forceinline__ void TmemLdWait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The same with the 16 values of TmemLd16Issue as operands, which keeps their uses behind the wait.
+__device__ __forceinline__ void TmemLdWait16(float *v)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
+                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
+                 :
+                 : "memory");
+}
 
 // 32 consecutive fp32 columns of this thread's TMEM lane, waited for.
 __device__ __forceinline__ void TmemLd32(uint32_t taddr, float *v)

@@ -261,3 +261,57 @@ def test_packed_weights_give_the_same_result(tile_n, N):
         for r, o in pairs:
             for off, n in zip(offs.tolist(), cnts.tolist()):
                 assert torch.equal(r[off:off + n].view(torch.uint8), o[off:off + n].view(torch.uint8))
+
+
+# The wide tile (two m-tiles per expert and two tiles per SM at least): K of one, five and eight 128-blocks, i.e. a scale group that is cut
+# short and whole ones; ragged and empty groups. `shift` moves the scales off 16 bytes and the result off 32.
+@pytest.mark.parametrize("K,shift", [(128, False), (640, False), (1024, False), (1024, True)])
+@pytest.mark.parametrize("mode", ["bf16", "swiglu"])
+def test_grouped_gemm_wide_tile(K, shift, mode):
+    import torch
+
+    from memfabric_hybrid_b200.ops import fp8_gemm as F
+
+    counts, N, dev = [1300, 0, 1, 129, 2047], 2816, "cuda"
+    offs, cnts, rows = _groups(counts, dev)
+    assert rows // 128 >= 2 * len(counts) and rows // 128 * (N // 256) >= 2 * 148
+    g = torch.Generator(device=dev).manual_seed(K)
+    a_q, a_s = F.quant_act_torch(torch.randn(rows, K, generator=g, device=dev))
+    w_q, w_s = F.quant_weight_torch(torch.randn(len(counts), N, K, generator=g, device=dev) * 0.05)
+    n_out = N // 2 if mode == "swiglu" else N
+    flat = torch.full((rows * n_out + 8,), float("nan"), dtype=torch.bfloat16, device=dev)
+    out = (flat[8:] if shift else flat[:-8]).view(rows, n_out)
+    if shift:
+        a_s, w_s = (torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape) for t in (a_s, w_s))
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    F.grouped_gemm(a_q, a_s, w_q, w_s, offs, cnts, mode=mode, out=out, status=status)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    ref = F.grouped_gemm_reference(a_q, a_s, w_q, w_s, offs, cnts, mode=mode)
+    for o, n, end in zip(offs.tolist(), counts, offs.tolist()[1:]):
+        # fp32 sums, one rounding to bf16 (2^-9 of the value) and what the sums lose where they cancel (2^-20 of the largest)
+        torch.testing.assert_close(out[o:o + n].float(), ref[o:o + n], rtol=2 ** -8, atol=2 ** -14 * float(ref.abs().max()))
+        assert bool(torch.isnan(out[o + n:end]).all())  # padding rows are never written
+
+
+# One block, a cut last trip of a warp (eight blocks) and several trips; row limits inside and outside of the buffer.
+@pytest.mark.parametrize("rows,K", [(1, 128), (3, 384), (17, 128), (700, 4096), (4001, 2048)])
+def test_quant_rows_is_the_rounded_quotient(rows, K):
+    import torch
+
+    from memfabric_hybrid_b200.ops import fp8_gemm as F
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randint(-2 ** 15, 2 ** 15, (rows, K), generator=g, device="cuda").to(torch.int16).view(torch.bfloat16)  # all exponents and signed zeros
+    x = torch.where(torch.isfinite(x), x, torch.full_like(x, -0.0))
+    x[:: 3] = torch.randn(x[:: 3].shape, generator=g, device="cuda").to(torch.bfloat16)
+    xb = x.float().view(rows, K // 128, 128)
+    sc = xb.abs().amax(-1).clamp_min(1e-10) * torch.tensor(1.0 / 448.0, dtype=torch.float32, device="cuda")
+    ref = (xb.double() / sc.double().unsqueeze(-1)).float().clamp(-448, 448).to(torch.float8_e4m3fn).view(rows, K).view(torch.uint8)
+    for limit in (None, 0, max(1, rows // 2), rows + 5):
+        n = rows if limit is None else min(rows, limit)
+        q = torch.full((rows, K), 85, dtype=torch.uint8, device="cuda")
+        s = torch.full((rows, K // 128), -1.0, device="cuda")
+        F.quant_rows_fp8(x, q, s, row_limit=None if limit is None else torch.tensor([limit], dtype=torch.int32, device="cuda"))
+        assert torch.equal(q[:n], ref[:n]) and torch.equal(s[:n], sc[:n])
+        assert bool((q[n:] == 85).all()) and bool((s[n:] == -1).all())
