@@ -106,9 +106,10 @@ class AllReduceRMSNorm:
         self.launches += 1
         if self.double_buffer:
             self._cur = 1 - self._cur
-        if self._results[0] != tokens:
-            self._results = (tokens, (self.out[:tokens], self.residual_out[:tokens]))
-        return self._results[1]
+        res = self._results
+        if res[0] != tokens:
+            res = self._results = (tokens, (self.out[:tokens], self.residual_out[:tokens]))
+        return res[1]
 
     def check_status(self) -> int:
         """Synchronises and returns the device status word (0 = fine, else MF_DEV_ERR_* | peer << 8)."""

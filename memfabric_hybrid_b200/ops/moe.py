@@ -141,20 +141,20 @@ class FusedMoE(_MoEBase):
                                   st.h1_sf.data_ptr(), st.y.data_ptr(), st.ret_y.data_ptr(), st.out.data_ptr(), st.cap, st.max_rows_ret, heap.world, hidden,
                                   topk, n_experts, inter, CH_DISPATCH, CH_COMBINE, timeout_ns, self.wait_ns,
                                   self._epoch_d.data_ptr() if device_epochs else 0, self._epoch_c.data_ptr() if device_epochs else 0)
-        self._weights_checked = None
         self._result = (max_tokens, st.out)
+        self._weight_shapes = [((self.el, n, k), (self.el, n // 32, k // 128, 32, 128), (self.el, n // 128, k // 128))
+                               for n, k in ((2 * inter, hidden), (hidden, inter))]
         torch.cuda.synchronize()
         heap.barrier()  # everybody's count matrix is zeroed before the first dispatch touches it
 
     def _weights(self):
-        """(address, scales' address, packed) of both projections. Shapes are looked at when a tensor is another than last time."""
-        t = (self.w13_q, self.w13_s, self.w2_q, self.w2_s)
-        if self._weights_checked is None or any(a is not b for a, b in zip(t, self._weights_checked)):
-            for q, s, n, k in ((t[0], t[1], 2 * self.inter, self.hidden), (t[2], t[3], self.hidden, self.inter)):
-                shape = (self.el, n // 32, k // 128, 32, 128) if q.dim() == 5 else (self.el, n, k)
-                assert tuple(q.shape) == shape and tuple(s.shape) == (self.el, n // 128, k // 128) and q.is_contiguous() and s.is_contiguous()
-            self._weights_checked = t
-        return t[0].data_ptr(), t[1].data_ptr(), int(t[0].dim() == 5), t[2].data_ptr(), t[3].data_ptr(), int(t[2].dim() == 5)
+        """(address, scales' address, packed) of both projections."""
+        out = []
+        for q, sc, (plain, blocks, scales) in ((self.w13_q, self.w13_s, self._weight_shapes[0]), (self.w2_q, self.w2_s, self._weight_shapes[1])):
+            packed = q.dim() == 5
+            assert q.shape == (blocks if packed else plain) and sc.shape == scales and q.is_contiguous() and sc.is_contiguous()
+            out += (q.data_ptr(), sc.data_ptr(), int(packed))
+        return out
 
     def _epoch(self, channel):
         return 0 if self.device_epochs else self.heap.next_epoch(channel)
@@ -183,9 +183,10 @@ class FusedMoE(_MoEBase):
         return self._out(T)
 
     def _out(self, T):
-        if self._result[0] != T:
-            self._result = (T, self.st.out[:T])
-        return self._result[1]
+        res = self._result
+        if res[0] != T:
+            res = self._result = (T, self.st.out[:T])
+        return res[1]
 
     def __call__(self, x, idx, w, stream=None):
         T = x.shape[0]

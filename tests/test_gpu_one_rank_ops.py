@@ -85,6 +85,21 @@ def test_moe_layer_skips_masked_pairs(heap):
     assert float(out[7].float().abs().max()) == 0.0
 
 
+def test_moe_layer_looks_at_its_weights_on_every_call(heap):
+    import torch
+
+    from memfabric_hybrid_b200.ops.moe import FusedMoE, route
+
+    T, H, E, K, I = 4, 256, 4, 2, 128
+    layer = FusedMoE(heap, T, H, E, K, I, *_weights(E, H, I, 6))
+    x = torch.ones(T, H, dtype=torch.bfloat16, device="cuda")
+    idx, tw = route(torch.randn(T, E, device="cuda"), K)
+    layer(x, idx, tw)
+    layer.w2_s.unsqueeze_(0)  # the same tensor, but no longer of the expected shape
+    with pytest.raises(AssertionError):
+        layer(x, idx, tw)
+
+
 def test_moe_overflow_is_reported_and_the_kernel_ends(heap):
     """Everything goes to one expert of a layer whose receive buffer holds a fraction of it."""
     import torch
