@@ -3,11 +3,9 @@
 // Each CTA brings 128 rows of A and 128 of the tile's 256 weight rows into its own shared memory and the tensor cores of both
 // SMs read both halves, so a K block costs each SM 32 KiB of operand traffic instead of the 48 KiB of the one-SM 128 x 256 tile:
 // one third less shared-memory fill per FLOP, and a ring of six stages instead of four in the same shared memory, i.e. more K
-// blocks in flight to cover the latency of L2 and DRAM. The one-SM kernel keeps the tensor pipe about 60 % busy with L2, DRAM
-// and the TMA unit all below 40 % of their peaks; the fill latency, not a throughput limit, paces it. Measured, the pair's longer
-// hand-shakes (commit to both CTAs, byte counts and arrivals crossing to the leader) cost what the deeper ring gains: 0.89 ms
-// against 0.83 ms for the one-SM kernel on the first FFN GEMM of the benchmark, equal on the second; the one-SM kernel stays
-// the default.
+// blocks in flight to cover the latency of L2 and DRAM. Measured, a K block takes 720 cycles, most of the wait being for scale
+// factors, against 600 of the one-SM kernel, and tiles of 256 rows pad more: 890 us against 840 us on the first FFN GEMM of
+// the benchmark, 530 against 470 us on the second; the one-SM kernel stays the default.
 //
 // Roles per CTA (384 threads): warp 0 TMA producer (per-CTA tiled loads, no multicast, completing on the LEADER's "full"
 // barrier), warp 2 scale-factor producer (this CTA's 128 A rows, all 256 weight columns; the atoms have a ring of their own —
@@ -62,6 +60,7 @@ struct SharedStorage2 {
     uint32_t tmemBase;
     int abortFlag;
     int tilePrefix[kMaxGroups + 1];
+    int groupOffset[kMaxGroups];  // of the caller's table: looked up for every tile by every role
 };
 
 struct Mx2Params {
@@ -146,6 +145,9 @@ __device__ __forceinline__ void TmemDeallocPair(uint32_t taddr, uint32_t cols)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 
+// The exponent byte of a power-of-two scale, four times.
+__device__ __forceinline__ uint32_t ScaleBytes(float f) { return ((__float_as_uint(f) >> 23) & 0xffu) * 0x01010101u; }
+
 __global__ void __launch_bounds__(kThreads, 1)
 mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const Mx2Params p)
 {
@@ -157,6 +159,7 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
     const int pairId = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
     for (int g = threadIdx.x; g < p.G; g += kThreads) {
+        s.groupOffset[g] = p.groupOffset[g];
         s.tilePrefix[g + 1] = ((p.groupCount[g] + 2 * BM - 1) / (2 * BM)) * NT;
     }
     if (threadIdx.x == 0) {
@@ -213,30 +216,32 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
-            const uint32_t leaderFull0 = MapToCta(SmemAddr(&s.full[0]), 0);
-            uint32_t it = 0;
-            for (int tile = pairId; tile < totalTiles && *abortFlag == 0; tile += pairs) {
-                int g, mt, nt;
-                decode(tile, g, mt, nt);
-                const int rowA = p.groupOffset[g] + mt * 2 * BM + (int)cta * BM;
-                const int rowB = g * p.N + nt * BN + (int)cta * BNH;
-                bool ok = true;
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % kStages, ph = (it / kStages) & 1;
-                    if (!MbarWaitBounded(&s.empty[st], ph ^ 1, abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    if (cta == 0) {
+        const bool elected = ElectOne();
+        const uint32_t rank = blockIdx.x & 1;
+        const uint32_t leaderFull0 = __reduce_or_sync(0xffffffffu, MapToCta(SmemAddr(&s.full[0]), 0));
+        uint32_t st = 0, ph = 0;
+        bool ok = true;
+        for (int tile = pairId; ok && __any_sync(0xffffffffu, tile < totalTiles); tile += pairs) {
+            int g, mt, nt;
+            decode(tile, g, mt, nt);
+            const int rowA = __reduce_max_sync(0xffffffffu, s.groupOffset[g] + mt * 2 * BM) + (int)rank * BM;
+            const int rowB = __reduce_max_sync(0xffffffffu, g * p.N + nt * BN) + (int)rank * BNH;
+            for (int kb = 0; kb < KB; kb++) {
+                if (!MbarWaitWarp(&s.empty[st], ph ^ 1, abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                if (elected) {
+                    if (rank == 0) {
                         MbarExpectTx(&s.full[st], 4 * kTileBytes);  // A and weight halves of both CTAs
                     }
                     const uint32_t bar = leaderFull0 + st * (uint32_t)sizeof(uint64_t);
                     TmaLoad2DPair(s.a[st], &tmapA, bar, kb * BK, rowA);
                     TmaLoad2DPair(s.b[st], &tmapB, bar, kb * BK, rowB);
                 }
-                if (!ok) {
-                    break;
+                if (++st == kStages) {
+                    st = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -247,13 +252,20 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
         const uint32_t leaderSfFull0 = MapToCta(SmemAddr(&s.sfFull[0]), 0);
         struct SfWords {
             uint32_t wa[4][4];
-            uint32_t wb[2][4];
+            float wb[2][4];
         };
         const bool vec = (KB & 3) == 0;
-        auto fetch = [&](int tile, int kb0, SfWords &w) {
+        // Where the words of a tile stand; then, per group of K blocks, nothing but loads: what is computed from them is computed when
+        // they are laid out, or their latency would be paid here, once per group on the path that feeds the MMAs.
+        int rowBase = 0;
+        const float *bBase = nullptr;
+        auto enter = [&](int tile) {
             int g, mt, nt;
             decode(tile, g, mt, nt);
-            const int rowBase = p.groupOffset[g] + mt * 2 * BM + (int)cta * BM + lane;
+            rowBase = s.groupOffset[g] + mt * 2 * BM + (int)cta * BM + lane;
+            bBase = p.bScale + ((size_t)g * (p.N / 128) + (size_t)nt * 2) * KB;
+        };
+        auto fetch = [&](int kb0, SfWords &w) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int r = rowBase + 32 * j;
@@ -278,13 +290,11 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
                     }
                 }
             }
-            const float *pb = p.bScale + ((size_t)g * (p.N / 128) + (size_t)nt * 2) * KB;
 #pragma unroll
             for (int a = 0; a < 2; a++) {
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    const float f = kb0 + k < KB ? pb[(size_t)a * KB + kb0 + k] : 1.f;
-                    w.wb[a][k] = ((__float_as_uint(f) >> 23) & 0xffu) * 0x01010101u;
+                    w.wb[a][k] = kb0 + k < KB ? bBase[(size_t)a * KB + kb0 + k] : 1.f;
                 }
             }
         };
@@ -293,7 +303,8 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
         SfWords cur, nxt;
         bool have = tile < totalTiles;
         if (have) {
-            fetch(tile, kb0, cur);
+            enter(tile);
+            fetch(kb0, cur);
         }
         while (have && *abortFlag == 0) {
             int tileN = tile, kbN = kb0 + 4;
@@ -303,7 +314,10 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
             }
             const bool haveNext = tileN < totalTiles;
             if (haveNext) {
-                fetch(tileN, kbN, nxt);
+                if (kbN == 0) {
+                    enter(tileN);
+                }
+                fetch(kbN, nxt);
             }
             const uint32_t buf = it & 1, ph = (it >> 1) & 1;
             const bool ok = MbarWaitBounded(&s.sfEmpty[buf], ph ^ 1, abortFlag);
@@ -317,7 +331,8 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
                     *reinterpret_cast<uint4 *>(s.sfa[slot] + lane * 16) = make_uint4(cur.wa[0][k], cur.wa[1][k], cur.wa[2][k], cur.wa[3][k]);
 #pragma unroll
                     for (int a = 0; a < 2; a++) {
-                        *reinterpret_cast<uint4 *>(s.sfb[slot] + a * 512 + lane * 16) = make_uint4(cur.wb[a][k], cur.wb[a][k], cur.wb[a][k], cur.wb[a][k]);
+                        const uint32_t e = ScaleBytes(cur.wb[a][k]);
+                        *reinterpret_cast<uint4 *>(s.sfb[slot] + a * 512 + lane * 16) = make_uint4(e, e, e, e);
                     }
                 }
                 FenceProxyAsyncShared();
@@ -337,47 +352,53 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader only)
-        if (lane == 0 && cta == 0) {
-            uint32_t it = 0, tl = 0, sg = 0;
-            for (int tile = pairId; tile < totalTiles && *abortFlag == 0; tile += pairs, tl++) {
-                if (!MbarWaitBounded(&s.tmemEmpty, (tl & 1) ^ 1, abortFlag)) {
+        if ((blockIdx.x & 1) == 0) {
+            const bool elected = ElectOne();
+            const uint32_t tmem = __reduce_or_sync(0xffffffffu, tmemBase);
+            const uint64_t aDesc0 = SmemDescSw128(SmemAddr(s.a[0])), bDesc0 = SmemDescSw128(SmemAddr(s.b[0]));
+            const uint64_t sfaDesc0 = SmemDescSfAtom(SmemAddr(s.sfa[0])), sfbDesc0 = SmemDescSfAtom(SmemAddr(s.sfb[0]));
+            uint32_t st = 0, ph = 0, sbuf = 0, sph = 0, tph = 0;
+            bool ok = true;
+            for (int tile = pairId; ok && __any_sync(0xffffffffu, tile < totalTiles); tile += pairs, tph ^= 1) {
+                if (!MbarWaitWarp(&s.tmemEmpty, tph ^ 1, abortFlag)) {
                     break;
                 }
-                const uint32_t d = tmemBase;
-                bool ok = true;
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % kStages, ph = (it / kStages) & 1;
-                    const uint32_t sbuf = sg & 1, slot = sbuf * kSfGroup + (kb % kSfGroup);
-                    if (kb % kSfGroup == 0 && !MbarWaitBounded(&s.sfFull[sbuf], (sg >> 1) & 1, abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    if (!MbarWaitBounded(&s.full[st], ph, abortFlag)) {
+                for (int kb = 0; kb < KB; kb++) {
+                    const uint32_t slot = sbuf * kSfGroup + ((uint32_t)kb & (kSfGroup - 1));
+                    const bool lastOfGroup = (kb & (kSfGroup - 1)) == kSfGroup - 1 || kb == KB - 1;
+                    if (((kb & (kSfGroup - 1)) == 0 && !MbarWaitWarp(&s.sfFull[sbuf], sph, abortFlag)) || !MbarWaitWarp(&s.full[st], ph, abortFlag)) {
                         ok = false;
                         break;
                     }
                     TcFenceAfter();
-                    const uint32_t sfa = tmemBase + kSfaCol + (kb & 1) * kSfSetCols, sfb = tmemBase + kSfbCol + (kb & 1) * kSfSetCols;
-                    TmemCpSfAtomPair(sfa, SmemDescSfAtom(SmemAddr(s.sfa[slot])));
-                    TmemCpSfAtomPair(sfb, SmemDescSfAtom(SmemAddr(s.sfb[slot])));
-                    TmemCpSfAtomPair(sfb + 4, SmemDescSfAtom(SmemAddr(s.sfb[slot] + 512)));
-                    const uint64_t aDesc = SmemDescSw128(SmemAddr(s.a[st]));
-                    const uint64_t bDesc = SmemDescSw128(SmemAddr(s.b[st]));
+                    if (elected) {
+                        const uint32_t sfa = tmem + kSfaCol + (kb & 1) * kSfSetCols, sfb = tmem + kSfbCol + (kb & 1) * kSfSetCols;
+                        TmemCpSfAtomPair(sfa, sfaDesc0 + (uint64_t)(slot * 32));
+                        TmemCpSfAtomPair(sfb, sfbDesc0 + (uint64_t)(slot * 64));
+                        TmemCpSfAtomPair(sfb + 4, sfbDesc0 + (uint64_t)(slot * 64 + 32));
+                        const uint64_t aDesc = aDesc0 + (uint64_t)(st * (uint32_t)(kTileBytes >> 4)), bDesc = bDesc0 + (uint64_t)(st * (uint32_t)(kTileBytes >> 4));
 #pragma unroll
-                    for (uint32_t k = 0; k < BK / 32; k++) {
-                        MmaMxF8Pair(d, aDesc + (uint64_t)(k * 2), bDesc + (uint64_t)(k * 2), InstrDescMxF8(2 * BM, BN, k), sfa | (k << 30), sfb | (k << 30),
-                                    (kb > 0 || k > 0) ? 1u : 0u);
+                        for (uint32_t k = 0; k < BK / 32; k++) {
+                            MmaMxF8Pair(tmem, aDesc + (uint64_t)(k * 2), bDesc + (uint64_t)(k * 2), InstrDescMxF8(2 * BM, BN, k), sfa | (k << 30),
+                                        sfb | (k << 30), (kb > 0 || k > 0) ? 1u : 0u);
+                        }
+                        MmaCommitPair(&s.empty[st]);
+                        if (lastOfGroup) {
+                            MmaCommitPair(&s.sfEmpty[sbuf]);
+                        }
+                        if (kb == KB - 1) {
+                            MmaCommitPair(&s.tmemFull);
+                        }
                     }
-                    MmaCommitPair(&s.empty[st]);
-                    if (kb % kSfGroup == kSfGroup - 1 || kb == KB - 1) {
-                        MmaCommitPair(&s.sfEmpty[sbuf]);
-                        sg++;
+                    if (lastOfGroup) {
+                        sbuf ^= 1;
+                        sph ^= sbuf ^ 1;
+                    }
+                    if (++st == kStages) {
+                        st = 0;
+                        ph ^= 1;
                     }
                 }
-                if (!ok) {
-                    break;
-                }
-                MmaCommitPair(&s.tmemFull);
             }
         }
     } else if (warp >= 4) {
@@ -393,7 +414,7 @@ mf_moe_grouped_gemm_mx2_kernel(const __grid_constant__ CUtensorMap tmapA, const 
             int g, mt, nt;
             decode(tile, g, mt, nt);
             const int rowLocal = mt * 2 * BM + (int)cta * BM + rowInTile;
-            const int row = p.groupOffset[g] + rowLocal;
+            const int row = s.groupOffset[g] + rowLocal;
             const bool valid = rowLocal < p.groupCount[g] && row < p.rowsTotal;
             if (!MbarWaitBounded(&s.tmemFull, tl & 1, abortFlag)) {
                 break;

@@ -23,6 +23,9 @@
 // BN = 224 (two accumulators of 224 columns, 4-stage ring) for the plain bf16 epilogue when N is a multiple of 224: nearly
 // the operand reuse of the 256-wide tile, and the epilogue of one tile runs under the MMAs of the next, which matters when K
 // is short (the second FFN GEMM: N = 7168 = 32 x 224, K = 2048).
+// What bounds it: a K block of a 256-wide tile takes 600 cycles of which the MMAs are 512 (724 cycles while the scale-factor warp computed
+// on words it had just asked for and one lane issued everything); 32768 rows, N 4096 / K 7168: 864 -> 781 us = 2.5 PFLOP/s, at
+// which the power limit holds the clock near 1.2 GHz.
 // Every mbarrier wait is bounded; on expiry the CTA sets *status, all roles drain and the CTA frees its TMEM and exits.
 // Gated form (mf_k_moe_grouped_gemm_mx_gated): the rows of A are being stored by other GPUs (the MoE dispatch of the peers)
 // while this kernel runs. The two warps that read A — the TMA producer and the scale-factor producer — start a tile only when
@@ -78,6 +81,7 @@ struct SharedStorage {
     int abortFlag;  // 0 running, 1 a pipeline wait expired, 2 an arrival wait expired
     int gated;
     int tilePrefix[kMaxGroups + 1];
+    int groupOffset[kMaxGroups];  // of the caller's table: looked up for every tile by every role
 };
 
 struct MxParams {
@@ -137,6 +141,9 @@ __device__ __forceinline__ uint32_t Ue8m0Ceil(float t)
     return e < 1u ? 1u : (e > 253u ? 253u : e);
 }
 
+// The exponent byte of a power-of-two scale, four times.
+__device__ __forceinline__ uint32_t ScaleBytes(float f) { return ((__float_as_uint(f) >> 23) & 0xffu) * 0x01010101u; }
+
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const MxParams p)
@@ -148,6 +155,7 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
     const int KB = p.K / BK, NT = p.N / BN;
 
     for (int g = threadIdx.x; g < p.G; g += kThreads) {
+        s.groupOffset[g] = p.groupOffset[g];
         s.tilePrefix[g + 1] = ((p.groupCount[g] + BM - 1) / BM) * NT;
     }
     if (threadIdx.x == 0) {
@@ -203,26 +211,32 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            uint32_t it = 0;
-            int lastGate = -1;
-            for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x) {
-                int g, mt, nt;
-                decode(tile, g, mt, nt);
-                const int rowA = p.groupOffset[g] + mt * BM;
-                const int rowB = g * p.N + nt * BN;
-                if (gated && (rowA >> 7) != lastGate) {
-                    if (!ArrivalWait(p.arrive + (rowA >> 7), min(BM, p.groupCount[g] - mt * BM), abortFlag, p.waitNs)) {
-                        break;
-                    }
+        const bool elected = ElectOne();
+        uint32_t st = 0, ph = 0;
+        int lastGate = -1;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && __any_sync(0xffffffffu, tile < totalTiles); tile += gridDim.x) {
+            int g, mt, nt;
+            decode(tile, g, mt, nt);
+            const int rowA = __reduce_max_sync(0xffffffffu, s.groupOffset[g] + mt * BM);
+            const int rowB = __reduce_max_sync(0xffffffffu, g * p.N + nt * BN);
+            if (gated && (rowA >> 7) != lastGate) {
+                bool here = true;
+                if (elected) {
+                    here = ArrivalWait(p.arrive + (rowA >> 7), min(BM, p.groupCount[g] - mt * BM), abortFlag, p.waitNs);
                     FenceProxyAsyncGlobal();  // the rows were stored through the generic proxy (by other GPUs); TMA reads them
-                    lastGate = rowA >> 7;
                 }
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % C::kStages, ph = (it / C::kStages) & 1;
-                    if (!MbarWaitBounded(&s.empty[st], ph ^ 1, abortFlag)) {
-                        break;
-                    }
+                if (!__all_sync(0xffffffffu, here)) {
+                    break;
+                }
+                lastGate = rowA >> 7;
+            }
+            for (int kb = 0; kb < KB; kb++) {
+                if (!MbarWaitWarp(&s.empty[st], ph ^ 1, abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                if (elected) {
                     MbarExpectTx(&s.full[st], C::kATile + C::kBTile);
                     TmaLoad2D(s.a[st], &tmapA, &s.full[st], kb * BK, rowA);
                     if (p.bPacked) {
@@ -230,6 +244,10 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
                     } else {
                         TmaLoad2D(s.b[st], &tmapB, &s.full[st], kb * BK, rowB);
                     }
+                }
+                if (++st == C::kStages) {
+                    st = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -240,13 +258,22 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
         // hand-shakes instead of being paid once per group on the path that feeds the MMAs.
         struct SfWords {
             uint32_t wa[4][4];
-            uint32_t wb[C::kAtomsB][C::kSfbWords][4];
+            float wb[C::kAtomsB][C::kSfbWords][4];
         };
         const bool vec = (KB & 3) == 0;
-        auto fetch = [&](int tile, int kb0, SfWords &w) {
+        // Where the words of a tile stand; then, per group of K blocks, nothing but loads: what is computed from them is computed when
+        // they are laid out, or their latency would be paid here, once per group on the path that feeds the MMAs.
+        int rowBase = 0;
+        const float *bBase = nullptr;
+        int colBase = 0;
+        auto enter = [&](int tile) {
             int g, mt, nt;
             decode(tile, g, mt, nt);
-            const int rowBase = p.groupOffset[g] + mt * BM + lane;
+            rowBase = s.groupOffset[g] + mt * BM + lane;
+            bBase = p.bScale + (size_t)g * (p.N / 128) * KB;
+            colBase = nt * BN;
+        };
+        auto fetch = [&](int kb0, SfWords &w) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int r = rowBase + 32 * j;
@@ -278,11 +305,10 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
 #pragma unroll
                 for (int j = 0; j < C::kSfbWords; j++) {
                     const int cin = a * 128 + 32 * j;
-                    const float *pb = p.bScale + ((size_t)g * (p.N / 128) + (size_t)((nt * BN + cin) / 128)) * KB;
+                    const float *pb = bBase + (size_t)((colBase + cin) / 128) * KB;
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        const float f = (cin < BN && kb0 + k < KB) ? pb[kb0 + k] : 1.f;
-                        w.wb[a][j][k] = ((__float_as_uint(f) >> 23) & 0xffu) * 0x01010101u;
+                        w.wb[a][j][k] = (cin < BN && kb0 + k < KB) ? pb[kb0 + k] : 1.f;
                     }
                 }
             }
@@ -293,7 +319,7 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
             if (lane == 0) {
                 int g, mt, nt;
                 decode(tile, g, mt, nt);
-                const int row0 = p.groupOffset[g] + mt * BM;
+                const int row0 = s.groupOffset[g] + mt * BM;
                 const int need = min(BM, p.groupCount[g] - mt * BM);
                 const int *ctr = p.arrive + (row0 >> 7);
                 ok = block ? (ArrivalWait(ctr, need, abortFlag, p.waitNs) ? 1 : 0) : (LdAcquireSys(ctr) >= need ? 1 : 0);
@@ -310,7 +336,8 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
             if (gated && !gate(tile, true)) {
                 have = false;
             } else {
-                fetch(tile, kb0, cur);
+                enter(tile);
+                fetch(kb0, cur);
             }
         }
         while (have && *abortFlag == 0) {
@@ -321,8 +348,11 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
             }
             const bool haveNext = tileN < totalTiles;
             bool fetched = false;
+            if (haveNext && kbN == 0) {
+                enter(tileN);
+            }
             if (haveNext && (!gated || kbN != 0 || gate(tileN, false))) {
-                fetch(tileN, kbN, nxt);
+                fetch(kbN, nxt);
                 fetched = true;
             }
             bool ok = true;
@@ -341,7 +371,8 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
                 for (int a = 0; a < C::kAtomsB; a++) {
                     // with one word per atom (the atom lies in one weight block) all four lanes-of-32 groups share it
                     *reinterpret_cast<uint4 *>(s.sfb[st] + a * 512 + lane * 16) =
-                        make_uint4(cur.wb[a][0][k], cur.wb[a][1 % C::kSfbWords][k], cur.wb[a][2 % C::kSfbWords][k], cur.wb[a][3 % C::kSfbWords][k]);
+                        make_uint4(ScaleBytes(cur.wb[a][0][k]), ScaleBytes(cur.wb[a][1 % C::kSfbWords][k]), ScaleBytes(cur.wb[a][2 % C::kSfbWords][k]),
+                                   ScaleBytes(cur.wb[a][3 % C::kSfbWords][k]));
                 }
                 FenceProxyAsyncShared();
                 __syncwarp();
@@ -357,7 +388,7 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
                 if (!gate(tileN, true)) {
                     break;
                 }
-                fetch(tileN, kbN, nxt);
+                fetch(kbN, nxt);
             }
             cur = nxt;
             tile = tileN;
@@ -366,42 +397,50 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            uint32_t it = 0, tl = 0;
-            for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x, tl++) {
-                const uint32_t buf = tl % C::kAccBufs, bph = (tl / C::kAccBufs) & 1;
-                if (!MbarWaitBounded(&s.tmemEmpty[buf], bph ^ 1, abortFlag)) {
+        const bool elected = ElectOne();
+        const uint32_t tmem = __reduce_or_sync(0xffffffffu, tmemBase);
+        const uint64_t aDesc0 = SmemDescSw128(SmemAddr(s.a[0])), bDesc0 = SmemDescSw128(SmemAddr(s.b[0]));
+        const uint64_t sfaDesc0 = SmemDescSfAtom(SmemAddr(s.sfa[0])), sfbDesc0 = SmemDescSfAtom(SmemAddr(s.sfb[0]));
+        uint32_t st = 0, ph = 0, buf = 0, bph = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && __any_sync(0xffffffffu, tile < totalTiles); tile += gridDim.x) {
+            if (!MbarWaitWarp(&s.tmemEmpty[buf], bph ^ 1, abortFlag)) {
+                break;
+            }
+            for (int kb = 0; kb < KB; kb++) {
+                if (!MbarWaitWarp(&s.full[st], ph, abortFlag)) {
+                    ok = false;
                     break;
                 }
-                const uint32_t d = tmemBase + buf * BN;
-                bool ok = true;
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % C::kStages, ph = (it / C::kStages) & 1;
-                    if (!MbarWaitBounded(&s.full[st], ph, abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    TcFenceAfter();
-                    TmemCpSfAtom(tmemBase + C::kSfaCol, SmemDescSfAtom(SmemAddr(s.sfa[st])));
+                TcFenceAfter();
+                if (elected) {
+                    const uint64_t sfbDesc = sfbDesc0 + (uint64_t)(st * (uint32_t)(32 * C::kAtomsB));
+                    TmemCpSfAtom(tmem + C::kSfaCol, sfaDesc0 + (uint64_t)(st * 32));
 #pragma unroll
                     for (int a = 0; a < C::kAtomsB; a++) {
-                        TmemCpSfAtom(tmemBase + C::kSfbCol + 4 * a, SmemDescSfAtom(SmemAddr(s.sfb[st] + a * 512)));
+                        TmemCpSfAtom(tmem + C::kSfbCol + 4 * a, sfbDesc + (uint64_t)(32 * a));
                     }
-                    const uint64_t aDesc = SmemDescSw128(SmemAddr(s.a[st]));
-                    const uint64_t bDesc = SmemDescSw128(SmemAddr(s.b[st]));
+                    const uint64_t aDesc = aDesc0 + (uint64_t)(st * (uint32_t)(C::kATile >> 4)), bDesc = bDesc0 + (uint64_t)(st * (uint32_t)(C::kBTile >> 4));
 #pragma unroll
                     for (uint32_t k = 0; k < BK / 32; k++) {
                         // 32 fp8 elements = 32 bytes further along K inside the 128-byte swizzled row: +2 in 16-byte units. The byte of
                         // the scale-factor columns that belongs to this K step rides in the top two address bits and the descriptor.
-                        MmaMxF8(d, aDesc + (uint64_t)(k * 2), bDesc + (uint64_t)(k * 2), InstrDescMxF8(BM, BN, k), (tmemBase + C::kSfaCol) | (k << 30),
-                                (tmemBase + C::kSfbCol) | (k << 30), (kb > 0 || k > 0) ? 1u : 0u);
+                        MmaMxF8(tmem + buf * BN, aDesc + (uint64_t)(k * 2), bDesc + (uint64_t)(k * 2), InstrDescMxF8(BM, BN, k),
+                                (tmem + C::kSfaCol) | (k << 30), (tmem + C::kSfbCol) | (k << 30), (kb > 0 || k > 0) ? 1u : 0u);
                     }
                     MmaCommit(&s.empty[st]);  // the stage (operands and scale atoms) may be refilled once these operations have read it
+                    if (kb == KB - 1) {
+                        MmaCommit(&s.tmemFull[buf]);
+                    }
                 }
-                if (!ok) {
-                    break;
+                if (++st == C::kStages) {
+                    st = 0;
+                    ph ^= 1;
                 }
-                MmaCommit(&s.tmemFull[buf]);
+            }
+            if (++buf == C::kAccBufs) {
+                buf = 0;
+                bph ^= 1;
             }
         }
     } else if (warp >= 4) {
@@ -416,7 +455,7 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
             int g, mt, nt;
             decode(tile, g, mt, nt);
             const uint32_t buf = tl % C::kAccBufs, bph = (tl / C::kAccBufs) & 1;
-            const int row = p.groupOffset[g] + mt * BM + rowInTile;
+            const int row = s.groupOffset[g] + mt * BM + rowInTile;
             const bool valid = mt * BM + rowInTile < p.groupCount[g] && row < p.rowsTotal;
             if (!MbarWaitBounded(&s.tmemFull[buf], bph, abortFlag)) {
                 break;

@@ -179,47 +179,62 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            uint32_t it = 0;
-            for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x) {
-                int g, mt, nt;
-                decode(tile, g, mt, nt);
-                const int rowA = s.groupOffset[g] + mt * BM;
-                const int rowB = g * p.N + nt * BN;
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % C::kStages, ph = (it / C::kStages) & 1;
-                    if (!MbarWaitBounded(&s.empty[st], ph ^ 1, abortFlag)) {
-                        break;
-                    }
+        const bool elected = ElectOne();
+        uint32_t st = 0, ph = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && __any_sync(0xffffffffu, tile < totalTiles); tile += gridDim.x) {
+            int g, mt, nt;
+            decode(tile, g, mt, nt);
+            const int rowA = __reduce_max_sync(0xffffffffu, s.groupOffset[g] + mt * BM);
+            const int rowB = __reduce_max_sync(0xffffffffu, g * p.N + nt * BN);
+            for (int kb = 0; kb < KB; kb++) {
+                if (!MbarWaitWarp(&s.empty[st], ph ^ 1, abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                if (elected) {
                     MbarExpectTx(&s.full[st], kTileBytes + C::kBTile);
                     TmaLoad2D(s.a[st], &tmapA, &s.full[st], kb * BK, rowA);
                     TmaLoad2D(s.b[st], &tmapB, &s.full[st], kb * BK, rowB);
+                }
+                if (++st == C::kStages) {
+                    st = 0;
+                    ph ^= 1;
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = InstrDescF8(BM, BN);
-            uint32_t it = 0;
-            for (int tile = blockIdx.x; tile < totalTiles && *abortFlag == 0; tile += gridDim.x) {
-                for (int kb = 0; kb < KB; kb++, it++) {
-                    const uint32_t st = it % C::kStages, ph = (it / C::kStages) & 1;
-                    const uint32_t buf = it % C::kAccBufs, bph = (it / C::kAccBufs) & 1;
-                    if (!MbarWaitBounded(&s.tmemEmpty[buf], bph ^ 1, abortFlag) || !MbarWaitBounded(&s.full[st], ph, abortFlag)) {
-                        break;
-                    }
-                    TcFenceAfter();
-                    const uint64_t aDesc = SmemDescSw128(SmemAddr(s.a[st]));
-                    const uint64_t bDesc = SmemDescSw128(SmemAddr(s.b[st]));
-                    const uint32_t d = tmemBase + buf * BN;
+        constexpr uint32_t idesc = InstrDescF8(BM, BN);
+        const bool elected = ElectOne();
+        const uint32_t tmem = __reduce_or_sync(0xffffffffu, tmemBase);
+        const uint64_t aDesc0 = SmemDescSw128(SmemAddr(s.a[0])), bDesc0 = SmemDescSw128(SmemAddr(s.b[0]));
+        uint32_t st = 0, ph = 0, buf = 0, bph = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && __any_sync(0xffffffffu, tile < totalTiles); tile += gridDim.x) {
+            for (int kb = 0; kb < KB; kb++) {
+                if (!MbarWaitWarp(&s.tmemEmpty[buf], bph ^ 1, abortFlag) || !MbarWaitWarp(&s.full[st], ph, abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                TcFenceAfter();
+                if (elected) {
+                    const uint64_t aDesc = aDesc0 + (uint64_t)(st * (uint32_t)(kTileBytes >> 4)), bDesc = bDesc0 + (uint64_t)(st * (uint32_t)(C::kBTile >> 4));
 #pragma unroll
                     for (int k = 0; k < BK / 32; k++) {
                         // 32 fp8 elements = 32 bytes further along K inside the 128-byte swizzled row: +2 in 16-byte units.
-                        MmaF8(d, aDesc + (uint64_t)(k * 2), bDesc + (uint64_t)(k * 2), idesc, k > 0 ? 1u : 0u);
+                        MmaF8(tmem + buf * BN, aDesc + (uint64_t)(k * 2), bDesc + (uint64_t)(k * 2), idesc, k > 0 ? 1u : 0u);
                     }
                     MmaCommit(&s.empty[st]);      // the smem stage may be refilled once these MMAs have read it
                     MmaCommit(&s.tmemFull[buf]);  // the partial product is complete in TMEM
+                }
+                if (++st == C::kStages) {
+                    st = 0;
+                    ph ^= 1;
+                }
+                if (++buf == C::kAccBufs) {
+                    buf = 0;
+                    bph ^= 1;
                 }
             }
         }

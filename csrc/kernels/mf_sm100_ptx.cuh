@@ -75,6 +75,21 @@ __device__ __forceinline__ bool MbarWaitBounded(uint64_t *bar, uint32_t parity, 
     return false;
 }
 
+// The same by a whole warp, with one answer for all lanes. The warps that feed the tensor cores run their loops uniformly and let one
+// elected lane issue: descriptors and addresses then stay in uniform registers, which is where the instructions want them. In a
+// loop of one lane they were moved there operand by operand, and issuing a K block took longer than its MMAs.
+__device__ __forceinline__ bool MbarWaitWarp(uint64_t *bar, uint32_t parity, volatile int *abortFlag)
+{
+    return __all_sync(0xffffffffu, MbarWaitBounded(bar, parity, abortFlag)) != 0;
+}
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool ElectOne()
+{
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
+
 // One 32-byte store (a whole sector) to global memory; the address must be 32-byte aligned.
 __device__ __forceinline__ void StGlobal32B(void *p, const uint32_t (&w)[8])
 {
