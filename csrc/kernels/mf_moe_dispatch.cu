@@ -34,8 +34,11 @@
 
 #include "mf/device/mf_shm_device.cuh"
 #include "mf_kernels.h"
+#include "mf_sm100_ptx.cuh"
 
 namespace cg = cooperative_groups;
+using mf::sm100::GridDependency;
+using mf::sm100::LaunchDependent;
 
 namespace {
 
@@ -121,6 +124,7 @@ template <bool EMULATED>
 __global__ void __launch_bounds__(kThreads, 4)
 mf_moe_dispatch_kernel(const __grid_constant__ mf_moe_dispatch_args_t own, const mf_moe_dispatch_args_t *__restrict__ emulated, int H, int K, int E, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
+    GridDependency();
     cg::grid_group grid = cg::this_grid();
     const mf_moe_dispatch_args_t &a = EMULATED ? emulated[blockIdx.y] : own;
     const uint64_t epoch = ResolveEpochD(a, epochArg);
@@ -556,6 +560,7 @@ template <bool ALONE, bool EMULATED>
 __global__ void __launch_bounds__(kThreads, 3)
 mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const mf_moe_combine_args_t *__restrict__ emulated, int H, int K, int EL, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
+    GridDependency();
     const mf_moe_combine_args_t &a = EMULATED ? emulated[blockIdx.y] : own;
     const uint64_t epoch = ResolveEpochD(a, epochArg);
     if (epoch == 0) {
@@ -815,7 +820,8 @@ static int LaunchCombine(const mf_moe_combine_args_t *argsHost, const mf_moe_com
     }
     void *kargs[] = {(void *)&own, (void *)&argsDev, (void *)&H, (void *)&K, (void *)&EL, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
     dim3 g((unsigned)grid, (unsigned)nEmulatedRanks, 1), b(kThreads, 1, 1);
-    cudaError_t e = alone ? cudaLaunchKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream)
+    cudaError_t e = alone ? LaunchDependent(mf_moe_combine_kernel<true, false>, (unsigned)grid, kThreads, 0, (cudaStream_t)stream, own, argsDev, H, K, EL,
+                                            channel, epoch, timeoutNs)
                           : cudaLaunchCooperativeKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();

@@ -154,10 +154,6 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KB = p.K / BK, NT = p.N / BN;
 
-    for (int g = threadIdx.x; g < p.G; g += kThreads) {
-        s.groupOffset[g] = p.groupOffset[g];
-        s.tilePrefix[g + 1] = ((p.groupCount[g] + BM - 1) / BM) * NT;
-    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < C::kStages; i++) {
             MbarInit(&s.full[i], 2);  // TMA thread (with the byte count) + scale-factor warp
@@ -168,13 +164,20 @@ mf_moe_grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmapA, const _
             MbarInit(&s.tmemEmpty[i], kEpiWarps);
         }
         s.abortFlag = 0;
-        s.gated = p.arrive != nullptr && (p.status == nullptr || *(volatile int *)p.status == 0) ? 1 : 0;
         MbarInitFence();
         TmaPrefetchDesc(&tmapA);
         TmaPrefetchDesc(&tmapB);
     }
     if (warp == 3) {
         TmemAlloc(&s.tmemBase, kTmemCols);
+    }
+    GridDependency();  // what stands above ran under the end of the kernel before
+    for (int g = threadIdx.x; g < p.G; g += kThreads) {
+        s.groupOffset[g] = p.groupOffset[g];
+        s.tilePrefix[g + 1] = ((p.groupCount[g] + BM - 1) / BM) * NT;
+    }
+    if (threadIdx.x == 0) {
+        s.gated = p.arrive != nullptr && (p.status == nullptr || *(volatile int *)p.status == 0) ? 1 : 0;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -640,8 +643,11 @@ int Launch(const CUtensorMap &mapA, const CUtensorMap &mapB, const MxParams &p, 
         return MF_K_LAUNCH_FAILED;
     }
     const int grid = ctas > 0 && ctas < sms ? ctas : sms;
-    mf_moe_grouped_gemm_mx_kernel<BN><<<grid, kThreads, smem, stream>>>(mapA, mapB, p);
-    return cudaGetLastError() == cudaSuccess ? MF_K_OK : MF_K_LAUNCH_FAILED;
+    if (LaunchDependent(mf_moe_grouped_gemm_mx_kernel<BN>, (unsigned)grid, kThreads, smem, stream, mapA, mapB, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MF_K_LAUNCH_FAILED;
+    }
+    return MF_K_OK;
 }
 
 int GemmMx(const void *a, const uint32_t *aSf, const void *b, const float *bScale, void *out, void *outSf, const int *groupOffset,

@@ -119,11 +119,6 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KB = p.K / BK, NT = p.N / BN;
 
-    for (int g = threadIdx.x; g < p.G; g += C::kThreads) {
-        s.groupOffset[g] = p.groupOffset[g];
-        s.groupCount[g] = p.groupCount[g];
-        s.tilePrefix[g + 1] = ((s.groupCount[g] + BM - 1) / BM) * NT;
-    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < C::kStages; i++) {
             MbarInit(&s.full[i], 1);
@@ -144,6 +139,12 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
     }
     if (warp == 0) {
         TmemAlloc(&s.tmemBase, kTmemCols);
+    }
+    GridDependency();  // what stands above ran under the end of the kernel before
+    for (int g = threadIdx.x; g < p.G; g += C::kThreads) {
+        s.groupOffset[g] = p.groupOffset[g];
+        s.groupCount[g] = p.groupCount[g];
+        s.tilePrefix[g + 1] = ((s.groupCount[g] + BM - 1) / BM) * NT;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -440,6 +441,7 @@ constexpr int kQuantUnroll = 4;
 __global__ void __launch_bounds__(256) mf_quant_rows_fp8_kernel(const __nv_bfloat16 *__restrict__ x, unsigned char *__restrict__ q,
                                                                 float *__restrict__ scale, int rows, int blocksPerRow, const int *__restrict__ rowLimit)
 {
+    GridDependency();
     const int lane = threadIdx.x & 31;
     const int limit = rowLimit != nullptr ? min(*rowLimit, rows) : rows;
     const long long total = (long long)limit * blocksPerRow;
@@ -553,8 +555,11 @@ int Launch(const void *a, const void *b, const GemmParams &p, int ctas, cudaStre
         return MF_K_LAUNCH_FAILED;
     }
     const int grid = ctas > 0 && ctas < sms ? ctas : sms;
-    mf_moe_grouped_gemm_kernel<BN><<<grid, Cfg<BN>::kThreads, smem, stream>>>(mapA, mapB, p);
-    return cudaGetLastError() == cudaSuccess ? MF_K_OK : MF_K_LAUNCH_FAILED;
+    if (LaunchDependent(mf_moe_grouped_gemm_kernel<BN>, (unsigned)grid, Cfg<BN>::kThreads, smem, stream, mapA, mapB, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MF_K_LAUNCH_FAILED;
+    }
+    return MF_K_OK;
 }
 
 }  // namespace
@@ -605,6 +610,10 @@ extern "C" int mf_k_quant_rows_fp8(const void *x, void *q, float *scale, int row
     if (blocks > 148 * 16) {
         blocks = 148 * 16;
     }
-    mf_quant_rows_fp8_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x, (unsigned char *)q, scale, rows, K / 128, rowLimit);
-    return cudaGetLastError() == cudaSuccess ? MF_K_OK : MF_K_LAUNCH_FAILED;
+    if (LaunchDependent(mf_quant_rows_fp8_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16 *)x, (unsigned char *)q, scale, rows,
+                        K / 128, rowLimit) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MF_K_LAUNCH_FAILED;
+    }
+    return MF_K_OK;
 }

@@ -90,6 +90,30 @@ __device__ __forceinline__ bool ElectOne()
     return e != 0;
 }
 
+// Programmatic dependent launch. Every thread of a kernel that is launched with LaunchDependent calls this before it touches global memory:
+// the next kernel of the stream may take the SMs that this one leaves (it waits here in turn, until this one is complete and
+// its writes are visible), and this one goes on when all before it is complete.
+__device__ __forceinline__ void GridDependency()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t LaunchDependent(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const A &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // One 32-byte store (a whole sector) to global memory; the address must be 32-byte aligned.
 __device__ __forceinline__ void StGlobal32B(void *p, const uint32_t (&w)[8])
 {

@@ -100,6 +100,40 @@ def test_moe_layer_looks_at_its_weights_on_every_call(heap):
         layer(x, idx, tw)
 
 
+def test_moe_layer_replays_and_follows_itself(heap):
+    """The launches of a layer overlap the end of the one before: captured three in a row, and eagerly with new inputs every time."""
+    import torch
+
+    from memfabric_hybrid_b200.ops.moe import FusedMoE, route
+
+    T, H, E, K, I = 64, 512, 8, 4, 256
+    layer = FusedMoE(heap, T, H, E, K, I, *_weights(E, H, I, 8), device_epochs=True)
+    g = torch.Generator(device="cuda").manual_seed(2)
+
+    def batch():
+        x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+        return (x,) + route(torch.randn(T, E, generator=g, device="cuda"), K)
+
+    inputs = batch()
+    ref = layer(*inputs).clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(3):
+            out = layer(*inputs)
+    for _ in range(5):
+        layer.st.out.zero_()
+        graph.replay()
+        assert torch.equal(out, ref)
+    for _ in range(30):
+        inputs = batch()
+        a = layer(*inputs).clone()
+        torch.cuda.synchronize()
+        layer(*batch())  # what follows must not reach into the call before it, nor be reached by it
+        assert torch.equal(layer(*inputs), a)
+    assert layer.check_status() == 0
+    del graph
+
+
 def test_moe_overflow_is_reported_and_the_kernel_ends(heap):
     """Everything goes to one expert of a layer whose receive buffer holds a fraction of it."""
     import torch
