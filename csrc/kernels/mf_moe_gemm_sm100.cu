@@ -16,7 +16,7 @@
 //   warps 2-3  bring the products sa * sb of four K-blocks at a time into a ring of two such groups, one group ahead and across
 //              tiles: a row's scales are a line of their own for every thread, and waiting for them once per K-block on the
 //              promotion path took longer than the MMAs. It also leaves the promotion threads few enough registers.
-// 8191 rows over 32 experts, SwiGLU GEMM N 4096 / K 7168: 486 -> 389 us; N 7168 / K 2048: 281 -> 215 us. What bounds it now: a partial
+// 8191 rows over 32 experts, SwiGLU GEMM N 4096 / K 7168: 486 -> 353 us; N 7168 / K 2048: 281 -> 196 us. What bounds it now: a partial
 // product is read from TMEM while the next one is made in the other accumulator, and the hand-over (commit, wait, load, arrive) is
 // not shorter than the MMAs of a K-block.
 // Tiles are enumerated on the device from group_offset/group_count (the host does not know the routing result), n fastest so
@@ -55,7 +55,8 @@ template <int BN>
 struct SharedStorage {
     alignas(1024) unsigned char a[Cfg<BN>::kStages][kTileBytes];
     alignas(1024) unsigned char b[Cfg<BN>::kStages][Cfg<BN>::kBTile];
-    float4 scale[2][BN / 128][BM];  // [group of four K-blocks][weight block][row]
+    // Read per K-block, not four at a time: with those in registers the promotion threads spilled (12 bytes, 389 instead of 353 us).
+    float scale[2][BN / 128][4][BM];  // [group of four K-blocks][weight block][K-block][row]
     uint64_t scaleFull[2];
     uint64_t scaleEmpty[2];
     uint64_t full[Cfg<BN>::kStages];
@@ -294,8 +295,10 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
             for (int c = 0; c < BN / 128; c++) {
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
-                    s.scale[buf][c][row0 + 32 * j] = make_float4(cur.a[j][0] * cur.b[c][0], cur.a[j][1] * cur.b[c][1], cur.a[j][2] * cur.b[c][2],
-                                                                 cur.a[j][3] * cur.b[c][3]);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        s.scale[buf][c][k][row0 + 32 * j] = cur.a[j][k] * cur.b[c][k];
+                    }
                 }
             }
             __syncwarp();
@@ -323,12 +326,6 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
             if (!MbarWaitBounded(&s.scaleFull[item & 1], (item >> 1) & 1, abortFlag)) {
                 break;
             }
-            float4 scale = s.scale[item & 1][part / 2][rowInTile];
-            __syncwarp();
-            if (lane == 0) {
-                MbarArrive(&s.scaleEmpty[item & 1]);
-            }
-            item++;
             const int n = min(4, KB - kb0);
             bool ok = true;
 #pragma unroll 1
@@ -340,7 +337,8 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
                 }
                 TcFenceAfter();
                 const uint32_t taddr = tmemBase + ((uint32_t)(quad * 32) << 16) + buf * BN + part * HC;
-                const uint64_t sc = PackF32x2(scale.x, scale.x);
+                const float scale = s.scale[item & 1][part / 2][k][rowInTile];
+                const uint64_t sc = PackF32x2(scale, scale);
 #pragma unroll
                 for (int c = 0; c < HC; c += 16) {
                     float v[16];
@@ -358,11 +356,15 @@ mf_moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __gr
                         FmaF32x2(acc2[(c + i) / 2], PackF32x2(v[i], v[i + 1]), sc);
                     }
                 }
-                scale = make_float4(scale.y, scale.z, scale.w, 0.f);
             }
             if (!ok) {
                 break;
             }
+            __syncwarp();
+            if (lane == 0) {
+                MbarArrive(&s.scaleEmpty[item & 1]);
+            }
+            item++;
             kb0 += 4;
             if (kb0 >= KB) {
                 int g, mt, nt;
@@ -592,8 +594,8 @@ extern "C" int mf_k_moe_grouped_gemm(const void *a, const float *aScale, const v
     p.rowsTotal = rowsTotal;
     p.wideStores = ((uintptr_t)out & 31) == 0 ? 1 : 0;
     p.vecScales = (K / BK) % 4 == 0 && ((uintptr_t)aScale & 15) == 0 && ((uintptr_t)bScale & 15) == 0 ? 1 : 0;
-    // The wide tile reads A half as often and hands a partial product over half as often: one K-block takes 1050 cycles instead of
-    // 2 x 720. It pays from two m-tiles per expert on if every SM still gets two tiles (8191 rows over 32 experts, N 4096 / K 7168: 389
+    // The wide tile reads A half as often and hands a partial product over half as often: one K-block takes about 950 cycles instead
+    // of 2 x 720. It pays from two m-tiles per expert on if every SM still gets two tiles (8191 rows over 32 experts, N 4096 / K 7168: 353
     // against 455 us); below that the weights' stream is what counts and the finer tiles end more evenly (2048 rows: 201 against 197 us).
     const long long mTiles = (rowsTotal + BM - 1) / BM;
     const bool wide = N % 256 == 0 && mTiles >= 2LL * G && mTiles * (N / 256) >= 2LL * 148;
