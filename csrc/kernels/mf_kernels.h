@@ -144,7 +144,8 @@ typedef struct {
     int *cursor;          // [E] scratch, zero before the first call (the kernel leaves it zero)
     int *expertOffset;    // out: [E/R + 1] first row of each local expert (multiples of 128); last = rows in use
     int *expertCount;     // out: [E/R] valid rows of each local expert
-    int *sendSlot;        // out (optional): [T, K] row each pair was written to on its owner
+    int4 *routed;         // out: [T, K] {row on the owner or -1, owner or -1, weight bits, 0} of each pair: combine reads nothing of the
+                          // caller's, whose tensors may be gone or changed by then
     int *status;          // device int, zero before launch
     int *arrive;          // heap, optional: [cap / 128] rows landed in each 128-row tile of the receive buffer (arrival mode: no
                           // closing barrier; the consumer waits per tile, see mf_k_moe_grouped_gemm_mx_gated). Between two
@@ -170,7 +171,7 @@ typedef struct {
     const int *expertOffset;  // as filled by dispatch
     const int *expertCount;
     void *retY;               // heap: [retRows][H] bf16 landing zone at the source rank, row = token * K + k
-    const int *topkIdx;       // [T, K] as given to dispatch
+    const int4 *routed;       // [T, K] as filled by dispatch
     void *out;                // [T, H] bf16
     int *status;
     unsigned long long *epochState;  // optional: as in mf_moe_dispatch_args_t (a separate pair of words for this kernel)
@@ -178,8 +179,6 @@ typedef struct {
     int cap;                  // rows of the receive buffer (and of y)
     int retRows;              // rows of every rank's landing zone (max tokens * K)
     int reserved;
-    const int *sendSlot;      // optional, both: [T, K] as filled by dispatch and [T, K] weights as given to it. With them a rank gathers the
-    const float *topkW;       // outputs of its own experts directly. The same choice on every rank.
 } mf_moe_combine_args_t;
 
 // H: hidden (multiple of 128), K: experts per token, E: experts in total (multiple of the rank count). Both kernels are

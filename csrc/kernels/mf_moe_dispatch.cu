@@ -296,9 +296,7 @@ mf_moe_dispatch_kernel(const __grid_constant__ mf_moe_dispatch_args_t own, const
                             mySlot = -1;  // the owner's buffer is full: this pair is dropped and the call reports the overflow
                         }
                     }
-                    if (a.sendSlot != nullptr) {
-                        a.sendSlot[t * K + lane] = mySlot;
-                    }
+                    a.routed[t * K + lane] = make_int4(mySlot, myOwner, __float_as_int(myW), 0);
                 }
                 // Pairs of one (token, owner) form groups of up to 1 + MF_MOE_MAX_SIBLINGS in k order; the first of a group leads it.
                 int before = 0, nsib = 0;
@@ -555,7 +553,7 @@ __device__ __forceinline__ void GatherGroup(float (&part)[2][8], uint32_t group,
 // Bound by the traffic of the expert outputs. A rank's own pairs are gathered by token from where dispatch put them: no landing
 // zone is written and read for them and no receive buffer is scanned for leaders (7 of 8 of its rows are followers when one rank
 // owns all experts). One rank, top-8, hidden 7168: 128 tokens 63 -> 8 us, 4096 tokens (530 MB) 247 -> 90 us.
-// ALONE: one rank with sendSlot and topkW and at most eight pairs a token; nothing waits on anything, so it is an ordinary launch.
+// ALONE: one rank and at most eight pairs a token; nothing waits on anything, so it is an ordinary launch.
 template <bool ALONE, bool EMULATED>
 __global__ void __launch_bounds__(kThreads, 3)
 mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const mf_moe_combine_args_t *__restrict__ emulated, int H, int K, int EL, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
@@ -591,9 +589,8 @@ mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const m
     // A call whose dispatch failed (overflow, timeout) moves no data; it still walks through the barriers so that the
     // peers' waits complete.
     const bool dead = ReadAbort(a.status, &abortFlag) != 0;
-    // The rows that this rank computed for its own tokens need no landing zone: dispatch left their places in sendSlot, and the
-    // source gathers them itself below.
-    const bool direct = ALONE || (a.sendSlot != nullptr && a.topkW != nullptr);
+    // The rows that this rank computed for its own tokens need no landing zone: dispatch left their places and weights in `routed`,
+    // and the source gathers them itself below.
 
     // ---- push: one row per (token, owner): the leader's output plus its siblings', weighted, to the source rank's
     //      landing zone [token][k of the leader][:]
@@ -611,7 +608,7 @@ mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const m
         const int4 meta = a.recvMeta[r];
         const uint32_t src = (uint32_t)meta.x;
         const int k = meta.z & 0xff, nsib = (meta.z >> 8) & 0xff;
-        if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || src >= R || (direct && src == m->rankId) || meta.y < 0 || k >= K || (long long)meta.y * K + k >= a.retRows ||
+        if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || src >= R || src == m->rankId || meta.y < 0 || k >= K || (long long)meta.y * K + k >= a.retRows ||
             nsib > MF_MOE_MAX_SIBLINGS) {
             continue;
         }
@@ -655,14 +652,10 @@ mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const m
         int myOwner = -1, mySlot = -1;
         float myW = 0.f;
         if (lane < K) {
-            const int e = a.topkIdx[t * K + lane];
-            if (e >= 0 && e < EL * (int)R) {
-                myOwner = e / EL;
-                if (direct && myOwner == (int)m->rankId) {
-                    mySlot = a.sendSlot[t * K + lane];
-                    myW = a.topkW[t * K + lane];
-                }
-            }
+            const int4 pair = a.routed[t * K + lane];
+            mySlot = pair.x;
+            myOwner = pair.y;
+            myW = __int_as_float(pair.z);
         }
         uint32_t same = 0;
         for (int j = 0; j < K; j++) {
@@ -684,7 +677,7 @@ mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const m
         for (; leaders != 0; leaders &= leaders - 1) {
             const int k = __ffs(leaders) - 1;
             const int owner = __shfl_sync(0xffffffffu, myOwner, k);
-            if (!direct || owner != (int)m->rankId) {
+            if (owner != (int)m->rankId) {
                 const char *rowp = reinterpret_cast<const char *>(a.retY) + ((size_t)t * K + k) * H * 2;
                 uint4 raw[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
                 if (has0) {
@@ -802,7 +795,7 @@ static int LaunchCombine(const mf_moe_combine_args_t *argsHost, const mf_moe_com
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
-    const bool alone = argsHost != nullptr && argsHost->sendSlot != nullptr && argsHost->topkW != nullptr && rankCount == 1 && K <= MF_MOE_MAX_SIBLINGS + 1;
+    const bool alone = argsHost != nullptr && rankCount == 1 && K <= MF_MOE_MAX_SIBLINGS + 1;
     const void *kernel = alone                 ? (const void *)mf_moe_combine_kernel<true, false>
                          : argsHost != nullptr ? (const void *)mf_moe_combine_kernel<false, false>
                                                : (const void *)mf_moe_combine_kernel<false, true>;

@@ -34,9 +34,9 @@ struct MoePlan {
     int Dispatch(uint64_t x, uint64_t idx, uint64_t w, int T, uint64_t epoch, bool overlap, int dedupMinPairs, uint64_t stream)
     {
         d.x = (const void *)x;
-        d.topkIdx = c.topkIdx = (const int *)idx;
-        d.topkW = c.topkW = (const float *)w;
-        d.T = T;
+        d.topkIdx = (const int *)idx;
+        d.topkW = (const float *)w;
+        d.T = c.T = T;
         d.arrive = overlap ? arrive : nullptr;
         d.dedupMinPairs = dedupMinPairs;
         // One CTA per token: small batches get a small grid (its grid-wide barriers are cheaper), large ones every SM.
@@ -57,11 +57,11 @@ struct MoePlan {
         return mf_k_moe_grouped_gemm_mx(h1Q, (const uint32_t *)h1Sf, (const void *)w2Q, (const float *)w2S, const_cast<void *>(c.y), nullptr, d.expertOffset,
                                         d.expertCount, el, rows, hidden, inter, mode2, 0, d.status, 0, (mf_stream_t)stream);
     }
-    int Combine(int T, uint64_t epoch, uint64_t stream)
+    // Of the tokens that were dispatched, whatever count the caller asks to see.
+    int Combine(uint64_t epoch, uint64_t stream)
     {
-        c.T = T;
         // One warp per 1 KiB piece of a returned row; alone, a rank has no rows to return and one warp sums each 1 KiB of a token.
-        const long long pieces = (long long)T * (world == 1 ? 1 : topk) * ((hidden / 8 + 63) / 64);
+        const long long pieces = (long long)c.T * (world == 1 ? 1 : topk) * ((hidden / 8 + 63) / 64);
         const int ctas = (int)((pieces + 7) / 8 < 65536 ? (pieces + 7) / 8 : 65536);
         return mf_k_moe_combine_rank(&c, world, hidden, topk, experts / world, combineChannel, epoch, timeoutNs, ctas > 1 ? ctas : 1, (mf_stream_t)stream);
     }
@@ -129,7 +129,7 @@ void BindOps(py::module_ &m)
     ops.attr("MOE_COMBINE_ARGS_BYTES") = (int)sizeof(mf_moe_combine_args_t);
     ops.def("pack_moe_dispatch_args", [](uint64_t meta, uint64_t x, uint64_t topkIdx, uint64_t topkW, uint64_t cnt, uint64_t recvX, uint64_t recvSf,
                                          uint64_t recvMeta, uint64_t recvSib, uint64_t localCnt, uint64_t cursor, uint64_t expertOffset, uint64_t expertCount,
-                                         uint64_t sendSlot, uint64_t status, int T, int cap, uint64_t arrive, int dedupMinPairs, uint64_t epochState) {
+                                         uint64_t routed, uint64_t status, int T, int cap, uint64_t arrive, int dedupMinPairs, uint64_t epochState) {
         mf_moe_dispatch_args_t a{};
         a.arrive = (int *)arrive;
         a.dedupMinPairs = dedupMinPairs;
@@ -147,20 +147,17 @@ void BindOps(py::module_ &m)
         a.cursor = (int *)cursor;
         a.expertOffset = (int *)expertOffset;
         a.expertCount = (int *)expertCount;
-        a.sendSlot = (int *)sendSlot;
+        a.routed = (int4 *)routed;
         a.status = (int *)status;
         a.T = T;
         a.cap = cap;
         return py::bytes((const char *)&a, sizeof(a));
     }, py::arg("meta"), py::arg("x"), py::arg("topk_idx"), py::arg("topk_w"), py::arg("cnt"), py::arg("recv_x"), py::arg("recv_sf"), py::arg("recv_meta"),
-            py::arg("recv_sib"), py::arg("local_cnt"), py::arg("cursor"), py::arg("expert_offset"), py::arg("expert_count"), py::arg("send_slot"),
+            py::arg("recv_sib"), py::arg("local_cnt"), py::arg("cursor"), py::arg("expert_offset"), py::arg("expert_count"), py::arg("routed"),
             py::arg("status"), py::arg("T"), py::arg("cap"), py::arg("arrive") = 0, py::arg("dedup_min_pairs") = 0, py::arg("epoch_state") = 0);
     ops.def("pack_moe_combine_args", [](uint64_t meta, uint64_t y, uint64_t recvMeta, uint64_t recvSib, uint64_t expertOffset, uint64_t expertCount,
-                                        uint64_t retY, uint64_t topkIdx, uint64_t out, uint64_t status, int T, int cap, int retRows, uint64_t epochState,
-                                        uint64_t sendSlot, uint64_t topkW) {
+                                        uint64_t retY, uint64_t routed, uint64_t out, uint64_t status, int T, int cap, int retRows, uint64_t epochState) {
         mf_moe_combine_args_t a{};
-        a.sendSlot = (const int *)sendSlot;
-        a.topkW = (const float *)topkW;
         a.epochState = (unsigned long long *)epochState;
         a.meta = (const void *)meta;
         a.y = (const void *)y;
@@ -169,7 +166,7 @@ void BindOps(py::module_ &m)
         a.expertOffset = (const int *)expertOffset;
         a.expertCount = (const int *)expertCount;
         a.retY = (void *)retY;
-        a.topkIdx = (const int *)topkIdx;
+        a.routed = (const int4 *)routed;
         a.out = (void *)out;
         a.status = (int *)status;
         a.T = T;
@@ -177,8 +174,7 @@ void BindOps(py::module_ &m)
         a.retRows = retRows;
         return py::bytes((const char *)&a, sizeof(a));
     }, py::arg("meta"), py::arg("y"), py::arg("recv_meta"), py::arg("recv_sib"), py::arg("expert_offset"), py::arg("expert_count"), py::arg("ret_y"),
-            py::arg("topk_idx"), py::arg("out"), py::arg("status"), py::arg("T"), py::arg("cap"), py::arg("ret_rows"), py::arg("epoch_state") = 0,
-            py::arg("send_slot") = 0, py::arg("topk_w") = 0);
+            py::arg("routed"), py::arg("out"), py::arg("status"), py::arg("T"), py::arg("cap"), py::arg("ret_rows"), py::arg("epoch_state") = 0);
     ops.def("moe_dispatch", [](uint64_t argsDev, int nEmulated, int rankCount, int H, int K, int E, uint32_t channel, uint64_t epoch, uint64_t timeoutNs,
                                int ctas, uint64_t stream) {
         return mf_k_moe_dispatch((const mf_moe_dispatch_args_t *)argsDev, nEmulated, rankCount, H, K, E, channel, epoch, timeoutNs, ctas,
@@ -241,7 +237,7 @@ void BindOps(py::module_ &m)
         });
     py::class_<MoePlan>(ops, "MoePlan")
         .def(py::init([](uint64_t meta, uint64_t cnt, uint64_t recvX, uint64_t recvSf, uint64_t recvMeta, uint64_t recvSib, uint64_t localCnt,
-                         uint64_t cursor, uint64_t expertOffset, uint64_t expertCount, uint64_t sendSlot, uint64_t arrive, uint64_t status, uint64_t h1Q,
+                         uint64_t cursor, uint64_t expertOffset, uint64_t expertCount, uint64_t routed, uint64_t arrive, uint64_t status, uint64_t h1Q,
                          uint64_t h1Sf, uint64_t y, uint64_t retY, uint64_t out, int cap, int retRows, int world, int hidden, int topk, int experts,
                          int inter, uint32_t dispatchChannel, uint32_t combineChannel, uint64_t timeoutNs, uint64_t waitNs, uint64_t epochD,
                          uint64_t epochC) {
@@ -260,8 +256,8 @@ void BindOps(py::module_ &m)
             p.c.expertOffset = (const int *)expertOffset;
             p.d.expertCount = (int *)expertCount;
             p.c.expertCount = (const int *)expertCount;
-            p.d.sendSlot = (int *)sendSlot;
-            p.c.sendSlot = (const int *)sendSlot;
+            p.d.routed = (int4 *)routed;
+            p.c.routed = (const int4 *)routed;
             p.d.status = p.c.status = (int *)status;
             p.d.epochState = (unsigned long long *)epochD;
             p.c.epochState = (unsigned long long *)epochC;
@@ -293,7 +289,7 @@ void BindOps(py::module_ &m)
             if (rc == MF_K_OK) {
                 rc = p.Experts(w13Q, w13S, w13Packed, w2Q, w2S, w2Packed, overlap, stream);
             }
-            return rc == MF_K_OK ? p.Combine(T, epochC, stream) : rc;
+            return rc == MF_K_OK ? p.Combine(epochC, stream) : rc;
         });
     ops.def("allreduce_rmsnorm", [](uint64_t argsDev, int nEmulated, int rankCount, int T, int H, float eps, int algo, uint32_t channel, uint64_t epoch,
                                     uint64_t timeoutNs, int ctas, uint64_t stream) {

@@ -82,7 +82,8 @@ class _RankState:
         self.cursor = torch.zeros(n_experts, dtype=torch.int32, device=device)
         self.expert_offset = torch.zeros(el + 1, dtype=torch.int32, device=device)
         self.expert_count = torch.zeros(el, dtype=torch.int32, device=device)
-        self.send_slot = torch.zeros(max_tokens * topk, dtype=torch.int32, device=device)
+        # row on the owner, owner and weight of every pair, from dispatch to combine
+        self.routed = torch.zeros(max_tokens * topk, 4, dtype=torch.int32, device=device)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self.max_rows_ret = max_tokens * topk
         self.h1_q = torch.empty(cap, inter, dtype=torch.float8_e4m3fn, device=device)
@@ -137,7 +138,7 @@ class FusedMoE(_MoEBase):
         st = self.st
         self._plan = _ops.MoePlan(heap.meta_ptr, st.cnt.data_ptr(), st.recv_x.data_ptr(), st.recv_s.data_ptr(), st.recv_m.data_ptr(),
                                   st.recv_sib.data_ptr(), st.local_cnt.data_ptr(), st.cursor.data_ptr(), st.expert_offset.data_ptr(),
-                                  st.expert_count.data_ptr(), st.send_slot.data_ptr(), st.arrive.data_ptr(), st.status.data_ptr(), st.h1_q.data_ptr(),
+                                  st.expert_count.data_ptr(), st.routed.data_ptr(), st.arrive.data_ptr(), st.status.data_ptr(), st.h1_q.data_ptr(),
                                   st.h1_sf.data_ptr(), st.y.data_ptr(), st.ret_y.data_ptr(), st.out.data_ptr(), st.cap, st.max_rows_ret, heap.world, hidden,
                                   topk, n_experts, inter, CH_DISPATCH, CH_COMBINE, timeout_ns, self.wait_ns,
                                   self._epoch_d.data_ptr() if device_epochs else 0, self._epoch_c.data_ptr() if device_epochs else 0)
@@ -176,7 +177,7 @@ class FusedMoE(_MoEBase):
 
     def combine(self, T, stream=None):
         s = stream.cuda_stream if stream is not None else current_stream_handle()
-        rc = self._plan.combine(T, self._epoch(CH_COMBINE), s)
+        rc = self._plan.combine(self._epoch(CH_COMBINE), s)
         if rc != 0:
             raise RuntimeError(f"moe_combine launch failed ({rc})")
         self.launches += 1
@@ -240,11 +241,11 @@ class EmulatedMoE(_MoEBase):
             st, rk = self.states[r], self.eheap.ranks[r]
             d += _ops.pack_moe_dispatch_args(rk.meta_ptr, xs[r].data_ptr(), idxs[r].data_ptr(), ws[r].data_ptr(), st.cnt.data_ptr(), st.recv_x.data_ptr(),
                                              st.recv_s.data_ptr(), st.recv_m.data_ptr(), st.recv_sib.data_ptr(), st.local_cnt.data_ptr(), st.cursor.data_ptr(),
-                                             st.expert_offset.data_ptr(), st.expert_count.data_ptr(), st.send_slot.data_ptr(), st.status.data_ptr(), T, st.cap,
+                                             st.expert_offset.data_ptr(), st.expert_count.data_ptr(), st.routed.data_ptr(), st.status.data_ptr(), T, st.cap,
                                              st.arrive.data_ptr() if self.overlap else 0, self.dedup_min_pairs)
             c += _ops.pack_moe_combine_args(rk.meta_ptr, st.y.data_ptr(), st.recv_m.data_ptr(), st.recv_sib.data_ptr(), st.expert_offset.data_ptr(),
-                                            st.expert_count.data_ptr(), st.ret_y.data_ptr(), idxs[r].data_ptr(), st.out.data_ptr(), st.status.data_ptr(),
-                                            T, st.cap, st.max_rows_ret, 0, st.send_slot.data_ptr(), ws[r].data_ptr())
+                                            st.expert_count.data_ptr(), st.ret_y.data_ptr(), st.routed.data_ptr(), st.out.data_ptr(), st.status.data_ptr(),
+                                            T, st.cap, st.max_rows_ret)
         dargs = torch.frombuffer(bytearray(d), dtype=torch.uint8).cuda()
         cargs = torch.frombuffer(bytearray(c), dtype=torch.uint8).cuda()
         s = torch.cuda.current_stream().cuda_stream

@@ -85,6 +85,57 @@ def test_moe_layer_skips_masked_pairs(heap):
     assert float(out[7].float().abs().max()) == 0.0
 
 
+def _routed_layer(heap, T, H, E, K, I, seed, **kw):
+    import torch
+
+    from memfabric_hybrid_b200.ops.moe import FusedMoE, route
+
+    layer = FusedMoE(heap, T, H, E, K, I, *_weights(E, H, I, seed), **kw)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    return (layer, x) + route(torch.randn(T, E, generator=g, device="cuda"), K)
+
+
+@pytest.mark.parametrize("change", ["gone", "in_place"])
+def test_combine_needs_nothing_of_what_dispatch_was_given(heap, change):
+    """Routing that was a temporary of the dispatch call, its memory handed out again; and routing changed before combine."""
+    import torch
+
+    T, K = 60, 4
+    layer, x, idx, tw = _routed_layer(heap, T, 512, 8, K, 128, 21)
+    want = layer(x, idx, tw * 2.5).clone()
+    torch.cuda.synchronize()
+    if change == "gone":
+        layer.dispatch(x, idx.clone(), tw * 2.5)
+        torch.cuda.synchronize()
+        reused = [torch.full((T, K), v, device="cuda", dtype=d) for d, v in ((torch.int32, 0), (torch.float32, 100.0)) for _ in range(4)]
+    else:
+        idx, tw = idx.clone(), tw * 2.5
+        layer.dispatch(x, idx, tw)
+        idx.zero_()
+        tw.fill_(100.0)
+    layer.experts()
+    assert torch.equal(layer.combine(T), want) and layer.check_status() == 0
+    if change == "gone":
+        del reused
+
+
+@pytest.mark.parametrize("asked", [1, 30, 64])
+def test_combine_sums_the_tokens_that_were_dispatched(heap, asked):
+    """Another count given to combine() selects rows of the result, it does not reach past the routing of this call."""
+    import torch
+
+    T, most = 40, 64
+    layer, x, idx, tw = _routed_layer(heap, most, 512, 8, 4, 128, 22)
+    x, idx, tw = x[:T].clone(), idx[:T].clone(), tw[:T].clone()
+    want = layer(x, idx, tw).clone()
+    layer.st.out.fill_(7.0)
+    layer.dispatch(x, idx, tw)
+    layer.experts()
+    assert layer.combine(asked).shape == (asked, 512)
+    assert torch.equal(layer.st.out[:T], want) and bool((layer.st.out[T:] == 7.0).all())
+
+
 def test_moe_layer_looks_at_its_weights_on_every_call(heap):
     import torch
 
