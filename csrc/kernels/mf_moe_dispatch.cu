@@ -520,11 +520,13 @@ __device__ __forceinline__ void GatherGroup(float (&part)[2][8], uint32_t group,
             const bool any = group != 0 && left > 0;
             const int j = any ? __ffs(group) - 1 : 0;
             const int row = __shfl_sync(0xffffffffu, myRow, j);
-            w[i] = __shfl_sync(0xffffffffu, myW, j);
+            const float weight = __shfl_sync(0xffffffffu, myW, j);
+            const bool taken = any && row >= 0 && row < rows;
+            w[i] = taken ? weight : 0.f;  // an infinite weight must not meet the zeros of a slot that holds no row
             group &= group - 1;
             left--;
             raw[i][0] = raw[i][1] = make_uint4(0u, 0u, 0u, 0u);
-            if (any && row >= 0 && row < rows) {
+            if (taken) {
                 const char *rowp = reinterpret_cast<const char *>(y) + (size_t)row * rowBytes + (size_t)v0 * 16;
                 if (v0 < vecs) {
                     raw[i][0] = mf_ld16(rowp);

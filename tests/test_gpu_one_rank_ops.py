@@ -136,6 +136,22 @@ def test_combine_sums_the_tokens_that_were_dispatched(heap, asked):
     assert torch.equal(layer.st.out[:T], want) and bool((layer.st.out[T:] == 7.0).all())
 
 
+@pytest.mark.parametrize("K", [1, 2, 3, 6])
+def test_combine_keeps_an_infinite_weight_infinite(heap, K):
+    """The rows of a token are read four at a time; the slots that hold no row add nothing, whatever the first weight is."""
+    import torch
+
+    T = 5
+    layer, x, idx, tw = _routed_layer(heap, T, 512, 8, K, 128, 23)
+    tw = tw.clone()
+    plain = layer(x, idx, tw).float()
+    tw[2, 0] = float("inf")
+    out = layer(x, idx, tw).float()
+    assert bool(out[2].isinf().all())
+    keep = [0, 1, 3, 4]
+    assert torch.equal(out[keep], plain[keep]) and layer.check_status() == 0
+
+
 def test_moe_layer_looks_at_its_weights_on_every_call(heap):
     import torch
 
