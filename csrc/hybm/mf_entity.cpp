@@ -752,29 +752,25 @@ uint32_t MemEntity::ReachTypes(uint32_t rank)
     return tags_->AllowedOps(opt_.rankId, rank, base & (opt_.dataOpType | OP_HOST_RDMA | OP_KERNEL_LDST | OP_COPY_ENGINE));
 }
 
-bool MemEntity::AddressInEntity(uint64_t addr, uint64_t len)
+bool MemEntity::AddressInEntity(uint64_t addr, uint64_t len, PlacedRange *placed)
 {
     // Window arithmetic is not enough: a rank that left (or died) leaves a hole in the window. Only ranges that are
     // backed right now — local slices, mapped peers, registered user memory — count.
     AllocatedRange a;
-    return VaManager::Instance().FindAllocated(addr, len, &a) && a.entityId == id_;
-}
-
-MemEntity::PlacedRange MemEntity::PlacementOf(uint64_t addr)
-{
-    // Inside one backed range of one window everything that placing an address looks at (class, visibility, owner, remoteness)
-    // is the same. Ranges outside the windows (registered user memory, other entities) are not remembered.
-    AllocatedRange a;
-    if (!VaManager::Instance().FindAllocated(addr, 1, &a) || a.entityId != id_) {
-        return PlacedRange{};
+    if (!VaManager::Instance().FindAllocated(addr, len, &a) || a.entityId != id_) {
+        return false;
     }
-    for (MemSegment *seg : {hbm_.get(), dram_.get()}) {
-        if (seg != nullptr && seg->InWindow(addr, 1)) {
-            const bool whole = seg->InWindow(a.gva, a.size) && seg->RankOf(a.gva) == seg->RankOf(a.gva + a.size - 1);
-            return whole ? PlacedRange{a.gva, a.gva + a.size} : PlacedRange{};
+    if (placed != nullptr) {
+        // Inside one backed range of one window everything that placing an address looks at (class, visibility, owner, remoteness)
+        // is the same. Ranges outside the windows (registered user memory) are not remembered.
+        *placed = PlacedRange{};
+        for (MemSegment *seg : {hbm_.get(), dram_.get()}) {
+            if (seg != nullptr && seg->InWindow(a.gva, a.size) && seg->RankOf(a.gva) == seg->RankOf(a.gva + a.size - 1)) {
+                *placed = PlacedRange{a.gva, a.gva + a.size};
+            }
         }
     }
-    return PlacedRange{};
+    return true;
 }
 
 uint32_t MemEntity::RankOfAddress(uint64_t addr)
@@ -924,8 +920,9 @@ int MemEntity::BatchCopyData(const BatchCopyParams &p, CopyDirection dir, void *
     size_t last = 0;
     // Blocks of one pool usually lie in one backed range per side. Once an element has been placed, every further one whose two
     // sides fall into the same two ranges belongs to the same group, so only the bounds are compared: about 2 ns an element
-    // instead of 75 ns for up to eight locked look-ups (3904 elements: 290 us -> 8 us). Index lists are only kept from
-    // the second group on.
+    // instead of 75 ns for up to six locked look-ups (3904 elements: 290 us -> 8 us). The ranges come from the look-ups that
+    // placing an element takes anyway, so a batch that never falls into them (local memory on one side, ranges that alternate)
+    // costs no more than without. Index lists are only kept from the second group on.
     PlacedRange seenSrc, seenDst;
     bool grouped = false;
     for (uint32_t i = 0; i < p.batchSize; i++) {
@@ -946,11 +943,12 @@ int MemEntity::BatchCopyData(const BatchCopyParams &p, CopyDirection dir, void *
             MF_ERROR("batch copy: element #" << i << " cannot be placed");
             return rc;
         }
+        seenSrc = seenDst = PlacedRange{};
         if (SrcClassOf(d) >= PC_GLOBAL_HOST) {
-            MF_CHECK_RET(AddressInEntity(sa, len), BM_INVALID_PARAM, "batch copy: source #" << i << " leaves the pool");
+            MF_CHECK_RET(AddressInEntity(sa, len, &seenSrc), BM_INVALID_PARAM, "batch copy: source #" << i << " leaves the pool");
         }
         if (DstClassOf(d) >= PC_GLOBAL_HOST) {
-            MF_CHECK_RET(AddressInEntity(da, len), BM_INVALID_PARAM, "batch copy: destination #" << i << " leaves the pool");
+            MF_CHECK_RET(AddressInEntity(da, len, &seenDst), BM_INVALID_PARAM, "batch copy: destination #" << i << " leaves the pool");
         }
         if (groups.empty() || !sameGroup(groups[last], d, opt)) {
             last = groups.size();
@@ -972,8 +970,6 @@ int MemEntity::BatchCopyData(const BatchCopyParams &p, CopyDirection dir, void *
         if (grouped) {
             groups[last].idx.push_back(i);
         }
-        seenSrc = PlacementOf(sa);
-        seenDst = PlacementOf(da);
     }
     if (!grouped && (groups[0].opt.srcRemote || groups[0].opt.dstRemote)) {
         groups[0].idx.resize(p.batchSize);

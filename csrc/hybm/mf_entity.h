@@ -66,15 +66,14 @@ public:
     int BatchCopyData(const BatchCopyParams &p, CopyDirection dir, void *stream, uint32_t flags);
     int Wait();
 
-    bool AddressInEntity(uint64_t addr, uint64_t len);
-    // Owner rank of a pooled address; RANK_MAX if the address is not pooled in this entity.
-    uint32_t RankOfAddress(uint64_t addr);
     // A backed address range whose every address is placed alike ([0, 0): none).
     struct PlacedRange {
         uint64_t begin{0}, end{0};
         bool Holds(uint64_t addr, uint64_t len) const { return addr >= begin && addr < end && (len == 0 ? 1 : len) <= end - addr; }
     };
-    PlacedRange PlacementOf(uint64_t addr);
+    bool AddressInEntity(uint64_t addr, uint64_t len, PlacedRange *placed = nullptr);
+    // Owner rank of a pooled address; RANK_MAX if the address is not pooled in this entity.
+    uint32_t RankOfAddress(uint64_t addr);
     PtrClass Classify(uint64_t addr, bool *deviceVisible);
     const DeviceMeta *DeviceMetaPtr() const { return devMeta_; }
     DeviceMeta HostMeta() const { return hostMeta_; }

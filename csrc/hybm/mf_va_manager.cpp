@@ -159,6 +159,7 @@ void VaManager::RemoveEntity(uint32_t entityId)
 bool VaManager::FindAllocated(uint64_t addr, uint64_t len, AllocatedRange *out)
 {
     std::lock_guard<std::mutex> g(mu_);
+    lookups_++;
     if (allocated_.empty()) {
         return false;
     }
@@ -178,6 +179,12 @@ bool VaManager::FindAllocated(uint64_t addr, uint64_t len, AllocatedRange *out)
         *out = a;
     }
     return true;
+}
+
+uint64_t VaManager::Lookups()
+{
+    std::lock_guard<std::mutex> g(mu_);
+    return lookups_;
 }
 
 bool VaManager::IsGva(uint64_t addr) { return FindReserved(addr, nullptr); }

@@ -51,6 +51,7 @@ public:
     void RemoveEntity(uint32_t entityId);
     // Range containing [addr, addr+len). len 0 is treated as 1.
     bool FindAllocated(uint64_t addr, uint64_t len, AllocatedRange *out);
+    uint64_t Lookups();  // calls of FindAllocated so far
     bool IsGva(uint64_t addr);
     PtrClass Classify(uint64_t addr);  // PC_GLOBAL_* if inside an allocated range, PC_UNKNOWN otherwise
     std::string Dump();
@@ -61,6 +62,7 @@ private:
     std::mutex mu_;
     std::map<uint64_t, ReservedRange> reserved_;
     std::map<uint64_t, AllocatedRange> allocated_;
+    uint64_t lookups_{0};
 };
 
 // Opaque slice handle (reference: src/hybm/csrc/mm/hybm_mem_slice.h:20-36): 40-bit magic | 16-bit index | 4-bit memory

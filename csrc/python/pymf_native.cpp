@@ -437,6 +437,7 @@ void BindNative(py::module_ &m)
         d["runtime"] = c.runtimeVersion;
         return d;
     });
+    n.def("va_lookups", []() { return hybm::VaManager::Instance().Lookups(); });
     n.def("data_op_stats", []() {
         hybm::DataOpStats st = hybm::GetDataOpStats();
         py::dict d;

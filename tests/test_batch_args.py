@@ -71,3 +71,27 @@ def test_elements_of_several_groups_keep_their_data(mf, pool, pattern):
     for i, k in enumerate(kinds):
         want = local if k == "l" else pooled
         assert (dst[64 * i:64 * i + 64] == want[64 * i:64 * i + 64]).all(), i
+
+
+@pytest.mark.parametrize("kind,per_element", [("local", 3), ("registered", 4), ("pool_then_registered", 3)])
+def test_placing_elements_that_share_no_range_costs_their_own_look_ups(mf, pool, kind, per_element):
+    """Elements with a side outside the pool's windows are placed one by one. Per element: two look-ups for the class of a side
+    outside the windows and its owner, and one per side that has to lie in the pool; none for remembering ranges that are of no use."""
+    n = 200
+    base = pool.dram()
+    outside = np.random.default_rng(11).integers(0, 256, 64 * n, dtype=np.uint8)
+    inside = _fill(base, 64 * n, 12)
+    dst = _fill(base + 4 * MiB, 64 * n, 13)
+    if kind != "local":
+        assert pool.handle.register(outside.ctypes.data, outside.size) == 0, mf.get_last_err_msg()
+    try:
+        from_pool = [kind == "pool_then_registered" and i % 2 == 0 for i in range(n)]
+        srcs = [base + 64 * i if p else outside.ctypes.data + 64 * i for i, p in enumerate(from_pool)]
+        before = mf.native.va_lookups()
+        assert pool.handle.copy_data_batch(srcs, [base + 4 * MiB + 64 * i for i in range(n)], [64] * n, n, mf.bm.BmCopyType.AUTO, 0) == 0
+        assert mf.native.va_lookups() - before <= per_element * n + 8
+        for i, p in enumerate(from_pool):
+            assert (dst[64 * i:64 * i + 64] == (inside if p else outside)[64 * i:64 * i + 64]).all(), i
+    finally:
+        if kind != "local":
+            assert pool.handle.unregister(outside.ctypes.data) == 0
