@@ -89,7 +89,6 @@ constexpr size_t kArenaDefault = 2u << 20;
 struct ThreadCtx {
     StageArena arena;
     std::vector<mf_copy_desc_t> scratch;
-    cudaEvent_t order{nullptr};  // see OrderAfterProducers
 };
 
 class KernelDataOp : public DataOperator {
@@ -116,7 +115,6 @@ public:
             return BM_NOT_SUPPORTED;
         }
         cudaStream_t s = opt.stream != nullptr ? (cudaStream_t)opt.stream : cu::ThreadStream(device_);
-        OrderAfterProducers(dir, opt, s);
         int rc = mf_k_xcopy(p.dest, p.src, p.dataSize, 0, (mf_stream_t)s);
         if (rc != MF_K_OK) {
             MF_ERROR("kernel engine: xcopy launch failed");
@@ -132,7 +130,6 @@ public:
         }
         ThreadCtx *ctx = Ctx();
         cudaStream_t s = opt.stream != nullptr ? (cudaStream_t)opt.stream : cu::ThreadStream(device_);
-        OrderAfterProducers(dir, opt, s);
         // All addresses and lengths multiples of 16: the bulk-copy kernel, else the load/store kernel.
         uint64_t total = 0, bits = 0;
         for (uint32_t i = 0; i < p.batchSize; i++) {
@@ -258,33 +255,6 @@ private:
         }
         MF_CHECK_RET(rc == MF_K_OK, BM_ERROR, "kernel engine: batch launch failed");
         return BM_OK;
-    }
-
-    // A call without a stream runs on this thread's own stream, which does not wait for the default one. Where one side is the
-    // caller's own device buffer, what was queued for that buffer on the default stream (a producer, a fill) has to come first:
-    // a copy that starts within microseconds at high priority would overtake it. An idle default stream costs one query;
-    // copies between pool addresses, which the library alone places, are not ordered.
-    void OrderAfterProducers(CopyDirection dir, const ExtOptions &opt, cudaStream_t s)
-    {
-        if (opt.stream != nullptr || (SrcClassOf(dir) != PC_LOCAL_DEVICE && DstClassOf(dir) != PC_LOCAL_DEVICE)) {
-            return;
-        }
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(cudaStreamLegacy, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-            (void)cudaGetLastError();  // another thread captures a graph: the default stream must not be touched
-            return;
-        }
-        if (cudaStreamQuery(cudaStreamLegacy) == cudaErrorNotReady) {
-            ThreadCtx *ctx = Ctx();
-            if (ctx->order == nullptr && cudaEventCreateWithFlags(&ctx->order, cudaEventDisableTiming) != cudaSuccess) {
-                (void)cudaGetLastError();
-                cudaStreamSynchronize(cudaStreamLegacy);
-                return;
-            }
-            cudaEventRecord(ctx->order, cudaStreamLegacy);
-            cudaStreamWaitEvent(s, ctx->order, 0);
-        }
-        (void)cudaGetLastError();
     }
 
     // Hands back the ranges whose kernels have finished; with `block` it waits for the oldest one.

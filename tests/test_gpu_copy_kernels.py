@@ -138,3 +138,30 @@ def test_enqueued_copies_keep_stream_order(mf, pool, kind):
         at = to
     torch.cuda.synchronize()
     assert torch.equal(device_tensor_from_gva(at, n), want)
+
+
+@pytest.mark.parametrize("form", ["single", "batch", "engine"])
+def test_a_copy_without_a_stream_does_not_wait_for_the_default_stream(mf, pool, form):
+    """Buffers of the caller's own device memory are copied while the default stream is busy with something else."""
+    import torch
+
+    n = {"single": 512 * KiB, "batch": 512 * KiB, "engine": 8 * MiB}[form]
+    mine = torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda")
+    host = torch.empty(n, dtype=torch.uint8).pin_memory()
+    to, T = pool.hbm() + 4 * MiB, mf.bm.BmCopyType
+    busy = torch.cuda.Event()
+    for turn in range(2):  # the first round loads the kernels
+        torch.cuda.synchronize()
+        torch.cuda._sleep(2000 if turn == 0 else 600_000_000)  # at least 0.3 s
+        busy.record()
+        if form == "batch":
+            rc = pool.handle.copy_data_batch([mine.data_ptr() + i * 4096 for i in range(n // 4096)], [to + i * 4096 for i in range(n // 4096)][::-1],
+                                             [4096] * (n // 4096), n // 4096, T.L2G, 0)
+        else:
+            rc = pool.handle.copy_data(mine.data_ptr(), to, n, T.L2G, 0)
+            if form == "engine":
+                rc |= pool.handle.copy_data(to, host.data_ptr(), n, T.G2H, 0)
+        still = not busy.query()
+        assert rc == 0, mf.get_last_err_msg()
+    assert still, "the copy waited for the default stream"
+    torch.cuda.synchronize()

@@ -296,6 +296,7 @@ def _two_rank_worker(rank, port, bar, q):
         assert (out == expect).all(), "peer DRAM push mismatch"
         # pull from the peer (remote read) and a batch of KV-like blocks
         pulled = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()  # the pool's synchronous copies run on the library's own stream, not on torch's
         assert pool.handle.copy_data(pool.hbm(peer) + 16 * MiB + 1, pulled.data_ptr(), n, T.G2L, 0) == 0
         assert (pulled.cpu().numpy() == np.random.default_rng(100 + rank).integers(0, 256, n, dtype=np.uint8)).all()
         assert pool.handle.get_rank_id_by_gva(pool.hbm(peer) + 5) == peer
