@@ -89,11 +89,18 @@ constexpr size_t kArenaDefault = 2u << 20;
 struct ThreadCtx {
     StageArena arena;
     std::vector<mf_copy_desc_t> scratch;
+    uint32_t index{0};  // which pair of fault words
 };
 
 class KernelDataOp : public DataOperator {
 public:
     explicit KernelDataOp(int device) : device_(device) {}
+    ~KernelDataOp() override
+    {
+        if (faults_ != nullptr) {
+            cudaFreeHost(faults_);
+        }
+    }
     uint32_t Type() const override { return OP_KERNEL_LDST; }
     const char *Name() const override { return "kernel_ldst"; }
 
@@ -101,6 +108,12 @@ public:
     {
         MF_CHECK_RET(cu::Available() && device_ >= 0, BM_NOT_SUPPORTED, "kernel engine: no GPU");
         MF_CUDA_CHECK_RET(cudaSetDevice(device_), BM_ERROR);
+        if (faults_ == nullptr) {
+            void *p = nullptr;
+            MF_CUDA_CHECK_RET(cudaHostAlloc(&p, kFaultPairs * 2 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), BM_ERROR);
+            std::memset(p, 0, kFaultPairs * 2 * sizeof(int));
+            faults_ = (int *)p;
+        }
         return BM_OK;
     }
 
@@ -115,12 +128,13 @@ public:
             return BM_NOT_SUPPORTED;
         }
         cudaStream_t s = opt.stream != nullptr ? (cudaStream_t)opt.stream : cu::ThreadStream(device_);
-        int rc = mf_k_xcopy(p.dest, p.src, p.dataSize, 0, (mf_stream_t)s);
+        int *fault = FaultWord(Ctx(), opt);
+        int rc = mf_k_xcopy(p.dest, p.src, p.dataSize, 0, fault, (mf_stream_t)s);
         if (rc != MF_K_OK) {
             MF_ERROR("kernel engine: xcopy launch failed");
             return BM_ERROR;
         }
-        return (opt.flags & FLAG_ASYNC_COPY) ? BM_OK : BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
+        return (opt.flags & FLAG_ASYNC_COPY) ? BM_OK : Finish(s, fault);
     }
 
     int BatchDataCopy(const BatchCopyParams &p, CopyDirection dir, const ExtOptions &opt) override
@@ -138,19 +152,35 @@ public:
         }
         int rc = BM_OK;
         if ((bits & 15) == 0) {
-            rc = BulkBatch(p, total, (mf_stream_t)s);
+            rc = BulkBatch(p, total, FaultWord(ctx, opt), (mf_stream_t)s);
         } else {
             rc = LoadStoreBatch(p, ctx, s);
         }
         if (rc != BM_OK) {
             return rc;
         }
-        return (opt.flags & FLAG_ASYNC_COPY) ? BM_OK : BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
+        return (opt.flags & FLAG_ASYNC_COPY) ? BM_OK : Finish(s, FaultWord(ctx, opt));
     }
 
-    int Wait() override { return BoundedStreamSync(device_, nullptr, DefaultSyncTimeoutMs()); }
+    int Wait() override { return Finish(nullptr, faults_ + 2 * Ctx()->index + 1); }
 
 private:
+    // Every thread has two words that a copy whose pipeline waits ran out sets: one for the calls that wait themselves, one for
+    // those that Wait() completes. Threads beyond the table share them, which can at worst report a failure to the wrong one.
+    static constexpr uint32_t kFaultPairs = 1024;
+    int *FaultWord(const ThreadCtx *ctx, const ExtOptions &opt) const { return faults_ + 2 * ctx->index + ((opt.flags & FLAG_ASYNC_COPY) ? 1 : 0); }
+    int Finish(cudaStream_t s, int *fault) const
+    {
+        const int rc = BoundedStreamSync(device_, s, DefaultSyncTimeoutMs());
+        volatile int *word = fault;
+        if (rc == BM_OK && *word != 0) {
+            *word = 0;
+            MF_ERROR("kernel engine: a bulk copy gave up waiting for its loads");
+            return BM_TIMEOUT;
+        }
+        return rc;
+    }
+
     static constexpr uint32_t kChunkShift = 15;
     static_assert((1u << kChunkShift) == MF_BATCH_CHUNK_BYTES, "chunk size of the load/store kernel");
 
@@ -187,7 +217,7 @@ private:
 
     // Pieces of the descriptor list ride in the parameters of one launch each; the first is short, so that the GPU starts early,
     // and the list of the next is written while it works (32 requests of 122 blocks: 179 us with one staged table).
-    static int BulkBatch(const BatchCopyParams &p, uint64_t total, mf_stream_t s)
+    static int BulkBatch(const BatchCopyParams &p, uint64_t total, int *fault, mf_stream_t s)
     {
         const uint32_t shift = mf_k_batch_bulk_shift(total), round = (1u << shift) - 1;
         thread_local std::unique_ptr<mf_copy_desc_t[]> piece(new mf_copy_desc_t[MF_BULK_INLINE_MAX]);
@@ -196,7 +226,7 @@ private:
         int launched = 0, rc = MF_K_OK;
         auto launch = [&]() {
             if (rc == MF_K_OK && n != 0) {
-                rc = mf_k_batch_bulk(d, n, chunks, shift, launched, s);
+                rc = mf_k_batch_bulk(d, n, chunks, shift, launched, mf_k_copy_wait_polls(), fault, s);
                 launched = 1;
                 room = MF_BULK_INLINE_MAX;
             }
@@ -332,11 +362,14 @@ private:
         if (it == ctxs.end()) {
             cudaSetDevice(device_);
             it = ctxs.try_emplace(this).first;
+            it->second.index = threads_.fetch_add(1, std::memory_order_relaxed) % kFaultPairs;
         }
         return &it->second;
     }
 
     int device_;
+    int *faults_{nullptr};  // pinned, kFaultPairs pairs
+    std::atomic<uint32_t> threads_{0};
 };
 
 // =============================================================================================== copy engine

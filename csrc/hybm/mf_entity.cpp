@@ -943,12 +943,12 @@ int MemEntity::BatchCopyData(const BatchCopyParams &p, CopyDirection dir, void *
             MF_ERROR("batch copy: element #" << i << " cannot be placed");
             return rc;
         }
-        seenSrc = seenDst = PlacedRange{};
+        PlacedRange nowSrc, nowDst;  // not the remembered ones themselves: those stay in registers
         if (SrcClassOf(d) >= PC_GLOBAL_HOST) {
-            MF_CHECK_RET(AddressInEntity(sa, len, &seenSrc), BM_INVALID_PARAM, "batch copy: source #" << i << " leaves the pool");
+            MF_CHECK_RET(AddressInEntity(sa, len, &nowSrc), BM_INVALID_PARAM, "batch copy: source #" << i << " leaves the pool");
         }
         if (DstClassOf(d) >= PC_GLOBAL_HOST) {
-            MF_CHECK_RET(AddressInEntity(da, len, &seenDst), BM_INVALID_PARAM, "batch copy: destination #" << i << " leaves the pool");
+            MF_CHECK_RET(AddressInEntity(da, len, &nowDst), BM_INVALID_PARAM, "batch copy: destination #" << i << " leaves the pool");
         }
         if (groups.empty() || !sameGroup(groups[last], d, opt)) {
             last = groups.size();
@@ -970,6 +970,8 @@ int MemEntity::BatchCopyData(const BatchCopyParams &p, CopyDirection dir, void *
         if (grouped) {
             groups[last].idx.push_back(i);
         }
+        seenSrc = nowSrc;
+        seenDst = nowDst;
     }
     if (!grouped && (groups[0].opt.srcRemote || groups[0].opt.dstRemote)) {
         groups[0].idx.resize(p.batchSize);

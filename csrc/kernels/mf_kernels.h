@@ -22,10 +22,13 @@ enum { MF_K_OK = 0, MF_K_INVALID = -2, MF_K_LAUNCH_FAILED = -1, MF_K_TIMEOUT = -
 // ------------------------------------------------------------------------------------------------ xcopy (K1 / K2)
 
 // Single copy of n bytes between any two device-visible addresses (local HBM, peer HBM over NVLink, pinned host).
-// ctas 0 = pick from the size.
-int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, mf_stream_t stream);
+// ctas 0 = pick from the size. The waits of the bulk-copy kernels (this one, mf_k_batch_bulk) are bounded by a number of polls,
+// mf_k_copy_wait_polls() in earnest; `fault` (a word of pinned host memory, may be NULL) becomes 1 when one of them ran out, i.e. when
+// the copy has completed without having moved everything.
+int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int *fault, mf_stream_t stream);
 int mf_k_xcopy_shaped(void *dst, const void *src, size_t n, uint32_t tile, uint32_t stages, uint32_t inflight, uint32_t blocked, int ctas,
-                      mf_stream_t stream);
+                      uint32_t waitPolls, int *fault, mf_stream_t stream);
+uint32_t mf_k_copy_wait_polls(void);
 
 typedef struct {
     uint64_t src;
@@ -48,7 +51,8 @@ int mf_k_batch_xcopy(const mf_copy_desc_t *descs, const mf_copy_desc_t *descsDev
 // pieces, each numbered from chunk 0, on one stream with nothing in between, `chained` set from the second on.
 enum { MF_BULK_FIRST_PIECE = 504, MF_BULK_INLINE_MAX = 1344 };
 uint32_t mf_k_batch_bulk_shift(uint64_t totalBytes);
-int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint32_t totalChunks, uint32_t chunkShift, int chained, mf_stream_t stream);
+int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint32_t totalChunks, uint32_t chunkShift, int chained, uint32_t waitPolls, int *fault,
+                    mf_stream_t stream);
 
 // ------------------------------------------------------------------------------------------------ allreduce + RMSNorm (K4)
 

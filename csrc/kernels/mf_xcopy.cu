@@ -70,9 +70,11 @@ constexpr size_t kTmaMinBytes = 24u << 20;
 
 __device__ __forceinline__ uint32_t SmemU32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool MbarWaitParity(uint64_t *bar, uint32_t parity)
+constexpr uint32_t kWaitPolls = 1u << 26;  // about a minute
+
+__device__ __forceinline__ bool MbarWaitParity(uint64_t *bar, uint32_t parity, uint32_t polls)
 {
-    for (uint32_t i = 0; i < (1u << 26); i++) {
+    for (uint32_t i = 0; i < polls; i++) {
         uint32_t ok;
         asm volatile(
             "{\n.reg .pred p;\n"
@@ -85,10 +87,32 @@ __device__ __forceinline__ bool MbarWaitParity(uint64_t *bar, uint32_t parity)
             return true;
         }
     }
-    return false;  // about a minute of polling: the caller stops issuing work
+    return false;
 }
 
 constexpr int kTmaMaxStages = 16;
+
+// Last step of a store thread that got `taken` loads before its wait for the next one ran out (a loader that gave up ends there too: what it
+// did not ask for never comes). The copy is incomplete: the word (host memory, may be missing) tells whoever waits for it. Loads that
+// are still on their way into the shared memory of this CTA are waited for, again within the limit, before the CTA gives it
+// up. The loader leaves the number that it issued, with kLoaderDone, when it ends, which its own limit sees to.
+constexpr uint32_t kLoaderDone = 1u << 31;
+__device__ __forceinline__ void GiveUp(uint64_t *full, uint32_t stages, const volatile uint32_t *loader, uint32_t taken, int *fault)
+{
+    if (fault != nullptr) {
+        *(volatile int *)fault = 1;
+        __threadfence_system();
+    }
+    uint32_t issued = *loader;
+    for (uint32_t i = 0; i < kWaitPolls && issued == 0; i++) {
+        __nanosleep(200);
+        issued = *loader;
+    }
+    issued &= ~kLoaderDone;
+    for (uint32_t it = taken; it < issued; it++) {
+        MbarWaitParity(&full[it % stages], (it / stages) & 1, kWaitPolls);
+    }
+}
 
 // Shape of the bulk-copy pipeline: bytes per tile (a multiple of 16), tiles of shared memory per CTA, how many stores may
 // still be reading shared memory before a tile is handed back to the loader, and whether a CTA walks the copy with a stride
@@ -98,6 +122,7 @@ struct TmaShape {
     uint32_t stages;
     uint32_t inflight;
     uint32_t blocked;
+    uint32_t polls;  // limit of every wait for a load
 };
 
 __device__ __forceinline__ void BulkWaitRead(uint32_t inflight)
@@ -113,11 +138,12 @@ __device__ __forceinline__ void BulkWaitRead(uint32_t inflight)
 }
 
 __global__ void __launch_bounds__(128, 1)
-mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict__ src, size_t n, TmaShape shape)
+mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict__ src, size_t n, TmaShape shape, int *fault)
 {
     extern __shared__ unsigned char tmaSmemRaw[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tmaSmemRaw) + 127) & ~(uintptr_t)127);
     __shared__ uint64_t full[kTmaMaxStages], empty[kTmaMaxStages];
+    __shared__ volatile uint32_t loader;
     const uint32_t kTmaTile = shape.tile, kTmaStages = shape.stages, kTmaStoresInFlight = shape.inflight;
     FollowPredecessor();
     // Unaligned head (up to the first 16-byte boundary of dst) and tail bytes go through ordinary loads/stores.
@@ -134,6 +160,7 @@ mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__rest
         }
     }
     if (threadIdx.x == 0) {
+        loader = 0;
         for (uint32_t i = 0; i < kTmaStages; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(SmemU32(&full[i])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(SmemU32(&empty[i])));
@@ -153,7 +180,7 @@ mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__rest
         uint32_t it = 0;
         for (size_t t = tBegin; t < tEnd; t += tStep, it++) {
             const uint32_t st = it % kTmaStages, ph = (it / kTmaStages) & 1;
-            if (!MbarWaitParity(&empty[st], ph ^ 1)) {
+            if (it >= kTmaStages && !MbarWaitParity(&empty[st], ph ^ 1, shape.polls)) {
                 break;
             }
             const size_t off = t * kTmaTile;
@@ -164,11 +191,13 @@ mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__rest
                          "l"(s0 + off), "r"(bytes), "r"(SmemU32(&full[st]))
                          : "memory");
         }
+        loader = kLoaderDone | it;
     } else if (threadIdx.x == 32) {
         uint32_t it = 0;
-        for (size_t t = tBegin; t < tEnd; t += tStep, it++) {
+        size_t t = tBegin;
+        for (; t < tEnd; t += tStep, it++) {
             const uint32_t st = it % kTmaStages, ph = (it / kTmaStages) & 1;
-            if (!MbarWaitParity(&full[st], ph)) {
+            if (!MbarWaitParity(&full[st], ph, shape.polls)) {
                 break;
             }
             const size_t off = t * kTmaTile;
@@ -185,6 +214,9 @@ mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__rest
             }
         }
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every store has landed before the CTA retires
+        if (t < tEnd) {
+            GiveUp(full, kTmaStages, &loader, it, fault);
+        }
     }
 }
 
@@ -246,14 +278,18 @@ mf_batch_xcopy_table_kernel(const mf_copy_desc_t *__restrict__ d, uint32_t count
 // A long list goes out as several launches, so that the GPU works on the first while the host prepares the next. The first
 // piece lets its dependents start only after its own wait, i.e. when everything before the batch is complete; the others therefore
 // begin at once, as SMs become free, and wait for the piece before them at their END, which keeps completion in stream order.
+// 24 bytes, like a descriptor: with eight more the launch of 168 of them (4064 instead of 4056 bytes) took 0.5 us longer.
 struct BulkBatch {
     uint32_t count;
     uint32_t totalChunks;
-    uint32_t chunkShift;
-    uint32_t stages;
-    uint32_t inflight;
-    uint32_t chained;  // a further piece of the batch whose first piece was launched just before
+    uint8_t chunkShift;
+    uint8_t stages;
+    uint8_t inflight;
+    uint8_t chained;  // a further piece of the batch whose first piece was launched just before
+    uint32_t polls;   // limit of every wait for a load
+    int *fault;
 };
+static_assert(sizeof(BulkBatch) == 24, "see above");
 template <int MAX>
 struct BulkBatchInline {
     BulkBatch b;
@@ -267,12 +303,15 @@ __device__ __forceinline__ void BulkBatchBody(const BulkBatch &b, const mf_copy_
     extern __shared__ unsigned char tmaSmemRaw[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tmaSmemRaw) + 127) & ~(uintptr_t)127);
     __shared__ uint64_t full[kTmaMaxStages], empty[kTmaMaxStages];
+    __shared__ volatile uint32_t loader;
     __shared__ uint64_t stageDst[kTmaMaxStages];
     __shared__ uint32_t stageLen[kTmaMaxStages];
+    const uint32_t stages = b.stages, shift = b.chunkShift;
     const uint32_t c0 = (uint32_t)((uint64_t)blockIdx.x * b.totalChunks / gridDim.x);
     const uint32_t c1 = (uint32_t)((uint64_t)(blockIdx.x + 1) * b.totalChunks / gridDim.x);
     if (threadIdx.x == 0) {
-        for (uint32_t i = 0; i < b.stages; i++) {
+        loader = 0;
+        for (uint32_t i = 0; i < stages; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(SmemU32(&full[i])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(SmemU32(&empty[i])));
         }
@@ -300,8 +339,9 @@ __device__ __forceinline__ void BulkBatchBody(const BulkBatch &b, const mf_copy_
         uint64_t src = __shfl_sync(0xffffffffu, mine.src, 0), dst = __shfl_sync(0xffffffffu, mine.dst, 0);
         uint32_t len = __shfl_sync(0xffffffffu, mine.len, 0), start = __shfl_sync(0xffffffffu, mine.chunkStart, 0);
         bool alive = true;
+        uint32_t issued = 0;
         for (uint32_t c = c0, it = 0; c < c1; c++, it++) {
-            if (((uint64_t)(c - start) << b.chunkShift) >= len) {
+            if (((uint64_t)(c - start) << shift) >= len) {
                 if (++cur == 32) {
                     window += 32;
                     cur = 0;
@@ -314,39 +354,47 @@ __device__ __forceinline__ void BulkBatchBody(const BulkBatch &b, const mf_copy_
                 start = __shfl_sync(0xffffffffu, mine.chunkStart, cur);
             }
             if (lane == 0 && alive) {
-                const uint32_t st = it % b.stages, ph = (it / b.stages) & 1;
-                const uint32_t off = (c - start) << b.chunkShift;
-                const uint32_t bytes = min(len - off, 1u << b.chunkShift);
-                alive = MbarWaitParity(&empty[st], ph ^ 1);
+                const uint32_t st = it % stages, ph = (it / stages) & 1;
+                const uint32_t off = (c - start) << shift;
+                const uint32_t bytes = min(len - off, 1u << shift);
+                alive = it < stages || MbarWaitParity(&empty[st], ph ^ 1, b.polls);
                 if (alive) {
+                    issued = it + 1;
                     stageDst[st] = dst + off;
                     stageLen[st] = bytes;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemU32(&full[st])), "r"(bytes) : "memory");
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                     SmemU32(tiles + ((size_t)st << b.chunkShift))),
+                                     SmemU32(tiles + ((size_t)st << shift))),
                                  "l"(src + off), "r"(bytes), "r"(SmemU32(&full[st]))
                                  : "memory");
                 }
             }
         }
+        if (lane == 0) {
+            loader = kLoaderDone | issued;
+        }
     } else if (threadIdx.x == 32) {
-        for (uint32_t it = 0; it < c1 - c0; it++) {
-            const uint32_t st = it % b.stages, ph = (it / b.stages) & 1;
-            if (!MbarWaitParity(&full[st], ph)) {
+        uint32_t it = 0;
+        for (; it < c1 - c0; it++) {
+            const uint32_t st = it % stages, ph = (it / stages) & 1;
+            if (!MbarWaitParity(&full[st], ph, b.polls)) {
                 break;
             }
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(stageDst[st]), "r"(SmemU32(tiles + ((size_t)st << b.chunkShift))),
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(stageDst[st]), "r"(SmemU32(tiles + ((size_t)st << shift))),
                          "r"(stageLen[st])
                          : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             BulkWaitRead(b.inflight);
             if (it >= b.inflight) {
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemU32(&empty[(it - b.inflight) % b.stages])) : "memory");
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemU32(&empty[(it - b.inflight) % stages])) : "memory");
             }
         }
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // every store of this CTA has landed
         if (b.chained) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        if (it < c1 - c0) {
+            GiveUp(full, stages, &loader, it, b.fault);
         }
     }
 }
@@ -502,7 +550,7 @@ static bool ShapeValid(const TmaShape &sh)
            sh.inflight >= 1 && sh.inflight < sh.stages && (sh.inflight <= 4 || sh.inflight == 6) && sh.blocked <= 1;
 }
 
-static int LaunchTma(void *dst, const void *src, size_t n, const TmaShape &shape, int ctas, int sms, mf_stream_t stream)
+static int LaunchTma(void *dst, const void *src, size_t n, const TmaShape &shape, int ctas, int sms, int *fault, mf_stream_t stream)
 {
     const size_t smem = (size_t)shape.stages * shape.tile + 128;
     if (!AllowSmem<mf_xcopy_tma_kernel>(220 * 1024 + 128)) {
@@ -512,15 +560,15 @@ static int LaunchTma(void *dst, const void *src, size_t n, const TmaShape &shape
     const size_t perSm = smem <= 110u * 1024 ? 2 : 1;  // two CTAs fit an SM when their tiles take less than half its shared memory
     const size_t full = (size_t)sms * perSm;
     size_t grid = ctas > 0 ? (size_t)ctas : (tiles < full ? tiles : full);
-    return LaunchCopy(mf_xcopy_tma_kernel, (unsigned)grid, 128, smem, stream, (unsigned char *)dst, (const unsigned char *)src, n, shape);
+    return LaunchCopy(mf_xcopy_tma_kernel, (unsigned)grid, 128, smem, stream, (unsigned char *)dst, (const unsigned char *)src, n, shape, fault);
 }
 
 // The bulk-copy kernel with an explicit pipeline shape, for tuning sweeps. Same preconditions as the automatic path: both
-// addresses congruent modulo 16. ctas 0 = one per SM.
+// addresses congruent modulo 16. ctas 0 = one per SM. waitPolls: limit of the pipeline's waits (0: the first one runs out at once).
 extern "C" int mf_k_xcopy_shaped(void *dst, const void *src, size_t n, uint32_t tile, uint32_t stages, uint32_t inflight, uint32_t blocked,
-                                 int ctas, mf_stream_t stream)
+                                 int ctas, uint32_t waitPolls, int *fault, mf_stream_t stream)
 {
-    const TmaShape shape{tile, stages, inflight, blocked};
+    const TmaShape shape{tile, stages, inflight, blocked, waitPolls};
     if (dst == nullptr || src == nullptr || n == 0 || ctas < 0 || !ShapeValid(shape) || ((((uintptr_t)dst) ^ ((uintptr_t)src)) & 15) != 0) {
         return MF_K_INVALID;
     }
@@ -528,10 +576,10 @@ extern "C" int mf_k_xcopy_shaped(void *dst, const void *src, size_t n, uint32_t 
     if (sms <= 0) {
         return MF_K_LAUNCH_FAILED;
     }
-    return LaunchTma(dst, src, n, shape, ctas, sms, stream);
+    return LaunchTma(dst, src, n, shape, ctas, sms, fault, stream);
 }
 
-extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, mf_stream_t stream)
+extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int *fault, mf_stream_t stream)
 {
     if (n == 0) {
         return MF_K_OK;
@@ -550,19 +598,19 @@ extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, mf_str
     if (useTma && ctas >= 0 && n >= kTmaMinBytes && ((((uintptr_t)dst) ^ ((uintptr_t)src)) & 15) == 0) {
         // MF_XCOPY_SHAPE="tile,stages,inflight,blocked" overrides the pipeline shape (read once).
         static const TmaShape forced = []() {
-            TmaShape sh{0, 0, 0, 0};
+            TmaShape sh{0, 0, 0, 0, kWaitPolls};
             const char *e = getenv("MF_XCOPY_SHAPE");
             unsigned a = 0, b = 0, c = 0, d = 0;
             if (e != nullptr && sscanf(e, "%u,%u,%u,%u", &a, &b, &c, &d) == 4) {
-                TmaShape cand{a, b, c, d};
+                TmaShape cand{a, b, c, d, kWaitPolls};
                 if (ShapeValid(cand)) {
                     sh = cand;
                 }
             }
             return sh;
         }();
-        const TmaShape shape = forced.tile != 0 ? forced : TmaShape{32 * 1024, 4, 2, 0};
-        return LaunchTma(dst, src, n, shape, ctas, sms, stream);
+        const TmaShape shape = forced.tile != 0 ? forced : TmaShape{32 * 1024, 4, 2, 0, kWaitPolls};
+        return LaunchTma(dst, src, n, shape, ctas, sms, fault, stream);
     }
     if (ctas < 0) {
         ctas = -ctas == 1 ? 0 : -ctas;  // negative: force the load/store kernel (with |ctas| CTAs, -1 = automatic)
@@ -622,7 +670,10 @@ static int LaunchBulkInline(const BulkBatch &b, const mf_copy_desc_t *descs, uns
     return LaunchCopy(mf_batch_bulk_inline_kernel<MAX>, grid, kBulkThreads, smem, stream, p);
 }
 
-extern "C" int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint32_t totalChunks, uint32_t chunkShift, int chained, mf_stream_t stream)
+extern "C" uint32_t mf_k_copy_wait_polls(void) { return kWaitPolls; }
+
+extern "C" int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint32_t totalChunks, uint32_t chunkShift, int chained, uint32_t waitPolls,
+                               int *fault, mf_stream_t stream)
 {
     if (count == 0 || totalChunks == 0) {
         return MF_K_OK;
@@ -638,7 +689,7 @@ extern "C" int mf_k_batch_bulk(const mf_copy_desc_t *descs, uint32_t count, uint
     const uint32_t stages = chunkShift >= 15 ? 4 : 8, inflight = stages / 2;
     const size_t smem = ((size_t)stages << chunkShift) + 128;
     const unsigned grid = totalChunks < (unsigned)sms ? totalChunks : (unsigned)sms;
-    const BulkBatch b{count, totalChunks, chunkShift, stages, inflight, chained ? 1u : 0u};
+    const BulkBatch b{count, totalChunks, (uint8_t)chunkShift, (uint8_t)stages, (uint8_t)inflight, (uint8_t)(chained ? 1 : 0), waitPolls, fault};
     // The launch copies the whole parameter block: 4 KiB cost nothing measurable, 32 KiB 3.5 us, so three sizes.
     if (count <= 168) {
         return LaunchBulkInline<168>(b, descs, grid, smem, stream);

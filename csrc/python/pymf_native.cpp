@@ -453,13 +453,37 @@ void BindNative(py::module_ &m)
         return d;
     });
     n.def("xcopy", [](uint64_t dst, uint64_t src, uint64_t nbytes, int ctas, uint64_t stream) {
-        return mf_k_xcopy((void *)dst, (const void *)src, nbytes, ctas, (mf_stream_t)stream);
+        return mf_k_xcopy((void *)dst, (const void *)src, nbytes, ctas, nullptr, (mf_stream_t)stream);
     }, py::arg("dst"), py::arg("src"), py::arg("nbytes"), py::arg("ctas") = 0, py::arg("stream") = 0);
     n.def("xcopy_shaped", [](uint64_t dst, uint64_t src, uint64_t nbytes, uint32_t tile, uint32_t stages, uint32_t inflight, uint32_t blocked,
-                             int ctas, uint64_t stream) {
-        return mf_k_xcopy_shaped((void *)dst, (const void *)src, nbytes, tile, stages, inflight, blocked, ctas, (mf_stream_t)stream);
+                             int ctas, uint64_t stream, int64_t waitPolls, uint64_t fault) {
+        return mf_k_xcopy_shaped((void *)dst, (const void *)src, nbytes, tile, stages, inflight, blocked, ctas,
+                                 waitPolls < 0 ? mf_k_copy_wait_polls() : (uint32_t)waitPolls, (int *)fault, (mf_stream_t)stream);
     }, py::arg("dst"), py::arg("src"), py::arg("nbytes"), py::arg("tile"), py::arg("stages"), py::arg("inflight"), py::arg("blocked") = 0,
-       py::arg("ctas") = 0, py::arg("stream") = 0);
+       py::arg("ctas") = 0, py::arg("stream") = 0, py::arg("wait_polls") = -1, py::arg("fault") = 0);
+    // The bulk-copy batch kernel by itself: one launch of at most MF_BULK_INLINE_MAX copies, all of them on the 16-byte grid.
+    n.def("batch_bulk", [](std::vector<uint64_t> srcs, std::vector<uint64_t> dsts, std::vector<uint64_t> sizes, uint64_t stream, int64_t waitPolls,
+                           uint64_t fault) {
+        if (srcs.size() != sizes.size() || dsts.size() != sizes.size() || sizes.size() > MF_BULK_INLINE_MAX) {
+            return (int)MF_K_INVALID;
+        }
+        uint64_t total = 0;
+        for (size_t i = 0; i < sizes.size(); i++) {
+            if (((srcs[i] | dsts[i] | sizes[i]) & 15) != 0 || sizes[i] == 0 || sizes[i] > (1u << 30)) {
+                return (int)MF_K_INVALID;
+            }
+            total += sizes[i];
+        }
+        const uint32_t shift = mf_k_batch_bulk_shift(total);
+        std::vector<mf_copy_desc_t> d;
+        uint32_t chunks = 0;
+        for (size_t i = 0; i < sizes.size(); i++) {
+            d.push_back(mf_copy_desc_t{srcs[i], dsts[i], (uint32_t)sizes[i], chunks});
+            chunks += (uint32_t)((sizes[i] + (1u << shift) - 1) >> shift);
+        }
+        return mf_k_batch_bulk(d.data(), (uint32_t)d.size(), chunks, shift, 0, waitPolls < 0 ? mf_k_copy_wait_polls() : (uint32_t)waitPolls, (int *)fault,
+                               (mf_stream_t)stream);
+    }, py::arg("srcs"), py::arg("dsts"), py::arg("sizes"), py::arg("stream") = 0, py::arg("wait_polls") = -1, py::arg("fault") = 0);
     n.def("copy_engine", [](uint64_t dst, uint64_t src, uint64_t nbytes, uint64_t stream) {
         return mf_k_memcpy_async((void *)dst, (const void *)src, nbytes, (mf_stream_t)stream);
     }, py::arg("dst"), py::arg("src"), py::arg("nbytes"), py::arg("stream") = 0);

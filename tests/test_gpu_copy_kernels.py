@@ -165,3 +165,28 @@ def test_a_copy_without_a_stream_does_not_wait_for_the_default_stream(mf, pool, 
         assert rc == 0, mf.get_last_err_msg()
     assert still, "the copy waited for the default stream"
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("polls", [-1, 0])
+@pytest.mark.parametrize("kernel", ["single", "batch"])
+def test_a_bulk_copy_that_gives_up_waiting_says_so(mf, pool, kernel, polls):
+    """With a limit of no polls at all the first wait for a load runs out; the loads that are on their way are waited for, the word is
+    set and the kernel ends. With the ordinary limit everything arrives and the word stays as it was."""
+    import torch
+
+    n = 26 * MiB
+    src, dst = _regions(pool, n)
+    fault = torch.zeros(1, dtype=torch.int32).pin_memory()
+    st = torch.cuda.current_stream().cuda_stream
+    if kernel == "single":
+        rc = mf.native.xcopy_shaped(dst.data_ptr(), src.data_ptr(), n, 32 * KiB, 4, 2, 0, 0, st, polls, fault.data_ptr())
+    else:
+        blk = n // 416
+        rc = mf.native.batch_bulk([src.data_ptr() + i * blk for i in range(416)], [dst.data_ptr() + i * blk for i in range(416)], [blk] * 416, st, polls,
+                                  fault.data_ptr())
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert int(fault[0]) == (1 if polls == 0 else 0)
+    assert torch.equal(dst, src) == (polls != 0)
+    # the context is as usable as before
+    assert pool.handle.copy_data(pool.hbm(), pool.hbm() + 96 * MiB, n, mf.bm.BmCopyType.G2G, 0) == 0 and torch.equal(dst, src)
