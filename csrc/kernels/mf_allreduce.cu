@@ -212,9 +212,9 @@ mf_residual_rmsnorm_kernel(const mf_allreduce_args_t a, int T, int H, float eps)
     for (int k = 0; k < VPT; k++) {
         const int vec = (int)threadIdx.x + k * kThreads;
         if (vec < vecsPerRow) {
-            xv[k] = mf_ld16((const char *)a.x + rowOff + (size_t)vec * 16);
+            xv[k] = mf_ld16_ordered((const char *)a.x + rowOff + (size_t)vec * 16);
             if (a.residual != nullptr) {
-                rv[k] = mf_ld16((const char *)a.residual + rowOff + (size_t)vec * 16);
+                rv[k] = mf_ld16_ordered((const char *)a.residual + rowOff + (size_t)vec * 16);
             }
             wv[k] = *reinterpret_cast<const uint4 *>((const char *)a.weight + (size_t)vec * 16);
         }

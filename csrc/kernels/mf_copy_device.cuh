@@ -8,11 +8,12 @@
 namespace mf {
 namespace dev {
 
-// Streaming 16-byte load: read-only path, no L1 allocation (every byte is touched once).
+// Streaming 16-byte load without L1 allocation (every byte is touched once). An ordinary load, not the non-coherent one: the copy kernels
+// are launched as programmatic dependents, so a copy may be resident while the ones before it still write what it reads.
 __device__ __forceinline__ uint4 LdStream16(const void *p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ void StStream16(void *p, const uint4 &v)
@@ -24,7 +25,7 @@ __device__ __forceinline__ void StStream16(void *p, const uint4 &v)
 // thread before the first store; what is left at the end takes less than one trip and has the same loads in flight, each
 // under its own bound.
 template <int UNROLL, int THREADS>
-__device__ __forceinline__ void CopyVec(uint4 *__restrict__ dst, const uint4 *__restrict__ src, unsigned n, unsigned tid)
+__device__ __forceinline__ void CopyVec(uint4 *dst, const uint4 *src, unsigned n, unsigned tid)
 {
     dst += tid;
     src += tid;
@@ -50,7 +51,7 @@ __device__ __forceinline__ void CopyVec(uint4 *__restrict__ dst, const uint4 *__
 __device__ __forceinline__ uint4 LdShared16(const void *p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 
@@ -69,7 +70,7 @@ __device__ __forceinline__ uint4 Realign16(const uint4 &a, const uint4 &b, unsig
 // neighbouring thread. Every source vector that is touched has at least one wanted byte, so nothing outside the pages of
 // the source is read. Narrow loads (two bytes for a bf16 slice at an odd element) need eight times the instructions.
 template <int UNROLL, int THREADS>
-__device__ __forceinline__ void CopyRealigned(uint4 *__restrict__ dst, const uint4 *__restrict__ src, unsigned nv, unsigned rel, unsigned tid)
+__device__ __forceinline__ void CopyRealigned(uint4 *dst, const uint4 *src, unsigned nv, unsigned rel, unsigned tid)
 {
     dst += tid;
     src += tid;

@@ -529,10 +529,10 @@ __device__ __forceinline__ void GatherGroup(float (&part)[2][8], uint32_t group,
             if (taken) {
                 const char *rowp = reinterpret_cast<const char *>(y) + (size_t)row * rowBytes + (size_t)v0 * 16;
                 if (v0 < vecs) {
-                    raw[i][0] = mf_ld16(rowp);
+                    raw[i][0] = mf_ld16_ordered(rowp);
                 }
                 if (v0 + 32 < vecs) {
-                    raw[i][1] = mf_ld16(rowp + 512);
+                    raw[i][1] = mf_ld16_ordered(rowp + 512);
                 }
             }
         }

@@ -440,9 +440,11 @@ constexpr int kQuantUnroll = 4;
 
 // Bound by DRAM: 12288 x 7168 in 57 us = 4.6 TB/s (96 us with one load in flight and divisions). K is a multiple of 128, so the rows are one sequence of 128-element blocks; sixteen lanes own a block, eight elements
 // each, and a warp takes 2 x kQuantUnroll consecutive blocks at once so that four 16-byte loads per lane are in flight.
-__global__ void __launch_bounds__(256) mf_quant_rows_fp8_kernel(const __nv_bfloat16 *__restrict__ x, unsigned char *__restrict__ q,
-                                                                float *__restrict__ scale, int rows, int blocksPerRow, const int *__restrict__ rowLimit)
+__global__ void __launch_bounds__(256) mf_quant_rows_fp8_kernel(const __nv_bfloat16 *x, unsigned char *q, float *scale, int rows, int blocksPerRow,
+                                                                const int *rowLimit)
 {
+    // No __restrict__: x and *rowLimit are written by kernels that this one may be resident with, so they must not be read by the
+    // non-coherent path.
     GridDependency();
     const int lane = threadIdx.x & 31;
     const int limit = rowLimit != nullptr ? min(*rowLimit, rows) : rows;

@@ -30,7 +30,8 @@ constexpr int kUnroll = 8;
 // Programmatic dependent launch: every copy kernel is launched with the stream-serialisation attribute, so the next one of the
 // stream may be scheduled while this one runs, and this one may have been scheduled while its predecessor ran; the wait returns
 // once the predecessor has completed and its writes are visible. Stream order is kept, only the launch latency between
-// back-to-back copies is hidden: 4.1 -> 2.2 us a copy up to 1 MiB, 6.2 -> 3.4 us at 8 MiB, 14.4 -> 13.0 us at 32 MiB. Without the
+// back-to-back copies is hidden (no parameter of these kernels is __restrict__: what a predecessor writes while this kernel is already
+// resident must not be read by the non-coherent path): 4.1 -> 2.2 us a copy up to 1 MiB, 6.2 -> 3.4 us at 8 MiB, 14.4 -> 13.0 us at 32 MiB. Without the
 // attribute both instructions do nothing.
 __device__ __forceinline__ void FollowPredecessor()
 {
@@ -39,7 +40,7 @@ __device__ __forceinline__ void FollowPredecessor()
 }
 
 __global__ void __launch_bounds__(kThreads, 2)
-mf_xcopy_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict__ src, size_t n, size_t tileBytes)
+mf_xcopy_kernel(unsigned char *dst, const unsigned char *src, size_t n, size_t tileBytes)
 {
     FollowPredecessor();
     // Tile 0 is stretched by `lead` bytes so that every later tile starts on a 16-byte boundary of dst.
@@ -138,7 +139,7 @@ __device__ __forceinline__ void BulkWaitRead(uint32_t inflight)
 }
 
 __global__ void __launch_bounds__(128, 1)
-mf_xcopy_tma_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict__ src, size_t n, TmaShape shape, int *fault)
+mf_xcopy_tma_kernel(unsigned char *dst, const unsigned char *src, size_t n, TmaShape shape, int *fault)
 {
     extern __shared__ unsigned char tmaSmemRaw[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tmaSmemRaw) + 127) & ~(uintptr_t)127);
@@ -227,8 +228,7 @@ struct BatchInline {
 };
 static_assert(sizeof(BatchInline) <= 4096 + 32, "inline batch must fit the classic kernel parameter space");
 
-__device__ __forceinline__ void BatchBody(const mf_copy_desc_t *__restrict__ d, uint32_t count, uint32_t totalChunks,
-                                          const uint32_t *__restrict__ chunkMap)
+__device__ __forceinline__ void BatchBody(const mf_copy_desc_t *d, uint32_t count, uint32_t totalChunks, const uint32_t *chunkMap)
 {
     for (uint32_t c = blockIdx.x; c < totalChunks; c += gridDim.x) {
         uint32_t lo = 0;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 2) mf_batch_xcopy_inline_kernel(cons
 
 // The chunk → descriptor map follows the descriptor table in the same device buffer.
 __global__ void __launch_bounds__(kThreads, 2)
-mf_batch_xcopy_table_kernel(const mf_copy_desc_t *__restrict__ d, uint32_t count, uint32_t totalChunks)
+mf_batch_xcopy_table_kernel(const mf_copy_desc_t *d, uint32_t count, uint32_t totalChunks)
 {
     FollowPredecessor();
     BatchBody(d, count, totalChunks, reinterpret_cast<const uint32_t *>(d + count));
@@ -298,7 +298,7 @@ struct BulkBatchInline {
 constexpr int kBulkThreads = 128;
 constexpr int kBulkSmemMax = 128 * 1024 + 128;
 
-__device__ __forceinline__ void BulkBatchBody(const BulkBatch &b, const mf_copy_desc_t *__restrict__ d)
+__device__ __forceinline__ void BulkBatchBody(const BulkBatch &b, const mf_copy_desc_t *d)
 {
     extern __shared__ unsigned char tmaSmemRaw[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tmaSmemRaw) + 127) & ~(uintptr_t)127);

@@ -141,12 +141,20 @@ __device__ __forceinline__ bool mf_wait_until_ge(const uint64_t *flag, uint64_t 
 
 /* 16-byte streaming accessors for heap data.
  * mf_ld16 uses the non-coherent read-only path: legal only for data that nobody writes while the calling kernel runs
- * (inputs produced by earlier kernels of the stream). Data that another GPU, or another CTA, writes during the kernel and
+ * (inputs produced by earlier kernels of the stream). A kernel launched as a programmatic dependent runs from the moment it is
+ * resident, i.e. while its predecessors still write: what they produce is read with mf_ld16_ordered after griddepcontrol.wait. Data that another GPU, or another CTA, writes during the kernel and
  * that becomes visible through a signal or barrier inside the kernel must be read with mf_ld16_coherent. */
 __device__ __forceinline__ uint4 mf_ld16(const void *p)
 {
     uint4 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+/* Ordinary load, kept out of the L1. */
+__device__ __forceinline__ uint4 mf_ld16_ordered(const void *p)
+{
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 /* Coherent variant for data another GPU may have written during this kernel (after an acquire on a flag). */

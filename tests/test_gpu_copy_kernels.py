@@ -190,3 +190,108 @@ def test_a_bulk_copy_that_gives_up_waiting_says_so(mf, pool, kernel, polls):
     assert torch.equal(dst, src) == (polls != 0)
     # the context is as usable as before
     assert pool.handle.copy_data(pool.hbm(), pool.hbm() + 96 * MiB, n, mf.bm.BmCopyType.G2G, 0) == 0 and torch.equal(dst, src)
+
+
+@pytest.mark.parametrize("n", [8 * KiB + 5, 24 * KiB + 1, 64 * KiB + 3, 256 * KiB + 1])
+@pytest.mark.parametrize("step", [1, 2, 7])
+def test_short_shifted_copies_keep_stream_order(mf, pool, n, step):
+    """Grids of a few CTAs, of which several copies are resident at once, read through the L1 what the copies just before them wrote
+    over the data that still older ones had read: other data every round."""
+    import torch
+
+    from memfabric_hybrid_b200.utils.tensors import device_tensor_from_gva
+
+    base, hop, G2G = pool.hbm(), MiB, mf.bm.BmCopyType.G2G
+    st = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(n + step)
+    first, ends, wants = device_tensor_from_gva(base, n), [], []
+    for _ in range(12):
+        data = torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda", generator=g)
+        first.copy_(data)
+        at = base
+        for i in range(31):
+            to = base + (hop if i % 2 == 0 else 0) + step * (i // 2 + 1)
+            assert pool.handle.copy_data_on_stream(at, to, n, G2G, st, 1) == 0, mf.get_last_err_msg()
+            at = to
+        ends.append(device_tensor_from_gva(at, n).clone())
+        wants.append(data)
+    for turn, (end, want) in enumerate(zip(ends, wants)):
+        assert torch.equal(end, want), turn
+
+
+@pytest.mark.parametrize("count", [505, 504 + 1344 + 1, 3000])
+def test_batches_in_several_pieces_replay_from_a_graph(mf, pool, count):
+    """A captured batch of several chained launches between two others: the second reads what the batch writes, the batch what the
+    first wrote; new data before every replay."""
+    import torch
+
+    blk = 4 * KiB
+    n = count * blk
+    order = np.random.default_rng(count).permutation(count)
+    src, dst = _regions(pool, n)
+    fresh, out = torch.empty_like(src), torch.empty_like(src)
+    perm = torch.from_numpy(order).cuda()
+    a, b = pool.hbm(), pool.hbm() + 96 * MiB
+    srcs, dsts = [a + i * blk for i in range(count)], [b + int(o) * blk for o in order]
+    stream = torch.cuda.Stream()
+    T = mf.bm.BmCopyType
+
+    def work():
+        h = stream.cuda_stream
+        assert pool.handle.copy_data_on_stream(fresh.data_ptr(), a, n, T.L2G, h, 1) == 0, mf.get_last_err_msg()
+        assert pool.handle.copy_data_batch_on_stream(srcs, dsts, [blk] * count, T.G2G, h, 1) == 0, mf.get_last_err_msg()
+        assert pool.handle.copy_data_on_stream(b, out.data_ptr(), n, T.G2L, h, 1) == 0, mf.get_last_err_msg()
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        work()  # loads the kernels
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            work()
+        g = torch.Generator(device="cuda").manual_seed(count)
+        for turn in range(6):
+            fresh.copy_(torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda", generator=g))
+            out.zero_()
+            for _ in range(2):
+                graph.replay()
+            assert torch.equal(out.view(count, blk)[perm], fresh.view(count, blk)), turn
+    torch.cuda.synchronize()
+    del graph
+
+
+def test_batches_of_two_threads_on_one_stream(mf, pool):
+    """Pieces of two batches are enqueued in any interleaving; each arrives whole, and what follows on the stream sees both."""
+    import threading
+
+    import torch
+
+    from memfabric_hybrid_b200.utils.tensors import device_tensor_from_gva
+
+    count, blk, rounds = 2500, 4 * KiB, 8
+    n = count * blk
+    st = torch.cuda.current_stream().cuda_stream
+    bases = [(pool.hbm() + k * 24 * MiB, pool.hbm() + 96 * MiB + k * 24 * MiB) for k in range(2)]
+    srcs = [device_tensor_from_gva(a, n) for a, _ in bases]
+    for k, s in enumerate(srcs):
+        s.random_(0, 256, generator=torch.Generator(device="cuda").manual_seed(k))
+    torch.cuda.synchronize()
+    orders = [[np.random.default_rng(10 * k + r).permutation(count) for r in range(rounds)] for k in range(2)]
+    rcs = []
+
+    def issue(k):
+        torch.cuda.set_device(0)
+        for r in range(rounds):
+            a, b = bases[k]
+            rcs.append(pool.handle.copy_data_batch_on_stream([a + i * blk for i in range(count)], [b + int(o) * blk for o in orders[k][r]], [blk] * count,
+                                                             mf.bm.BmCopyType.G2G, st, 1))
+
+    threads = [threading.Thread(target=issue, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    seen = [device_tensor_from_gva(b, n).clone() for _, b in bases]
+    assert rcs == [0] * (2 * rounds)
+    for k in range(2):
+        assert torch.equal(seen[k].view(count, blk)[torch.from_numpy(orders[k][-1]).cuda()], srcs[k].view(count, blk)), k
