@@ -594,7 +594,8 @@ static int LaunchAllReduce(const mf_allreduce_args_t *argsHost, const mf_allredu
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
-    if (argsHost != nullptr && rankCount == 1) {
+    // One rank that leaves the choice to the library; a named algorithm or a CTA count is what the caller wants to run.
+    if (argsHost != nullptr && rankCount == 1 && algo == MF_AR_AUTO && ctas <= 0) {
         return LaunchOneRank(*argsHost, T, H, eps, stream);
     }
     const mf_allreduce_args_t own = argsHost != nullptr ? *argsHost : mf_allreduce_args_t{};

@@ -84,7 +84,8 @@ enum { MF_AR_AUTO = 0, MF_AR_ONESHOT = 1, MF_AR_TWOSHOT = 2, MF_AR_NVLS = 3, MF_
 // be used with host-side epochs any more). H: multiple of 8, at most 16384. timeoutNs 0 = 2 s.
 int mf_k_allreduce_rmsnorm(const mf_allreduce_args_t *argsDev, int nEmulatedRanks, int rankCount, int T, int H, float eps, int algo,
                            uint32_t channel, uint64_t epoch, uint64_t timeoutNs, int ctas, mf_stream_t stream);
-// The same for a real rank, its block passed by value: nothing has to be uploaded when a pointer changes, and a CUDA graph holds it.
+// The same for a real rank, its block passed by value: nothing has to be uploaded when a pointer changes, and a CUDA graph holds it. One
+// rank with MF_AR_AUTO and no CTA count runs a kernel of its own that needs neither barriers nor the epoch.
 int mf_k_allreduce_rmsnorm_rank(const mf_allreduce_args_t *argsHost, int rankCount, int T, int H, float eps, int algo, uint32_t channel, uint64_t epoch,
                                 uint64_t timeoutNs, int ctas, mf_stream_t stream);
 

@@ -85,7 +85,7 @@ class AllReduceRMSNorm:
             raise ValueError("tokens exceeds max_tokens")
         a = ALGOS[algo]
         nbytes = tokens * self.hidden * 2
-        if a == _ops.AR_AUTO:
+        if a == _ops.AR_AUTO and not (self.heap.world == 1 and ctas <= 0):  # one rank by itself: a kernel of its own, picked below
             if nbytes <= ONESHOT_MAX_BYTES:
                 a = _ops.AR_ONESHOT_NOTAIL if self.double_buffer else _ops.AR_ONESHOT
             elif self.heap.multicast_ptr and self.heap.world > 2:

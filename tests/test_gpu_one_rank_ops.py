@@ -238,3 +238,42 @@ def test_epilogue(heap, T, H):
         assert torch.equal(h.float(), ref_h)  # one rounding of an exact sum of two bf16 numbers
         torch.testing.assert_close(out.float(), ref_out, rtol=2 ** -7, atol=1e-6)  # bf16 rounding (2^-8) and 32-bit sums
     heap._bump.used = mark
+
+
+def _launched(call):
+    """Names of the kernels that `call` launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return " ".join(e.key for e in prof.key_averages())
+
+
+@pytest.mark.parametrize("algo,ctas,kernel", [("auto", 0, "residual_rmsnorm"), ("oneshot", 0, "oneshot"), ("twoshot", 0, "twoshot"), ("auto", 4, "oneshot"),
+                                              ("twoshot", 8, "twoshot")])
+def test_epilogue_of_one_rank_runs_the_algorithm_that_was_named(heap, algo, ctas, kernel):
+    import torch
+
+    from memfabric_hybrid_b200.ops.allreduce import AllReduceRMSNorm, reference
+
+    T, H = 24, 2048
+    mark = heap._bump.used
+    ar = AllReduceRMSNorm(heap, T, H)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, res = (torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    w = torch.ones(H, dtype=torch.bfloat16, device="cuda")
+    ref_out, ref_h = reference([x], res, w, 1e-6)
+
+    def call():
+        ar.x[:T].copy_(x)
+        call.got = ar(T, res, w, algo=algo, ctas=ctas)
+
+    call()
+    assert kernel in _launched(call)
+    out, h = call.got
+    assert torch.equal(h.float(), ref_h) and ar.check_status() == 0
+    torch.testing.assert_close(out.float(), ref_out, rtol=2 ** -7, atol=1e-6)
+    heap._bump.used = mark
