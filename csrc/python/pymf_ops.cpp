@@ -15,9 +15,6 @@ namespace {
 struct AllReducePlan {
     mf_allreduce_args_t a{};
     int world{1}, hidden{0};
-    float eps{0.f};
-    uint32_t channel{0};
-    uint64_t timeoutNs{0};
 };
 
 // What one MoE layer of a rank keeps between calls, and the launches of a call: in Python the four of them took about 60 us,
@@ -28,7 +25,7 @@ struct MoePlan {
     void *h1Q{nullptr}, *h1Sf{nullptr};
     int world{1}, hidden{0}, topk{0}, experts{0}, inter{0};
     uint32_t dispatchChannel{0}, combineChannel{0};
-    uint64_t timeoutNs{0}, waitNs{0};
+    uint64_t timeoutNs{0}, waitNs{0};  // limits of the layer, set anew by every call
     int *arrive{nullptr};
 
     int Dispatch(uint64_t x, uint64_t idx, uint64_t w, int T, uint64_t epoch, bool overlap, int dedupMinPairs, uint64_t stream)
@@ -213,8 +210,7 @@ void BindOps(py::module_ &m)
     }, py::arg("args_dev"), py::arg("n_emulated"), py::arg("rank_count"), py::arg("channel"), py::arg("epoch"), py::arg("timeout_ns") = 0,
             py::arg("ctas") = 0, py::arg("stream") = 0);
     py::class_<AllReducePlan>(ops, "AllReducePlan")
-        .def(py::init([](uint64_t meta, uint64_t residualOut, uint64_t out, uint64_t status, uint64_t epochState, int world, int hidden, float eps,
-                         uint32_t channel, uint64_t timeoutNs) {
+        .def(py::init([](uint64_t meta, uint64_t residualOut, uint64_t out, uint64_t status, uint64_t epochState, int world, int hidden) {
             AllReducePlan p;
             p.a.meta = (const void *)meta;
             p.a.residualOut = (void *)residualOut;
@@ -223,24 +219,21 @@ void BindOps(py::module_ &m)
             p.a.epochState = (unsigned long long *)epochState;
             p.world = world;
             p.hidden = hidden;
-            p.eps = eps;
-            p.channel = channel;
-            p.timeoutNs = timeoutNs;
             return p;
         }))
-        .def("run", [](const AllReducePlan &p, uint64_t x, uint64_t residual, uint64_t weight, int T, int algo, uint64_t epoch, int ctas, uint64_t stream) {
+        .def("run", [](const AllReducePlan &p, uint64_t x, uint64_t residual, uint64_t weight, int T, float eps, int algo, uint32_t channel, uint64_t epoch,
+                       uint64_t timeoutNs, int ctas, uint64_t stream) {
             mf_allreduce_args_t a = p.a;
             a.x = (const void *)x;
             a.residual = (const void *)residual;
             a.weight = (const void *)weight;
-            return mf_k_allreduce_rmsnorm_rank(&a, p.world, T, p.hidden, p.eps, algo, p.channel, epoch, p.timeoutNs, ctas, (mf_stream_t)stream);
+            return mf_k_allreduce_rmsnorm_rank(&a, p.world, T, p.hidden, eps, algo, channel, epoch, timeoutNs, ctas, (mf_stream_t)stream);
         });
     py::class_<MoePlan>(ops, "MoePlan")
         .def(py::init([](uint64_t meta, uint64_t cnt, uint64_t recvX, uint64_t recvSf, uint64_t recvMeta, uint64_t recvSib, uint64_t localCnt,
                          uint64_t cursor, uint64_t expertOffset, uint64_t expertCount, uint64_t routed, uint64_t arrive, uint64_t status, uint64_t h1Q,
                          uint64_t h1Sf, uint64_t y, uint64_t retY, uint64_t out, int cap, int retRows, int world, int hidden, int topk, int experts,
-                         int inter, uint32_t dispatchChannel, uint32_t combineChannel, uint64_t timeoutNs, uint64_t waitNs, uint64_t epochD,
-                         uint64_t epochC) {
+                         int inter, uint32_t dispatchChannel, uint32_t combineChannel, uint64_t epochD, uint64_t epochC) {
             MoePlan p;
             p.d.meta = p.c.meta = (const void *)meta;
             p.d.cnt = (int *)cnt;
@@ -276,15 +269,20 @@ void BindOps(py::module_ &m)
             p.inter = inter;
             p.dispatchChannel = dispatchChannel;
             p.combineChannel = combineChannel;
-            p.timeoutNs = timeoutNs;
-            p.waitNs = waitNs;
             return p;
         }))
+        .def("limits", [](MoePlan &p, uint64_t timeoutNs, uint64_t waitNs) {
+            p.timeoutNs = timeoutNs;
+            p.waitNs = waitNs;
+        })
         .def("dispatch", &MoePlan::Dispatch)
         .def("experts", &MoePlan::Experts)
         .def("combine", &MoePlan::Combine)
         .def("run", [](MoePlan &p, uint64_t x, uint64_t idx, uint64_t w, int T, uint64_t w13Q, uint64_t w13S, int w13Packed, uint64_t w2Q, uint64_t w2S,
-                       int w2Packed, uint64_t epochD, uint64_t epochC, bool overlap, int dedupMinPairs, uint64_t stream) {
+                       int w2Packed, uint64_t epochD, uint64_t epochC, bool overlap, int dedupMinPairs, uint64_t timeoutNs, uint64_t waitNs,
+                       uint64_t stream) {
+            p.timeoutNs = timeoutNs;
+            p.waitNs = waitNs;
             int rc = p.Dispatch(x, idx, w, T, epochD, overlap, dedupMinPairs, stream);
             if (rc == MF_K_OK) {
                 rc = p.Experts(w13Q, w13S, w13Packed, w2Q, w2S, w2Packed, overlap, stream);

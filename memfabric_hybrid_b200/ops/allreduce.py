@@ -71,7 +71,7 @@ class AllReduceRMSNorm:
             # current host-side epoch (the same number on every rank), so that flags left by earlier host-epoch calls are stale.
             self._epoch_state = torch.tensor([heap.next_epoch(channel), 0], dtype=torch.int64, device=dev)
         self._plan = _ops.AllReducePlan(heap.meta_ptr, self.residual_out.data_ptr(), self.out.data_ptr(), self.status.data_ptr(),
-                                        self._epoch_state.data_ptr() if device_epochs else 0, heap.world, hidden, eps, channel, timeout_ns)
+                                        self._epoch_state.data_ptr() if device_epochs else 0, heap.world, hidden)
         self._x_ptrs = [x.data_ptr() for x in self._xs]
         self._results = (max_tokens, (self.out, self.residual_out))  # views of the last token count: making them costs as much as a launch
 
@@ -100,7 +100,8 @@ class AllReduceRMSNorm:
             raise RuntimeError("the NVLS algorithm needs a heap created with nvls=True on a platform with multicast")
         s = stream.cuda_stream if stream is not None else current_stream_handle()
         epoch = 0 if self.device_epochs else self.heap.next_epoch(self.channel)
-        rc = self._plan.run(self._x_ptrs[self._cur], residual.data_ptr() if residual is not None else 0, weight.data_ptr(), tokens, a, epoch, ctas, s)
+        rc = self._plan.run(self._x_ptrs[self._cur], residual.data_ptr() if residual is not None else 0, weight.data_ptr(), tokens,
+                            self.eps, a, self.channel, epoch, self.timeout_ns, ctas, s)
         if rc != 0:
             raise RuntimeError(f"allreduce_rmsnorm launch failed ({rc})")
         self.launches += 1

@@ -140,7 +140,7 @@ class FusedMoE(_MoEBase):
                                   st.recv_sib.data_ptr(), st.local_cnt.data_ptr(), st.cursor.data_ptr(), st.expert_offset.data_ptr(),
                                   st.expert_count.data_ptr(), st.routed.data_ptr(), st.arrive.data_ptr(), st.status.data_ptr(), st.h1_q.data_ptr(),
                                   st.h1_sf.data_ptr(), st.y.data_ptr(), st.ret_y.data_ptr(), st.out.data_ptr(), st.cap, st.max_rows_ret, heap.world, hidden,
-                                  topk, n_experts, inter, CH_DISPATCH, CH_COMBINE, timeout_ns, self.wait_ns,
+                                  topk, n_experts, inter, CH_DISPATCH, CH_COMBINE,
                                   self._epoch_d.data_ptr() if device_epochs else 0, self._epoch_c.data_ptr() if device_epochs else 0)
         self._result = (max_tokens, st.out)
         self._weight_shapes = [((self.el, n, k), (self.el, n // 32, k // 128, 32, 128), (self.el, n // 128, k // 128))
@@ -162,6 +162,7 @@ class FusedMoE(_MoEBase):
 
     def dispatch(self, x, idx, w, stream=None):
         s = stream.cuda_stream if stream is not None else current_stream_handle()
+        self._plan.limits(self.timeout_ns, self.wait_ns)
         rc = self._plan.dispatch(x.data_ptr(), idx.data_ptr(), w.data_ptr(), x.shape[0], self._epoch(CH_DISPATCH), self.overlap, self.dedup_min_pairs, s)
         if rc != 0:
             raise RuntimeError(f"moe_dispatch launch failed ({rc})")
@@ -169,6 +170,7 @@ class FusedMoE(_MoEBase):
 
     def experts(self, stream=None):
         s = stream.cuda_stream if stream is not None else current_stream_handle()
+        self._plan.limits(self.timeout_ns, self.wait_ns)
         rc = self._plan.experts(*self._weights(), self.overlap, s)
         if rc != 0:
             raise RuntimeError(f"moe_grouped_gemm_mx launch failed ({rc})")
@@ -177,6 +179,7 @@ class FusedMoE(_MoEBase):
 
     def combine(self, T, stream=None):
         s = stream.cuda_stream if stream is not None else current_stream_handle()
+        self._plan.limits(self.timeout_ns, self.wait_ns)
         rc = self._plan.combine(self._epoch(CH_COMBINE), s)
         if rc != 0:
             raise RuntimeError(f"moe_combine launch failed ({rc})")
@@ -193,7 +196,7 @@ class FusedMoE(_MoEBase):
         T = x.shape[0]
         s = stream.cuda_stream if stream is not None else current_stream_handle()
         rc = self._plan.run(x.data_ptr(), idx.data_ptr(), w.data_ptr(), T, *self._weights(), self._epoch(CH_DISPATCH), self._epoch(CH_COMBINE),
-                            self.overlap, self.dedup_min_pairs, s)
+                            self.overlap, self.dedup_min_pairs, self.timeout_ns, self.wait_ns, s)
         if rc != 0:
             raise RuntimeError(f"MoE layer launch failed ({rc})")
         self.launches += 4

@@ -277,3 +277,48 @@ def test_epilogue_of_one_rank_runs_the_algorithm_that_was_named(heap, algo, ctas
     assert torch.equal(h.float(), ref_h) and ar.check_status() == 0
     torch.testing.assert_close(out.float(), ref_out, rtol=2 ** -7, atol=1e-6)
     heap._bump.used = mark
+
+
+def test_epilogue_reads_its_settings_on_every_call(heap):
+    import torch
+
+    from memfabric_hybrid_b200.ops.allreduce import AllReduceRMSNorm, reference
+
+    T, H = 6, 1024
+    mark = heap._bump.used
+    ar = AllReduceRMSNorm(heap, T, H)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    w = torch.ones(H, dtype=torch.bfloat16, device="cuda")
+    for eps in (1e-6, 0.5, 1e-6):
+        ar.eps = eps
+        ar.x[:T].copy_(x)
+        torch.testing.assert_close(ar(T, None, w)[0].float(), reference([x], None, w, eps)[0], rtol=2 ** -7, atol=1e-6)
+    heap._bump.used = mark
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_moe_layer_reads_its_limits_on_every_call(heap, whole):
+    """A dispatch in arrival mode whose tiles never fill up: the first GEMM gives up after the layer's present `wait_ns`."""
+    import time
+
+    import torch
+
+    layer, x, idx, tw = _routed_layer(heap, 16, 256, 4, 2, 128, 31, overlap=True)
+    layer(x, idx, tw)
+    assert layer.check_status() == 0
+    took = {}
+    for wait_ns in (1_000_000, 700_000_000):
+        layer.wait_ns = wait_ns
+        if whole:
+            layer(x, idx, tw)
+            assert layer.check_status() == 0
+        layer.dispatch(x, idx, tw)
+        layer.st.arrive.zero_()  # as if the senders' counts had been lost
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        layer.experts()
+        torch.cuda.synchronize()
+        took[wait_ns] = time.perf_counter() - t0
+        assert layer.check_status() == 4  # the arrival wait ran out
+        layer.st.status.zero_()
+    assert took[1_000_000] < 0.3 < took[700_000_000], took
