@@ -143,7 +143,7 @@ class FusedMoE(_MoEBase):
                                   topk, n_experts, inter, CH_DISPATCH, CH_COMBINE,
                                   self._epoch_d.data_ptr() if device_epochs else 0, self._epoch_c.data_ptr() if device_epochs else 0)
         self._result = (max_tokens, st.out)
-        self._weight_shapes = [((self.el, n, k), (self.el, n // 32, k // 128, 32, 128), (self.el, n // 128, k // 128))
+        self._weight_shapes = [((self.el, n, k), (self.el, n // 32, k // 128, 32, 128), self.el * (n // 128) * (k // 128))
                                for n, k in ((2 * inter, hidden), (hidden, inter))]
         torch.cuda.synchronize()
         heap.barrier()  # everybody's count matrix is zeroed before the first dispatch touches it
@@ -153,7 +153,8 @@ class FusedMoE(_MoEBase):
         out = []
         for q, sc, (plain, blocks, scales) in ((self.w13_q, self.w13_s, self._weight_shapes[0]), (self.w2_q, self.w2_s, self._weight_shapes[1])):
             packed = q.dim() == 5
-            assert q.shape == (blocks if packed else plain) and sc.shape == scales and q.is_contiguous() and sc.is_contiguous()
+            # the scales in order, whatever shape the caller keeps them in
+            assert q.shape == (blocks if packed else plain) and sc.numel() >= scales and q.is_contiguous() and sc.is_contiguous()
             out += (q.data_ptr(), sc.data_ptr(), int(packed))
         return out
 

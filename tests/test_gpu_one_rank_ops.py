@@ -161,8 +161,16 @@ def test_moe_layer_looks_at_its_weights_on_every_call(heap):
     layer = FusedMoE(heap, T, H, E, K, I, *_weights(E, H, I, 6))
     x = torch.ones(T, H, dtype=torch.bfloat16, device="cuda")
     idx, tw = route(torch.randn(T, E, device="cuda"), K)
-    layer(x, idx, tw)
-    layer.w2_s.unsqueeze_(0)  # the same tensor, but no longer of the expected shape
+    want = layer(x, idx, tw).clone()
+    layer.w2_s.unsqueeze_(0)  # the same scales in another shape are as good
+    layer.w13_s = layer.w13_s.flatten()
+    assert torch.equal(layer(x, idx, tw), want)
+    layer.w2_q.transpose_(1, 2)  # the same tensor, but its rows no longer follow one another
+    with pytest.raises(AssertionError):
+        layer(x, idx, tw)
+    layer.w2_q.transpose_(1, 2)
+    layer.w2_s.squeeze_(0)
+    layer.w2_s = layer.w2_s[1:]  # too few scales
     with pytest.raises(AssertionError):
         layer(x, idx, tw)
 
