@@ -212,16 +212,23 @@ mf_residual_rmsnorm_kernel(const mf_allreduce_args_t a, int T, int H, float eps)
     for (int k = 0; k < VPT; k++) {
         const int vec = (int)threadIdx.x + k * kThreads;
         if (vec < vecsPerRow) {
-            xv[k] = mf_ld16_ordered((const char *)a.x + rowOff + (size_t)vec * 16);
             if (a.residual != nullptr) {
                 rv[k] = mf_ld16_ordered((const char *)a.residual + rowOff + (size_t)vec * 16);
             }
             wv[k] = *reinterpret_cast<const uint4 *>((const char *)a.weight + (size_t)vec * 16);
         }
     }
+    // Before x is touched: the check is there to stop that access. What it does not look at is already on its way.
     if (mf_check_bounds_enabled(m) && !mf_shm_in_own_window(m, a.x, (uint64_t)T * H * 2)) {
         Fail(a, MF_DEV_ERR_BOUNDS);
         return;
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; k++) {
+        const int vec = (int)threadIdx.x + k * kThreads;
+        if (vec < vecsPerRow) {
+            xv[k] = mf_ld16_ordered((const char *)a.x + rowOff + (size_t)vec * 16);
+        }
     }
     float ss = 0.f;
     Acc8 acc[VPT];

@@ -330,3 +330,34 @@ def test_moe_layer_reads_its_limits_on_every_call(heap, whole):
         assert layer.check_status() == 4  # the arrival wait ran out
         layer.st.status.zero_()
     assert took[1_000_000] < 0.3 < took[700_000_000], took
+
+
+@pytest.mark.parametrize("H", [512, 8192, 16384])
+def test_epilogue_of_one_rank_checks_its_input_first(heap, H):
+    """With the bounds check on, an input outside the heap (valid memory here) is refused before anything is read or written."""
+    import torch
+
+    from memfabric_hybrid_b200.ops.allreduce import AllReduceRMSNorm
+
+    T = 7
+    mark = heap._bump.used
+    ar = AllReduceRMSNorm(heap, T, H)
+    outside = torch.ones(T, H, dtype=torch.bfloat16, device="cuda")
+    w = torch.ones(H, dtype=torch.bfloat16, device="cuda")
+    ar.out.fill_(3.0)
+    ar.residual_out.fill_(3.0)
+    heap.set_check_bounds(True)
+    try:
+        inside = list(ar._x_ptrs)
+        ar._x_ptrs = [outside.data_ptr()] * 2
+        ar(T, outside, w)
+        assert ar.check_status() == 2  # MF_DEV_ERR_BOUNDS
+        assert bool((ar.out == 3.0).all()) and bool((ar.residual_out == 3.0).all())
+        ar.status.zero_()
+        ar._x_ptrs = inside
+        ar.x.zero_()
+        ar(T, outside, w)
+        assert ar.check_status() == 0 and bool((ar.residual_out == 1.0).all())
+    finally:
+        heap.set_check_bounds(False)
+    heap._bump.used = mark
