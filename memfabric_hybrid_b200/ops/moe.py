@@ -142,7 +142,7 @@ class FusedMoE(_MoEBase):
                                   st.h1_sf.data_ptr(), st.y.data_ptr(), st.ret_y.data_ptr(), st.out.data_ptr(), st.cap, st.max_rows_ret, heap.world, hidden,
                                   topk, n_experts, inter, CH_DISPATCH, CH_COMBINE,
                                   self._epoch_d.data_ptr() if device_epochs else 0, self._epoch_c.data_ptr() if device_epochs else 0)
-        self._result = (max_tokens, st.out)
+        self._rows = (max_tokens, st.out[:max_tokens])  # never handed out itself: callers get aliases
         self._weight_shapes = [((self.el, n, k), (self.el, n // 32, k // 128, 32, 128), self.el * (n // 128) * (k // 128))
                                for n, k in ((2 * inter, hidden), (hidden, inter))]
         torch.cuda.synchronize()
@@ -188,10 +188,10 @@ class FusedMoE(_MoEBase):
         return self._out(T)
 
     def _out(self, T):
-        res = self._result
-        if res[0] != T:
-            res = self._result = (T, self.st.out[:T])
-        return res[1]
+        rows = self._rows
+        if rows[0] != T:
+            rows = self._rows = (T, self.st.out[:T])
+        return rows[1][...]
 
     def __call__(self, x, idx, w, stream=None):
         T = x.shape[0]

@@ -361,3 +361,33 @@ def test_epilogue_of_one_rank_checks_its_input_first(heap, H):
     finally:
         heap.set_check_bounds(False)
     heap._bump.used = mark
+
+
+@pytest.mark.parametrize("n", [12, 5])
+def test_results_are_tensors_of_their_own(heap, n):
+    """What a caller does to the shape of a result stays with that tensor: the next call returns the ordinary one."""
+    import torch
+
+    from memfabric_hybrid_b200.models.llama import ParamSpec
+    from memfabric_hybrid_b200.ops.allreduce import AllReduceRMSNorm
+    from memfabric_hybrid_b200.ops.reshard import Resharder, ReshardPlan
+
+    T, H = 12, 512
+    mark = heap._bump.used
+    ar = AllReduceRMSNorm(heap, T, H)
+    w = torch.ones(H, dtype=torch.bfloat16, device="cuda")
+    layer, x, idx, tw = _routed_layer(heap, T, H, 4, 2, 128, 41)
+    rs = Resharder(heap, ReshardPlan([ParamSpec("a", (256, 128), "col", True), ParamSpec("b", (64,), "rep", False)], 1, 0, 1, fp8=True))
+    calls = [lambda: ar(n, None, w), lambda: (layer(x[:n], idx[:n], tw[:n]),), lambda: (*rs()["a"], rs()["b"])]
+    for call in calls:
+        shapes = [t.shape for t in call()]
+        first = call()
+        for t in first:
+            t.unsqueeze_(0)
+            t.transpose_(0, 1)
+        again = call()
+        assert [t.shape for t in again] == shapes
+        assert all(t is not f for t, f in zip(again, first))
+        assert all(t.data_ptr() == f.data_ptr() for t, f in zip(again, first))
+    assert ar.out.shape == (T, H) and layer.st.out.shape == (T, H)
+    heap._bump.used = mark
