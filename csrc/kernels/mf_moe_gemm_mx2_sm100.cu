@@ -23,9 +23,11 @@
 #include <cstdlib>
 
 #include "mf_kernels.h"
+#include "mf_launch.cuh"
 #include "mf_sm100_ptx.cuh"
 
 using namespace mf::sm100;
+using mf::AllowSmem;
 
 namespace {
 
@@ -595,14 +597,9 @@ extern "C" int mf_k_moe_grouped_gemm_mx_2sm(const void *a, const uint32_t *aSf, 
     p.mode = mode;
     p.rowsTotal = rowsTotal;
     p.wideStores = ((uintptr_t)out & 31) == 0 ? 1 : 0;
-    static bool attrSet = false;
     const size_t smem = sizeof(SharedStorage2) + 1024;
-    if (!attrSet) {
-        if (cudaFuncSetAttribute(mf_moe_grouped_gemm_mx2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return MF_K_LAUNCH_FAILED;
-        }
-        attrSet = true;
+    if (!AllowSmem<mf_moe_grouped_gemm_mx2_kernel>(smem)) {
+        return MF_K_LAUNCH_FAILED;
     }
     const int sms = mf_k_sm_count();
     if (sms < 2) {
@@ -622,7 +619,13 @@ extern "C" int mf_k_moe_grouped_gemm_mx_2sm(const void *a, const uint32_t *aSf, 
     // The kernel is persistent with a static tile walk: every pair must be resident from the start, or the pairs of a second
     // wave would only begin when a first-wave pair has finished ALL its tiles. Not every SM can be paired (a pair needs two
     // free SMs of one cluster-scheduling group), so the number of pairs that fit at once is asked for, not assumed.
-    static int maxPairs = 0;
+    static std::atomic<int> fit[64];  // per device; AllowSmem has refused others
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MF_K_LAUNCH_FAILED;
+    }
+    int maxPairs = fit[dev].load(std::memory_order_relaxed);
     if (maxPairs == 0) {
         cfg.gridDim = dim3((unsigned)(sms & ~1));
         int n = 0;
@@ -631,6 +634,7 @@ extern "C" int mf_k_moe_grouped_gemm_mx_2sm(const void *a, const uint32_t *aSf, 
             return MF_K_LAUNCH_FAILED;
         }
         maxPairs = n;
+        fit[dev].store(n, std::memory_order_relaxed);
     }
     int pairsWanted = (ctas > 0 && ctas < sms ? ctas : sms) / 2;
     if (pairsWanted > maxPairs) {

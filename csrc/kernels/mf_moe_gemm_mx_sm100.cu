@@ -39,9 +39,11 @@
 #include <cstdlib>
 
 #include "mf_kernels.h"
+#include "mf_launch.cuh"
 #include "mf_sm100_ptx.cuh"
 
 using namespace mf::sm100;
+using mf::AllowSmem;
 
 namespace {
 
@@ -629,14 +631,9 @@ bool MakeMapPacked(CUtensorMap *m, const void *base, uint64_t rows, uint64_t K, 
 template <int BN>
 int Launch(const CUtensorMap &mapA, const CUtensorMap &mapB, const MxParams &p, int ctas, cudaStream_t stream)
 {
-    static bool attrSet = false;
     const size_t smem = sizeof(SharedStorage<BN>) + 1024;
-    if (!attrSet) {
-        if (cudaFuncSetAttribute(mf_moe_grouped_gemm_mx_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return MF_K_LAUNCH_FAILED;
-        }
-        attrSet = true;
+    if (!AllowSmem<mf_moe_grouped_gemm_mx_kernel<BN>>(smem)) {
+        return MF_K_LAUNCH_FAILED;
     }
     const int sms = mf_k_sm_count();
     if (sms <= 0) {

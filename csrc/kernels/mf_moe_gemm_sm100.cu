@@ -30,9 +30,11 @@
 #include <cstdlib>
 
 #include "mf_kernels.h"
+#include "mf_launch.cuh"
 #include "mf_sm100_ptx.cuh"
 
 using namespace mf::sm100;
+using mf::AllowSmem;
 
 namespace {
 
@@ -545,14 +547,9 @@ int Launch(const void *a, const void *b, const GemmParams &p, int ctas, cudaStre
     if (!MakeMap(&mapA, a, (uint64_t)p.rowsTotal, (uint64_t)p.K, BM) || !MakeMap(&mapB, b, (uint64_t)p.G * p.N, (uint64_t)p.K, BN)) {
         return MF_K_LAUNCH_FAILED;
     }
-    static bool attrSet = false;
     const size_t smem = sizeof(SharedStorage<BN>) + 1024;
-    if (!attrSet) {
-        if (cudaFuncSetAttribute(mf_moe_grouped_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return MF_K_LAUNCH_FAILED;
-        }
-        attrSet = true;
+    if (!AllowSmem<mf_moe_grouped_gemm_kernel<BN>>(smem)) {
+        return MF_K_LAUNCH_FAILED;
     }
     const int sms = mf_k_sm_count();
     if (sms <= 0) {

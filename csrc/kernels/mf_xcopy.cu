@@ -14,13 +14,15 @@
 // 512-thread CTAs at two per SM (128 KiB in flight per SM — enough to cover HBM3e and NVLink latency), persistent grid.
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 
 #include "mf_copy_device.cuh"
 #include "mf_kernels.h"
+#include "mf_launch.cuh"
+
+using mf::AllowSmem;
 
 namespace {
 
@@ -507,26 +509,6 @@ int LaunchCopy(void (*kernel)(Params...), unsigned grid, unsigned threads, size_
         return MF_K_LAUNCH_FAILED;
     }
     return MF_K_OK;
-}
-
-// Dynamic shared memory above 48 KiB has to be allowed once per kernel and device.
-template <auto KERNEL>
-bool AllowSmem(size_t bytes)
-{
-    static std::atomic<bool> allowed[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    if (!allowed[dev].load(std::memory_order_relaxed)) {
-        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
-        }
-        allowed[dev].store(true, std::memory_order_relaxed);
-    }
-    return true;
 }
 
 int LaunchResult()
