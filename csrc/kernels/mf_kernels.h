@@ -131,6 +131,10 @@ int mf_k_moe_grouped_gemm_mx_2sm(const void *a, const uint32_t *aSf, const void 
                                  const int *groupOffset, const int *groupCount, int G, int rowsTotal, int N, int K, int mode, int *status, int ctas,
                                  mf_stream_t stream);
 
+// Columns per tile that the two GEMMs choose by themselves when `ctas` CTAs are to run (tests look at the rules through these).
+int mf_k_gemm_tile(int G, int rowsTotal, int N, int ctas);
+int mf_k_gemm_mx_tile(int G, int rowsTotal, int N, int mode, int ctas);
+
 // ------------------------------------------------------------------------------------------------ MoE dispatch / combine (K5a, K5c)
 
 // Per-rank argument blocks (device memory). "heap" fields must sit at the same offset of the symmetric heap on every rank.

@@ -669,22 +669,8 @@ int GemmMx(const void *a, const uint32_t *aSf, const void *b, const float *bScal
         return MF_K_INVALID;  // TMA base addresses, the 16-byte scale-word loads and the 16-byte epilogue stores need 16-byte alignment
     }
     if (tileN == 0) {
-        // Wide tiles when every SM gets at least two of them even so; otherwise more, narrower tiles balance better. The plain
-        // bf16 epilogue prefers the double-buffered 224-column tile where N allows it.
-        const long long mTiles = (rowsTotal + BM - 1) / BM;
-        static const bool auto224 = []() {
-            const char *e = getenv("MF_GEMM_TILE224");
-            return e != nullptr && e[0] == '1';
-        }();
-        // Measured on the second FFN GEMM (N 7168, K 2048): with at most one m-tile per expert (decode) the 224-column tile is 4 %
-        // faster than the 256-column one, with 1024 rows per expert it is 6 % slower, so it is chosen for the former only
-        // (MF_GEMM_TILE224=1 forces it wherever it applies).
-        const bool fewRows = mTiles <= (long long)G;
-        if ((auto224 || fewRows) && epi == MF_GEMM_EPI_BF16 && N % 224 == 0 && mTiles * (N / 224) >= 2LL * 148) {
-            tileN = 224;
-        } else {
-            tileN = (N % 256 == 0 && mTiles * (N / 256) >= 2LL * 148) ? 256 : 128;
-        }
+        const int sms = mf_k_sm_count();
+        tileN = mf_k_gemm_mx_tile(G, rowsTotal, N, mode, ctas > 0 && ctas < sms ? ctas : sms);
     }
     if ((tileN == 256 && N % 256 != 0) || (tileN == 224 && (N % 224 != 0 || epi != MF_GEMM_EPI_BF16))) {
         return MF_K_INVALID;
@@ -719,6 +705,25 @@ int GemmMx(const void *a, const uint32_t *aSf, const void *b, const float *bScal
 }
 
 }  // namespace
+
+extern "C" int mf_k_gemm_mx_tile(int G, int rowsTotal, int N, int mode, int ctas)
+{
+    // Wide tiles when every SM gets at least two of them even so; otherwise more, narrower tiles balance better. The plain
+    // bf16 epilogue prefers the double-buffered 224-column tile where N allows it.
+    const long long mTiles = (rowsTotal + BM - 1) / BM;
+    static const bool auto224 = []() {
+        const char *e = getenv("MF_GEMM_TILE224");
+        return e != nullptr && e[0] == '1';
+    }();
+    // Measured on the second FFN GEMM (N 7168, K 2048): with at most one m-tile per expert (decode) the 224-column tile is 4 %
+    // faster than the 256-column one, with 1024 rows per expert it is 6 % slower, so it is chosen for the former only
+    // (MF_GEMM_TILE224=1 forces it wherever it applies).
+    const bool fewRows = mTiles <= (long long)G;
+    if ((auto224 || fewRows) && (mode & 15) == MF_GEMM_EPI_BF16 && N % 224 == 0 && mTiles * (N / 224) >= 2LL * ctas) {
+        return 224;
+    }
+    return N % 256 == 0 && mTiles * (N / 256) >= 2LL * ctas ? 256 : 128;
+}
 
 extern "C" int mf_k_moe_grouped_gemm_mx(const void *a, const uint32_t *aSf, const void *b, const float *bScale, void *out, void *outSf,
                                         const int *groupOffset, const int *groupCount, int G, int rowsTotal, int N, int K, int mode, int tileN,

@@ -593,12 +593,18 @@ extern "C" int mf_k_moe_grouped_gemm(const void *a, const float *aScale, const v
     p.rowsTotal = rowsTotal;
     p.wideStores = ((uintptr_t)out & 31) == 0 ? 1 : 0;
     p.vecScales = (K / BK) % 4 == 0 && ((uintptr_t)aScale & 15) == 0 && ((uintptr_t)bScale & 15) == 0 ? 1 : 0;
+    const int sms = mf_k_sm_count();
+    const bool wide = mf_k_gemm_tile(G, rowsTotal, N, ctas > 0 && ctas < sms ? ctas : sms) == 256;
+    return wide ? Launch<256>(a, b, p, ctas, (cudaStream_t)stream) : Launch<128>(a, b, p, ctas, (cudaStream_t)stream);
+}
+
+extern "C" int mf_k_gemm_tile(int G, int rowsTotal, int N, int ctas)
+{
     // The wide tile reads A half as often and hands a partial product over half as often: one K-block takes about 950 cycles instead
     // of 2 x 720. It pays from two m-tiles per expert on if every SM still gets two tiles (8191 rows over 32 experts, N 4096 / K 7168: 353
     // against 455 us); below that the weights' stream is what counts and the finer tiles end more evenly (2048 rows: 201 against 197 us).
     const long long mTiles = (rowsTotal + BM - 1) / BM;
-    const bool wide = N % 256 == 0 && mTiles >= 2LL * G && mTiles * (N / 256) >= 2LL * 148;
-    return wide ? Launch<256>(a, b, p, ctas, (cudaStream_t)stream) : Launch<128>(a, b, p, ctas, (cudaStream_t)stream);
+    return N % 256 == 0 && mTiles >= 2LL * G && mTiles * (N / 256) >= 2LL * ctas ? 256 : 128;
 }
 
 extern "C" int mf_k_quant_rows_fp8(const void *x, void *q, float *scale, int rows, int K, const int *rowLimit, mf_stream_t stream)
