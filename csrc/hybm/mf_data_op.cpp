@@ -62,6 +62,12 @@ int BoundedStreamSync(int device, void *stream, uint32_t timeoutMs)
     }
 }
 
+static bool TouchesHost(CopyDirection d)
+{
+    PtrClass s = SrcClassOf(d), t = DstClassOf(d);
+    return s == PC_LOCAL_HOST || s == PC_GLOBAL_HOST || t == PC_LOCAL_HOST || t == PC_GLOBAL_HOST;
+}
+
 // =============================================================================================== kernel engine
 
 namespace {
@@ -129,7 +135,8 @@ public:
         }
         cudaStream_t s = opt.stream != nullptr ? (cudaStream_t)opt.stream : cu::ThreadStream(device_);
         int *fault = FaultWord(Ctx(), opt);
-        int rc = mf_k_xcopy(p.dest, p.src, p.dataSize, 0, fault, (mf_stream_t)s);
+        const bool sameHbm = opt.srcRank == opt.dstRank && !TouchesHost(dir);
+        int rc = mf_k_xcopy(p.dest, p.src, p.dataSize, 0, sameHbm ? 1 : 0, fault, (mf_stream_t)s);
         if (rc != MF_K_OK) {
             MF_ERROR("kernel engine: xcopy launch failed");
             return BM_ERROR;
@@ -643,11 +650,6 @@ int ComposeDataOp::Initialize()
 }
 
 static bool HostOnly(CopyDirection d) { return d == DIR_LH_TO_GH || d == DIR_GH_TO_LH || d == DIR_GH_TO_GH; }
-static bool TouchesHost(CopyDirection d)
-{
-    PtrClass s = SrcClassOf(d), t = DstClassOf(d);
-    return s == PC_LOCAL_HOST || s == PC_GLOBAL_HOST || t == PC_LOCAL_HOST || t == PC_GLOBAL_HOST;
-}
 
 static uint64_t PeerCopyEngineMin()
 {

@@ -22,10 +22,13 @@ enum { MF_K_OK = 0, MF_K_INVALID = -2, MF_K_LAUNCH_FAILED = -1, MF_K_TIMEOUT = -
 // ------------------------------------------------------------------------------------------------ xcopy (K1 / K2)
 
 // Single copy of n bytes between any two device-visible addresses (local HBM, peer HBM over NVLink, pinned host).
-// ctas 0 = pick from the size. The waits of the bulk-copy kernels (this one, mf_k_batch_bulk) are bounded by a number of polls,
+// ctas 0 = pick from the size; sameHbm: both sides lie in the memory of the GPU that copies. The waits of the bulk-copy kernels (this one, mf_k_batch_bulk) are bounded by a number of polls,
 // mf_k_copy_wait_polls() in earnest; `fault` (a word of pinned host memory, may be NULL) becomes 1 when one of them ran out, i.e. when
 // the copy has completed without having moved everything.
-int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int *fault, mf_stream_t stream);
+int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int sameHbm, int *fault, mf_stream_t stream);
+// The rule by which it takes the bulk-copy kernel (returns 1 and {tile, stages, stores in flight, contiguous runs}) or the load/store
+// kernel (0).
+int mf_k_xcopy_shape(uint64_t dst, uint64_t src, size_t n, int sameHbm, uint32_t shape[4]);
 int mf_k_xcopy_shaped(void *dst, const void *src, size_t n, uint32_t tile, uint32_t stages, uint32_t inflight, uint32_t blocked, int ctas,
                       uint32_t waitPolls, int *fault, mf_stream_t stream);
 uint32_t mf_k_copy_wait_polls(void);

@@ -68,8 +68,13 @@ mf_xcopy_kernel(unsigned char *dst, const unsigned char *src, size_t n, size_t t
 // copies (a shallow pipeline interleaves DRAM reads and writes more regularly than a deep one): 32 KiB tiles, 4 stages, 2
 // stores in flight, one CTA per SM, strided walk: 12.9 / 23.0 / 44.0 / 83.5 / 325 us at 32 / 64 / 128 / 256 / 1024 MiB, against 13.3 /
 // 25.4 / 50.0 / 97.5 / 376 us of the load/store kernel. Below kTmaMinBytes the load/store kernel is the faster one (3.6 and 6.2 us
-// at 8 and 16 MiB against 3.5 and 6.7 us, 3.1 against 3.3 us at 4 MiB). Over NVLink every shape runs at the link's rate.
+// at 8 and 16 MiB against 3.5 and 6.7 us, 3.1 against 3.3 us at 4 MiB). That was measured, and is the rule, where both sides lie in
+// this GPU's memory. Over a link (a peer's memory, the host's) every shape runs at the link's rate from the sizes that were measured
+// there; what was in place for those measurements stays: bulk copies from 4 MiB on, 16 KiB tiles with one store in flight,
+// 32 KiB tiles in contiguous runs from 256 MiB on.
 constexpr size_t kTmaMinBytes = 24u << 20;
+constexpr size_t kTmaMinBytesLink = 4u << 20;
+constexpr size_t kTmaLargeLink = 256u << 20;
 
 __device__ __forceinline__ uint32_t SmemU32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -561,7 +566,23 @@ extern "C" int mf_k_xcopy_shaped(void *dst, const void *src, size_t n, uint32_t 
     return LaunchTma(dst, src, n, shape, ctas, sms, fault, stream);
 }
 
-extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int *fault, mf_stream_t stream)
+extern "C" int mf_k_xcopy_shape(uint64_t dst, uint64_t src, size_t n, int sameHbm, uint32_t shape[4])
+{
+    TmaShape pick{32 * 1024, 4, 2, 0, 0};
+    if (((dst ^ src) & 15) != 0 || n < (sameHbm ? kTmaMinBytes : kTmaMinBytesLink)) {
+        return 0;
+    }
+    if (!sameHbm) {
+        pick = n >= kTmaLargeLink ? TmaShape{32 * 1024, 4, 2, 1, 0} : TmaShape{16 * 1024, 4, 1, 0, 0};
+    }
+    shape[0] = pick.tile;
+    shape[1] = pick.stages;
+    shape[2] = pick.inflight;
+    shape[3] = pick.blocked;
+    return 1;
+}
+
+extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int sameHbm, int *fault, mf_stream_t stream)
 {
     if (n == 0) {
         return MF_K_OK;
@@ -577,7 +598,8 @@ extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int *f
         const char *e = getenv("MF_XCOPY_TMA");
         return !(e != nullptr && e[0] == '0');
     }();
-    if (useTma && ctas >= 0 && n >= kTmaMinBytes && ((((uintptr_t)dst) ^ ((uintptr_t)src)) & 15) == 0) {
+    uint32_t pick[4];
+    if (useTma && ctas >= 0 && mf_k_xcopy_shape((uint64_t)dst, (uint64_t)src, n, sameHbm, pick) != 0) {
         // MF_XCOPY_SHAPE="tile,stages,inflight,blocked" overrides the pipeline shape (read once).
         static const TmaShape forced = []() {
             TmaShape sh{0, 0, 0, 0, kWaitPolls};
@@ -591,7 +613,7 @@ extern "C" int mf_k_xcopy(void *dst, const void *src, size_t n, int ctas, int *f
             }
             return sh;
         }();
-        const TmaShape shape = forced.tile != 0 ? forced : TmaShape{32 * 1024, 4, 2, 0, kWaitPolls};
+        const TmaShape shape = forced.tile != 0 ? forced : TmaShape{pick[0], pick[1], pick[2], pick[3], kWaitPolls};
         return LaunchTma(dst, src, n, shape, ctas, sms, fault, stream);
     }
     if (ctas < 0) {

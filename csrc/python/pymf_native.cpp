@@ -452,9 +452,16 @@ void BindNative(py::module_ &m)
         d["remote_elems"] = st.remoteElems;
         return d;
     });
-    n.def("xcopy", [](uint64_t dst, uint64_t src, uint64_t nbytes, int ctas, uint64_t stream) {
-        return mf_k_xcopy((void *)dst, (const void *)src, nbytes, ctas, nullptr, (mf_stream_t)stream);
-    }, py::arg("dst"), py::arg("src"), py::arg("nbytes"), py::arg("ctas") = 0, py::arg("stream") = 0);
+    n.def("xcopy", [](uint64_t dst, uint64_t src, uint64_t nbytes, int ctas, uint64_t stream, bool sameHbm) {
+        return mf_k_xcopy((void *)dst, (const void *)src, nbytes, ctas, sameHbm ? 1 : 0, nullptr, (mf_stream_t)stream);
+    }, py::arg("dst"), py::arg("src"), py::arg("nbytes"), py::arg("ctas") = 0, py::arg("stream") = 0, py::arg("same_hbm") = true);
+    n.def("xcopy_shape", [](uint64_t dst, uint64_t src, uint64_t nbytes, bool sameHbm) -> py::object {
+        uint32_t s[4];
+        if (mf_k_xcopy_shape(dst, src, nbytes, sameHbm ? 1 : 0, s) == 0) {
+            return py::none();
+        }
+        return py::make_tuple(s[0], s[1], s[2], s[3]);
+    }, py::arg("dst"), py::arg("src"), py::arg("nbytes"), py::arg("same_hbm"));
     n.def("xcopy_shaped", [](uint64_t dst, uint64_t src, uint64_t nbytes, uint32_t tile, uint32_t stages, uint32_t inflight, uint32_t blocked,
                              int ctas, uint64_t stream, int64_t waitPolls, uint64_t fault) {
         return mf_k_xcopy_shaped((void *)dst, (const void *)src, nbytes, tile, stages, inflight, blocked, ctas,
