@@ -191,7 +191,7 @@ class FusedMoE(_MoEBase):
         rows = self._rows
         if rows[0] != T:
             rows = self._rows = (T, self.st.out[:T])
-        return rows[1][...]
+        return rows[1].detach()
 
     def __call__(self, x, idx, w, stream=None):
         T = x.shape[0]

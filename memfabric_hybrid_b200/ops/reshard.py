@@ -107,7 +107,7 @@ class Resharder:
 
     def views(self):
         """name -> bf16 tensor, or (float8_e4m3fn tensor, fp32 scales [rows/128, cols/128]) for quantised parameters."""
-        return {name: (v[0][...], v[1][...]) if isinstance(v, tuple) else v[...] for name, v in self._views.items()}
+        return {name: (v[0].detach(), v[1].detach()) if isinstance(v, tuple) else v.detach() for name, v in self._views.items()}
 
     def _make_views(self):
         import torch

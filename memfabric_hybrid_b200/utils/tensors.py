@@ -6,12 +6,19 @@ import ctypes
 import numpy as np
 
 
+_torch_c = None
+
+
 def current_stream_handle() -> int:
     """cudaStream_t of the calling thread's current stream on its current device, without building the Stream object (which
     takes about as long as a kernel launch)."""
-    import torch
+    global _torch_c
+    if _torch_c is None:
+        import torch
 
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        torch.cuda.init()
+        _torch_c = torch._C
+    return _torch_c._cuda_getCurrentRawStream(_torch_c._cuda_getDevice())
 
 
 class _CudaBlob:
