@@ -2,7 +2,7 @@
 """Small, self-ending single-GPU cases for profiler captures: each runs ONE kernel of the library a few times on inputs that
 are larger than L2 (126 MB) where DRAM figures matter but hold at most a few GB on the device.
 
-    python benchmarks/profile_cases.py xcopy | peer | batch | gemm | gemm_2sm | gemm2 | allreduce | dispatch | reshard
+    python benchmarks/profile_cases.py xcopy | shifted | peer | batch | gemm | gemm_2sm | gemm2 | gemm_fp32 | allreduce | epilogue | dispatch | moe_rank | reshard
 
 `peer` needs two GPUs in ONE process (no second rank): GPU 0 pushes 256 MiB into GPU 1's memory over NVLink, so the link's byte
 counters (nvltx__bytes / nvlrx__bytes) can be read next to the kernel's duration.
@@ -33,6 +33,22 @@ def case_xcopy():
         assert mf.native.xcopy(b.data_ptr(), a.data_ptr(), n, -1, s) == 0   # load/store variant
     torch.cuda.synchronize()
     assert torch.equal(a, b)
+
+
+def case_shifted():
+    """Addresses that differ modulo 16: vectors put together from two neighbours."""
+    import torch
+    import memfabric_hybrid_b200 as mf
+
+    n = 256 << 20
+    a = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+    b = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    mf.native.fill_pattern(a.data_ptr(), n + 64, 1, s)
+    for _ in range(3):
+        assert mf.native.xcopy(b.data_ptr(), a.data_ptr() + 2, n, 0, s) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(a[2:2 + n], b[:n])
 
 
 def case_peer():
@@ -72,7 +88,7 @@ def case_batch():
     srcs = [int(a.data_ptr() + o) for o in so]
     dsts = [int(b.data_ptr() + o) for o in do]
     for _ in range(4):
-        assert mf.native.batch_xcopy_inline(srcs, dsts, [int(x) for x in sizes], 0, s) == 0
+        assert mf.native.batch_bulk(srcs, dsts, [int(x) for x in sizes], s) == 0
     torch.cuda.synchronize()
 
 
@@ -123,6 +139,78 @@ def case_gemm2():
     for _ in range(3):
         F.grouped_gemm_mx(a_q, a_s, w_q, w_s, offs, cnts, mode="bf16", out=out)
     torch.cuda.synchronize()
+
+
+def case_gemm_fp32():
+    """The GEMM with free-form fp32 scales: the first FFN GEMM's shape with SwiGLU and the second's, 8 experts x 512 rows."""
+    import torch
+    from memfabric_hybrid_b200.ops import fp8_gemm as F
+
+    G, per = 8, 512
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rows = G * per
+    offs = torch.arange(0, rows + 1, per, dtype=torch.int32, device="cuda")
+    cnts = torch.full((G,), per, dtype=torch.int32, device="cuda")
+    for N, K, mode in ((4096, 7168, "swiglu"), (7168, 2048, "bf16")):
+        q, sc = F.quant_rows_fp8(torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16))
+        w_q = torch.empty(G, N, K, dtype=torch.float8_e4m3fn, device="cuda")
+        w_s = torch.empty(G, N // 128, K // 128, dtype=torch.float32, device="cuda")
+        for e in range(G):
+            w_q[e], w_s[e] = F.quant_weight_torch(torch.randn(N, K, generator=g, device="cuda") * 0.02)
+        torch.cuda.synchronize()
+        F.grouped_gemm(q, sc, w_q, w_s, offs, cnts, mode=mode)
+        torch.cuda.synchronize()
+
+
+def _one_rank_heap(nbytes):
+    import socket
+
+    from memfabric_hybrid_b200.parallel.heap import SymmetricHeap
+
+    with socket.socket() as s:
+        s.bind(("127.0.0.1", 0))
+        port = s.getsockname()[1]
+    return SymmetricHeap(0, 1, 0, nbytes, store_url=f"tcp://127.0.0.1:{port}")
+
+
+def case_epilogue():
+    """Residual add + RMSNorm of one rank: 32 rows (decode), then 8192 rows (537 MB of traffic)."""
+    import torch
+    from memfabric_hybrid_b200.ops.allreduce import AllReduceRMSNorm
+
+    heap = _one_rank_heap(1 << 30)
+    H, w = 8192, torch.ones(8192, dtype=torch.bfloat16, device="cuda")
+    for T in (32, 8192):
+        ar = AllReduceRMSNorm(heap, T, H, double_buffer=False)
+        res = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+        ar.x.normal_()
+        torch.cuda.synchronize()
+        for _ in range(2):
+            ar(T, res, w)
+            torch.cuda.synchronize()
+        assert ar.check_status() == 0
+    heap.close()
+
+
+def case_moe_rank():
+    """Dispatch and combine of one rank that owns all experts: 2048 tokens, hidden 7168, top-8 of 32."""
+    import torch
+    from memfabric_hybrid_b200.ops import fp8_gemm as F
+    from memfabric_hybrid_b200.ops.moe import FusedMoE, route
+
+    T, H, E, K, I = 2048, 7168, 32, 8, 256
+    heap = _one_rank_heap(1 << 30)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    w13 = F.quant_weight_mx_torch(torch.randn(E, 2 * I, H, generator=g, device="cuda") * 0.01)
+    w2 = F.quant_weight_mx_torch(torch.randn(E, H, I, generator=g, device="cuda") * 0.02)
+    layer = FusedMoE(heap, T, H, E, K, I, *w13, *w2, capacity_factor=1.25)
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    idx, w = route(torch.randn(T, E, generator=g, device="cuda"), K)
+    for _ in range(2):
+        layer(x, idx, w)
+        torch.cuda.synchronize()
+    assert layer.check_status() == 0
+    heap.close()
 
 
 def case_allreduce():
@@ -190,5 +278,5 @@ if __name__ == "__main__":
     import torch
 
     torch.cuda.set_device(0)
-    {"xcopy": case_xcopy, "peer": case_peer, "batch": case_batch, "gemm": case_gemm, "gemm_2sm": case_gemm_2sm, "gemm2": case_gemm2, "allreduce": case_allreduce, "dispatch": case_dispatch, "reshard": case_reshard}[sys.argv[1]]()
+    globals()["case_" + sys.argv[1]]()
     print("ok", sys.argv[1])

@@ -5,19 +5,21 @@ from __future__ import annotations
 
 def smoke_all(verbose: bool = False) -> dict:
     """Launches every kernel family on `cuda:<current>` with small inputs and checks each result against its PyTorch oracle:
-    single copies through both copy kernels, the inline and the table batch copy, all-reduce + RMSNorm (one-shot and two-shot,
-    four emulated ranks), MoE dispatch → block-scaled grouped GEMMs → combine (two emulated ranks), the fp32-scale grouped
-    GEMM and the row quantiser, and the weight reshard (bf16 and fp8, four emulated ranks). Returns {name: True}; raises on
-    the first mismatch."""
+    single copies through both copy kernels, the inline, the table and the bulk batch copy, all-reduce + RMSNorm (one-shot and
+    two-shot, four emulated ranks; one real rank), MoE dispatch → block-scaled grouped GEMMs → combine (two emulated ranks; one
+    real rank), the fp32-scale grouped GEMM and the row quantiser, and the weight reshard (bf16 and fp8, four emulated ranks).
+    Returns {name: True}; raises on the first mismatch."""
+    import socket
+
     import numpy as np
     import torch
 
     from .. import native
     from ..models import LlamaConfig, param_specs
-    from ..parallel.heap import EmulatedHeap
+    from ..parallel.heap import EmulatedHeap, SymmetricHeap
     from . import fp8_gemm as F
-    from .allreduce import emulated_allreduce, reference
-    from .moe import EmulatedMoE, moe_reference, route
+    from .allreduce import AllReduceRMSNorm, emulated_allreduce, reference
+    from .moe import EmulatedMoE, FusedMoE, moe_reference, route
     from .reshard import ReshardPlan, emulated_reshard, reference_reshard
 
     done = {}
@@ -29,8 +31,8 @@ def smoke_all(verbose: bool = False) -> dict:
         if verbose:
             print("smoke:", name, "ok", flush=True)
 
-    # ---- single copies: bulk-copy kernel (>= 4 MiB, congruent addresses), load/store kernel (misaligned), small copy
-    n = 6 << 20
+    # ---- single copies: bulk-copy kernel (>= 24 MiB, congruent addresses), load/store kernel (misaligned), small copy
+    n = 24 << 20
     a = torch.empty(n + 64, dtype=torch.uint8, device=dev)
     b = torch.zeros(n + 64, dtype=torch.uint8, device=dev)
     native.fill_pattern(a.data_ptr(), n + 64, 5, s)
@@ -45,9 +47,9 @@ def smoke_all(verbose: bool = False) -> dict:
     assert torch.equal(a[7:7 + n], b[3:3 + n]) and torch.equal(a[1:41], b[n + 8:n + 48])
     mark("xcopy_ldst")
 
-    # ---- batch copies: 100 descriptors ride in the kernel parameters, 400 go through the staged table
+    # ---- batch copies: 100 descriptors ride in the kernel parameters, 400 go through the staged table, 500 through the bulk copy engine
     rng = np.random.default_rng(0)
-    for count, name in ((100, "batch_inline"), (400, "batch_table")):
+    for count, name in ((100, "batch_inline"), (400, "batch_table"), (500, "batch_bulk")):
         blk = 8192
         src = torch.randint(0, 256, (count * blk,), dtype=torch.uint8, device=dev)
         dst = torch.zeros(count * blk, dtype=torch.uint8, device=dev)
@@ -56,6 +58,8 @@ def smoke_all(verbose: bool = False) -> dict:
         dsts = [dst.data_ptr() + int(p) * blk for p in perm]
         if count <= 168:
             assert native.batch_xcopy_inline(srcs, dsts, [blk] * count, 0, s) == 0
+        elif name == "batch_bulk":
+            assert native.batch_bulk(srcs, dsts, [blk] * count, s) == 0
         else:
             assert native.batch_xcopy_noalloc(srcs, dsts, [blk] * count, s) == 0
         torch.cuda.synchronize()
@@ -79,6 +83,32 @@ def smoke_all(verbose: bool = False) -> dict:
         for r in range(world):
             torch.testing.assert_close(outs[r].float(), ref_out, atol=2e-2, rtol=2e-2)
         mark("allreduce_" + algo)
+
+    # ---- the same, and the MoE layer, on a heap of one real rank: argument blocks by value, kernels without barriers
+    with socket.socket() as sock:
+        sock.bind(("127.0.0.1", 0))
+        port = sock.getsockname()[1]
+    own = SymmetricHeap(0, 1, torch.cuda.current_device(), 64 << 20, store_url=f"tcp://127.0.0.1:{port}")
+    ar = AllReduceRMSNorm(own, T, H)
+    ar.x[:T].copy_(xs[0])
+    out, h = ar(T, res, w)
+    ref_out, ref_h = reference(xs[:1], res, w, 1e-6)
+    assert ar.check_status() == 0 and torch.equal(h.float(), ref_h)
+    torch.testing.assert_close(out.float(), ref_out, atol=2e-2, rtol=2e-2)
+    mark("epilogue_one_rank")
+    T, H, E, K, I = 48, 1024, 8, 4, 256
+    gate, up = (torch.randn(E, I, H, generator=g, device=dev) * H ** -0.5 for _ in range(2))
+    weights = F.quant_weight_mx_torch(F.interleave_gate_up(gate, up)) + F.quant_weight_mx_torch(torch.randn(E, H, I, generator=g, device=dev) * I ** -0.5)
+    x = torch.randn(T, H, generator=g, device=dev).to(torch.bfloat16)
+    idx, tw = route(torch.randn(T, E, generator=g, device=dev), K)
+    layer = FusedMoE(own, T, H, E, K, I, *weights)
+    out, ref = layer(x, idx, tw), moe_reference([x], [idx], [tw], [weights], E, I)[0]
+    assert layer.check_status() == 0
+    assert float((out.float() - ref).abs().max()) <= 1e-1 * float(ref.abs().max())
+    assert float((out.float() - ref).abs().mean()) <= 4e-3 * float(ref.abs().max())
+    mark("moe_one_rank")
+    del ar, layer, out, h
+    own.close()
 
     # ---- MoE layer on two emulated ranks: dispatch, block-scaled GEMMs (both tile widths are picked by size), combine
     world, T, H, E, K, I = 2, 48, 1024, 8, 4, 256
