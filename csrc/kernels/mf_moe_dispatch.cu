@@ -552,16 +552,84 @@ __device__ __forceinline__ void GatherGroup(float (&part)[2][8], uint32_t group,
     }
 }
 
-// Bound by the traffic of the expert outputs. A rank's own pairs are gathered by token from where dispatch put them: no landing
-// zone is written and read for them and no receive buffer is scanned for leaders (7 of 8 of its rows are followers when one rank
-// owns all experts). One rank, top-8, hidden 7168: 128 tokens 63 -> 8 us, 4096 tokens (530 MB) 247 -> 90 us.
-// ALONE: one rank and at most eight pairs a token; nothing waits on anything, so it is an ordinary launch.
-template <bool ALONE, bool EMULATED>
+// One rank. Bound by the traffic of the expert outputs: they are gathered by token from where dispatch put them, no landing zone is
+// written and read and no receive buffer is scanned for leaders (7 of 8 of its rows are followers). Nothing waits on anything, so it
+// is an ordinary launch. Top-8, hidden 7168, in a loop: 128 tokens 61 -> 6 us, 4096 tokens (530 MB) 247 -> 85 us.
+template <bool MANY>  // more pairs a token than one group holds
+__global__ void __launch_bounds__(kThreads, 3)
+mf_moe_combine_alone_kernel(const __grid_constant__ mf_moe_combine_args_t a, int H, int K, uint64_t epochArg)
+{
+    GridDependency();
+    const uint64_t epoch = ResolveEpochD(a, epochArg);
+    if (epoch == 0) {
+        FailD(a.status, MF_DEV_ERR_BOUNDS);  // neither an epoch argument nor a device-resident epoch
+        return;
+    }
+    const MfDeviceMeta *m = reinterpret_cast<const MfDeviceMeta *>(a.meta);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warpsTotal = gridDim.x * kWarps;
+    __shared__ int abortFlag;
+    if (mf_check_bounds_enabled(m) && !mf_shm_in_own_window(m, a.retY, (uint64_t)a.retRows * H * 2)) {
+        FailD(a.status, MF_DEV_ERR_BOUNDS);
+        FinishEpochD(a, epochArg, epoch);
+        return;
+    }
+    if (ReadAbort(a.status, &abortFlag) != 0) {  // a call whose dispatch failed (overflow) moves no data
+        FinishEpochD(a, epochArg, epoch);
+        return;
+    }
+    // Work unit = (token, chunk of 64 vectors); lane k holds pair k.
+    const int vecs = H / 8, units = (vecs + 63) / 64;
+    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)a.T * units; u += warpsTotal) {
+        const int t = (int)(u / units), v0 = (int)(u % units) * 64 + lane;
+        int mySlot = -1, myOwner = -1;
+        float myW = 0.f;
+        if (lane < K) {
+            const int4 pair = a.routed[t * K + lane];
+            mySlot = pair.x;
+            myOwner = pair.y;
+            myW = __int_as_float(pair.z);
+        }
+        uint32_t pairs = __ballot_sync(0xffffffffu, myOwner >= 0);
+        float acc[2][8];
+        if (!MANY) {
+            GatherGroup(acc, pairs, MF_MOE_MAX_SIBLINGS + 1, mySlot, myW, a.y, (size_t)H * 2, a.cap, v0, vecs);
+        } else {
+            // Groups of eight in k order, each rounded like a partial sum that travels.
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                acc[0][q] = acc[1][q] = 0.f;
+            }
+            while (pairs != 0) {
+                float part[2][8];
+                GatherGroup(part, pairs, MF_MOE_MAX_SIBLINGS + 1, mySlot, myW, a.y, (size_t)H * 2, a.cap, v0, vecs);
+                const uint4 rounded[2] = {PackRow(part[0]), PackRow(part[1])};
+                AddRow(acc, rounded);
+                for (int i = 0; i < MF_MOE_MAX_SIBLINGS + 1; i++) {
+                    pairs &= pairs - 1;
+                }
+            }
+        }
+        char *o = reinterpret_cast<char *>(a.out) + ((size_t)t * H + (size_t)v0 * 8) * 2;
+        if (v0 < vecs) {
+            mf_st16(o, PackRow(acc[0]));
+        }
+        if (v0 + 32 < vecs) {
+            mf_st16(o + 512, PackRow(acc[1]));
+        }
+    }
+    FinishEpochD(a, epochArg, epoch);
+}
+
+// Several ranks. Every pair travels as a partial sum through the landing zone, those of a rank's own tokens too: a form that gathered these
+// directly, in units of 64 instead of 128 vectors, left too few loads in flight for groups of one or two rows (emulated ranks, 4096
+// tokens in all, hidden 7168, top-8 of 32: 2 / 4 / 8 ranks 220 / 238 / 263 us, that form 308 / 346 / 421 us).
+template <bool EMULATED>
 __global__ void __launch_bounds__(kThreads, 3)
 mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const mf_moe_combine_args_t *__restrict__ emulated, int H, int K, int EL, uint32_t channel, uint64_t epochArg, uint64_t timeoutNs)
 {
-    GridDependency();
-    const mf_moe_combine_args_t &a = EMULATED ? emulated[blockIdx.y] : own;
+    cg::grid_group grid = cg::this_grid();
+    const mf_moe_combine_args_t a = EMULATED ? emulated[blockIdx.y] : own;
     const uint64_t epoch = ResolveEpochD(a, epochArg);
     if (epoch == 0) {
         FailD(a.status, MF_DEV_ERR_BOUNDS);  // neither an epoch argument nor a device-resident epoch
@@ -578,28 +646,26 @@ mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const m
         FinishEpochD(a, epochArg, epoch);
         return;
     }
-    for (int i = threadIdx.x; i <= EL && !ALONE; i += kThreads) {
+    for (int i = threadIdx.x; i <= EL; i += kThreads) {
         offs[i] = a.expertOffset[i];
         if (i < EL) {
             cnts[i] = a.expertCount[i];
         }
     }
     __syncthreads();
-    const int rows = ALONE ? 0 : min(offs[EL], a.cap);
+    const int rows = min(offs[EL], a.cap);
     const int vecs = H / 8;
     const uint32_t R = m->rankCount;
     // A call whose dispatch failed (overflow, timeout) moves no data; it still walks through the barriers so that the
     // peers' waits complete.
     const bool dead = ReadAbort(a.status, &abortFlag) != 0;
-    // The rows that this rank computed for its own tokens need no landing zone: dispatch left their places and weights in `routed`,
-    // and the source gathers them itself below.
 
     // ---- push: one row per (token, owner): the leader's output plus its siblings', weighted, to the source rank's
     //      landing zone [token][k of the leader][:]
-    // Work unit = (row, chunk of 64 vectors): a leader with many siblings is spread over several warps.
-    const int units = (vecs + 63) / 64;
-    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)rows * units && !dead && !ALONE; u += warpsTotal) {
-        const int r = (int)(u / units), v0 = (int)(u % units) * 64 + lane;
+    // Work unit = (row, chunk of 128 vectors): a leader with many siblings is spread over several warps.
+    const int chunks = (vecs + 127) / 128;
+    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)rows * chunks && !dead; u += warpsTotal) {
+        const int r = (int)(u / chunks), ch = (int)(u % chunks);
         int el = 0;
         while (el + 1 < EL && offs[el + 1] <= r) {
             el++;
@@ -610,99 +676,135 @@ mf_moe_combine_kernel(const __grid_constant__ mf_moe_combine_args_t own, const m
         const int4 meta = a.recvMeta[r];
         const uint32_t src = (uint32_t)meta.x;
         const int k = meta.z & 0xff, nsib = (meta.z >> 8) & 0xff;
-        if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || src >= R || src == m->rankId || meta.y < 0 || k >= K || (long long)meta.y * K + k >= a.retRows ||
+        if ((meta.z & MF_MOE_META_FOLLOWER) != 0 || src >= R || meta.y < 0 || k >= K || (long long)meta.y * K + k >= a.retRows ||
             nsib > MF_MOE_MAX_SIBLINGS) {
             continue;
         }
-        // Lane 0 holds the leader's row, lanes 1..nsib those of its siblings.
-        int2 mine = make_int2(r, meta.w);
-        if (lane >= 1 && lane <= nsib) {
-            mine = a.recvSib[(size_t)r * MF_MOE_MAX_SIBLINGS + lane - 1];
-        }
-        float part[2][8];
-        GatherGroup(part, (2u << nsib) - 1, MF_MOE_MAX_SIBLINGS + 1, mine.x, __int_as_float(mine.y), a.y, (size_t)H * 2, rows, v0, vecs);
-        char *dst = reinterpret_cast<char *>(mf_shm_peer(m, a.retY, src)) + ((size_t)meta.y * K + k) * H * 2;
-        if (v0 < vecs) {
-            mf_st16(dst + (size_t)v0 * 16, PackRow(part[0]));
-        }
-        if (v0 + 32 < vecs) {
-            mf_st16(dst + (size_t)(v0 + 32) * 16, PackRow(part[1]));
-        }
-    }
-    if (!ALONE) {
-        __threadfence_system();
-        cg::grid_group grid = cg::this_grid();
-        grid.sync();
-        if (blockIdx.x == 0) {
-            int rc = mf_barrier_cta(m, channel, 0, epoch, timeoutNs);
-            if (rc != MF_DEV_OK) {
-                FailD(a.status, rc);
+        const int2 *sd = a.recvSib + (size_t)r * MF_MOE_MAX_SIBLINGS;
+        int rowOf[MF_MOE_MAX_SIBLINGS + 1];
+        float wOf[MF_MOE_MAX_SIBLINGS + 1];
+        rowOf[0] = r;
+        wOf[0] = __int_as_float(meta.w);
+        int n = 1;
+        for (int i = 0; i < nsib; i++) {
+            const int2 e = sd[i];
+            if (e.x >= 0 && e.x < rows) {
+                rowOf[n] = e.x;
+                wOf[n] = __int_as_float(e.y);
+                n++;
             }
         }
-        grid.sync();
+        char *dst = reinterpret_cast<char *>(mf_shm_peer(m, a.retY, src)) + ((size_t)meta.y * K + k) * H * 2;
+        // The lane's four vectors of the chunk are loaded together for every addend, so that four 16-byte loads per lane are
+        // in flight (the rows of a group lie far apart: latency, not bandwidth, would pace a one-at-a-time loop).
+        const int vEnd = min(vecs, (ch + 1) * 128);
+        const int v0 = ch * 128 + lane;
+        float acc[4][8];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                acc[j][q] = 0.f;
+            }
+        }
+        for (int i = 0; i < n; i++) {
+            const char *rowp = reinterpret_cast<const char *>(a.y) + (size_t)rowOf[i] * H * 2;
+            uint4 raw[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                raw[j] = v0 + 32 * j < vEnd ? mf_ld16(rowp + (size_t)(v0 + 32 * j) * 16) : make_uint4(0u, 0u, 0u, 0u);
+            }
+            const float w = wOf[i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[j]);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float2 f = __bfloat1622float2(h[q]);
+                    acc[j][2 * q] = fmaf(w, f.x, acc[j][2 * q]);
+                    acc[j][2 * q + 1] = fmaf(w, f.y, acc[j][2 * q + 1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (v0 + 32 * j < vEnd) {
+                uint4 pk;
+                __nv_bfloat162 *hp = reinterpret_cast<__nv_bfloat162 *>(&pk);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    hp[q] = __floats2bfloat162_rn(acc[j][2 * q], acc[j][2 * q + 1]);
+                }
+                mf_st16(dst + (size_t)(v0 + 32 * j) * 16, pk);
+            }
+        }
     }
+    __threadfence_system();
+    grid.sync();
+    if (blockIdx.x == 0) {
+        int rc = mf_barrier_cta(m, channel, 0, epoch, timeoutNs);
+        if (rc != MF_DEV_OK) {
+            FailD(a.status, rc);
+        }
+    }
+    grid.sync();
     if (ReadAbort(a.status, &abortFlag) != 0) {
         FinishEpochD(a, epochArg, epoch);
         return;
     }
-    // ---- add the owners' partial sums (fp32, fixed order): pair k carries one iff no earlier pair of its group (the pairs of the
-    //      token on one owner, eight at most, in k order) does. Work unit = (token, chunk of 64 vectors).
-    for (long long u = (long long)blockIdx.x * kWarps + warp; u < (long long)a.T * units; u += warpsTotal) {
-        const int t = (int)(u / units), v0 = (int)(u % units) * 64 + lane, v1 = v0 + 32;
-        const bool has0 = v0 < vecs, has1 = v1 < vecs;
-        // Lane k holds pair k: where its partial sum or its expert's output stands and which lanes belong to its group.
-        int myOwner = -1, mySlot = -1;
-        float myW = 0.f;
-        if (lane < K) {
-            const int4 pair = a.routed[t * K + lane];
-            mySlot = pair.x;
-            myOwner = pair.y;
-            myW = __int_as_float(pair.z);
-        }
-        uint32_t same = 0;
+    // ---- add the owners' partial sums (fp32, fixed order): pair k carries one iff no earlier pair of the token has the same owner
+    for (int t = blockIdx.x * kWarps + warp; t < a.T; t += warpsTotal) {
+        const char *base = reinterpret_cast<const char *>(a.retY) + (size_t)t * K * H * 2;
+        char *o = reinterpret_cast<char *>(a.out) + (size_t)t * H * 2;
+        const int myOwner = lane < K ? a.routed[t * K + lane].y : -1;  // lane k holds pair k
+        int before = 0;
         for (int j = 0; j < K; j++) {
-            same |= __shfl_sync(0xffffffffu, myOwner, j) == myOwner ? 1u << j : 0u;
+            before += __shfl_sync(0xffffffffu, myOwner, j) == myOwner && j < lane ? 1 : 0;
         }
-        const int before = __popc(same & ((1u << lane) - 1));
-        uint32_t leaders = __ballot_sync(0xffffffffu, myOwner >= 0 && before % (MF_MOE_MAX_SIBLINGS + 1) == 0);
-        char *o = reinterpret_cast<char *>(a.out) + ((size_t)t * H + (size_t)v0 * 8) * 2;
-        float acc[2][8];
-        if (ALONE) {  // one group holds everything
-            GatherGroup(acc, __ballot_sync(0xffffffffu, myOwner >= 0), MF_MOE_MAX_SIBLINGS + 1, mySlot, myW, a.y, (size_t)H * 2, a.cap, v0, vecs);
-            leaders = 0;
-        } else {
+        const uint32_t leaders = __ballot_sync(0xffffffffu, myOwner >= 0 && before % (MF_MOE_MAX_SIBLINGS + 1) == 0);
+        // Four vectors per lane and trip, loaded together for every partial sum (same reason as above).
+        for (int vb = lane; vb < vecs; vb += 128) {
+            float acc[4][8];
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                acc[0][q] = acc[1][q] = 0.f;
-            }
-        }
-        for (; leaders != 0; leaders &= leaders - 1) {
-            const int k = __ffs(leaders) - 1;
-            const int owner = __shfl_sync(0xffffffffu, myOwner, k);
-            if (owner != (int)m->rankId) {
-                const char *rowp = reinterpret_cast<const char *>(a.retY) + ((size_t)t * K + k) * H * 2;
-                uint4 raw[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-                if (has0) {
-                    raw[0] = mf_ld16_coherent(rowp + (size_t)v0 * 16);
+            for (int j = 0; j < 4; j++) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    acc[j][q] = 0.f;
                 }
-                if (has1) {
-                    raw[1] = mf_ld16_coherent(rowp + (size_t)v1 * 16);
-                }
-                AddRow(acc, raw);
-                continue;
             }
-            // This group's outputs are here: weighted in k order, and rounded like a partial sum that travels.
-            float part[2][8];
-            const uint32_t group = __shfl_sync(0xffffffffu, same, k) & (0xffffffffu << k);
-            GatherGroup(part, group, MF_MOE_MAX_SIBLINGS + 1, mySlot, myW, a.y, (size_t)H * 2, a.cap, v0, vecs);
-            uint4 rounded[2] = {PackRow(part[0]), PackRow(part[1])};
-            AddRow(acc, rounded);
-        }
-        if (has0) {
-            mf_st16(o, PackRow(acc[0]));
-        }
-        if (has1) {
-            mf_st16(o + 512, PackRow(acc[1]));
+            for (int k = 0; k < K; k++) {
+                if ((leaders >> k & 1u) == 0) {
+                    continue;
+                }
+                const char *rowp = base + (size_t)k * H * 2;
+                uint4 raw[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    raw[j] = vb + 32 * j < vecs ? mf_ld16_coherent(rowp + (size_t)(vb + 32 * j) * 16) : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[j]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        float2 f = __bfloat1622float2(h[i]);
+                        acc[j][2 * i] += f.x;
+                        acc[j][2 * i + 1] += f.y;
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (vb + 32 * j < vecs) {
+                    uint4 pk;
+                    __nv_bfloat162 *hp = reinterpret_cast<__nv_bfloat162 *>(&pk);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        hp[i] = __floats2bfloat162_rn(acc[j][2 * i], acc[j][2 * i + 1]);
+                    }
+                    mf_st16(o + (size_t)(vb + 32 * j) * 16, pk);
+                }
+            }
         }
     }
     FinishEpochD(a, epochArg, epoch);
@@ -797,10 +899,11 @@ static int LaunchCombine(const mf_moe_combine_args_t *argsHost, const mf_moe_com
     if (timeoutNs == 0) {
         timeoutNs = 2000000000ull;
     }
-    const bool alone = argsHost != nullptr && rankCount == 1 && K <= MF_MOE_MAX_SIBLINGS + 1;
-    const void *kernel = alone                 ? (const void *)mf_moe_combine_kernel<true, false>
-                         : argsHost != nullptr ? (const void *)mf_moe_combine_kernel<false, false>
-                                               : (const void *)mf_moe_combine_kernel<false, true>;
+    const bool alone = argsHost != nullptr && rankCount == 1;
+    auto aloneKernel = K > MF_MOE_MAX_SIBLINGS + 1 ? mf_moe_combine_alone_kernel<true> : mf_moe_combine_alone_kernel<false>;
+    const void *kernel = alone                 ? (const void *)aloneKernel
+                         : argsHost != nullptr ? (const void *)mf_moe_combine_kernel<false>
+                                               : (const void *)mf_moe_combine_kernel<true>;
     const mf_moe_combine_args_t own = argsHost != nullptr ? *argsHost : mf_moe_combine_args_t{};
     int cap = CoopCap(kernel, 0);
     if (cap <= 0) {
@@ -815,8 +918,7 @@ static int LaunchCombine(const mf_moe_combine_args_t *argsHost, const mf_moe_com
     }
     void *kargs[] = {(void *)&own, (void *)&argsDev, (void *)&H, (void *)&K, (void *)&EL, (void *)&channel, (void *)&epoch, (void *)&timeoutNs};
     dim3 g((unsigned)grid, (unsigned)nEmulatedRanks, 1), b(kThreads, 1, 1);
-    cudaError_t e = alone ? LaunchDependent(mf_moe_combine_kernel<true, false>, (unsigned)grid, kThreads, 0, (cudaStream_t)stream, own, argsDev, H, K, EL,
-                                            channel, epoch, timeoutNs)
+    cudaError_t e = alone ? LaunchDependent(aloneKernel, (unsigned)grid, kThreads, 0, (cudaStream_t)stream, own, H, K, epoch)
                           : cudaLaunchCooperativeKernel(kernel, g, b, kargs, 0, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();

@@ -57,8 +57,8 @@ struct MoePlan {
     // Of the tokens that were dispatched, whatever count the caller asks to see.
     int Combine(uint64_t epoch, uint64_t stream)
     {
-        // One warp per 1 KiB piece of a returned row; alone, a rank has no rows to return and one warp sums each 1 KiB of a token.
-        const long long pieces = (long long)c.T * (world == 1 ? 1 : topk) * ((hidden / 8 + 63) / 64);
+        // One warp per 2 KiB piece of a returned row; alone, a rank has no rows to return and one warp sums each 1 KiB of a token.
+        const long long pieces = world == 1 ? (long long)c.T * ((hidden / 8 + 63) / 64) : (long long)c.T * topk * ((hidden / 8 + 127) / 128);
         const int ctas = (int)((pieces + 7) / 8 < 65536 ? (pieces + 7) / 8 : 65536);
         return mf_k_moe_combine_rank(&c, world, hidden, topk, experts / world, combineChannel, epoch, timeoutNs, ctas > 1 ? ctas : 1, (mf_stream_t)stream);
     }
