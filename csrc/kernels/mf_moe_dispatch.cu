@@ -48,8 +48,9 @@ constexpr int kMaxExperts = 1024;
 constexpr int kMaxTopk = 32;
 // A token routed to several experts of one owner crosses the link once and is replicated by the owner when the call moves at
 // least this many (token, expert) pairs per rank on average; below it the scan of the receive buffer that the replication
-// needs costs more than the link time it saves (measured on two GPUs, top-8 of 64 experts: 128 tokens per rank 45 us without
-// and 109 us with it, 4096 tokens per rank 233 us without and 190 us with it).
+// needs costs more than the link time it saves. Measured on two GPUs, top-8 of 64 experts, with the dispatch that worked a token per
+// warp: 128 tokens per rank 45 us without and 109 us with it, 4096 tokens per rank 233 us without and 190 us with it. The
+// present form (a CTA per token, the replication unchanged) has not run on several GPUs; the line stands where it was.
 constexpr int kDedupMinPairsPerRank = 8192;
 
 __device__ __forceinline__ void FailD(int *status, int code)

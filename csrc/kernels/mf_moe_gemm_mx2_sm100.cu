@@ -4,8 +4,9 @@
 // SMs read both halves, so a K block costs each SM 32 KiB of operand traffic instead of the 48 KiB of the one-SM 128 x 256 tile:
 // one third less shared-memory fill per FLOP, and a ring of six stages instead of four in the same shared memory, i.e. more K
 // blocks in flight to cover the latency of L2 and DRAM. Measured, a K block takes 720 cycles, most of the wait being for scale
-// factors, against 600 of the one-SM kernel, and tiles of 256 rows pad more: 890 us against 840 us on the first FFN GEMM of
-// the benchmark, 530 against 470 us on the second; the one-SM kernel stays the default.
+// factors, against 600 of the one-SM kernel, and tiles of 256 rows pad more. At 1024 rows per expert (32 experts) the first FFN GEMM
+// takes 1091 us alone against 763 us and the second 583 against 542 us; in a loop, where the power limit sets the clock, 925 against 942
+// and 536 against 540 us. With 64 rows per expert it is a third slower either way. The one-SM kernel stays the default.
 //
 // Roles per CTA (384 threads): warp 0 TMA producer (per-CTA tiled loads, no multicast, completing on the LEADER's "full"
 // barrier), warp 2 scale-factor producer (this CTA's 128 A rows, all 256 weight columns; the atoms have a ring of their own —

@@ -24,8 +24,8 @@
 // the operand reuse of the 256-wide tile, and the epilogue of one tile runs under the MMAs of the next, which matters when K
 // is short (the second FFN GEMM: N = 7168 = 32 x 224, K = 2048).
 // What bounds it: a K block of a 256-wide tile takes 600 cycles of which the MMAs are 512 (724 cycles while the scale-factor warp computed
-// on words it had just asked for and one lane issued everything); 32768 rows, N 4096 / K 7168: 864 -> 781 us = 2.5 PFLOP/s, at
-// which the power limit holds the clock near 1.2 GHz.
+// on words it had just asked for and one lane issued everything); 32768 rows, N 4096 / K 7168: 864 -> 763-781 us alone = 2.5 PFLOP/s;
+// in a loop the power limit holds the clock near 1.2 GHz (842-942 us).
 // Every mbarrier wait is bounded; on expiry the CTA sets *status, all roles drain and the CTA frees its TMEM and exits.
 // Gated form (mf_k_moe_grouped_gemm_mx_gated): the rows of A are being stored by other GPUs (the MoE dispatch of the peers)
 // while this kernel runs. The two warps that read A — the TMA producer and the scale-factor producer — start a tile only when
@@ -715,9 +715,12 @@ extern "C" int mf_k_gemm_mx_tile(int G, int rowsTotal, int N, int mode, int ctas
         const char *e = getenv("MF_GEMM_TILE224");
         return e != nullptr && e[0] == '1';
     }();
-    // Measured on the second FFN GEMM (N 7168, K 2048): with at most one m-tile per expert (decode) the 224-column tile is 4 %
-    // faster than the 256-column one, with 1024 rows per expert it is 6 % slower, so it is chosen for the former only
-    // (MF_GEMM_TILE224=1 forces it wherever it applies).
+    // Measured on the second FFN GEMM (N 7168, K 2048, 32 experts; us alone / in a loop at the power limit, tiles of 128, 224, 256):
+    //   rows per expert   64: 110 / 104   108 /  97   120 /  98        512: 368 / 346   286 / 300   298 / 292
+    //                    256: 196 / 188   171 / 170   183 / 168       1024: 718 / 656   523 / 563   542 / 540
+    // so the 224-column tile is chosen for at most one m-tile per expert (decode), where it is ahead both ways (MF_GEMM_TILE224=1
+    // forces it wherever it applies). First FFN GEMM (N 4096, K 7168), tiles of 128 and 256: 210 / 199 and 202 / 187 at 64 rows,
+    // 364 / 344 and 263 / 303 at 256, 1353 / 1134 and 763 / 942 at 1024.
     const bool fewRows = mTiles <= (long long)G;
     if ((auto224 || fewRows) && (mode & 15) == MF_GEMM_EPI_BF16 && N % 224 == 0 && mTiles * (N / 224) >= 2LL * ctas) {
         return 224;

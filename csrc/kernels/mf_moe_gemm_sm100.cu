@@ -16,9 +16,9 @@
 //   warps 2-3  bring the products sa * sb of four K-blocks at a time into a ring of two such groups, one group ahead and across
 //              tiles: a row's scales are a line of their own for every thread, and waiting for them once per K-block on the
 //              promotion path took longer than the MMAs. It also leaves the promotion threads few enough registers.
-// 8191 rows over 32 experts, SwiGLU GEMM N 4096 / K 7168: 486 -> 353 us; N 7168 / K 2048: 281 -> 196 us. What bounds it now: a partial
-// product is read from TMEM while the next one is made in the other accumulator, and the hand-over (commit, wait, load, arrive) is
-// not shorter than the MMAs of a K-block.
+// 8191 rows over 32 experts, SwiGLU GEMM N 4096 / K 7168: 486 -> 353 us; N 7168 / K 2048: 281 -> 196 us. What bounds it now is the
+// promotion: a K-block takes about 950 cycles of the wide tile and 720 of the narrow one, whose four accumulators leave the hand-over
+// out of the way, against 512 and 256 of its MMAs. Each warp reads its 64 columns by four loads that it waits for one by one.
 // Tiles are enumerated on the device from group_offset/group_count (the host does not know the routing result), n fastest so
 // that concurrently running CTAs share an A tile and stream one expert's weights through L2.
 // Every mbarrier wait is bounded; on expiry the CTA sets *status, all roles drain and the CTA frees its TMEM and exits.
