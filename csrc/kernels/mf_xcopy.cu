@@ -68,7 +68,8 @@ mf_xcopy_kernel(unsigned char *dst, const unsigned char *src, size_t n, size_t t
 // copies (a shallow pipeline interleaves DRAM reads and writes more regularly than a deep one): 32 KiB tiles, 4 stages, 2
 // stores in flight, one CTA per SM, strided walk: 12.9 / 23.0 / 44.0 / 83.5 / 325 us at 32 / 64 / 128 / 256 / 1024 MiB, against 13.3 /
 // 25.4 / 50.0 / 97.5 / 376 us of the load/store kernel. Below kTmaMinBytes the load/store kernel is the faster one (3.6 and 6.2 us
-// at 8 and 16 MiB against 3.5 and 6.7 us, 3.1 against 3.3 us at 4 MiB). That was measured, and is the rule, where both sides lie in
+// at 8 and 16 MiB against 3.5 and 6.7 us, 3.1 against 3.3 us at 4 MiB; with data that is not in the L2 7.2 against 7.9 us at 16 MiB,
+// 9.0 against 9.3 at 20, 10.4 against 9.9 at 23). That was measured, and is the rule, where both sides lie in
 // this GPU's memory. Over a link (a peer's memory, the host's) every shape runs at the link's rate from the sizes that were measured
 // there; what was in place for those measurements stays: bulk copies from 4 MiB on, 16 KiB tiles with one store in flight,
 // 32 KiB tiles in contiguous runs from 256 MiB on.
